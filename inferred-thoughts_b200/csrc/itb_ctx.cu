@@ -124,7 +124,7 @@ extern "C" void itb_destroy(itb_ctx* c) {
     cudaStreamSynchronize(c->stream);
     free_map(c->mirrors); free_map(c->states); free_map(c->kv);
     for (auto& w : c->weights) { cudaFree(w.second.a); cudaFree(w.second.b); cudaFree(w.second.scale2); }
-    cudaFree(c->pair_off); cudaFree(c->pair_list);
+    cudaFree(c->pair_off); cudaFree(c->pair_list); cudaFree(c->pair_tiles);
     itb_tc_free(c);
     cudaFree(c->route_ids); cudaFree(c->route_w); cudaFree(c->xq); cudaFree(c->xs); cudaFree(c->tmp_f32);
     cudaStreamDestroy(c->stream);
@@ -299,27 +299,29 @@ __global__ void k_repack_q8(const uint8_t* __restrict__ raw, int8_t* __restrict_
     dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
     dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
 }
-// One thread per NVFP4 block of 64: 4 scale codes + 32 bytes whose byte 8s+j holds element 16s+j (low)
-// and 16s+j+8 (high) -> scale plane and element-ordered nibbles (byte i of a sub-block = elements 2i, 2i+1).
-__global__ void k_repack_fp4(const uint8_t* __restrict__ raw, uint8_t* __restrict__ nib, uint8_t* __restrict__ sc, size_t nb) {
+// One thread per NVFP4 block of 64: 4 scale codes + 32 bytes whose byte 8s+j holds element 16s+j (low) and 16s+j+8 (high) -> the
+// row's 32 bytes and 4 scales of its tile (DevFp4's layout).
+__global__ void k_repack_fp4(const uint8_t* __restrict__ raw, uint8_t* __restrict__ nib, uint8_t* __restrict__ sc, int kgs, int n_out, size_t pad_out, size_t nb) {
     size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     const uint8_t* p = raw + b * 36;
-    uint8_t out[32];
+    const int kg = (int)(b % kgs); const size_t er = b / kgs; const int row = (int)(er % n_out); const size_t e = er / n_out;
+    uint8_t out[32], so[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         uint8_t c = p[s];
-        sc[b * 4 + s] = c == 0x7f ? 0 : c;
-        uint8_t e[16];
+        so[s] = c == 0x7f ? 0 : c;
+        uint8_t v[16];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { e[j] = p[4 + 8 * s + j] & 0xf; e[j + 8] = p[4 + 8 * s + j] >> 4; }
+        for (int j = 0; j < 8; ++j) { v[j] = p[4 + 8 * s + j] & 0xf; v[j + 8] = p[4 + 8 * s + j] >> 4; }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) out[8 * s + i] = e[2 * i] | (e[2 * i + 1] << 4);
+        for (int i = 0; i < 8; ++i) out[8 * (i >> 1) + 4 * (s >> 1) + 2 * (s & 1) + (i & 1)] = v[2 * i] | (v[2 * i + 1] << 4);
     }
-    uint4* dst = (uint4*)(nib + b * 32);
+    uint4* dst = (uint4*)(nib + e * pad_out * kgs * 32 + fp4_nib_at(row, kg, kgs));
     const uint4* src = (const uint4*)out;
     dst[0] = src[0];
     dst[1] = src[1];
+    *(uint32_t*)(sc + e * pad_out * kgs * 4 + fp4_sc_at(row, kg, kgs)) = *(const uint32_t*)so;
 }
 __global__ void k_f16_to_f32(const uint16_t* __restrict__ raw, float* __restrict__ out, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -328,8 +330,9 @@ __global__ void k_f16_to_f32(const uint16_t* __restrict__ raw, float* __restrict
 void itb_repack_q8(cudaStream_t st, const uint8_t* raw, int8_t* q, uint16_t* s, size_t nb) {
     if (nb) k_repack_q8<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(raw, q, s, nb);
 }
-void itb_repack_fp4(cudaStream_t st, const uint8_t* raw, uint8_t* nib, uint8_t* sc, size_t nb) {
-    if (nb) k_repack_fp4<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(raw, nib, sc, nb);
+void itb_repack_fp4(cudaStream_t st, const uint8_t* raw, uint8_t* nib, uint8_t* sc, size_t n_in, size_t n_out, size_t n_expert) {
+    const size_t nb = n_in / 64 * n_out * n_expert;
+    if (nb) k_repack_fp4<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(raw, nib, sc, (int)(n_in / 64), (int)n_out, fp4_rows_pad(n_out), nb);
 }
 void itb_f16_to_f32(cudaStream_t st, const uint16_t* raw, float* out, size_t n) {
     if (n) k_f16_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(raw, out, n);
@@ -361,8 +364,9 @@ const WeightEntry* itb_weight(itb_ctx* c, const uint8_t* data, size_t bytes, uin
     // Every plane is allocated before any kernel runs; on a failure everything allocated so far is given back and the
     // caller gets "out of device memory" instead of a kernel writing through a null pointer.
     const bool want_s2 = scale && scale_bytes >= n_expert * 4;
-    const size_t a_bytes = ty == ITB_F32 ? 0 : ty == ITB_F16 ? elems * 4 : ty == ITB_Q8_0 ? elems : elems / 2;
-    const size_t b_bytes = ty == ITB_Q8_0 ? elems / 32 * 2 : ty == ITB_NVFP4 ? elems / 16 : 0;
+    const size_t padded = fp4_rows_pad(n_out) * n_in * n_expert;      // NVFP4: whole tiles of 16 rows
+    const size_t a_bytes = ty == ITB_F32 ? 0 : ty == ITB_F16 ? elems * 4 : ty == ITB_Q8_0 ? elems : padded / 2;
+    const size_t b_bytes = ty == ITB_Q8_0 ? elems / 32 * 2 : ty == ITB_NVFP4 ? padded / 16 : 0;
     bool oom = false;
     if (a_bytes && cudaMalloc(&w.a, a_bytes) != cudaSuccess) { w.a = nullptr; oom = true; }
     if (!oom && b_bytes && cudaMalloc(&w.b, b_bytes) != cudaSuccess) { w.b = nullptr; oom = true; }
@@ -382,8 +386,8 @@ const WeightEntry* itb_weight(itb_ctx* c, const uint8_t* data, size_t bytes, uin
         itb_repack_q8(c->stream, raw, (int8_t*)w.a, (uint16_t*)w.b, elems / 32);
         w.bytes = elems + elems / 16;
     } else {
-        itb_repack_fp4(c->stream, raw, (uint8_t*)w.a, (uint8_t*)w.b, elems / 64);
-        w.bytes = elems / 2 + elems / 16;
+        itb_repack_fp4(c->stream, raw, (uint8_t*)w.a, (uint8_t*)w.b, n_in, n_out, n_expert);
+        w.bytes = padded / 2 + padded / 16;
     }
     if (want_s2) cudaMemcpyAsync(w.scale2, scale, n_expert * 4, cudaMemcpyHostToDevice, c->stream);
     e = cudaStreamSynchronize(c->stream);

@@ -25,6 +25,7 @@ void itb_synth_fp4_raw(cudaStream_t st, uint64_t key, size_t per_expert, size_t 
 #include "itb_fused.cuh"
 #include "itb_mega.cuh"
 #include "itb_rows.cuh"
+#include "itb_exp.cuh"
 #include "itb_attn_exact.cuh"
 #include "itb_attn_mma.cuh"
 #include "itb_gdn_chunk.cuh"
@@ -128,8 +129,9 @@ static int adopt_raw(itb_model* m, const std::string& name, uint32_t ty, size_t 
         itb_repack_q8(c->stream, raw, (int8_t*)t.a, (uint16_t*)t.b, elems / 32);
         t.bytes = elems + elems / 16;
     } else if (ty == ITB_NVFP4) {
+        elems = n_in * fp4_rows_pad(n_out) * e_cnt;          // whole tiles of 16 rows
         if (!two(elems / 2, elems / 16)) return 1;
-        itb_repack_fp4(c->stream, raw, (uint8_t*)t.a, (uint8_t*)t.b, elems / 64);
+        itb_repack_fp4(c->stream, raw, (uint8_t*)t.a, (uint8_t*)t.b, n_in, n_out, e_cnt);
         t.scale2 = scale2_dev;
         t.bytes = elems / 2 + elems / 16;
     } else return 1;
@@ -457,6 +459,7 @@ struct EpState {
     // pairs it received (every one names a local expert), the per-rank counts of all ranks
     int8_t* sxq = nullptr; float* sxs = nullptr; int32_t* sids = nullptr;   // [R*K] rows in owner order
     int8_t* rxq = nullptr; float* rxs = nullptr; int32_t* rids = nullptr;   // received pairs (capacity a2a_cap)
+    __half* rxh = nullptr;                                                  // received rows as the expert kernels read them
     float* o_back = nullptr;                                                // this rank's pairs' outputs, in owner order
     int32_t* owner = nullptr; int* own_off = nullptr; int* own_list = nullptr;
     int* cnt_dev = nullptr; int* cnt_host = nullptr;                        // [W][W]: cnt[s][d] = pairs rank s sends to rank d
@@ -637,12 +640,13 @@ struct itb_engine {
     float* scores = nullptr; size_t scores_cap = 0;    // exact attention: [rows][n_head][n_ctx] scores (grown on demand)
     float *router = nullptr, *shlogit = nullptr, *sg = nullptr, *su = nullptr, *h = nullptr, *logits = nullptr;
     int8_t* xq = nullptr; float* xs = nullptr;
+    __half *xh = nullptr, *hh = nullptr;                     // activation rows of the experts in multi-row passes (f16, exp_pos order): router input, gated rows
     int32_t* route_ids = nullptr; float* route_w = nullptr;  // [n_layer][B][n_used]
     int32_t* history = nullptr; int* step_counter = nullptr; uint32_t history_cap = 0;
     int* err = nullptr; float* arg_v = nullptr; int* arg_i = nullptr;
     int8_t *aq = nullptr, *hq = nullptr, *sq = nullptr; float *as = nullptr, *hs = nullptr, *ss = nullptr;  // producer-quantised activations
     float* gdn_scratch = nullptr; size_t gdn_scratch_cap = 0;     // chunk-parallel delta rule: W, Qg, Kd, U, P of every (chunk, value head) of a pass
-    float *h_all = nullptr, *o_all = nullptr, *shd = nullptr, *qkvc2 = nullptr; int *pair_off = nullptr, *pair_list = nullptr;  // grouped experts (multi-row path)
+    float *h_all = nullptr, *o_all = nullptr, *shd = nullptr, *qkvc2 = nullptr; int *pair_off = nullptr, *pair_list = nullptr; int4* pair_tiles = nullptr;  // grouped experts (multi-row path)
     int32_t* prompt = nullptr; size_t prompt_cap = 0;
     int n_split = 1, n_split_rows = 4;
     uint32_t R = 0;                                   // rows the multi-row pass can hold (>= B)
@@ -829,10 +833,7 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
     if (!attrs_set) {
         set_smem((const void*)k_in_proj, 200 * 1024); set_smem((const void*)k_out_proj, 200 * 1024);
         set_smem((const void*)k_moe_glu, 100 * 1024);
-        set_smem((const void*)k_moe_down<1>, 100 * 1024); set_smem((const void*)k_moe_down<2>, 100 * 1024);
-        set_smem((const void*)k_moe_down<4>, 100 * 1024); set_smem((const void*)k_moe_down<8>, 100 * 1024);
-        set_smem((const void*)k_moe_down<1, true>, 100 * 1024); set_smem((const void*)k_moe_down<2, true>, 100 * 1024);
-        set_smem((const void*)k_moe_down<4, true>, 100 * 1024); set_smem((const void*)k_moe_down<8, true>, 100 * 1024);
+        set_smem((const void*)k_moe_down<false>, 200 * 1024); set_smem((const void*)k_moe_down<true>, 200 * 1024);
         set_smem((const void*)k_gdn_core<128>, 100 * 1024); set_smem((const void*)k_gdn_core<64>, 100 * 1024);
         attrs_set = true;
     }
@@ -979,20 +980,11 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
         if (e->ep) { w.o_pairs = e->o_all; w.own_row = e->ep->rank; w.shd = e->shd; }
         if (p2p) for (int r = 0; r < W; ++r) w.o_rows[r] = (float*)(e->ep->peer[r] + e->ep->off_o + (size_t)il * e->ep->o_layer);
         {
-            int slots = 32 >> lanes_shift(d.expert_ff / 32), need = ((int)d.n_expert_used + slots - 1) / slots;
-            int rp = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
-            dim3 grid(std::max(1, std::min(sms, (H + NWG - 1) / NWG)), RW);
+            dim3 grid(H / 16, RW);
             w.tl_slot = tl++;
-            size_t smem_d = moe_down_smem(d.n_expert_used, d.expert_ff, d.shared_ff, rp);
-            if (e->ep) {
-                if (rp == 1) launch_k(pdl, k_moe_down<1, true>, grid, TPB, smem_d, st, w);
-                else if (rp == 2) launch_k(pdl, k_moe_down<2, true>, grid, TPB, smem_d, st, w);
-                else if (rp == 4) launch_k(pdl, k_moe_down<4, true>, grid, TPB, smem_d, st, w);
-                else launch_k(pdl, k_moe_down<8, true>, grid, TPB, smem_d, st, w);
-            } else if (rp == 1) launch_k(pdl, k_moe_down<1>, grid, TPB, smem_d, st, w);
-            else if (rp == 2) launch_k(pdl, k_moe_down<2>, grid, TPB, smem_d, st, w);
-            else if (rp == 4) launch_k(pdl, k_moe_down<4>, grid, TPB, smem_d, st, w);
-            else launch_k(pdl, k_moe_down<8>, grid, TPB, smem_d, st, w);
+            const size_t smem_d = moe_down_smem(d.n_expert_used, d.expert_ff, d.shared_ff);
+            if (e->ep) launch_k(pdl, k_moe_down<true>, grid, TPB, smem_d, st, w);
+            else launch_k(pdl, k_moe_down<false>, grid, TPB, smem_d, st, w);
         }
         if (p2p) {
             // the served picks' rows were stored straight into their owners' regions: tell every rank, then combine this rank's
@@ -1129,15 +1121,15 @@ static bool ep_a2a_prepare(itb_engine* e) {
     if (q->a2a_cap >= cap) return true;
     cudaStreamSynchronize(e->c->stream);
     bool ok = cudaMalloc(&q->sxq, mine * H) == cudaSuccess && cudaMalloc(&q->sxs, mine * (H / 32) * 4) == cudaSuccess && cudaMalloc(&q->sids, mine * 4) == cudaSuccess &&
-              cudaMalloc(&q->rxq, cap * H) == cudaSuccess && cudaMalloc(&q->rxs, cap * (H / 32) * 4) == cudaSuccess && cudaMalloc(&q->rids, cap * 4) == cudaSuccess &&
+              cudaMalloc(&q->rxq, cap * H) == cudaSuccess && cudaMalloc(&q->rxh, cap * H * 2) == cudaSuccess && cudaMalloc(&q->rxs, cap * (H / 32) * 4) == cudaSuccess && cudaMalloc(&q->rids, cap * 4) == cudaSuccess &&
               cudaMalloc(&q->o_back, mine * H * 4) == cudaSuccess && cudaMalloc(&q->owner, mine * 4) == cudaSuccess && cudaMalloc(&q->own_off, (W + 1) * 4) == cudaSuccess &&
               cudaMalloc(&q->own_list, mine * 4) == cudaSuccess && cudaMalloc(&q->cnt_dev, W * (W + 1) * 4) == cudaSuccess &&
               cudaMallocHost(&q->cnt_host, W * (W + 1) * 4) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
-        cudaFree(q->sxq); cudaFree(q->sxs); cudaFree(q->sids); cudaFree(q->rxq); cudaFree(q->rxs); cudaFree(q->rids); cudaFree(q->o_back); cudaFree(q->owner);
+        cudaFree(q->sxq); cudaFree(q->sxs); cudaFree(q->sids); cudaFree(q->rxq); cudaFree(q->rxh); cudaFree(q->rxs); cudaFree(q->rids); cudaFree(q->o_back); cudaFree(q->owner);
         cudaFree(q->own_off); cudaFree(q->own_list); cudaFree(q->cnt_dev); if (q->cnt_host) cudaFreeHost(q->cnt_host);
-        q->sxq = q->rxq = nullptr; q->sxs = q->rxs = q->o_back = nullptr; q->sids = q->rids = q->owner = nullptr; q->own_off = q->own_list = q->cnt_dev = q->cnt_host = nullptr;
+        q->sxq = q->rxq = nullptr; q->rxh = nullptr; q->sxs = q->rxs = q->o_back = nullptr; q->sids = q->rids = q->owner = nullptr; q->own_off = q->own_list = q->cnt_dev = q->cnt_host = nullptr;
         return itb_fail_msg(e->c, "expert-parallel engine: out of device memory for the all-to-all buffers");
     }
     q->a2a_cap = cap;
@@ -1215,17 +1207,12 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     static bool attrs_set = false;
     if (!attrs_set) {
         set_smem((const void*)k_gemm_q8<4>, 200 * 1024); set_smem((const void*)k_gemm_q8<1>, 200 * 1024);
-        set_smem((const void*)k_glu_grouped, 200 * 1024); set_smem((const void*)k_down_grouped, 200 * 1024);
         set_smem((const void*)k_matmul_f32_rows<20>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<24>, 64 * 1024);
         set_smem((const void*)k_matmul_f32_rows<28>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<32>, 64 * 1024);
         set_smem((const void*)k_tile_q8<1, 256, 4>, 226 * 1024); set_smem((const void*)k_tile_q8<4, 256, 2>, 226 * 1024);
         set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
         set_smem((const void*)k_sgemm_serial_small<false>, sgemm_small_smem()); set_smem((const void*)k_sgemm_serial_small<true>, sgemm_small_smem());
         set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
-        set_smem((const void*)k_tile_glu<1, 256, 1>, 226 * 1024); set_smem((const void*)k_tile_down<1, 256, 1>, 226 * 1024);
-        set_smem((const void*)k_tile_glu<2, 256, 1>, 226 * 1024); set_smem((const void*)k_tile_down<2, 256, 1>, 226 * 1024);
-        set_smem((const void*)k_tile_glu<4, 256, 1>, 226 * 1024); set_smem((const void*)k_tile_down<4, 256, 1>, 226 * 1024);
-        set_smem((const void*)k_tile_glu<4, 256, 2>, 226 * 1024); set_smem((const void*)k_tile_down<4, 256, 2>, 226 * 1024);
         set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
         attrs_set = true;
     }
@@ -1249,10 +1236,10 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         const bool skinny = R <= 32;
         if (skinny && k % 256 == 0) {
             const int ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (R + 31) / 32), 256, tile_smem<MK_Q8, 1, 256, 4>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
+            k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
         } else if (!skinny && k % 256 == 0) {
             const int ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (R + 63) / 64), 256, tile_smem<MK_Q8, 4, 256, 2>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
+            k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (R + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
         } else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(w.n_in), st>>>(w, xq, xs, R, out, stride, mode);
         else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (R + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), st>>>(w, xq, xs, R, out, stride, mode);
         launches++;
@@ -1269,7 +1256,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             int tiles = 0;
             for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; p.tiles[i] = (w[i]->n_out + 31) / 32; tiles += p.tiles[i]; }
             const int k = w[0]->n_in, ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8_multi<1, 256, 4><<<dim3(tiles, (R + 31) / 32), 256, tile_smem<MK_Q8, 1, 256, 4>(k), st>>>(p, xq, xs, R, ns);
+            k_tile_q8_multi<1, 256, 4><<<dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(p, xq, xs, R, ns);
             launches++;
             return;
         }
@@ -1285,11 +1272,10 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             launches++;
             return;
         }
-        const int nb = w.n_in / 32, nsb = w.n_in / 16, gsh = lanes_shift(nb), nw = 8;
         const int gx = std::max(1, std::min((w.n_out + 31) / 32, 2 * sms));
-        const size_t smem = (size_t)w.n_in + (size_t)nb * 4 + (size_t)nw * terms_floats(4, gsh, nsb) * 4;
+        const size_t smem = matmul_fp4_smem(w.n_in);
         set_smem((const void*)k_matmul_fp4, smem);
-        k_matmul_fp4<<<dim3(gx, rows), nw * 32, smem, st>>>(w, nullptr, 1, 0, xq, xs, out);
+        k_matmul_fp4<<<dim3(gx, rows), 256, smem, st>>>(w, nullptr, 1, 0, xq, xs, out);
         launches++;
         if (has_s) { const size_t n = (size_t)rows * w.n_out; k_scale<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, sc); launches++; }
     };
@@ -1436,7 +1422,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             gemm(L.wo, e->aq, e->as, e->x, H, 1);
         }
         // routed FFN
-        k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs); launches++;
+        k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, e->ep ? nullptr : e->xh); launches++;
         if (!L.shared4[0].nib && !L.shared4[1].nib) {
             const DevQ8* ws[2] = {&L.shared_gate, &L.shared_up}; float* os[2] = {e->sg, e->su}; const size_t ss[2] = {(size_t)d.shared_ff, (size_t)d.shared_ff};
             gemm_multi(2, ws, os, ss, e->xq, e->xs);
@@ -1533,8 +1519,9 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                 Lg = tier_stack(e, il, 0, L.gate); Lu = tier_stack(e, il, 1, L.up); Ld = tier_stack(e, il, 2, L.down);
             }
             if (P > 0) {
-            if (E <= 1024) k_group_pairs_fast<<<1, 1024, (size_t)E * 4, st>>>(ids_src, P, E, e->pair_off, e->pair_list);
-            else k_group_pairs<<<1, 256, (size_t)E * 4, st>>>(ids_src, P, E, e->pair_off, e->pair_list);
+            const int e_here = e->ep ? std::max(1, E / W) : E;        // an expert-parallel rank serves all the pairs it sees with its own E / W experts
+            const int tile_cap = exp_tile_cap(P, e_here, ff, sms), max_tiles = exp_max_tiles(P, E, tile_cap);
+            k_group_pairs_fast<<<1, 1024, (size_t)E * 4, st>>>(ids_src, P, E, e->pair_off, e->pair_list, e->pair_tiles, e->pair_off + E + 1, tile_cap);
             launches++;
             const cudaStreamCaptureStatus cap_st = cap_rows;
             if (c->fp4tc && n_tok > 1 && !e->ep && !e->tier && cap_st == cudaStreamCaptureStatusNone && itb_tc_shape_ok(Lg) && itb_tc_shape_ok(Lu) && itb_tc_shape_ok(Ld)) {
@@ -1544,24 +1531,21 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                     !itb_tc_experts(c, st, Ld, nullptr, e->h_all, 1, e->pair_off, e->pair_list, P, e->o_all)) return launches;
                 launches += 6;
             } else {
-                // rows per expert decide the tile shape (a tile's empty token columns cost as much as full ones)
-                const bool tile_w = H % 256 == 0 && ff % 256 == 0;
-                // up to 32 rows per expert: 128 weight rows x 8*NJ tokens per block (every weight decoded by one warp); more: 64 x 64
-                // (an expert-parallel rank serves all the pairs it sees with its own E / W experts)
-                const int e_here = e->ep ? std::max(1, E / W) : E;
-                const int per_e = (P + e_here - 1) / e_here, nj = per_e <= 8 ? 1 : per_e <= 16 ? 2 : per_e <= 32 ? 4 : 0;
-                const int ns_g = std::min(H / 256, TILE_STAGES), ns_d = std::min(ff / 256, TILE_STAGES);
-#define GLU_TILE(NJ, TH) k_tile_glu<NJ, 256, TH><<<dim3(E, (ff + 128 / TH - 1) / (128 / TH)), 256, tile_smem<MK_FP4, NJ, 256, TH>(H), st>>>(Lg, Lu, xq_src, xs_src, Kt, e->pair_off, e->pair_list, e->h_all, ns_g)
-#define DOWN_TILE(NJ, TH) k_tile_down<NJ, 256, TH><<<dim3(E, (H + 128 / TH - 1) / (128 / TH)), 256, tile_smem<MK_FP4, NJ, 256, TH>(ff), st>>>(Ld, e->hq, e->hs, e->pair_off, e->pair_list, e->o_all, ns_d)
-                if (tile_w) { if (nj == 1) GLU_TILE(1, 1); else if (nj == 2) GLU_TILE(2, 1); else if (nj == 4) GLU_TILE(4, 1); else GLU_TILE(4, 2); }
-                else k_glu_grouped<<<dim3(E, (ff + MMA_ROWS - 1) / MMA_ROWS), 256, gemm_smem(H), st>>>(Lg, Lu, xq_src, xs_src, Kt, e->pair_off, e->pair_list, e->h_all);
-                launches++;
-                k_quant_rows<<<P, 128, 0, st>>>(e->h_all, ff, e->hq, e->hs); launches++;
-                if (tile_w) { if (nj == 1) DOWN_TILE(1, 1); else if (nj == 2) DOWN_TILE(2, 1); else if (nj == 4) DOWN_TILE(4, 1); else DOWN_TILE(4, 2); }
-#undef GLU_TILE
-#undef DOWN_TILE
-                else k_down_grouped<<<dim3(E, (H + MMA_ROWS - 1) / MMA_ROWS), 256, gemm_smem(ff), st>>>(Ld, e->hq, e->hs, e->pair_off, e->pair_list, e->o_all);
-                launches++;
+                // bit-exact: every expert's pairs against its weights, the gated row quantised on its way out (itb_exp.cuh)
+                __half* xh = e->xh;
+                if (e->ep) {
+                    // the rows came from every rank as int8
+                    const size_t n16 = (a2a ? (size_t)P : (size_t)W * R) * (H / 16);
+                    if (a2a) xh = e->ep->rxh;
+                    k_q8_to_h<<<(unsigned)((n16 + 255) / 256), 256, 0, st>>>(xq_src, n16, xh); launches++;
+                }
+                ExpArgs ea{};
+                ea.wa = Lg; ea.wb = Lu; ea.xh = xh; ea.xs = xs_src; ea.div = Kt; ea.tiles = e->pair_tiles; ea.n_tiles = e->pair_off + E + 1; ea.list = e->pair_list; ea.oh = e->hh; ea.os = e->hs;
+                exp_run(ea, true, max_tiles, tile_cap, st);
+                ExpArgs ed{};
+                ed.wa = Ld; ed.xh = e->hh; ed.xs = e->hs; ed.div = 1; ed.tiles = ea.tiles; ed.n_tiles = ea.n_tiles; ed.list = e->pair_list; ed.out = e->o_all;
+                exp_run(ed, false, max_tiles, tile_cap, st);
+                launches += 2;
             }
             }
             const float* o_src = e->o_all;
@@ -1668,16 +1652,15 @@ static int engine_create(itb_model* m, uint32_t n_ctx, uint32_t n_seq, int world
               dalloc(E, &e->route_ids, (size_t)d.n_layer * R * K) && dalloc(E, &e->route_w, (size_t)d.n_layer * R * K) &&
               dalloc(E, &e->step_counter, B) && dalloc(E, &e->err, 1) && dalloc(E, &e->arg_v, B * ARGMAX_PARTS) && dalloc(E, &e->arg_i, B * ARGMAX_PARTS) &&
               dalloc(E, &e->aq, R * std::max(vd, qd)) && dalloc(E, &e->as, R * std::max(vd, qd) / 32) &&
-              dalloc(E, &e->hq, W * R * K * d.expert_ff) && dalloc(E, &e->hs, W * R * K * d.expert_ff / 32) &&
+              dalloc(E, &e->xh, W * R * H) && dalloc(E, &e->hh, W * R * K * d.expert_ff) && dalloc(E, &e->hq, W * B * K * d.expert_ff) && dalloc(E, &e->hs, W * R * K * d.expert_ff / 32) &&
               dalloc(E, &e->sq, R * d.shared_ff) && dalloc(E, &e->ss, R * d.shared_ff / 32) &&
               dalloc(E, &e->xn, R * H) && dalloc(E, &e->qh, R * key_dim) && dalloc(E, &e->kh, R * key_dim) && dalloc(E, &e->vh, R * vd) &&
               dalloc(E, &e->gb, R * d.ssm_dt_rank * 2) && dalloc(E, &e->core, R * vd) && dalloc(E, &e->xlast, B * H) &&
               dalloc(E, &e->h_all, W * R * K * d.expert_ff) && dalloc(E, &e->o_all, W * R * K * H) && dalloc(E, &e->shd, R * H) &&
-              dalloc(E, &e->qkvc2, R * cd) && dalloc(E, &e->pair_off, (size_t)d.n_expert + 1) && dalloc(E, &e->pair_list, W * R * K);
+              dalloc(E, &e->qkvc2, R * cd) && dalloc(E, &e->pair_off, (size_t)d.n_expert + 2) && dalloc(E, &e->pair_tiles, (size_t)d.n_expert + W * R * K / 8 + 1) && dalloc(E, &e->pair_list, W * R * K);
     if (!ok) { for (void* p : e->allocs) cudaFree(p); return 1; }
     e->host_pos.assign(B, 0);
     cudaEventCreate(&e->ev0); cudaEventCreate(&e->ev1);
-    cudaMemsetAsync(e->h_all, 0, W * R * K * d.expert_ff * sizeof(float), c->stream);   // pairs served elsewhere are quantised too: keep them finite
     if (world > 1) {
         e->ep = new EpState();
         e->ep->world = world;
@@ -1826,7 +1809,7 @@ extern "C" void itb_engine_destroy(itb_engine* e) {
         cudaFreeHost(q->agree_host);
         for (int r = 0; r < q->world && r < 8; ++r) if (r != q->rank && q->peer[r]) cudaIpcCloseMemHandle(q->peer[r]);
         cudaFree(q->region); cudaFree(q->seq); cudaFree(q->peer_dev);
-        cudaFree(q->sxq); cudaFree(q->sxs); cudaFree(q->sids); cudaFree(q->rxq); cudaFree(q->rxs); cudaFree(q->rids); cudaFree(q->o_back); cudaFree(q->owner);
+        cudaFree(q->sxq); cudaFree(q->sxs); cudaFree(q->sids); cudaFree(q->rxq); cudaFree(q->rxh); cudaFree(q->rxs); cudaFree(q->rids); cudaFree(q->o_back); cudaFree(q->owner);
         cudaFree(q->own_off); cudaFree(q->own_list); cudaFree(q->cnt_dev); if (q->cnt_host) cudaFreeHost(q->cnt_host);
         delete q; e->ep = nullptr;
     }
@@ -1921,7 +1904,7 @@ static bool mega_prepare(itb_engine* e) {
     if (!coop) return no("no cooperative launch on this device");
     const int G = sms;
     auto per_block = [&](int n) { return (n + G - 1) / G + 1; };
-    const int gdn_rows = per_block(n_v * sk), down_rows = per_block(H);
+    const int gdn_rows = per_block(n_v * sk), down_rows = 16 * ((H / 16 + G - 1) / G);
     if (gdn_rows > MG_CT || (gdn_rows + sk - 1) / sk + 1 > MG_MAX_LOCAL_HEADS) return no("too many delta-rule rows per block");
     // shared-memory layout
     const int nmax = std::max(H, std::max(vd, qd));

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
                 float* cs = p.conv_state + (size_t)b * p.conv_state_stride;
                 const float* cw = p.conv_w;
                 const int kernel = p.conv_kernel;
-                rows_batched<MK_Q8, 2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh, [&](int row, float v) {
+                rows_batched<2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh, [&](int row, float v) {
                     float* past = cs + (size_t)row * keep;
                     const bool pre = row - conv_lo < CONV_CAP;
                     const float* pin = pre ? cpre + (row - conv_lo) * 8 : past;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
                     past[keep - 1] = v;
                 });
             } else {
-                rows_batched<MK_Q8, 2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh,
+                rows_batched<2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh,
                                           [&](int row, float v) { o[row] = v; });
             }
         }
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(NWG * 32) k_out_proj(OutProj p) {
     __syncthreads();
     TL(TLK_OUT_PROJ, 2);
     float* x = p.x + (size_t)b * p.x_stride;
-    rows_batched<MK_Q8, 1, 4>((const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, b0 + r0, b0 + r1, aq, as, terms, p.br, gsh,
+    rows_batched<1, 4>((const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, b0 + r0, b0 + r1, aq, as, terms, p.br, gsh,
                               [&](int row, float v) { x[row] += v; });
     if (wid == 0) l2_hint(p.hint, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, threadIdx.x & 31);
     TL(TLK_OUT_PROJ, 3);
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     __shared__ float s_sum;
     __shared__ float s_cand_p[MOE_CAND];        // the first n_used of every 32-group: probability and id
     __shared__ int s_cand_i[MOE_CAND];
-    const int n = p.n_embd, nb = n / 32, nsb = n / 16, gsh = lanes_shift(nb), ff = p.gate.n_out, upp = ff / 32;
+    const int n = p.n_embd, nb = n / 32, nsb = n / 16, ff = p.gate.n_out, upp = ff / 32;
     const int b = blockIdx.y, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int unit = blockIdx.x, n_units = p.n_used * upp;
     TL(TLK_MOE_GLU, 0);
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     float* probs = (float*)smem;                  // [n_expert rounded up to 32]
     int8_t* xq = (int8_t*)(probs + ((p.n_expert + 31) & ~31));
     float* xs = (float*)(xq + n);
-    float* terms = xs + nb + wid * terms_floats(4, gsh, nsb);
+    float* terms = xs + nb;                       // [64 rows][nsb + 1]
     {
         // softmax numerators (src/ops/naive.rs:362-376) by the whole block: every warp finds the max itself
         const float* lg = p.router + (size_t)b * p.n_expert;
@@ -616,22 +616,21 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     const int pick = unit / upp, row0 = (unit % upp) * 32;
     const int el = s_ids[pick] - p.gate.expert_lo;
     if (el < 0 || el >= p.gate.n_expert) return;   // this pick's expert lives on another device
-    // 64 row-dots (32 gate rows, 32 up rows) spread over the block's warps
+    // four 16-row tiles (two of gate, two of up), four warps to a tile and a quarter of k each; the terms meet in shared memory and a
+    // lane per row folds them in order
     const size_t eo = (size_t)el * ff;
     const bool has_g = p.gate.scale2 != nullptr, has_u = p.up.scale2 != nullptr;
     const float sg2 = has_g ? p.gate.scale2[el] : 1.0f, su2 = has_u ? p.up.scale2[el] : 1.0f;   // in flight under the row dots
-    int k0, k1;
-    share(64, blockDim.x >> 5, wid, k0, k1);
-    const uint8_t* gn = p.gate.nib + eo * (n / 2); const uint8_t* gs = p.gate.sc + eo * nsb;
-    const uint8_t* un = p.up.nib + eo * (n / 2); const uint8_t* us = p.up.sc + eo * nsb;
-    rows_list<MK_FP4, 4, 2>(k1 - k0, n, terms, gsh,
-        [&](int k, const uint8_t*& pa, const uint8_t*& pb, const int8_t*& q, const float*& s) {
-            const int kk = k0 + k, row = row0 + (kk & 31);
-            pa = (kk < 32 ? gn : un) + (size_t)row * (n / 2);
-            pb = (kk < 32 ? gs : us) + (size_t)row * nsb;
-            q = xq; s = xs;
-        },
-        [&](int k, float v) { s_gu[k0 + k] = v; });
+    {
+        const int kgs = n / 64, tile = wid >> 2;
+        int g0, g1;
+        share(kgs, 4, wid & 3, g0, g1);
+        const DevFp4& w = tile < 2 ? p.gate : p.up;
+        const size_t ro = eo + row0 + (tile & 1) * 16;                 // a multiple of 16: rows before it fill whole tiles
+        fp4_tile_terms<4>(w.nib + ro * (n / 2), w.sc + ro * nsb, g0, g1, xq, xs, terms + tile * 16 * (nsb + 1), nsb + 1);
+    }
+    __syncthreads();
+    if (tid < 64) s_gu[tid] = fold_terms(terms + tid * (nsb + 1), nsb);
     if (p.down_nib && b < 4 && wid == (int)(blockDim.x >> 5) - 1) {
         // this pick's down-projection weights, which the next kernel streams: into L2 while this one runs (the pick's blocks share them out)
         L2Hint h{};
@@ -654,15 +653,15 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     TL(TLK_MOE_GLU, 5);
 }
 size_t moe_glu_smem(int n_expert, int n) {
-    int nb = n / 32, gsh = lanes_shift(nb);
-    return (size_t)((n_expert + 31) & ~31) * 4 + n + (size_t)nb * 4 + (size_t)NWG * terms_floats(4, gsh, n / 16) * 4 + 64;
+    return (size_t)((n_expert + 31) & ~31) * 4 + n + (size_t)(n / 32) * 4 + (size_t)64 * (n / 16 + 1) * 4 + 64;
 }
 
 // ------------------------------------------------------------------------------------------------------
 // Routed experts, second half, with the whole FFN tail fused: down projections of the picks and of the
 // shared expert, the weighted sum in pick order, the sigmoid-gated shared term and the residual add
-// (src/model/qwen35.rs:1659-1699, src/ops/mod.rs:1134-1171, src/model/qwen35.rs:1090). A warp takes one
-// output row at a time and runs all its streams (picks + shared) in one pass, so their loads share one round trip.
+// (src/model/qwen35.rs:1659-1699, src/ops/mod.rs:1134-1171, src/model/qwen35.rs:1090). A block takes a tile of 16 output rows: its warps
+// share the (pick, slice of k) pieces of the tile and the shared expert's rows among themselves, every load issued before the
+// first dot; a lane per (pick, row) folds that row's terms in order, and a lane per row combines.
 struct MoeDown {
     const int8_t* hq; const float* hs; int n_used, ff;
     const int32_t* ids; const float* wts;
@@ -679,113 +678,104 @@ struct MoeDown {
     float* o_rows[8];                               // non-null: row b's picks go to o_rows[b][k][n_out] (rank b's memory) instead of o_pairs
     int tl_slot;
 };
-template <int RP, bool PAIRS = false>
+constexpr int DOWN_KG = 4;                      // 64-element groups of k per piece
+template <bool PAIRS = false>
 __global__ void __launch_bounds__(NWG * 32) k_moe_down(MoeDown p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_el[16];
     __shared__ float s_wt[16];
     __shared__ float s_g;
     __shared__ int s_loc[16], s_nloc;        // picks whose expert is stored here, in pick order (expert-parallel pairs mode)
-    const int ff = p.ff, sff = p.sff, nbf = ff / 32, nbs = sff / 32, nsb = ff / 16;
-    const int gf = lanes_shift(nbf), gs = lanes_shift(nbs);
+    const int ff = p.ff, sff = p.sff, nbf = ff / 32, nbs = sff / 32, nsb = ff / 16, kgs = ff / 64, K = p.n_used;
     const int b = blockIdx.y, tid = threadIdx.x, wid = tid >> 5, nw = blockDim.x >> 5, lane = tid & 31;
-    const int n_out = p.down.n_out;
-    int8_t* hq = (int8_t*)smem;                           // [n_used][ff]
-    float* hs = (float*)(hq + p.n_used * ff);             // [n_used][nbf]
-    int8_t* sq = (int8_t*)(hs + p.n_used * nbf);          // [sff]
+    const int n_out = p.down.n_out, row0 = blockIdx.x * 16;
+    int8_t* hq = (int8_t*)smem;                           // [K][ff]
+    float* hs = (float*)(hq + K * ff);                    // [K][nbf]
+    int8_t* sq = (int8_t*)(hs + K * nbf);                 // [sff]
     float* ss = (float*)(sq + sff);                       // [nbs]
-    const int tf = max(terms_floats(RP, gf, nsb), terms_floats(1, gs, nbs));
-    float* terms = ss + nbs + wid * (tf + 32);
-    float* outv = terms + tf;                             // this warp's per-stream results
-    int b0, b1, r0, r1;
-    share(n_out, gridDim.x, blockIdx.x, b0, b1);
-    share(b1 - b0, nw, wid, r0, r1);
+    float* terms = ss + nbs;                              // [K][16][nsb + 1]
+    float* sterms = terms + K * 16 * (nsb + 1);           // [16][nbs + 1]
+    float* outv = sterms + 16 * (nbs + 1);                // [16 rows][K + 2]
+    constexpr bool pairs = PAIRS;            // compile-time: the one-GPU kernel carries none of the expert-parallel branches
+    const bool shared_here = pairs ? b == p.own_row : !p.local_only;
     TL(TLK_MOE_DOWN, 0);
     pdl_trigger();
+    // the shared expert's weights do not depend on the routing: this thread's first 32-element unit is on its way before the wait
+    UnitW su{};
+    const int su_row = row0 + tid / nbs, su_u = tid % nbs;
+    const bool su_in = shared_here && tid < 16 * nbs;
+    if (su_in) unit_load(su, (const uint8_t*)p.shared_down.q + (size_t)su_row * sff, (const uint8_t*)p.shared_down.s + (size_t)su_row * (sff / 16), su_u);
     pdl_wait();
     TL(TLK_MOE_DOWN, 1);
-    for (int i = tid; i < p.n_used * ff / 16; i += blockDim.x) ((uint4*)hq)[i] = ((const uint4*)(p.hq + (size_t)b * p.n_used * ff))[i];
-    for (int i = tid; i < p.n_used * nbf; i += blockDim.x) hs[i] = p.hs[(size_t)b * p.n_used * nbf + i];
-    constexpr bool pairs = PAIRS;            // compile-time: the one-GPU kernel carries none of the expert-parallel branches
+    if (tid < K) {
+        int el = p.ids[(size_t)b * K + tid] - p.down.expert_lo;
+        s_el[tid] = (el < 0 || el >= p.down.n_expert) ? -1 : el;
+        s_wt[tid] = p.wts[(size_t)b * K + tid];
+    }
+    for (int i = tid; i < K * ff / 16; i += blockDim.x) ((uint4*)hq)[i] = ((const uint4*)(p.hq + (size_t)b * K * ff))[i];
+    for (int i = tid; i < K * nbf; i += blockDim.x) hs[i] = p.hs[(size_t)b * K * nbf + i];
     const size_t shb = pairs ? 0 : (size_t)b;        // where this row's shared-expert activation and gate logit sit
-    if (!pairs || b == p.own_row) {
+    if (shared_here) {
         for (int i = tid; i < sff / 16; i += blockDim.x) ((uint4*)sq)[i] = ((const uint4*)(p.sq + shb * sff))[i];
         for (int i = tid; i < nbs; i += blockDim.x) ss[i] = p.ss[shb * nbs + i];
     }
-    if (tid < p.n_used) {
-        int el = p.ids[(size_t)b * p.n_used + tid] - p.down.expert_lo;
-        s_el[tid] = (el < 0 || el >= p.down.n_expert) ? -1 : el;
-        s_wt[tid] = p.wts[(size_t)b * p.n_used + tid];
-    }
     if (tid == 32 && !pairs) s_g = sigmoid_f(p.logit[b]);
     __syncthreads();
-    if (pairs && tid == 0) { int n = 0; for (int k = 0; k < p.n_used; ++k) if (s_el[k] >= 0) s_loc[n++] = k; s_nloc = n; }
+    if (pairs && tid == 0) { int n = 0; for (int k = 0; k < K; ++k) if (s_el[k] >= 0) s_loc[n++] = k; s_nloc = n; }
     if (pairs) __syncthreads();
     TL(TLK_MOE_DOWN, 2);
     const bool has_s = p.down.scale2 != nullptr;
     float* x = p.x + (size_t)b * p.x_stride;
     // lane k keeps pick k's second scale; the load is issued here and first used after the row dots, so it costs no round trip
-    const float s2k = (has_s && lane < p.n_used && s_el[lane] >= 0) ? p.down.scale2[s_el[lane]] : 1.0f;
+    const int ck = tid % K, cr = tid / K;                 // the (pick, row) chain this thread folds
+    const float s2k = (has_s && cr < 16 && s_el[ck] >= 0) ? p.down.scale2[s_el[ck]] : 1.0f;
+    const int slices = (kgs + DOWN_KG - 1) / DOWN_KG, n_items = (pairs ? s_nloc : K) * slices;
 #pragma unroll 1
-    for (int row = b0 + r0; row < b0 + r1; ++row) {
-        // routed picks: item k = pick k of this row (pairs mode: the k-th LOCAL pick, so no row of an absent expert is read)
-        rows_list<MK_FP4, RP>(pairs ? s_nloc : p.n_used, ff, terms, gf,
-            [&](int k, const uint8_t*& pa, const uint8_t*& pb, const int8_t*& q, const float*& s) {
-                const int pk = pairs ? s_loc[k] : k;
-                const int el = max(s_el[pk], 0);
-                pa = p.down.nib + ((size_t)el * n_out + row) * (ff / 2);
-                pb = p.down.sc + ((size_t)el * n_out + row) * nsb;
-                q = hq + pk * ff; s = hs + pk * nbf;
-            },
-            [&](int k, float v) { outv[pairs ? s_loc[k] : k] = v; });
-        float sh = 0.0f;
-        if (pairs) {
-            if (b == p.own_row) {
-                rows_list<MK_Q8, 1>(1, sff, terms, gs,
-                    [&](int, const uint8_t*& pa, const uint8_t*& pb, const int8_t*& q, const float*& s) {
-                        pa = (const uint8_t*)p.shared_down.q + (size_t)row * sff;
-                        pb = (const uint8_t*)p.shared_down.s + (size_t)row * (sff / 16);
-                        q = sq; s = ss;
-                    },
-                    [&](int, float v) { p.shd[row] = v; });
-            }
-            __syncwarp();
-            if (lane < p.n_used && s_el[lane] >= 0) {
-                float* orow = p.o_rows[0] ? p.o_rows[b] + (size_t)lane * n_out : p.o_pairs + ((size_t)b * p.n_used + lane) * n_out;
-                orow[row] = has_s ? outv[lane] * s2k : outv[lane];
-            }
-            __syncwarp();
-            continue;
+    for (int it = wid; it < n_items; it += nw) {
+        const int pk = pairs ? s_loc[it / slices] : it / slices, g0 = (it % slices) * DOWN_KG, el = s_el[pk];
+        if (el < 0) continue;
+        const size_t ro = (size_t)el * n_out + row0;
+        fp4_tile_terms<DOWN_KG / 2>(p.down.nib + ro * (ff / 2), p.down.sc + ro * nsb, g0, min(kgs, g0 + DOWN_KG), hq + pk * ff, hs + pk * nbf, terms + pk * 16 * (nsb + 1), nsb + 1);
+    }
+    if (su_in) unit_terms(su, *(const uint4*)(sq + su_u * 32), *(const uint4*)(sq + su_u * 32 + 16), ss[su_u], sterms + (tid / nbs) * (nbs + 1), su_u);
+    if (shared_here)
+        for (int i = tid + blockDim.x; i < 16 * nbs; i += blockDim.x) {
+            const int r = i / nbs, u = i % nbs;
+            UnitW w;
+            unit_load(w, (const uint8_t*)p.shared_down.q + (size_t)(row0 + r) * sff, (const uint8_t*)p.shared_down.s + (size_t)(row0 + r) * (sff / 16), u);
+            unit_terms(w, *(const uint4*)(sq + u * 32), *(const uint4*)(sq + u * 32 + 16), ss[u], sterms + r * (nbs + 1), u);
         }
-        if (!p.local_only) {
-            rows_list<MK_Q8, 1>(1, sff, terms, gs,
-                [&](int, const uint8_t*& pa, const uint8_t*& pb, const int8_t*& q, const float*& s) {
-                    pa = (const uint8_t*)p.shared_down.q + (size_t)row * sff;
-                    pb = (const uint8_t*)p.shared_down.s + (size_t)row * (sff / 16);
-                    q = sq; s = ss;
-                },
-                [&](int, float v) { outv[31] = v; });
+    const bool live = tid < K * 16 && s_el[ck] >= 0;
+    const float xold = tid < 16 && !pairs && !p.local_only ? x[row0 + tid] : 0.0f;
+    __syncthreads();
+    if (live) {
+        float v = fold_terms(terms + (ck * 16 + cr) * (nsb + 1), nsb);
+        if (has_s) v = v * s2k;
+        if (pairs) (p.o_rows[0] ? p.o_rows[b] + (size_t)ck * n_out : p.o_pairs + ((size_t)b * K + ck) * n_out)[row0 + cr] = v;
+        else outv[cr * (K + 2) + ck] = v;
+    }
+    // the shared expert's rows fold on the warps after the picks'
+    const int st = tid - ((K * 16 + 31) & ~31);
+    if (shared_here && st >= 0 && st < 16) {
+        const float v = fold_terms(sterms + st * (nbs + 1), nbs);
+        if (pairs) p.shd[row0 + st] = v; else outv[st * (K + 2) + K] = v;
+    }
+    if (pairs) return;
+    __syncthreads();
+    if (tid < 16) {
+        float acc = 0.0f;                                   // experts in pick order from zero, shared last
+        for (int k = 0; k < K; ++k) {
+            if (s_el[k] < 0) continue;
+            acc += s_wt[k] * outv[tid * (K + 2) + k];
         }
-        __syncwarp();
-        if (has_s && lane < p.n_used) outv[lane] = outv[lane] * s2k;
-        __syncwarp();
-        if (lane == 0) {
-            float acc = 0.0f;                                   // experts in pick order from zero, shared last
-            for (int k = 0; k < p.n_used; ++k) {
-                if (s_el[k] < 0) continue;
-                acc += s_wt[k] * outv[k];
-            }
-            if (p.local_only) p.partial[(size_t)b * n_out + row] = acc;
-            else { sh = outv[31]; acc += sh * s_g; x[row] += acc; }
-        }
-        __syncwarp();
+        if (p.local_only) p.partial[(size_t)b * n_out + row0 + tid] = acc;
+        else { acc += outv[tid * (K + 2) + K] * s_g; x[row0 + tid] = xold + acc; }
     }
     TL(TLK_MOE_DOWN, 3);
 }
-size_t moe_down_smem(int n_used, int ff, int sff, int rp) {
-    int gf = lanes_shift(ff / 32), gs = lanes_shift(sff / 32);
-    int tf = std::max(terms_floats(rp, gf, ff / 16), terms_floats(1, gs, sff / 32));
-    return (size_t)n_used * ff + (size_t)n_used * (ff / 32) * 4 + sff + (size_t)(sff / 32) * 4 + (size_t)NWG * (tf + 32) * 4 + 64;
+size_t moe_down_smem(int n_used, int ff, int sff) {
+    return (size_t)n_used * ff + (size_t)n_used * (ff / 32) * 4 + sff + (size_t)(sff / 32) * 4 +
+           ((size_t)n_used * 16 * (ff / 16 + 1) + 16 * (sff / 32 + 1) + 16 * (n_used + 2)) * 4 + 64;
 }
 
 // ------------------------------------------------------------------------------------------------------

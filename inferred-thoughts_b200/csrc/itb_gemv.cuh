@@ -20,13 +20,23 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     return v;
 }
 
+// Where element e of a 32-element activation block stands in the f16 rows the many-row expert kernels read (itb_exp.cuh): the 8
+// elements a lane of an MMA quad multiplies (4 of each 16-element half) lie together, so one 16-byte read feeds two MMAs. The
+// NVFP4 nibbles lie the same way (k_repack_fp4).
+__host__ __device__ __forceinline__ int exp_pos(int e) { return ((e & 15) >> 2) * 8 + (e >> 4) * 4 + (e & 3); }
+__device__ __forceinline__ uint32_t f16x2_of_ints(int a, int b) {
+    const __half2 h = __halves2half2(__int2half_rn(a), __int2half_rn(b));
+    return *(const uint32_t*)&h;
+}
+
 // ---- activation prologues ------------------------------------------------------------------------
 // RMSNorm of one row into shared memory: f32 squares, f64 accumulation (tree), (x*scale)*w
 // (src/ops/naive.rs:139-152, :633-640). `red` holds blockDim.x/32 doubles.
 // With xq/xs given, the vector path also quantises the normalised row to Q8_0 in the same pass (8 consecutive lanes hold
-// one 32-block; src/ops/naive.rs:653-675) and returns true; otherwise the caller quantises from xn.
+// one 32-block; src/ops/naive.rs:653-675) and returns true; otherwise the caller quantises from xn. xh: the quants also as f16
+// in the order of exp_pos.
 __device__ __forceinline__ bool block_rms_norm(const float* __restrict__ x, const float* __restrict__ w, int n, float eps,
-                                               float* xn, double* red, int8_t* xq = nullptr, float* xs = nullptr) {
+                                               float* xn, double* red, int8_t* xq = nullptr, float* xs = nullptr, __half* xh = nullptr) {
     const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if ((n & 3) == 0 && n <= 16 * (int)blockDim.x && ((((uintptr_t)x) | ((uintptr_t)w) | ((uintptr_t)xn)) & 15) == 0) {
         // the row and the norm weights as float4, every load in flight before the first use: one memory round trip
@@ -68,6 +78,7 @@ __device__ __forceinline__ bool block_rms_norm(const float* __restrict__ x, cons
                     q.x = (signed char)fminf(127.0f, fmaxf(-128.0f, roundf(o.x * id))); q.y = (signed char)fminf(127.0f, fmaxf(-128.0f, roundf(o.y * id)));
                     q.z = (signed char)fminf(127.0f, fmaxf(-128.0f, roundf(o.z * id))); q.w = (signed char)fminf(127.0f, fmaxf(-128.0f, roundf(o.w * id)));
                     ((char4*)xq)[i] = q;
+                    if (xh) *(uint2*)(xh + (size_t)(i >> 3) * 32 + exp_pos((i & 7) * 4)) = make_uint2(f16x2_of_ints(q.x, q.y), f16x2_of_ints(q.z, q.w));
                     if ((i & 7) == 0) xs[i >> 3] = __half2float(__float2half_rn(d));
                 }
             }
@@ -130,49 +141,69 @@ __device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t se
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
-__device__ __forceinline__ int fp4_dot8(uint32_t w, uint32_t a0, uint32_t a1) {
+// A 16-byte unit of 32 codes (word t: elements 4t..4t+3 of the first 16 in the low half, of the second 16 in the high half)
+// against 32 int8 values (xa: the first 16, xb: the second): the two sub-blocks' integer dots.
+__device__ __forceinline__ void fp4_unit_dots(const uint4& w, const uint4& xa, const uint4& xb, int& s0, int& s1) {
     const uint32_t P0 = 0x03020100u, P1 = 0x0c080604u;
-    uint32_t n = w ^ 0x88888888u;
-    int pos = __dp4a((int)prmt_raw(P0, P1, w), (int)a0, 0);
-    pos = __dp4a((int)prmt_raw(P0, P1, w >> 16), (int)a1, pos);
-    int neg = __dp4a((int)prmt_raw(P0, P1, n), (int)a0, 0);
-    neg = __dp4a((int)prmt_raw(P0, P1, n >> 16), (int)a1, neg);
-    return pos - neg;
+    const uint32_t ww[4] = {w.x, w.y, w.z, w.w}, a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {xb.x, xb.y, xb.z, xb.w};
+    int p0 = 0, n0 = 0, p1 = 0, n1 = 0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const uint32_t v = ww[t], n = v ^ 0x88888888u;
+        p0 = __dp4a((int)prmt_raw(P0, P1, v), (int)a[t], p0);
+        n0 = __dp4a((int)prmt_raw(P0, P1, n), (int)a[t], n0);
+        p1 = __dp4a((int)prmt_raw(P0, P1, v >> 16), (int)b[t], p1);
+        n1 = __dp4a((int)prmt_raw(P0, P1, n >> 16), (int)b[t], n1);
+    }
+    s0 = p0 - n0; s1 = p1 - n1;
 }
 
-// Matrix kinds the row cores understand. Plane A: Q8_0 int8 quants (n_in bytes per row) or NVFP4 nibbles
-// (n_in/2); plane B: f16 scales per 32 (n_in/16 bytes per row) or UE4M3 codes per 16 (n_in/16).
-enum { MK_Q8 = 0, MK_FP4 = 1 };
-template <int KIND> __host__ __device__ __forceinline__ int plane_a_bytes(int n_in) { return KIND == MK_Q8 ? n_in : n_in / 2; }
-__host__ __device__ __forceinline__ int plane_b_bytes(int n_in) { return n_in / 16; }
-// f32 terms per row: one per Q8_0 block of 32, or one per NVFP4 sub-block of 16.
-template <int KIND> __host__ __device__ __forceinline__ int row_terms(int n_in) { return KIND == MK_Q8 ? n_in / 32 : n_in / 16; }
-
-// One lane's 32-element unit of one row: 32 bytes (Q8_0) or 16 bytes (NVFP4) of weights plus the 2 scale bytes.
+// One lane's 32-element unit of one Q8_0 row: 32 quants and the f16 scale.
 struct UnitW { uint4 a, b; uint32_t s; };
-template <int KIND>
 __device__ __forceinline__ void unit_load(UnitW& w, const uint8_t* pa, const uint8_t* pb, int u) {
-    if (KIND == MK_Q8) { w.a = ld_stream16(pa + u * 32); w.b = ld_stream16(pa + u * 32 + 16); }
-    else w.a = ld_stream16(pa + u * 16);
+    w.a = ld_stream16(pa + u * 32); w.b = ld_stream16(pa + u * 32 + 16);
     w.s = __ldg((const uint16_t*)(pb + u * 2));
 }
-// The unit's f32 term(s) into t (row's term array), against the activation unit xa|xb with scale dx.
-template <int KIND>
+// The unit's f32 term into t (row's term array), against the activation unit xa|xb with scale dx.
 __device__ __forceinline__ void unit_terms(const UnitW& w, const uint4& xa, const uint4& xb, float dx, float* t, int u) {
-    if (KIND == MK_Q8) {
-        int s = 0;
-        s = __dp4a((int)w.a.x, (int)xa.x, s); s = __dp4a((int)w.a.y, (int)xa.y, s);
-        s = __dp4a((int)w.a.z, (int)xa.z, s); s = __dp4a((int)w.a.w, (int)xa.w, s);
-        s = __dp4a((int)w.b.x, (int)xb.x, s); s = __dp4a((int)w.b.y, (int)xb.y, s);
-        s = __dp4a((int)w.b.z, (int)xb.z, s); s = __dp4a((int)w.b.w, (int)xb.w, s);
-        t[u] = i2f_small(s) * (f16_bits_to_f32((uint16_t)w.s) * dx);           // src/ops/naive.rs:701
-    } else {
-        int s0 = fp4_dot8(w.a.x, xa.x, xa.y) + fp4_dot8(w.a.y, xa.z, xa.w);
-        int s1 = fp4_dot8(w.a.z, xb.x, xb.y) + fp4_dot8(w.a.w, xb.z, xb.w);
-        float d0, d1;
-        ue4m3x2_half(w.s, d0, d1);
-        t[2 * u] = dx * d0 * i2f_small(s0);                                    // src/ops/naive.rs:730
-        t[2 * u + 1] = dx * d1 * i2f_small(s1);
+    int s = 0;
+    s = __dp4a((int)w.a.x, (int)xa.x, s); s = __dp4a((int)w.a.y, (int)xa.y, s);
+    s = __dp4a((int)w.a.z, (int)xa.z, s); s = __dp4a((int)w.a.w, (int)xa.w, s);
+    s = __dp4a((int)w.b.x, (int)xb.x, s); s = __dp4a((int)w.b.y, (int)xb.y, s);
+    s = __dp4a((int)w.b.z, (int)xb.z, s); s = __dp4a((int)w.b.w, (int)xb.w, s);
+    t[u] = i2f_small(s) * (f16_bits_to_f32((uint16_t)w.s) * dx);           // src/ops/naive.rs:701
+}
+// One NVFP4 row's 64 elements (v0 | v1: its 32 bytes, s4: its 4 scale codes) against 64 int8 activations with two block scales:
+// the four sub-blocks' f32 terms.
+__device__ __forceinline__ void fp4_group_terms(const uint4& v0, const uint4& v1, uint32_t s4, const int8_t* xq, const float* xs, float* t) {
+    const uint4* x = (const uint4*)xq;
+    int a, b;
+    float d0, d1;
+    fp4_unit_dots(make_uint4(v0.x, v0.z, v1.x, v1.z), x[0], x[1], a, b);
+    ue4m3x2_half(s4 & 0xffffu, d0, d1);
+    t[0] = xs[0] * d0 * i2f_small(a); t[1] = xs[0] * d1 * i2f_small(b);           // src/ops/naive.rs:730
+    fp4_unit_dots(make_uint4(v0.y, v0.w, v1.y, v1.w), x[2], x[3], a, b);
+    ue4m3x2_half(s4 >> 16, d0, d1);
+    t[2] = xs[1] * d0 * i2f_small(a); t[3] = xs[1] * d1 * i2f_small(b);
+}
+// A warp on one 16-row tile of an NVFP4 matrix (nib, sc: the tile), groups [g0, g1) of 64 elements: lane = (row, group parity), so a
+// trip reads two groups, 1 KB in one piece. UB trips are loaded before the first dot. Terms go to t[row * stride + term].
+template <int UB>
+__device__ __forceinline__ void fp4_tile_terms(const uint8_t* __restrict__ nib, const uint8_t* __restrict__ sc, int g0, int g1, const int8_t* xq, const float* xs, float* t, int stride) {
+    const int lane = threadIdx.x & 31, r = lane & 15, par = lane >> 4;
+#pragma unroll 1
+    for (int k0 = g0 + par; k0 < g1; k0 += 2 * UB) {
+        uint4 v[UB][2]; uint32_t s[UB];
+#pragma unroll
+        for (int i = 0; i < UB; ++i)
+            if (k0 + 2 * i < g1) {
+                const uint8_t* p = nib + (size_t)(k0 + 2 * i) * 512 + r * 32;
+                v[i][0] = ld_stream16(p); v[i][1] = ld_stream16(p + 16);
+                s[i] = __ldg((const uint32_t*)(sc + (size_t)(k0 + 2 * i) * 64 + r * 4));
+            }
+#pragma unroll
+        for (int i = 0; i < UB; ++i)
+            if (k0 + 2 * i < g1) { const int k = k0 + 2 * i; fp4_group_terms(v[i][0], v[i][1], s[i], xq + k * 64, xs + k * 2, t + r * stride + k * 4); }
     }
 }
 // Ascending fold of one row's terms.
@@ -186,13 +217,13 @@ __device__ __forceinline__ float fold_terms(const float* t, int nt) {
 // Rows [r0, r1) of one matrix (planes pa/pb, row 0 first) against one quantised activation (xq, xs in shared
 // memory). terms: warp-private shared scratch of terms_floats(RP, gsh, row_terms) floats. epi(row, value) is
 // called by one lane per row. UB units per lane and trip are loaded before the first dot.
-template <int KIND, int RP, int UB, class Epi>
+template <int RP, int UB, class Epi>
 __device__ __forceinline__ void rows_direct_ub(const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r0, int r1,
                                             const int8_t* xq, const float* xs, float* terms, int gsh, Epi epi) {
     const int G = 1 << gsh, lane = threadIdx.x & 31, sub = lane & (G - 1), slot = lane >> gsh;
     const int SLOTS = 32 >> gsh, ROWS = RP * SLOTS;
-    const int nunits = n_in >> 5, nt = row_terms<KIND>(n_in), stride = nt + 1;
-    const int arb = plane_a_bytes<KIND>(n_in), brb = plane_b_bytes(n_in);
+    const int nunits = n_in >> 5, nt = n_in >> 5, stride = nt + 1;
+    const int arb = n_in, brb = n_in / 16;
 #pragma unroll 1
     for (int r = r0; r < r1; r += ROWS) {
 #pragma unroll 1
@@ -204,7 +235,7 @@ __device__ __forceinline__ void rows_direct_ub(const uint8_t* __restrict__ pa, c
                 if (row < r1) {
 #pragma unroll
                     for (int h = 0; h < UB; ++h)
-                        if (u0 + h * G < nunits) unit_load<KIND>(w[h][i], pa + (size_t)row * arb, pb + (size_t)row * brb, u0 + h * G);
+                        if (u0 + h * G < nunits) unit_load(w[h][i], pa + (size_t)row * arb, pb + (size_t)row * brb, u0 + h * G);
                 }
             }
 #pragma unroll
@@ -215,7 +246,7 @@ __device__ __forceinline__ void rows_direct_ub(const uint8_t* __restrict__ pa, c
                     const float dx = xs[u];
 #pragma unroll
                     for (int i = 0; i < RP; ++i)
-                        if (r + i * SLOTS + slot < r1) unit_terms<KIND>(w[h][i], xa, xb, dx, terms + (i * SLOTS + slot) * stride, u);
+                        if (r + i * SLOTS + slot < r1) unit_terms(w[h][i], xa, xb, dx, terms + (i * SLOTS + slot) * stride, u);
                 }
             }
         }
@@ -225,58 +256,16 @@ __device__ __forceinline__ void rows_direct_ub(const uint8_t* __restrict__ pa, c
     }
 }
 
-// A list of independent row-dots, each with its own weight row and its own activation: item k of [0, n) is
-// described by src(k, pa, pb, xq, xs) (weight planes of THE ROW, activation in shared memory). One pass
-// takes RP*(32/G) items with every load issued before the first dot; epi(k, value) by one lane per item.
-template <int KIND, int RP, int UB = 1, class Src, class Epi>
-__device__ __forceinline__ void rows_list(int n, int n_in, float* terms, int gsh, Src src, Epi epi) {
-    const int G = 1 << gsh, lane = threadIdx.x & 31, sub = lane & (G - 1), slot = lane >> gsh;
-    const int SLOTS = 32 >> gsh, ROWS = RP * SLOTS;
-    const int nunits = n_in >> 5, nt = row_terms<KIND>(n_in), stride = nt + 1;
-#pragma unroll 1
-    for (int k0 = 0; k0 < n; k0 += ROWS) {
-        const uint8_t *pa[RP], *pb[RP];
-        const int8_t* xq[RP];
-        const float* xs[RP];
-#pragma unroll
-        for (int i = 0; i < RP; ++i) {
-            int k = k0 + i * SLOTS + slot;
-            if (k < n) src(k, pa[i], pb[i], xq[i], xs[i]);
-        }
-#pragma unroll 1
-        for (int u0 = sub; u0 < nunits; u0 += UB * G) {
-            UnitW w[UB][RP];
-#pragma unroll
-            for (int h = 0; h < UB; ++h)
-#pragma unroll
-                for (int i = 0; i < RP; ++i)
-                    if (k0 + i * SLOTS + slot < n && u0 + h * G < nunits) unit_load<KIND>(w[h][i], pa[i], pb[i], u0 + h * G);
-#pragma unroll
-            for (int h = 0; h < UB; ++h)
-#pragma unroll
-                for (int i = 0; i < RP; ++i)
-                    if (k0 + i * SLOTS + slot < n && u0 + h * G < nunits) {
-                        const int u = u0 + h * G;
-                        const uint4 xa = *(const uint4*)(xq[i] + u * 32), xb = *(const uint4*)(xq[i] + u * 32 + 16);
-                        unit_terms<KIND>(w[h][i], xa, xb, xs[i][u], terms + (i * SLOTS + slot) * stride, u);
-                    }
-        }
-        __syncwarp();
-        if (lane < ROWS && k0 + lane < n) epi(k0 + lane, fold_terms(terms + lane * stride, nt));
-        __syncwarp();
-    }
-}
-
 // As rows_direct_ub, but the terms of up to `br` rows are collected first and then folded by `br` lanes at
 // once: the fold is a serial chain per row, so folding one or two rows at a time leaves most lanes idle and
 // costs as many instructions as the dots themselves. terms: br * (row_terms + 1) floats, warp-private.
-template <int KIND, int RP, int UB, class Epi>
+template <int RP, int UB, class Epi>
 __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r0, int r1,
                                              const int8_t* xq, const float* xs, float* terms, int br, int gsh, Epi epi) {
     const int G = 1 << gsh, lane = threadIdx.x & 31, sub = lane & (G - 1), slot = lane >> gsh;
     const int SLOTS = 32 >> gsh, ROWS = RP * SLOTS;
-    const int nunits = n_in >> 5, nt = row_terms<KIND>(n_in), stride = nt + 1;
-    const int arb = plane_a_bytes<KIND>(n_in), brb = plane_b_bytes(n_in);
+    const int nunits = n_in >> 5, nt = n_in >> 5, stride = nt + 1;
+    const int arb = n_in, brb = n_in / 16;
     br = min(br, 32) / ROWS * ROWS;   // whole passes per batch (the caller sizes terms for at least one pass)
 #pragma unroll 1
     for (int rb = r0; rb < r1; rb += br) {
@@ -292,7 +281,7 @@ __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, con
                     if (row < rend) {
 #pragma unroll
                         for (int h = 0; h < UB; ++h)
-                            if (u0 + h * G < nunits) unit_load<KIND>(w[h][i], pa + (size_t)row * arb, pb + (size_t)row * brb, u0 + h * G);
+                            if (u0 + h * G < nunits) unit_load(w[h][i], pa + (size_t)row * arb, pb + (size_t)row * brb, u0 + h * G);
                     }
                 }
 #pragma unroll
@@ -304,7 +293,7 @@ __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, con
 #pragma unroll
                         for (int i = 0; i < RP; ++i) {
                             const int row = r + i * SLOTS + slot;
-                            if (row < rend) unit_terms<KIND>(w[h][i], xa, xb, dx, terms + (row - rb) * stride, u);
+                            if (row < rend) unit_terms(w[h][i], xa, xb, dx, terms + (row - rb) * stride, u);
                         }
                     }
                 }
@@ -316,21 +305,15 @@ __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, con
     }
 }
 
-template <int KIND, int RP, class Epi>
+template <int RP, class Epi>
 __device__ __forceinline__ void rows_direct(const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r0, int r1,
                                             const int8_t* xq, const float* xs, float* terms, int gsh, Epi epi) {
-    rows_direct_ub<KIND, RP, 2>(pa, pb, n_in, r0, r1, xq, xs, terms, gsh, epi);
+    rows_direct_ub<RP, 2>(pa, pb, n_in, r0, r1, xq, xs, terms, gsh, epi);
 }
 template <int RP, class Epi>
 __device__ __forceinline__ void q8_rows(const DevQ8& w, int r0, int r1, const int8_t* xq, const float* xs, float* terms, int gsh, Epi epi) {
-    rows_direct<MK_Q8, RP>((const uint8_t*)w.q, (const uint8_t*)w.s, w.n_in, r0, r1, xq, xs, terms, gsh, epi);
+    rows_direct<RP>((const uint8_t*)w.q, (const uint8_t*)w.s, w.n_in, r0, r1, xq, xs, terms, gsh, epi);
 }
-template <int RP, class Epi>
-__device__ __forceinline__ void fp4_rows(const uint8_t* nib, const uint8_t* sc, int n_in, int r0, int r1, const int8_t* xq,
-                                         const float* xs, float* terms, int gsh, Epi epi) {
-    rows_direct<MK_FP4, RP>(nib, sc, n_in, r0, r1, xq, xs, terms, gsh, epi);
-}
-
 // ---- F32 rows --------------------------------------------------------------------------------------
 // EXACT: serial-k left fold per output like the CPU path (src/ops/naive.rs:845-849). A warp takes one row at a time: the lanes
 // fetch the weights (coalesced) and put the products w[k] * x[k] of a tile of the row into the warp's shared scratch, then

@@ -20,9 +20,12 @@ struct DevQ8 {
     const uint16_t* s = nullptr;
     int n_in = 0, n_out = 0;
 };
-// NVFP4 stack repacked from 36-byte blocks (src/quant/mod.rs:338-357): nibbles [E][n_out][n_in/2] with
-// nibble k of byte-pair order = element order (low nibble first), scales [E][n_out][n_in/16] UE4M3 codes
-// with bit 7 cleared and 0x7f mapped to 0 (both read as the reference reads them, src/quant/mod.rs:271-284).
+// NVFP4 stack repacked from 36-byte blocks (src/quant/mod.rs:338-357), tiles of 16 rows x 64 elements of k, k fastest:
+// nibbles [E][n_out / 16][n_in / 64][16 rows][32 B], scales [E][n_out / 16][n_in / 64][16 rows][4] UE4M3 codes with bit 7 cleared
+// and 0x7f mapped to 0 (both read as the reference reads them, src/quant/mod.rs:271-284); n_out rounded up to 16. Word 2t + u of a
+// row's 32 bytes holds elements 4t..4t+3 (low half) and 16+4t..16+4t+3 (high half) of the u-th 32 of its 64 elements, low nibble
+// first: what the lane of an MMA quad multiplies is one 8-byte read (itb_exp.cuh), a warp that dots 16 rows reads 512 contiguous
+// bytes, and any group of 16 rows is contiguous.
 struct DevFp4 {
     const uint8_t* nib = nullptr;
     const uint8_t* sc = nullptr;
@@ -31,7 +34,11 @@ struct DevFp4 {
     int expert_lo = 0;              // first expert stored (expert-parallel shard); ids are global
     const int* slot_map = nullptr;  // tiered experts: global id -> slot in the HBM pool (nib/sc/scale2 are the pool), -1 = not resident
 };
+__host__ __device__ inline size_t fp4_rows_pad(size_t n_out) { return (n_out + 15) & ~(size_t)15; }
 #ifdef __CUDACC__
+// Byte offsets of (row, 64-element group) inside one matrix.
+__device__ __forceinline__ size_t fp4_nib_at(int row, int kg, int kgs) { return ((size_t)(row >> 4) * kgs + kg) * 512 + (row & 15) * 32; }
+__device__ __forceinline__ size_t fp4_sc_at(int row, int kg, int kgs) { return ((size_t)(row >> 4) * kgs + kg) * 64 + (row & 15) * 4; }
 // Where expert `e` of a stack lives on this device: its index into nib/sc/scale2, or -1 (stored elsewhere / not resident).
 __device__ __forceinline__ int fp4_slot(const DevFp4& w, int e) {
     if (w.slot_map) return w.slot_map[e];
@@ -78,7 +85,7 @@ struct itb_ctx {
     std::unordered_map<const void*, WeightEntry> weights;
     // current device route (src/ops/cuda/ops/mod.rs:299-302)
     int32_t* route_ids = nullptr;
-    int* pair_off = nullptr; int* pair_list = nullptr; size_t pair_cap = 0, pair_experts = 0;   // pairs grouped by expert (many-row expert matmuls)
+    int* pair_off = nullptr; int* pair_list = nullptr; void* pair_tiles = nullptr; size_t pair_cap = 0, pair_experts = 0;   // pairs grouped by expert (many-row expert matmuls)
     float* route_w = nullptr;
     size_t route_cap = 0, route_n_tok = 0, route_n_used = 0;
     // scratch for activation quantisation
@@ -146,7 +153,7 @@ bool itb_ensure_xq(itb_ctx* c, size_t n_elems);
 
 // repack (itb_ctx.cu): raw reference-layout bytes on the device -> kernel layouts
 void itb_repack_q8(cudaStream_t st, const uint8_t* raw, int8_t* q, uint16_t* s, size_t n_blocks_total);
-void itb_repack_fp4(cudaStream_t st, const uint8_t* raw, uint8_t* nib, uint8_t* sc, size_t n_blocks64_total);
+void itb_repack_fp4(cudaStream_t st, const uint8_t* raw, uint8_t* nib, uint8_t* sc, size_t n_in, size_t n_out, size_t n_expert);
 void itb_f16_to_f32(cudaStream_t st, const uint16_t* raw, float* out, size_t n);
 
 // ------------------------------------------------------------------ device helpers

@@ -293,31 +293,36 @@ __global__ void k_matmul_q8(DevQ8 w, const int8_t* xq_g, const float* xs_g, floa
 
 // NVFP4 rows for (token,pick) pairs: pair i uses expert ids[i] (or expert 0 when ids is null), activation row
 // x_row(i) and writes out row i, times the expert's second scale (src/ops/mod.rs:1049-1088).
-__global__ void k_matmul_fp4(DevFp4 w, const int32_t* ids, int n_used, int rows_mode, const int8_t* xq_g, const float* xs_g, float* out) {
+// A block takes 32 rows (two 16-row tiles) at a time, four warps to a tile and a quarter of k each.
+__global__ void __launch_bounds__(256) k_matmul_fp4(DevFp4 w, const int32_t* ids, int n_used, int rows_mode, const int8_t* xq_g, const float* xs_g, float* out) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int RP = 4;
-    int nb = w.n_in / 32, nsb = w.n_in / 16, gsh = lanes_shift(nb);
+    const int n = w.n_in, nb = n / 32, nsb = n / 16, kgs = n / 64, tid = threadIdx.x, wid = tid >> 5;
     int8_t* xq = (int8_t*)smem;
-    float* xs = (float*)(smem + w.n_in);
-    float* terms = xs + nb + (threadIdx.x >> 5) * terms_floats(RP, gsh, nsb);
+    float* xs = (float*)(smem + n);
+    float* terms = xs + nb;                                              // [32][nsb + 1]
     size_t i = blockIdx.y;
     int e = ids ? ids[i] : 0;
     size_t xr = rows_mode == 0 ? i : rows_mode == 1 ? i / n_used : 0;  // rows==picks / rows==n_tok / single row
-    for (int k = threadIdx.x; k < w.n_in / 16; k += blockDim.x) ((uint4*)xq)[k] = ((const uint4*)(xq_g + xr * w.n_in))[k];
-    for (int k = threadIdx.x; k < nb; k += blockDim.x) xs[k] = xs_g[xr * nb + k];
-    __syncthreads();
+    for (int k = tid; k < n / 16; k += 256) ((uint4*)xq)[k] = ((const uint4*)(xq_g + xr * n))[k];
+    for (int k = tid; k < nb; k += 256) xs[k] = xs_g[xr * nb + k];
     int el = e - w.expert_lo;
     if (el < 0 || el >= w.n_expert) return;  // not stored on this device (expert-parallel shard)
-    const uint8_t* nib = w.nib + (size_t)el * w.n_out * (w.n_in / 2);
-    const uint8_t* sc = w.sc + (size_t)el * w.n_out * nsb;
-    float s2 = w.scale2 ? w.scale2[el] : 1.0f;
-    bool has_s2 = w.scale2 != nullptr;
-    int b0, b1, r0, r1;
-    share(w.n_out, gridDim.x, blockIdx.x, b0, b1);
-    share(b1 - b0, blockDim.x >> 5, threadIdx.x >> 5, r0, r1);
+    const size_t pad = fp4_rows_pad(w.n_out);
+    const uint8_t* nib = w.nib + (size_t)el * pad * (n / 2);
+    const uint8_t* sc = w.sc + (size_t)el * pad * nsb;
+    const float s2 = w.scale2 ? w.scale2[el] : 1.0f;
     float* o = out + i * w.n_out;
-    fp4_rows<RP>(nib, sc, w.n_in, b0 + r0, b0 + r1, xq, xs, terms, gsh, [&](int row, float v) { o[row] = has_s2 ? v * s2 : v; });
+    int g0, g1;
+    share(kgs, 4, wid & 3, g0, g1);
+    for (int r0 = blockIdx.x * 32; r0 < w.n_out; r0 += gridDim.x * 32) {
+        __syncthreads();                                                  // the activation is staged; the previous rows are folded
+        const int row = r0 + (wid >> 2) * 16;
+        if (row < w.n_out) fp4_tile_terms<4>(nib + (size_t)row * (n / 2), sc + (size_t)row * nsb, g0, g1, xq, xs, terms + (wid >> 2) * 16 * (nsb + 1), nsb + 1);
+        __syncthreads();
+        if (tid < 32 && r0 + tid < w.n_out) { const float v = fold_terms(terms + tid * (nsb + 1), nsb); o[r0 + tid] = w.scale2 ? v * s2 : v; }
+    }
 }
+static inline size_t matmul_fp4_smem(int n) { return (size_t)n + (size_t)(n / 32) * 4 + (size_t)32 * (n / 16 + 1) * 4; }
 
 // Multi-token matmuls on the int8 MMA path: grid (row tiles, token tiles of 32). A warp owns 16 rows and NJ of
 // the tile's 4 groups of 8 tokens: NJ=4, 8 warps and 128 rows per block when there are many token tiles (prefill);

@@ -174,12 +174,21 @@ __device__ __forceinline__ int glu_units(const MegaParams& p) { return p.n_used 
 struct DownPlan { int o0, o1, nr, pc, nchunks; uint32_t ra, rb; };
 __device__ __forceinline__ DownPlan down_plan(const MegaParams& p) {
     DownPlan d;
-    share(p.H, gridDim.x, blockIdx.x, d.o0, d.o1);
+    share(p.H / 16, gridDim.x, blockIdx.x, d.o0, d.o1);      // whole 16-row tiles: a tile of an expert's matrix is one contiguous piece
+    d.o0 *= 16; d.o1 *= 16;
     d.nr = d.o1 - d.o0;
     d.ra = (uint32_t)p.ff / 2; d.rb = (uint32_t)p.ff / 16;
     d.pc = d.nr ? max(1, min(p.n_used, p.slot_b / (int)(d.nr * (d.ra + d.rb)))) : p.n_used;
     d.nchunks = d.nr ? (p.n_used + d.pc - 1) / d.pc : 0;
     return d;
+}
+
+// The shared expert's down rows of this block: the same output rows as the routed picks'.
+__device__ __forceinline__ RowPlan down_shared_plan(const MegaParams& p, const DevQ8& w, int slot_bytes) {
+    RowPlan pl = q8_plan(w, slot_bytes);
+    const DownPlan d = down_plan(p);
+    pl.r0 = d.o0; pl.r1 = d.o1; pl.nchunks = (d.nr + pl.rc - 1) / pl.rc;
+    return pl;
 }
 
 // ------------------------------------------------------------------------------------------------ producers
@@ -248,7 +257,7 @@ __device__ __noinline__ void mg_producer_static(const MegaParams& p, MegaCtl* ct
             } else if (type == MS_OUT) {
                 const DevQ8 w = st->w; ok = prod_rows(p, ctl, r, q8_plan(w, r.slot_bytes), (const uint8_t*)w.q, (const uint8_t*)w.s, s);
             } else if (type == MS_DOWN) {
-                const DevQ8 w = st->shared_down; ok = prod_rows(p, ctl, r, q8_plan(w, r.slot_bytes), (const uint8_t*)w.q, (const uint8_t*)w.s, s);
+                const DevQ8 w = st->shared_down; ok = prod_rows(p, ctl, r, down_shared_plan(p, w, r.slot_bytes), (const uint8_t*)w.q, (const uint8_t*)w.s, s);
             }
         }
         __syncwarp();
@@ -332,19 +341,12 @@ __device__ __forceinline__ void q8_row_terms(const uint8_t* wa, const uint8_t* w
         }
     }
 }
-__device__ __forceinline__ void fp4_row_terms(const uint8_t* wa, const uint8_t* wb, int n_in, const int8_t* xq, const float* xs, float* t) {
-    const int lane = threadIdx.x & 31, np = n_in >> 5;
-#pragma unroll 2
-    for (int pp = lane; pp < np; pp += 32) {
-        const uint4 w = *(const uint4*)(wa + pp * 16);
-        const uint4 xa = *(const uint4*)(xq + pp * 32), xb = *(const uint4*)(xq + pp * 32 + 16);
-        const int s0 = fp4_dot8(w.x, xa.x, xa.y) + fp4_dot8(w.y, xa.z, xa.w);
-        const int s1 = fp4_dot8(w.z, xb.x, xb.y) + fp4_dot8(w.w, xb.z, xb.w);
-        float d0, d1;
-        ue4m3x2_half(((const uint16_t*)wb)[pp], d0, d1);
-        const float dx = xs[pp];
-        t[2 * pp] = dx * d0 * i2f_small(s0);                                                      // src/ops/naive.rs:730
-        t[2 * pp + 1] = dx * d1 * i2f_small(s1);
+// Row r of a span of 16-row tiles (nibbles at wa, scales at wb), a lane per 64 elements.
+__device__ __forceinline__ void fp4_row_terms(const uint8_t* wa, const uint8_t* wb, int r, int n_in, const int8_t* xq, const float* xs, float* t) {
+    const int lane = threadIdx.x & 31, kgs = n_in >> 6;
+    for (int kg = lane; kg < kgs; kg += 32) {
+        const uint4* w = (const uint4*)(wa + fp4_nib_at(r, kg, kgs));
+        fp4_group_terms(w[0], w[1], *(const uint32_t*)(wb + fp4_sc_at(r, kg, kgs)), xq + kg * 64, xs + kg * 2, t + kg * 4);
     }
 }
 
@@ -364,7 +366,7 @@ struct Pending {
 
 // Consume a RowPlan's chunks of a quantised matrix from ring `r`: warp w takes rows w, w + MG_NW, ... of every chunk.
 // `claim(row)` runs on the lane that will fold `row`, when the row is taken (prefetch of epilogue operands).
-template <int KIND, class Claim, class Epi>
+template <class Claim, class Epi>
 __device__ __forceinline__ void consume_rows(const MegaParams& p, MegaCtl* ctl, Ring& r, const RowPlan& pl, int n_in, const int8_t* xq, const float* xs,
                                              Pending& pd, int stage, Claim claim, Epi epi) {
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -379,8 +381,7 @@ __device__ __forceinline__ void consume_rows(const MegaParams& p, MegaCtl* ctl, 
             if (pd.n == pd.cap) pd.flush(epi);
             if (lane == pd.n) claim(c0 + i);
             float* t = pd.next(c0 + i);
-            if (KIND == MK_Q8) q8_row_terms(slot + (size_t)i * pl.ra, pb + (size_t)i * pl.rb, n_in, xq, xs, t);
-            else fp4_row_terms(slot + (size_t)i * pl.ra, pb + (size_t)i * pl.rb, n_in, xq, xs, t);
+            q8_row_terms(slot + (size_t)i * pl.ra, pb + (size_t)i * pl.rb, n_in, xq, xs, t);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(r.empty_bar());
@@ -479,15 +480,15 @@ __device__ __forceinline__ void mg_stage_rows(const MegaParams& p, MegaCtl* ctl,
                 for (int k = 0; k < 6; ++k) if (k + 1 < keep) pst[k] = past[k + 1];
                 pst[keep - 1] = v;
             };
-            consume_rows<MK_Q8>(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, claim, epi);
+            consume_rows(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, claim, epi);
             pd.flush(epi);
         } else if (st.flags & MSF_ARGMAX) {
             auto epi = [&](int row, float v) { o[row] = v; if (best_i == 0x7fffffff || v > best_v || (v == best_v && row < best_i)) { best_v = v; best_i = row; } };
-            consume_rows<MK_Q8>(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
+            consume_rows(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
             pd.flush(epi);
         } else {
             auto epi = [&](int row, float v) { o[row] = v; };
-            consume_rows<MK_Q8>(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
+            consume_rows(p, ctl, ra, pl, n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
             pd.flush(epi);
         }
     }
@@ -657,7 +658,7 @@ __device__ __forceinline__ void mg_stage_out(const MegaParams& p, MegaCtl* ctl, 
     pd.init(sm.terms + wid * p.tw_floats, nb, p.tw_floats);
     float* x = p.x;
     auto epi = [&](int row, float v) { x[row] += v; };
-    consume_rows<MK_Q8>(p, ctl, ra, q8_plan(w, ra.slot_bytes), n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
+    consume_rows(p, ctl, ra, q8_plan(w, ra.slot_bytes), n, sm.xq, sm.xs, pd, s, [](int) {}, epi);
     pd.flush(epi);
 }
 
@@ -936,7 +937,7 @@ __device__ __forceinline__ void mg_stage_glu(const MegaParams& p, MegaCtl* ctl, 
             for (int i = wid; have && i < 32; i += MG_NW) {
                 if (pd.n == pd.cap) pd.flush(epi);
                 float* t = pd.next(half * 32 + i);
-                fp4_row_terms(slot + (size_t)i * (n / 2), pb + (size_t)i * nsb, n, sm.xq, sm.xs, t);
+                fp4_row_terms(slot, pb, i, n, sm.xq, sm.xs, t);
             }
             pd.flush(epi);
             __syncwarp();
@@ -997,7 +998,7 @@ __device__ __forceinline__ void mg_stage_down(const MegaParams& p, MegaCtl* ctl,
             const uint8_t* base = slot + (size_t)k * (ab + bb);
             if (pd.n == pd.cap) pd.flush(epi);
             float* t = pd.next(r * (K + 1) + k0 + k);
-            fp4_row_terms(base + (size_t)r * d.ra, base + ab + (size_t)r * d.rb, ff, hq + (size_t)(k0 + k) * ff, hs + (k0 + k) * nbf, t);
+            fp4_row_terms(base, base + ab, r, ff, hq + (size_t)(k0 + k) * ff, hs + (k0 + k) * nbf, t);
         }
         pd.flush(epi);
         __syncwarp();
@@ -1007,11 +1008,11 @@ __device__ __forceinline__ void mg_stage_down(const MegaParams& p, MegaCtl* ctl,
     // shared expert's down projection: item (row r) -> outv[r * (K + 1) + K]
     {
         const DevQ8 w = st.shared_down;
-        const RowPlan pl = q8_plan(w, ra.slot_bytes);
+        const RowPlan pl = down_shared_plan(p, w, ra.slot_bytes);
         pd.init(sm.terms + wid * p.tw_floats, nbs, p.tw_floats);
         const int o0 = d.o0;
         auto epi_s = [&](int row, float v) { outv[(row - o0) * (K + 1) + K] = v; };
-        consume_rows<MK_Q8>(p, ctl, ra, pl, sff, sq, ss, pd, s, [](int) {}, epi_s);
+        consume_rows(p, ctl, ra, pl, sff, sq, ss, pd, s, [](int) {}, epi_s);
         pd.flush(epi_s);
     }
     csync();

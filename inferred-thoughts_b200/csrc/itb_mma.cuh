@@ -104,11 +104,12 @@ __device__ __forceinline__ void mma_fp4_rows16(const uint8_t* nib, const uint8_t
                                                const float* ss, int jb, float (&acc)[NJ][4]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int nsb = k / 16, nb = k / 32, stride = mma_act_stride(k);
-    const int ra = min(r0 + g, n_rows - 1), rb = min(r0 + g + 8, n_rows - 1);
-    const uint8_t* pa = nib + (size_t)ra * (k / 2) + 2 * t;   // 4 codes = 2 bytes per thread and sub-block
-    const uint8_t* pb = nib + (size_t)rb * (k / 2) + 2 * t;
-    const uint8_t* sa = sc + (size_t)ra * nsb;
-    const uint8_t* sb = sc + (size_t)rb * nsb;
+    (void)n_rows;                                             // rows past the matrix lie in its last (padded) tile of 16
+    const int kgs = k / 64;
+    const uint8_t* pa = nib + fp4_nib_at(r0 + g, 0, kgs) + 8 * t;   // 4 codes = 2 bytes per thread and sub-block
+    const uint8_t* pb = nib + fp4_nib_at(r0 + g + 8, 0, kgs) + 8 * t;
+    const uint8_t* sa = sc + fp4_sc_at(r0 + g, 0, kgs);
+    const uint8_t* sb = sc + fp4_sc_at(r0 + g + 8, 0, kgs);
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
@@ -120,8 +121,9 @@ __device__ __forceinline__ void mma_fp4_rows16(const uint8_t* nib, const uint8_t
         for (int u = 0; u < UNR; ++u) {
             const int s = min(s0 + u, nsb - 1);
             // elements 4t..4t+3 of the sub-block on both sides (any fixed bijection of k is fine)
-            wa[u] = __ldg((const uint16_t*)(pa + s * 8)); wb[u] = __ldg((const uint16_t*)(pb + s * 8));
-            ca[u] = __ldg(sa + s); cb[u] = __ldg(sb + s);
+            const int o = (s >> 2) * 512 + ((s >> 1) & 1) * 4 + (s & 1) * 2, so = (s >> 2) * 64 + (s & 3);
+            wa[u] = __ldg((const uint16_t*)(pa + o)); wb[u] = __ldg((const uint16_t*)(pb + o));
+            ca[u] = __ldg(sa + so); cb[u] = __ldg(sb + so);
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {

@@ -5,6 +5,7 @@
 #include "itb_gdn_chunk.cuh"
 #include "itb_attn_mma.cuh"
 #include "itb_rows.cuh"
+#include "itb_exp.cuh"
 
 static inline unsigned blocks_for(size_t n, int per = 256) { return (unsigned)((n + per - 1) / per); }
 
@@ -219,14 +220,14 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od)
 }
 
 // The pairs of a pass sorted by expert: pair_off[e .. e+1) bounds expert e's slots of pair_list.
-static bool group_pairs(itb_ctx* c, const int32_t* ids, size_t n_pairs, size_t E) {
+static bool group_pairs(itb_ctx* c, const int32_t* ids, size_t n_pairs, size_t E, int cap = 64) {
     if (c->pair_cap < n_pairs || c->pair_experts < E) {
         cudaStreamSynchronize(c->stream);
-        cudaFree(c->pair_off); cudaFree(c->pair_list); c->pair_off = nullptr; c->pair_list = nullptr; c->pair_cap = 0; c->pair_experts = 0;
-        if (cudaMalloc(&c->pair_off, (E + 1) * 4) != cudaSuccess || cudaMalloc(&c->pair_list, n_pairs * 4) != cudaSuccess) return itb_fail_msg(c, "experts: out of device memory");
+        cudaFree(c->pair_off); cudaFree(c->pair_list); cudaFree(c->pair_tiles); c->pair_off = nullptr; c->pair_list = nullptr; c->pair_tiles = nullptr; c->pair_cap = 0; c->pair_experts = 0;
+        if (cudaMalloc(&c->pair_off, (E + 2) * 4) != cudaSuccess || cudaMalloc(&c->pair_list, n_pairs * 4) != cudaSuccess || cudaMalloc(&c->pair_tiles, (E + n_pairs / 8 + 1) * sizeof(int4)) != cudaSuccess) return itb_fail_msg(c, "experts: out of device memory");
         c->pair_cap = n_pairs; c->pair_experts = E;
     }
-    k_group_pairs_fast<<<1, 1024, E * 4, c->stream>>>(ids, (int)n_pairs, (int)E, c->pair_off, c->pair_list);
+    k_group_pairs_fast<<<1, 1024, E * 4, c->stream>>>(ids, (int)n_pairs, (int)E, c->pair_off, c->pair_list, (int4*)c->pair_tiles, c->pair_off + E + 1, cap);
     ITB_LAUNCHED(c);
     return true;
 }
@@ -259,32 +260,11 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const int32_t* ids, siz
         return;
     }
     DevFp4 dw{(const uint8_t*)w->a, (const uint8_t*)w->b, w->scale2, (int)w->n_in, (int)w->n_out, (int)w->n_expert, 0};
-    if (ids && n_pairs >= 16 && w->n_in % 256 == 0 && w->n_expert <= 1024) {
-        // many pairs: group them by expert and run each expert's rows through the int8-MMA tiles, so an expert's weights
-        // are read once (the reference groups the same way, kernels/moe.cuh:62-133 there)
-        const size_t E = w->n_expert;
-        if (!group_pairs(c, ids, n_pairs, E)) return;
-        const int per_e = (int)((n_pairs + E - 1) / E), nj = per_e <= 8 ? 1 : per_e <= 16 ? 2 : per_e <= 32 ? 4 : 0;
-        const int ns = std::min((int)w->n_in / 256, TILE_STAGES);
-        const int div = rows_mode == 0 ? 1 : rows_mode == 1 ? n_used : 0x7fffffff;
-#define EXP_TILE(NJ, TH)                                                                                                          \
-    do {                                                                                                                         \
-        cudaFuncSetAttribute(k_tile_down<NJ, 256, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);                 \
-        k_tile_down<NJ, 256, TH><<<dim3((unsigned)E, (unsigned)((w->n_out + 128 / TH - 1) / (128 / TH))), 256,                    \
-                                   tile_smem<MK_FP4, NJ, 256, TH>((int)w->n_in), c->stream>>>(dw, c->xq, c->xs, c->pair_off, c->pair_list, od, ns, div); \
-    } while (0)
-        if (nj == 1) EXP_TILE(1, 1); else if (nj == 2) EXP_TILE(2, 1); else if (nj == 4) EXP_TILE(4, 1); else EXP_TILE(4, 2);
-#undef EXP_TILE
-        ITB_LAUNCHED(c);
-        return;
-    }
-    int nb = (int)w->n_in / 32, nsb = (int)w->n_in / 16, gsh = lanes_shift(nb), nw = 8;
     int gx = (int)std::min<size_t>((w->n_out + 31) / 32, (size_t)c->sm_count * 2);
     if (gx < 1) gx = 1;
-    size_t smem = w->n_in + nb * 4 + (size_t)nw * terms_floats(4, gsh, nsb) * 4;
-    dim3 grid(gx, (unsigned)n_pairs);
+    const size_t smem = matmul_fp4_smem((int)w->n_in);
     cudaFuncSetAttribute(k_matmul_fp4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_matmul_fp4<<<grid, nw * 32, smem, c->stream>>>(dw, ids, n_used, rows_mode, c->xq, c->xs, od);
+    k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, c->xq, c->xs, od);
     ITB_LAUNCHED(c);
 }
 
@@ -369,8 +349,31 @@ static bool stage_route(itb_ctx* c, const itb_route_t* r, size_t n_expert) {
     c->route_n_tok = r->n_tok; c->route_n_used = r->n_used;
     return true;
 }
+// Many pairs: grouped by expert, an expert's rows through the tensor-core form of the CPU arithmetic (itb_exp.cuh), so its weights
+// are read once (the reference groups the same way, kernels/moe.cuh:62-133 there). u: the up stack of a gated pair, or null.
+// False: too few pairs, or a stack it does not take.
+static bool experts_grouped(itb_ctx* c, const itb_experts* g, const itb_experts* u, const itb_route_t* r, const float* xd, size_t x_len, float* od) {
+    const size_t n_pairs = r->n_tok * r->n_used, rows = x_len / g->n_in, k = g->n_in;
+    if (g->ggml_type != ITB_NVFP4 || (u && u->ggml_type != ITB_NVFP4) || n_pairs < 16 || g->n_expert > 1024 || g->n_out % 32) return false;
+    const WeightEntry* wg = itb_weight(c, g->data, g->bytes, g->ggml_type, g->n_in, g->n_out, g->n_expert, g->scale, g->scale_bytes);
+    const WeightEntry* wu = u ? itb_weight(c, u->data, u->bytes, u->ggml_type, u->n_in, u->n_out, u->n_expert, u->scale, u->scale_bytes) : nullptr;
+    if (!wg || (u && !wu)) return true;                       // failed loudly
+    const int E = (int)g->n_expert, cap = exp_tile_cap((int)n_pairs, E, (int)(u ? g->n_out : g->n_out / 2), c->sm_count);
+    if (!itb_ensure_xq(c, rows * k * 2) || !group_pairs(c, c->route_ids, n_pairs, g->n_expert, cap)) return true;
+    __half* xh = (__half*)c->xq;
+    k_quant_rows_h<<<(unsigned)rows, 256, 0, c->stream>>>(xd, (int)k, xh, c->xs);
+    ITB_LAUNCHED(c);
+    ExpArgs a{};
+    a.wa = DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0};
+    if (wu) a.wb = DevFp4{(const uint8_t*)wu->a, (const uint8_t*)wu->b, wu->scale2, (int)wu->n_in, (int)wu->n_out, (int)wu->n_expert, 0};
+    a.xh = xh; a.xs = c->xs; a.div = rows == n_pairs ? 1 : rows > 1 ? (int)r->n_used : 0x7fffffff; a.tiles = (const int4*)c->pair_tiles; a.n_tiles = c->pair_off + E + 1; a.list = c->pair_list; a.out = od;
+    exp_run(a, wu != nullptr, exp_max_tiles((int)n_pairs, E, cap), cap, c->stream);
+    ITB_LAUNCHED(c);
+    return true;
+}
 static void experts_dev(itb_ctx* c, const itb_experts* w, const itb_route_t* r, const float* xd, size_t x_len, float* od) {
     if (w->ggml_type != ITB_NVFP4) { itb_fail_msg(c, "routed experts: only NVFP4 has a kernel here"); return; }  // src/ops/mod.rs:29-55
+    if (experts_grouped(c, w, nullptr, r, xd, x_len, od)) return;
     const WeightEntry* we = itb_weight(c, w->data, w->bytes, w->ggml_type, w->n_in, w->n_out, w->n_expert, w->scale, w->scale_bytes);
     if (!we) return;
     size_t n_pairs = r->n_tok * r->n_used, rows = x_len / w->n_in;
@@ -397,7 +400,7 @@ extern "C" void itb_moe_glu(itb_ctx* c, const itb_experts* gate, const itb_exper
     const float* xd = itb_mirror_in(c, x, x_len);
     float* od = itb_mirror_out(c, out, out_len); float* sd = itb_mirror_out(c, scratch, out_len);
     if (!xd || !od || !sd) return;
-    if (experts_tc(c, gate, up, r, xd, x_len, od)) return;
+    if (experts_tc(c, gate, up, r, xd, x_len, od) || experts_grouped(c, gate, up, r, xd, x_len, od)) return;
     experts_dev(c, gate, r, xd, x_len, od);
     experts_dev(c, up, r, xd, x_len, sd);
     EW_LAUNCH(c, k_silu_mul, out_len, od, sd, out_len);

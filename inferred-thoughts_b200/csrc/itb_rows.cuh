@@ -166,20 +166,22 @@ __global__ void __launch_bounds__(256) k_sgemm_serial_small(DevF32 w0, const flo
 }
 
 // RMSNorm + Q8_0 quantisation of each row (src/ops/naive.rs:139-152, :653-675): normalised f32 row, int8 quants,
-// scales. grid = rows, block 256.
-__global__ void __launch_bounds__(256) k_norm_quant(const float* x, const float* w, int n, float eps, float* xn_out, int8_t* xq, float* xs) {
+// scales; xh (optional): the quants as f16 for the expert kernels (exp_pos order). grid = rows, block 256.
+__global__ void __launch_bounds__(256) k_norm_quant(const float* x, const float* w, int n, float eps, float* xn_out, int8_t* xq, float* xs, __half* xh = nullptr) {
     extern __shared__ __align__(16) unsigned char smem[];
     double* red = (double*)smem;
     float* xn = (float*)(red + 32);
     const size_t r = blockIdx.x;
-    if (block_rms_norm(x + r * n, w, n, eps, xn, red, xq + r * n, xs + r * (n / 32))) {   // quantised in the same pass
+    if (block_rms_norm(x + r * n, w, n, eps, xn, red, xq + r * n, xs + r * (n / 32), xh ? xh + r * n : nullptr)) {   // quantised in the same pass
         if (xn_out) for (int i = threadIdx.x; i < n / 4; i += blockDim.x) ((float4*)(xn_out + r * n))[i] = ((const float4*)xn)[i];
         return;
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int b = wid; b < n / 32; b += nw) {
         float v = xn[b * 32 + lane], d;
-        xq[r * n + b * 32 + lane] = warp_quant_q8(v, &d);
+        const int8_t q = warp_quant_q8(v, &d);
+        xq[r * n + b * 32 + lane] = q;
+        if (xh) xh[r * n + b * 32 + exp_pos(lane)] = __int2half_rn((int)q);
         if (lane == 0) xs[r * (n / 32) + b] = d;
         if (xn_out) xn_out[r * n + b * 32 + lane] = v;
     }
@@ -521,121 +523,6 @@ __global__ void k_route_rows(const float* router, int n_rows, int n_expert, int 
         for (int k = 0; k < n_used; ++k) { ids_out[(size_t)r * n_used + k] = ids[k]; w_out[(size_t)r * n_used + k] = wts[k]; }
 }
 
-// Counting sort of the pairs by expert, ascending pair index inside an expert. One block, thread e owns expert e.
-// off: [n_expert + 1], list: [n_pairs] pair indices.
-__global__ void k_group_pairs(const int32_t* ids, int n_pairs, int n_expert, int* off, int* list) {
-    extern __shared__ int cnt[];
-    for (int e = threadIdx.x; e < n_expert; e += blockDim.x) {
-        int c = 0;
-        for (int i = 0; i < n_pairs; ++i) c += ids[i] == e;
-        cnt[e] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int e = 0; e < n_expert; ++e) { off[e] = acc; acc += cnt[e]; }
-        off[n_expert] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n_expert; e += blockDim.x) {
-        int at = off[e];
-        for (int i = 0; i < n_pairs; ++i) if (ids[i] == e) list[at++] = i;
-    }
-}
-
-// Activation rows of up to 32 listed pairs into the MMA tile: pair p reads row p / div of (xq, xs).
-__device__ __forceinline__ void stage_pairs(const int8_t* xq, const float* xs, int k, const int* list, int n, int div, int8_t* sq, float* ss) {
-    const int nb = k / 32, stride = mma_act_stride(k);
-    for (int i = threadIdx.x; i < MMA_TOK * (k / 16); i += blockDim.x) {
-        int t = i / (k / 16), c = i % (k / 16);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (t < n) v = *(const uint4*)(xq + (size_t)(list[t] / div) * k + c * 16);
-        *(uint4*)(sq + (size_t)t * stride + c * 16) = v;
-    }
-    for (int i = threadIdx.x; i < MMA_TOK * nb; i += blockDim.x) {
-        int t = i / nb;
-        ss[i] = t < n ? xs[(size_t)(list[t] / div) * nb + i % nb] : 0.0f;
-    }
-    __syncthreads();
-}
-
-// Gate and up of one expert for its pairs, SiLU-gated: h[pair][row] (src/ops/mod.rs:1105-1117). grid (n_expert, ff/128).
-__global__ void __launch_bounds__(256) k_glu_grouped(DevFp4 gate, DevFp4 up, const int8_t* xq, const float* xs, int n_used,
-                                                     const int* off, const int* list, float* h) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int e = blockIdx.x, k = gate.n_in, ff = gate.n_out, nsb = k / 16;
-    const int p0 = off[e], p1 = off[e + 1];
-    if (p0 >= p1) return;
-    const int el = fp4_slot(gate, e);
-    if (el < 0) return;
-    int8_t* sq = (int8_t*)smem;
-    float* ss = (float*)(sq + (size_t)MMA_TOK * mma_act_stride(k));
-    const int r0 = blockIdx.y * MMA_ROWS + (threadIdx.x >> 5) * 16;
-    const size_t eo = (size_t)el * ff;
-    const bool has_g = gate.scale2 != nullptr, has_u = up.scale2 != nullptr;
-    const float sg2 = has_g ? gate.scale2[el] : 1.0f, su2 = has_u ? up.scale2[el] : 1.0f;
-    for (int t0 = p0; t0 < p1; t0 += MMA_TOK) {
-        const int n = min(MMA_TOK, p1 - t0);
-        __syncthreads();
-        stage_pairs(xq, xs, k, list + t0, n, n_used, sq, ss);
-        if (r0 < ff) {
-            float g[4][4], u[4][4];
-            mma_fp4_rows16<4, 8>(gate.nib + eo * (k / 2), gate.sc + eo * nsb, k, ff, r0, sq, ss, 0, g);
-            mma_fp4_rows16<4, 8>(up.nib + eo * (k / 2), up.sc + eo * nsb, k, ff, r0, sq, ss, 0, u);
-            const int lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int t = 8 * j + 2 * tq + (i & 1), row = r0 + gq + (i >> 1) * 8;
-                    if (t < n && row < ff) {
-                        float gv = has_g ? g[j][i] * sg2 : g[j][i], uv = has_u ? u[j][i] * su2 : u[j][i];
-                        h[(size_t)list[t0 + t] * ff + row] = silu_f(gv) * uv;
-                    }
-                }
-        }
-    }
-}
-
-// Down projection of one expert for its pairs: o[pair][row], times the expert's second scale
-// (src/ops/mod.rs:1049-1088). grid (n_expert, n_out/128). Activation rows are per pair (div = 1).
-__global__ void __launch_bounds__(256) k_down_grouped(DevFp4 down, const int8_t* hq, const float* hs, const int* off, const int* list, float* o) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int e = blockIdx.x, k = down.n_in, n_out = down.n_out, nsb = k / 16;
-    const int p0 = off[e], p1 = off[e + 1];
-    if (p0 >= p1) return;
-    const int el = fp4_slot(down, e);
-    if (el < 0) return;
-    int8_t* sq = (int8_t*)smem;
-    float* ss = (float*)(sq + (size_t)MMA_TOK * mma_act_stride(k));
-    const int r0 = blockIdx.y * MMA_ROWS + (threadIdx.x >> 5) * 16;
-    const size_t eo = (size_t)el * n_out;
-    const bool has_s = down.scale2 != nullptr;
-    const float s2 = has_s ? down.scale2[el] : 1.0f;
-    for (int t0 = p0; t0 < p1; t0 += MMA_TOK) {
-        const int n = min(MMA_TOK, p1 - t0);
-        __syncthreads();
-        stage_pairs(hq, hs, k, list + t0, n, 1, sq, ss);
-        if (r0 < n_out) {
-            float acc[4][4];
-            mma_fp4_rows16<4, 8>(down.nib + eo * (k / 2), down.sc + eo * nsb, k, n_out, r0, sq, ss, 0, acc);
-            mma_foreach<4>(acc, r0, n_out, 0, [&](int t, int row, float v) {
-                if (t < n) o[(size_t)list[t0 + t] * n_out + row] = has_s ? v * s2 : v;
-            });
-        }
-    }
-}
-
-// Q8_0 quantisation of rows of f32 (block per row).
-__global__ void k_quant_rows(const float* x, int n, int8_t* xq, float* xs) {
-    const size_t r = blockIdx.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int b = wid; b < n / 32; b += nw) {
-        float d;
-        xq[r * n + b * 32 + lane] = warp_quant_q8(x[r * n + b * 32 + lane], &d);
-        if (lane == 0) xs[r * (n / 32) + b] = d;
-    }
-}
 // silu(gate) * up of the shared expert per row, quantised (src/model/qwen35.rs:1669-1678). block per row.
 __global__ void k_shared_act_rows(const float* sg, const float* su, int n, int8_t* q, float* s) {
     const size_t r = blockIdx.x;
@@ -666,9 +553,13 @@ namespace {
 // Pairs grouped by expert without a serial scan: counts by shared-memory atomics, an exclusive scan, then each
 // pair takes the next free place of its expert. The order inside an expert depends on scheduling; results do
 // not, since every pair is computed on its own. One block.
-__global__ void __launch_bounds__(1024) k_group_pairs_fast(const int32_t* ids, int n_pairs, int n_expert, int* off, int* list) {
+// tiles (optional): the pairs cut into tiles of at most `cap` (a multiple of 8), an expert's pairs evenly over its tiles, as
+// (expert, first slot, pairs, 0), largest first so that no long tile starts last; *n_tiles of them.
+__global__ void __launch_bounds__(1024) k_group_pairs_fast(const int32_t* ids, int n_pairs, int n_expert, int* off, int* list, int4* tiles = nullptr, int* n_tiles = nullptr, int cap = 64) {
     extern __shared__ int cnt[];    // [n_expert] counts, then cursors
     __shared__ int s_off[1025];
+    __shared__ int s_bucket[9], s_start[9];       // tiles by groups of 8 pairs (1..8)
+    if (threadIdx.x < 9) s_bucket[threadIdx.x] = 0;
     for (int e = threadIdx.x; e < n_expert; e += blockDim.x) cnt[e] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) atomicAdd(&cnt[ids[i]], 1);
@@ -687,8 +578,19 @@ __global__ void __launch_bounds__(1024) k_group_pairs_fast(const int32_t* ids, i
         if (threadIdx.x == 0) off[n_expert] = carry;
     }
     __syncthreads();
+    // this thread's expert (at most 1024 of them): its tiles' size and the sizes' count
+    const int te = threadIdx.x, tc = tiles && te < n_expert ? cnt[te] : 0, nt = (tc + cap - 1) / cap;
+    const int per = nt ? (((tc + nt - 1) / nt) + 7) & ~7 : 8;
+    for (int i = 0; i < nt; ++i) { const int m = min(per, tc - i * per); if (m > 0) atomicAdd(&s_bucket[(m + 7) >> 3], 1); }
+    __syncthreads();
+    if (threadIdx.x == 0 && tiles) {
+        int at = 0;
+        for (int b = 8; b >= 1; --b) { s_start[b] = at; at += s_bucket[b]; }
+        *n_tiles = at;
+    }
     for (int e = threadIdx.x; e < n_expert; e += blockDim.x) cnt[e] = 0;
     __syncthreads();
+    for (int i = 0; i < nt; ++i) { const int m = min(per, tc - i * per); if (m > 0) tiles[atomicAdd(&s_start[(m + 7) >> 3], 1)] = make_int4(te, s_off[te] + i * per, m, 0); }
     for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) { const int e = ids[i]; list[s_off[e] + atomicAdd(&cnt[e], 1)] = i; }
 }
 

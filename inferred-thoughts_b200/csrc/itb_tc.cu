@@ -313,11 +313,14 @@ __global__ void k_tc_tile_weights(const uint8_t* nib, const uint8_t* sc, int n_e
     const int kb = (int)(idx % kbs); const size_t er = idx / kbs;
     const int row = (int)(er % n_out); const int e = (int)(er / n_out);
     const int mt = row / TC_M, r = row % TC_M;
-    const uint4* src = (const uint4*)(nib + ((size_t)e * n_out + row) * (n_in / 2) + kb * 32);
+    const size_t eo = (size_t)e * n_out * kbs;                // n_out is a multiple of 128 here: no padding rows
+    const uint4* src = (const uint4*)(nib + eo * 32 + fp4_nib_at(row, kb, kbs));
+    const uint4 v0 = src[0], v1 = src[1];
     uint8_t* blk = w_img + (((size_t)e * (n_out / TC_M) + mt) * kbs + kb) * 4096;
-    *(uint4*)(blk + (r >> 3) * 128 + (r & 7) * 16) = src[0];
-    *(uint4*)(blk + 2048 + (r >> 3) * 128 + (r & 7) * 16) = src[1];
-    const uint32_t s4 = *(const uint32_t*)(sc + ((size_t)e * n_out + row) * (n_in / 16) + kb * 4);
+    // back to element order: a word holds elements of both halves of a 32-element unit
+    *(uint4*)(blk + (r >> 3) * 128 + (r & 7) * 16) = make_uint4(__byte_perm(v0.x, v0.z, 0x5410), __byte_perm(v1.x, v1.z, 0x5410), __byte_perm(v0.x, v0.z, 0x7632), __byte_perm(v1.x, v1.z, 0x7632));
+    *(uint4*)(blk + 2048 + (r >> 3) * 128 + (r & 7) * 16) = make_uint4(__byte_perm(v0.y, v0.w, 0x5410), __byte_perm(v1.y, v1.w, 0x5410), __byte_perm(v0.y, v0.w, 0x7632), __byte_perm(v1.y, v1.w, 0x7632));
+    const uint32_t s4 = *(const uint32_t*)(sc + eo * 4 + fp4_sc_at(row, kb, kbs));
     *(uint32_t*)(sf_img + (((size_t)e * (n_out / TC_M) + mt) * kbs + kb) * 512 + (r & 31) * 16 + (r >> 5) * 4) = s4;
 }
 

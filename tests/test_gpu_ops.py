@@ -299,6 +299,30 @@ def test_grouped_expert_matmuls_config2_exact(ops, cfg2_experts, n_tok):
     exact(o, o_want, "matmul_experts(down)")
 
 
+@pytest.mark.parametrize("E,H,ff", [(5, 192, 64), (20, 192, 4160)])
+def test_grouped_expert_tiles_at_their_edges(ops, E, H, ff):
+    """Tiles of up to 16 pairs (few experts: spread over the SMs) and of up to 64: experts with no pair, 1, 8, 9, 64, 65 and 130 of them,
+    rows that end inside a block of rows and a stage of k."""
+    from inferred_thoughts_b200 import host
+    gb, gs = nvfp4_weights(E, ff, H, 150); ub, us = nvfp4_weights(E, ff, H, 151); db, ds = nvfp4_weights(E, H, ff, 152)
+    gs *= 300; us *= 300; ds *= 300
+    counts = [0, 1, 8, 9, 130] if E == 5 else [0, 1, 8, 9, 130, 64, 65] + [1] * 13
+    ids = np.random.default_rng(5).permutation(np.repeat(np.arange(E), counts)).astype(np.int32)
+    n = ids.size
+    x = noise(n * H, 153)
+    h = keep(np.zeros(n * ff, np.float32)); scratch = keep(np.zeros_like(h)); o = keep(np.zeros(n * H, np.float32))
+    G, U, D = host.Experts(gb, host.NVFP4, H, ff, E, gs), host.Experts(ub, host.NVFP4, H, ff, E, us), host.Experts(db, host.NVFP4, ff, H, E, ds)
+    ops.begin_pass(n)
+    route = host.Route.host(ids.astype(np.uint64), None, 1)
+    ops.moe_glu(G, U, route, x, h, scratch); ops.matmul_experts(D, route, h, o)
+    ops.host_needs(h); ops.host_needs(o); ops.check()
+    h_want = np.zeros_like(h); o_want = np.zeros_like(o)
+    L.orc_moe_glu(gb, gs.ctypes.data, ub, us.ctypes.data, H, ff, E, ids, n, 1, x, x.size, h_want, 0)
+    close(h, h_want, 8 * EPS, "moe_glu (through silu)")
+    L.orc_matmul_experts(db, ff, H, E, ds.ctypes.data, ids, n, 1, h, h.size, o_want, 0)
+    exact(o, o_want, "matmul_experts(down)")
+
+
 def test_grouped_expert_matmuls_at_8192_tokens_repeat_the_small_case(ops, cfg2_experts):
     """At the microbenchmark's largest size the CPU check is too slow; instead 8,192 tokens made of 16 copies of 512 distinct
     ones must give 16 copies of the 512-token result (the tiles are 64 tokens wide there, 16 wide at 512 tokens)."""
