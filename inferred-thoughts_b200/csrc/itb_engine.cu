@@ -1206,12 +1206,9 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     uint64_t launches = 0;
     static bool attrs_set = false;
     if (!attrs_set) {
-        set_smem((const void*)k_gemm_q8<4>, 200 * 1024); set_smem((const void*)k_gemm_q8<1>, 200 * 1024);
         set_smem((const void*)k_matmul_f32_rows<20>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<24>, 64 * 1024);
         set_smem((const void*)k_matmul_f32_rows<28>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<32>, 64 * 1024);
-        set_smem((const void*)k_tile_q8<1, 256, 4>, 226 * 1024); set_smem((const void*)k_tile_q8<4, 256, 2>, 226 * 1024);
         set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
-        set_smem((const void*)k_sgemm_serial_small<false>, sgemm_small_smem()); set_smem((const void*)k_sgemm_serial_small<true>, sgemm_small_smem());
         set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
         set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
         attrs_set = true;
@@ -1220,28 +1217,10 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     // direct-load MMA kernels otherwise.
     cudaStreamCaptureStatus cap_rows = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cap_rows);
-    const bool q8tc = c->q8tc && n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone;
     const bool f16tc = c->f16tc && n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone;
     // same: this matmul reads the quantised rows the previous one read (their tensor-core images are still current)
     auto gemm_n = [&](const DevQ8& w, const int8_t* xq, const float* xs, float* out, size_t stride, int mode, int R, bool same = false) {
-        const int k = w.n_in;
-        if (f16tc && R >= 64 && itb_tc_f16_shape_ok(w)) {
-            // many rows, dense=f16tc (tolerance class): both operands dequantised to f16, one tcgen05 GEMM with f32 accumulators
-            if (itb_tc_f16_gemm(c, st, w, xq, xs, R, out, stride, mode, same)) { launches++; return; }
-        }
-        if (q8tc && R >= 64 && itb_tc_q8_shape_ok(w)) {
-            // many rows, dense=q8tc: integer dots of 128 x 128 (row, token) pairs per tcgen05 MMA, scaled and summed in the CPU's order
-            if (itb_tc_q8_gemm(c, st, w, xq, xs, R, out, stride, mode, same)) { launches++; return; }
-        }
-        const bool skinny = R <= 32;
-        if (skinny && k % 256 == 0) {
-            const int ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
-        } else if (!skinny && k % 256 == 0) {
-            const int ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (R + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, xq, xs, R, out, stride, mode, ns);
-        } else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(w.n_in), st>>>(w, xq, xs, R, out, stride, mode);
-        else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (R + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), st>>>(w, xq, xs, R, out, stride, mode);
+        dense_q8(c, st, w, xq, xs, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone, same);
         launches++;
     };
     auto gemm = [&](const DevQ8& w, const int8_t* xq, const float* xs, float* out, size_t stride, int mode, bool same = false) { gemm_n(w, xq, xs, out, stride, mode, R, same); };
@@ -1280,14 +1259,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         if (has_s) { const size_t n = (size_t)rows * w.n_out; k_scale<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, sc); launches++; }
     };
     auto f32mm = [&](const DevF32& w, const float* x, float* out) {
-        if (!c->exact && f16tc && w.n_in % SGS_K == 0 && R >= 64) {
-            // tolerance-class passes: the serial-order tiles with fused multiply-adds (a chain per (row, output), k in order)
-            const int big = ((w.n_out + SG_T - 1) / SG_T) * ((R + SG_T - 1) / SG_T);
-            if (big >= sms / 2) k_sgemm_serial<true><<<dim3((w.n_out + SG_T - 1) / SG_T, (R + SG_T - 1) / SG_T), 256, 0, st>>>(w, x, R, out);
-            else k_sgemm_serial_small<true><<<dim3((w.n_out + 15) / 16, (R + 15) / 16), 256, sgemm_small_smem(), st>>>(w, x, R, out);
-            launches++;
-            return;
-        }
+        if (!c->exact && f16tc && sgemm_chain_ok(w.n_in) && R >= 64) { sgemm_chain<true>(st, sms, w, x, R, out); launches++; return; }   // tolerance-class passes: fused multiply-adds
         if (!c->exact && w.n_in % 512 == 0 && w.n_in <= 4096) {
             const dim3 g((w.n_out + 7) / 8, (R + F32_TOK - 1) / F32_TOK);
             const size_t sm = (size_t)F32_TOK * w.n_in * 4;
@@ -1299,14 +1271,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             launches++;
             return;
         }
-        if (c->exact && w.n_in % SGS_K == 0) {
-            // a chain per (row, output), a thread per 4 x 4 of them, k in order (also for a few rows: the tile's k loop is as long as a row's chain either way)
-            const int big = ((w.n_out + SG_T - 1) / SG_T) * ((R + SG_T - 1) / SG_T);
-            if (big >= sms / 2) k_sgemm_serial<false><<<dim3((w.n_out + SG_T - 1) / SG_T, (R + SG_T - 1) / SG_T), 256, 0, st>>>(w, x, R, out);
-            else k_sgemm_serial_small<false><<<dim3((w.n_out + 15) / 16, (R + 15) / 16), 256, sgemm_small_smem(), st>>>(w, x, R, out);
-            launches++;
-            return;
-        }
+        if (c->exact && sgemm_chain_ok(w.n_in)) { sgemm_chain<false>(st, sms, w, x, R, out); launches++; return; }   // also for a few rows: the tile's k loop is as long as a row's chain either way
         const int nw = 4;
         dim3 g(std::max(1, std::min(2 * sms, (w.n_out + 31) / 32)), R);
         size_t sm = (size_t)w.n_in * 4 + (size_t)nw * 32 * 33 * 4;
@@ -1314,14 +1279,11 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         else k_matmul_f32<false><<<g, nw * 32, sm, st>>>(w, x, out);
         launches++;
     };
-    // two F32 matrices over the same rows: one launch where both take the small serial-order tiles, else one after the other
+    // two F32 matrices over the same rows: one launch where both take the serial-order tiles, else one after the other
     auto f32mm2 = [&](const DevF32& wa, float* oa, const DevF32& wb, float* ob, const float* x) {
         const bool fused = !c->exact && f16tc && R >= 64;
-        const int big_a = ((wa.n_out + SG_T - 1) / SG_T) * ((R + SG_T - 1) / SG_T), big_b = ((wb.n_out + SG_T - 1) / SG_T) * ((R + SG_T - 1) / SG_T);
-        if ((c->exact || fused) && wa.n_in == wb.n_in && wa.n_in % SGS_K == 0 && big_a < sms / 2 && big_b < sms / 2) {
-            const dim3 g((std::max(wa.n_out, wb.n_out) + 15) / 16, (R + 15) / 16, 2);
-            if (fused) k_sgemm_serial_small<true><<<g, 256, sgemm_small_smem(), st>>>(wa, x, R, oa, wb, ob);
-            else k_sgemm_serial_small<false><<<g, 256, sgemm_small_smem(), st>>>(wa, x, R, oa, wb, ob);
+        if ((c->exact || fused) && wa.n_in == wb.n_in && sgemm_chain_ok(wa.n_in)) {
+            if (fused) sgemm_chain<true>(st, sms, wa, x, R, oa, wb, ob); else sgemm_chain<false>(st, sms, wa, x, R, oa, wb, ob);
             launches++;
             return;
         }
@@ -2155,7 +2117,7 @@ extern "C" int itb_engine_decode(itb_engine* e, const uint32_t* tokens, float* l
     ITB_CUDA_RET(c, cudaMemcpyAsync(e->tokens, tokens, e->B * 4, cudaMemcpyHostToDevice, st), 1);
     if (!run_steps(e, 1, true)) return 1;
     if (next_out) cudaMemcpyAsync(next_out, e->next, e->B * 4, cudaMemcpyDeviceToHost, st);
-    if (logits_out) cudaMemcpyAsync(logits_out, e->logits, (size_t)e->B * e->m->d.n_vocab * 4, cudaMemcpyDeviceToHost, st);
+    if (logits_out && !itb_download(c, logits_out, e->logits, (size_t)e->B * e->m->d.n_vocab * 4)) return 1;
     ITB_CUDA_RET(c, cudaStreamSynchronize(st), 1);
     cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1);
     return check_flag(e) ? 0 : 1;
@@ -2248,7 +2210,7 @@ extern "C" int itb_engine_prefill(itb_engine* e, const uint32_t* tokens, size_t 
         off += nt * e->B;
     }
     cudaEventRecord(e->ev1, st);
-    if (logits_out) cudaMemcpyAsync(logits_out, e->logits, (size_t)e->B * e->m->d.n_vocab * 4, cudaMemcpyDeviceToHost, st);
+    if (logits_out && !itb_download(c, logits_out, e->logits, (size_t)e->B * e->m->d.n_vocab * 4)) return 1;
     ITB_CUDA_RET(c, cudaStreamSynchronize(st), 1);
     cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1);
     return check_flag(e) && c->error.empty() ? 0 : 1;

@@ -69,8 +69,10 @@ struct WeightEntry {
     size_t bytes = 0;
 };
 
+struct HostPipe;                 // pinned staging and copy threads of one context (itb_ctx.cu)
 struct itb_ctx {
     int device = 0;
+    HostPipe* pipe = nullptr;
     cudaStream_t stream = nullptr;
     std::string error;       // sticky first error
     std::string error_out;   // storage handed back by take_error
@@ -88,6 +90,7 @@ struct itb_ctx {
     int* pair_off = nullptr; int* pair_list = nullptr; void* pair_tiles = nullptr; size_t pair_cap = 0, pair_experts = 0;   // pairs grouped by expert (many-row expert matmuls)
     float* route_w = nullptr;
     size_t route_cap = 0, route_n_tok = 0, route_n_used = 0;
+    size_t route_grouped = 0; int route_tile_cap = 0;      // expert count and tile size pair_off / pair_list / pair_tiles were made for (0: not for this route)
     // scratch for activation quantisation
     int8_t* xq = nullptr; float* xs = nullptr; size_t xq_cap = 0;
     float* tmp_f32 = nullptr; size_t tmp_cap = 0;
@@ -140,6 +143,10 @@ bool itb_fail_msg(itb_ctx* c, const std::string& msg);
         if (e__ != cudaSuccess) itb_fail((c), "kernel launch", e__);     \
     } while (0)
 
+// Pageable host memory <-> device on the context's stream, through the context's pinned staging. itb_upload returns when the host
+// bytes have been read (the caller may change them), itb_download when they are there. False: failed (sticky error set).
+bool itb_upload(itb_ctx* c, void* dev, const void* host, size_t bytes);
+bool itb_download(itb_ctx* c, void* host, const void* dev, size_t bytes);
 // mirrors (itb_ctx.cu)
 float* itb_mirror_in(itb_ctx* c, const float* host, size_t len);
 float* itb_mirror_out(itb_ctx* c, const float* host, size_t len);

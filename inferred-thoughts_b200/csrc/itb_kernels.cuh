@@ -253,6 +253,16 @@ __global__ void k_route(const float* probs, int n_expert, int n_used, int32_t* i
     block_topk(probs + t * n_expert, n_expert, n_used, ids + t * n_used, wts + t * n_used, sval, sidx);
 }
 
+// The same, a warp per token (up to 1,024 experts): no block barriers between the rounds.
+__global__ void __launch_bounds__(128) k_route_warp(const float* probs, int n_tok, int n_expert, int n_used, int32_t* ids_out, float* w_out) {
+    const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (t >= n_tok) return;
+    int32_t ids[16]; float wts[16];
+    warp_topk_any(probs + (size_t)t * n_expert, n_expert, n_used, ids, wts);
+    if (lane == 0)
+        for (int k = 0; k < n_used; ++k) { ids_out[(size_t)t * n_used + k] = ids[k]; w_out[(size_t)t * n_used + k] = wts[k]; }
+}
+
 // Weighted expert sum + gated shared expert (src/ops/mod.rs:1134-1171): ascending picks, shared last.
 __global__ void k_moe_finish(float* out, size_t at, int n, const float* rows, const float* wts, int n_used, size_t n_tok,
                              const float* shared, const float* logit, size_t logit_at) {
@@ -320,6 +330,34 @@ __global__ void __launch_bounds__(256) k_matmul_fp4(DevFp4 w, const int32_t* ids
         if (row < w.n_out) fp4_tile_terms<4>(nib + (size_t)row * (n / 2), sc + (size_t)row * nsb, g0, g1, xq, xs, terms + (wid >> 2) * 16 * (nsb + 1), nsb + 1);
         __syncthreads();
         if (tid < 32 && r0 + tid < w.n_out) { const float v = fold_terms(terms + tid * (nsb + 1), nsb); o[r0 + tid] = w.scale2 ? v * s2 : v; }
+    }
+}
+// The same for a gated pair of stacks and few (token, pick) pairs: 16 gate rows and the same 16 up rows at a time, out = silu(gate) * up
+// (src/ops/mod.rs:1105-1117). grid (ceil(n_out / 16), pairs).
+__global__ void __launch_bounds__(256) k_matmul_fp4_glu(DevFp4 wg, DevFp4 wu, const int32_t* ids, int n_used, int rows_mode, const int8_t* xq_g, const float* xs_g, float* out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int n = wg.n_in, nb = n / 32, nsb = n / 16, kgs = n / 64, tid = threadIdx.x, wid = tid >> 5, row = blockIdx.x * 16;
+    int8_t* xq = (int8_t*)smem;
+    float* xs = (float*)(smem + n);
+    float* terms = xs + nb;                                              // [32][nsb + 1]
+    const size_t i = blockIdx.y, xr = rows_mode == 0 ? i : rows_mode == 1 ? i / n_used : 0;
+    const int el = ids[i] - wg.expert_lo;
+    if (el < 0 || el >= wg.n_expert) return;
+    for (int k = tid; k < n / 16; k += 256) ((uint4*)xq)[k] = ((const uint4*)(xq_g + xr * n))[k];
+    for (int k = tid; k < nb; k += 256) xs[k] = xs_g[xr * nb + k];
+    const DevFp4& w = wid < 4 ? wg : wu;
+    const size_t ro = (size_t)el * fp4_rows_pad(w.n_out) + row;
+    const float sg = wg.scale2 ? wg.scale2[el] : 1.0f, su = wu.scale2 ? wu.scale2[el] : 1.0f;
+    int g0, g1;
+    share(kgs, 4, wid & 3, g0, g1);
+    __syncthreads();
+    fp4_tile_terms<4>(w.nib + ro * (n / 2), w.sc + ro * nsb, g0, g1, xq, xs, terms + (wid >> 2) * 16 * (nsb + 1), nsb + 1);
+    __syncthreads();
+    if (tid < 32) {
+        float v = fold_terms(terms + tid * (nsb + 1), nsb);
+        if (tid < 16 ? wg.scale2 != nullptr : wu.scale2 != nullptr) v = v * (tid < 16 ? sg : su);
+        const float u = __shfl_down_sync(0xffffffffu, v, 16);
+        if (tid < 16 && row + tid < wg.n_out) out[i * wg.n_out + row + tid] = silu_f(v) * u;
     }
 }
 static inline size_t matmul_fp4_smem(int n) { return (size_t)n + (size_t)(n / 32) * 4 + (size_t)32 * (n / 16 + 1) * 4; }

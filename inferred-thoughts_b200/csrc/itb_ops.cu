@@ -187,6 +187,14 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
 }
 
 // ------------------------------------------------------------------ matmuls
+// Raises a kernel's shared-memory limit when a launch needs more than any before it (the call costs a microsecond of host time).
+static void once_smem(const void* fn, size_t bytes) {
+    static thread_local std::unordered_map<const void*, size_t> have;
+    size_t& h = have[fn];
+    if (bytes <= h || bytes <= 48 * 1024) return;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    h = bytes;
+}
 static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in) {
     if (!itb_ensure_xq(c, n_rows * n_in)) return false;
     k_quant_q8<<<(unsigned)n_rows, 256, 0, c->stream>>>(xd, (int)n_in, c->xq, c->xs);
@@ -194,18 +202,10 @@ static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_i
     return true;
 }
 
-static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od) {
+static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od, bool same) {
     DevQ8 dw{(const int8_t*)w->a, (const uint16_t*)w->b, (int)w->n_in, (int)w->n_out};
-    if (c->f16tc && n_tok >= 64 && itb_tc_f16_shape_ok(dw) && itb_tc_f16_gemm(c, c->stream, dw, c->xq, c->xs, (int)n_tok, od, w->n_out, 0, false)) {
-        ITB_LAUNCHED(c);      // opts dense=f16tc: many rows as one f16 tensor-core GEMM (tolerance class)
-        return;
-    }
     if (n_tok >= 2 && w->n_in % 32 == 0 && gemm_smem((int)w->n_in) <= 200 * 1024) {
-        // several tokens: every weight row is read once per 32 tokens, on the int8 tensor-core path
-        size_t sm = gemm_smem((int)w->n_in);
-        cudaFuncSetAttribute(k_gemm_q8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        dim3 g((unsigned)((w->n_out + MMA_ROWS - 1) / MMA_ROWS), (unsigned)((n_tok + MMA_TOK - 1) / MMA_TOK));
-        k_gemm_q8<4><<<g, 256, sm, c->stream>>>(dw, c->xq, c->xs, (int)n_tok, od, w->n_out, 0);
+        dense_q8(c, c->stream, dw, c->xq, c->xs, (int)n_tok, od, w->n_out, 0, true, same);       // every weight row read once per token tile
         ITB_LAUNCHED(c);
         return;
     }
@@ -214,7 +214,7 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od)
     if (gx < 1) gx = 1;
     size_t smem = w->n_in + nb * 4 + (size_t)nw * terms_floats(4, gsh, nb) * 4;
     dim3 grid(gx, (unsigned)n_tok);
-    cudaFuncSetAttribute(k_matmul_q8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    once_smem((const void*)k_matmul_q8, smem);
     k_matmul_q8<<<grid, nw * 32, smem, c->stream>>>(dw, c->xq, c->xs, od);
     ITB_LAUNCHED(c);
 }
@@ -222,11 +222,15 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od)
 // The pairs of a pass sorted by expert: pair_off[e .. e+1) bounds expert e's slots of pair_list.
 static bool group_pairs(itb_ctx* c, const int32_t* ids, size_t n_pairs, size_t E, int cap = 64) {
     if (c->pair_cap < n_pairs || c->pair_experts < E) {
+        c->route_grouped = 0;
         cudaStreamSynchronize(c->stream);
         cudaFree(c->pair_off); cudaFree(c->pair_list); cudaFree(c->pair_tiles); c->pair_off = nullptr; c->pair_list = nullptr; c->pair_tiles = nullptr; c->pair_cap = 0; c->pair_experts = 0;
         if (cudaMalloc(&c->pair_off, (E + 2) * 4) != cudaSuccess || cudaMalloc(&c->pair_list, n_pairs * 4) != cudaSuccess || cudaMalloc(&c->pair_tiles, (E + n_pairs / 8 + 1) * sizeof(int4)) != cudaSuccess) return itb_fail_msg(c, "experts: out of device memory");
         c->pair_cap = n_pairs; c->pair_experts = E;
     }
+    // the route's pairs stay grouped for the other matmuls over it (gate + up, then down)
+    if (c->route_grouped == E && c->route_tile_cap == cap) return true;
+    c->route_grouped = E; c->route_tile_cap = cap;
     k_group_pairs_fast<<<1, 1024, E * 4, c->stream>>>(ids, (int)n_pairs, (int)E, c->pair_off, c->pair_list, (int4*)c->pair_tiles, c->pair_off + E + 1, cap);
     ITB_LAUNCHED(c);
     return true;
@@ -252,7 +256,7 @@ static bool experts_tc(itb_ctx* c, const itb_experts* g, const itb_experts* u, c
 static void launch_fp4(itb_ctx* c, const WeightEntry* w, const int32_t* ids, size_t n_pairs, int n_used, int rows_mode, float* od) {
     if (!ids && n_pairs >= 2 && gemm_smem((int)w->n_in) <= 200 * 1024) {
         size_t sm = gemm_smem((int)w->n_in);
-        cudaFuncSetAttribute(k_gemm_fp4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        once_smem((const void*)k_gemm_fp4, sm);
         dim3 g((unsigned)((w->n_out + MMA_ROWS - 1) / MMA_ROWS), (unsigned)((n_pairs + MMA_TOK - 1) / MMA_TOK));
         k_gemm_fp4<<<g, 256, sm, c->stream>>>((const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, c->xq, c->xs,
                                              (int)n_pairs, od, w->n_out, 1.0f, 0);
@@ -263,34 +267,41 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const int32_t* ids, siz
     int gx = (int)std::min<size_t>((w->n_out + 31) / 32, (size_t)c->sm_count * 2);
     if (gx < 1) gx = 1;
     const size_t smem = matmul_fp4_smem((int)w->n_in);
-    cudaFuncSetAttribute(k_matmul_fp4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    once_smem((const void*)k_matmul_fp4, smem);
     k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, c->xq, c->xs, od);
     ITB_LAUNCHED(c);
 }
 
 static void launch_f32(itb_ctx* c, const WeightEntry* w, const float* xd, size_t n_tok, float* od) {
     DevF32 dw{(const float*)w->a, (int)w->n_in, (int)w->n_out};
+    if (sgemm_chain_ok(dw.n_in) && (c->exact || (c->f16tc && n_tok >= 64))) {
+        // a chain per (token, output); fused multiply-adds in the tolerance-class mode of many-token passes
+        if (c->exact) sgemm_chain<false>(c->stream, c->sm_count, dw, xd, (int)n_tok, od); else sgemm_chain<true>(c->stream, c->sm_count, dw, xd, (int)n_tok, od);
+        ITB_LAUNCHED(c);
+        return;
+    }
     int nw = 4;
     int gx = (int)std::min<size_t>((w->n_out + 31) / 32, (size_t)c->sm_count * 2);
     if (gx < 1) gx = 1;
     size_t smem = w->n_in * 4 + (size_t)nw * 32 * 33 * 4;
     dim3 grid(gx, (unsigned)n_tok);
     if (c->exact) {
-        cudaFuncSetAttribute(k_matmul_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        once_smem((const void*)k_matmul_f32<true>, smem);
         k_matmul_f32<true><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
     } else {
-        cudaFuncSetAttribute(k_matmul_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        once_smem((const void*)k_matmul_f32<false>, smem);
         k_matmul_f32<false><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
     }
     ITB_LAUNCHED(c);
 }
 
-static void matmul_dev(itb_ctx* c, const itb_weights* w, const float* xd, size_t n_tok, float* od) {
+// same: c->xq / c->xs already hold these rows (the second matrix of a pair).
+static void matmul_dev(itb_ctx* c, const itb_weights* w, const float* xd, size_t n_tok, float* od, bool same = false) {
     const WeightEntry* we = itb_weight(c, w->data, w->bytes, w->ggml_type, w->n_in, w->n_out, 1, nullptr, 0);
     if (!we) return;
-    if (we->ty == ITB_Q8_0) { if (quantize_rows(c, xd, n_tok, w->n_in)) launch_q8(c, we, n_tok, od); }
-    else if (we->ty == ITB_NVFP4) { if (quantize_rows(c, xd, n_tok, w->n_in)) launch_fp4(c, we, nullptr, n_tok, 1, 0, od); }
-    else launch_f32(c, we, xd, n_tok, od);
+    if (we->ty != ITB_Q8_0 && we->ty != ITB_NVFP4) { launch_f32(c, we, xd, n_tok, od); return; }
+    if (!same && !quantize_rows(c, xd, n_tok, w->n_in)) return;
+    if (we->ty == ITB_Q8_0) launch_q8(c, we, n_tok, od, same); else launch_fp4(c, we, nullptr, n_tok, 1, 0, od);
 }
 
 extern "C" void itb_matmul(itb_ctx* c, const itb_weights* w, const float* x, size_t x_len, float* out, size_t out_len) {
@@ -307,8 +318,10 @@ extern "C" void itb_matmul_pair(itb_ctx* c, const itb_weights* a, const itb_weig
     const float* xd = itb_mirror_in(c, x, x_len);
     float* oa = itb_mirror_out(c, out_a, out_a_len); float* ob = itb_mirror_out(c, out_b, out_b_len);
     if (!xd || !oa || !ob) return;
+    auto quantised = [](const itb_weights* w) { return w->ggml_type == ITB_Q8_0 || w->ggml_type == ITB_NVFP4; };
     matmul_dev(c, a, xd, nt, oa);
-    matmul_dev(c, b, xd, nt, ob);
+    if (!c->error.empty()) return;
+    matmul_dev(c, b, xd, nt, ob, quantised(a) && quantised(b));
 }
 
 // ------------------------------------------------------------------ routing and experts
@@ -319,8 +332,10 @@ extern "C" void itb_route(itb_ctx* c, float* probs, size_t len, size_t n_expert,
     size_t nt = len / n_expert;
     const float* p = itb_mirror_in(c, probs, len);
     if (!p || !itb_ensure_route(c, nt * n_used)) return;
-    k_route<<<(unsigned)nt, 256, 0, c->stream>>>(p, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
+    if (n_expert <= 1024) k_route_warp<<<(unsigned)((nt + 3) / 4), 128, 0, c->stream>>>(p, (int)nt, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
+    else k_route<<<(unsigned)nt, 256, 0, c->stream>>>(p, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
     ITB_LAUNCHED(c);
+    c->route_grouped = 0;
     c->route_n_tok = nt; c->route_n_used = n_used;
     out->on_device = 1; out->n_used = n_used; out->n_tok = nt; out->ids = nullptr; out->weights = nullptr;
 }
@@ -346,6 +361,7 @@ static bool stage_route(itb_ctx* c, const itb_route_t* r, size_t n_expert) {
     cudaMemcpyAsync(c->route_ids, ids.data(), n * 4, cudaMemcpyHostToDevice, c->stream);
     if (r->weights) cudaMemcpyAsync(c->route_w, r->weights, n * 4, cudaMemcpyHostToDevice, c->stream);
     cudaStreamSynchronize(c->stream);
+    c->route_grouped = 0;
     c->route_n_tok = r->n_tok; c->route_n_used = r->n_used;
     return true;
 }
@@ -401,6 +417,21 @@ extern "C" void itb_moe_glu(itb_ctx* c, const itb_experts* gate, const itb_exper
     float* od = itb_mirror_out(c, out, out_len); float* sd = itb_mirror_out(c, scratch, out_len);
     if (!xd || !od || !sd) return;
     if (experts_tc(c, gate, up, r, xd, x_len, od) || experts_grouped(c, gate, up, r, xd, x_len, od)) return;
+    if (gate->ggml_type == ITB_NVFP4 && up->ggml_type == ITB_NVFP4) {
+        // few pairs: both halves and the gating in one kernel
+        const WeightEntry* wg = itb_weight(c, gate->data, gate->bytes, gate->ggml_type, gate->n_in, gate->n_out, gate->n_expert, gate->scale, gate->scale_bytes);
+        const WeightEntry* wu = itb_weight(c, up->data, up->bytes, up->ggml_type, up->n_in, up->n_out, up->n_expert, up->scale, up->scale_bytes);
+        const size_t n_pairs = r->n_tok * r->n_used, rows = x_len / gate->n_in;
+        if (!wg || !wu || !quantize_rows(c, xd, rows, gate->n_in)) return;
+        const size_t smem = matmul_fp4_smem((int)gate->n_in);
+        once_smem((const void*)k_matmul_fp4_glu, smem);
+        k_matmul_fp4_glu<<<dim3((unsigned)((gate->n_out + 15) / 16), (unsigned)n_pairs), 256, smem, c->stream>>>(
+            DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0},
+            DevFp4{(const uint8_t*)wu->a, (const uint8_t*)wu->b, wu->scale2, (int)wu->n_in, (int)wu->n_out, (int)wu->n_expert, 0}, c->route_ids, (int)r->n_used,
+            rows == n_pairs ? 0 : rows > 1 ? 1 : 2, c->xq, c->xs, od);
+        ITB_LAUNCHED(c);
+        return;
+    }
     experts_dev(c, gate, r, xd, x_len, od);
     experts_dev(c, up, r, xd, x_len, sd);
     EW_LAUNCH(c, k_silu_mul, out_len, od, sd, out_len);
@@ -410,7 +441,7 @@ extern "C" void itb_moe_finish(itb_ctx* c, float* out, size_t out_len, size_t at
     size_t nt = r->n_tok;
     if (rows_len != nt * r->n_used * n || at + nt * n > out_len) { itb_fail_msg(c, "moe_finish: bad shape"); return; }
     if (!stage_route(c, r, r->on_device ? 16 : 4096)) return;   // the combine reads the weights only; ids just have to be sane
-    float* od = itb_mirror_inout(c, out, out_len);
+    float* od = at == 0 && nt * n == out_len ? itb_mirror_out(c, out, out_len) : itb_mirror_inout(c, out, out_len);     // written whole: nothing to bring in
     const float* rd = itb_mirror_in(c, rows, rows_len); const float* sh = itb_mirror_in(c, shared, nt * n);
     const float* lg = itb_mirror_in(c, logit, logit_at + nt);
     if (!od || !rd || !sh || !lg) return;

@@ -53,116 +53,120 @@ __global__ void __launch_bounds__(256) k_matmul_f32_rows(DevF32 w, const float* 
 
 // F32 matrix against many rows in the CPU path's own order (src/ops/naive.rs:49-56: a left fold over k of w[o][k] * x[r][k],
 // product and sum rounded separately). With many rows there is a chain per (row, output), so no chain needs to be spread over
-// lanes: a thread owns a 4 x 4 block of outputs and walks k in order -- a plain tiled SGEMM whose k loop is never reassociated
-// or fused. grid (ceil(n_out / 64), ceil(n_rows / 64)), block 256; k tiles of 32 through shared memory, next tile in flight.
-// FUSED (tolerance class, with opts dense=bf16tc): the same walk with one fused multiply-add per step -- half the instructions, and
-// sums that differ from the CPU's by the product's rounding only.
-constexpr int SG_T = 64, SG_K = 32;
-template <bool FUSED = false>
-__global__ void __launch_bounds__(256) k_sgemm_serial(DevF32 w, const float* __restrict__ x, int n_rows, float* out) {
-    __shared__ float ws[2][SG_K][SG_T + 4], xs[2][SG_K][SG_T + 4];      // [k][output] and [k][row]: a thread reads 4 consecutive of each
-    const int o0 = blockIdx.x * SG_T, r0 = blockIdx.y * SG_T, n = w.n_in;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;             // outputs 4*tx.., rows 4*ty..
-    // loader: thread -> (line 0..63 of the tile, 8 consecutive k)
-    const int ll = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 8;
-    const float* wsrc = w.w + (size_t)min(o0 + ll, w.n_out - 1) * n + lk;
-    const float* xsrc = x + (size_t)min(r0 + ll, n_rows - 1) * n + lk;
-    float4 wa, wb, xa, xb;
-    auto fetch = [&](int k0) {
-        wa = __ldg((const float4*)(wsrc + k0)); wb = __ldg((const float4*)(wsrc + k0 + 4));
-        xa = __ldg((const float4*)(xsrc + k0)); xb = __ldg((const float4*)(xsrc + k0 + 4));
-    };
-    auto stash = [&](int buf) {
-        ws[buf][lk][ll] = wa.x; ws[buf][lk + 1][ll] = wa.y; ws[buf][lk + 2][ll] = wa.z; ws[buf][lk + 3][ll] = wa.w;
-        ws[buf][lk + 4][ll] = wb.x; ws[buf][lk + 5][ll] = wb.y; ws[buf][lk + 6][ll] = wb.z; ws[buf][lk + 7][ll] = wb.w;
-        xs[buf][lk][ll] = xa.x; xs[buf][lk + 1][ll] = xa.y; xs[buf][lk + 2][ll] = xa.z; xs[buf][lk + 3][ll] = xa.w;
-        xs[buf][lk + 4][ll] = xb.x; xs[buf][lk + 5][ll] = xb.y; xs[buf][lk + 6][ll] = xb.z; xs[buf][lk + 7][ll] = xb.w;
-    };
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    fetch(0); stash(0);
-    __syncthreads();
-    const int nk = n / SG_K;
-    for (int t = 0; t < nk; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < nk) fetch((t + 1) * SG_K);
-#pragma unroll
-        for (int kk = 0; kk < SG_K; ++kk) {
-            const float4 wv = *(const float4*)&ws[buf][kk][4 * tx], xv = *(const float4*)&xs[buf][kk][4 * ty];
-            const float wq[4] = {wv.x, wv.y, wv.z, wv.w}, xq[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = FUSED ? fmaf(wq[j], xq[i], acc[i][j]) : __fadd_rn(acc[i][j], __fmul_rn(wq[j], xq[i]));
-        }
-        if (t + 1 < nk) stash(buf ^ 1);
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = r0 + 4 * ty + i;
-        if (r >= n_rows) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int o = o0 + 4 * tx + j;
-            if (o < w.n_out) out[(size_t)r * w.n_out + o] = acc[i][j];
-        }
-    }
-}
-
-// The same for few rows or few outputs, where 64 x 64 tiles would leave most SMs idle: a thread per (row, output), 16 x 16 of
-// them per block; every thread's k loop is the row's whole chain either way, so the small tile costs nothing but reuse. With
-// so few blocks the global loads are what must not be waited for: tiles of 128 k arrive through a four-stage cp.async ring
-// (three tiles in flight while one is folded). grid (ceil(n_out / 16), ceil(n_rows / 16)), block 256, dynamic shared memory
-// sgemm_small_smem(); n_in a multiple of 128.
-constexpr int SGS_K = 128, SGS_ST = SGS_K + 4, SGS_STAGES = 4;
-constexpr size_t sgemm_small_smem() { return (size_t)SGS_STAGES * 2 * 16 * SGS_ST * 4; }
-// Two matrices over the same rows in one launch (blockIdx.z picks; w1.w null: one matrix): the router and the shared expert's
-// gate, or alpha and beta -- each alone is a handful of blocks walking a 2,048-long chain, and one after the other they cost twice.
-template <bool FUSED = false>
-__global__ void __launch_bounds__(256) k_sgemm_serial_small(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
+// lanes: a thread owns MR x MO of them and walks k in order -- a tiled SGEMM whose k loop is never reassociated or fused. Tiles of
+// KT k arrive through an NST-stage cp.async ring, lines KT + 4 floats apart; a thread's outputs and rows are TO / MO and TR / MR
+// apart, so the 16-byte reads of a warp fall on distinct banks. FUSED (tolerance class): the same walk with one fused multiply-add
+// per step. Two matrices over the same rows in one launch (blockIdx.z picks; w1.w null: one): the router and the shared expert's
+// gate, or alpha and beta -- each alone is a handful of blocks walking a 2,048-long chain.
+// grid (ceil(n_out / TO), ceil(n_rows / TR), 1 or 2), block 128; n_in a multiple of KT.
+// What bounds the two shapes: 16 x 16 (2 chains to a thread, a warp to a scheduler) the chain itself, 4 cycles a step, which the
+// shared-memory reads just keep up with (a thread per output at 256 threads read twice as much per step and took twice as long);
+// 32 x 64 the f32 pipe (16 chains, 32 operations for 8 reads of 4 steps).
+template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
+__global__ void __launch_bounds__(128) k_sgemm_chain(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
+    static_assert((TO / MO) * (TR / MR) == 128, "a thread per MO x MR outputs");
+    constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, PIECES = (TO + TR) * (KT / 4) / 128;
     extern __shared__ __align__(16) unsigned char smem[];
-    float* ring = (float*)smem;                    // [stage][w | x][16 lines][SGS_ST]
+    float* ring = (float*)smem;                    // [stage][TO weight lines | TR activation lines][ST]
     const DevF32 w = blockIdx.z ? w1 : w0;
     float* out = blockIdx.z ? out1 : out0;
-    if ((int)blockIdx.x * 16 >= w.n_out) return;
-    const int o0 = blockIdx.x * 16, r0 = blockIdx.y * 16, n = w.n_in, nk = n / SGS_K;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;            // output o0 + tx, row r0 + ty
+    const int o0 = blockIdx.x * TO, r0 = blockIdx.y * TR, n = w.n_in, nk = n / KT;
+    if (o0 >= w.n_out) return;
+    const int tx = threadIdx.x % NX, ty = threadIdx.x / NX;
+    const float* src[PIECES];
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int c = threadIdx.x + 128 * i, line = c / (KT / 4), k4 = (c % (KT / 4)) * 4;
+        src[i] = (line < TO ? w.w + (size_t)min(o0 + line, w.n_out - 1) * n : x + (size_t)min(r0 + line - TO, n_rows - 1) * n) + k4;
+    }
     auto fetch = [&](int t) {
         if (t < nk) {
-            float* st = ring + (size_t)(t % SGS_STAGES) * 2 * 16 * SGS_ST;
+            float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int c = threadIdx.x + 256 * i, m = c >> 9, line = (c & 511) >> 5, k4 = (c & 31) * 4;      // 2 matrices x 16 lines x 32 chunks
-                const float* src = m ? x + (size_t)min(r0 + line, n_rows - 1) * n : w.w + (size_t)min(o0 + line, w.n_out - 1) * n;
-                cp_async16(st + (m * 16 + line) * SGS_ST + k4, src + (size_t)t * SGS_K + k4, true);
+            for (int i = 0; i < PIECES; ++i) {
+                const int c = threadIdx.x + 128 * i;
+                cp_async16(st + (c / (KT / 4)) * ST + (c % (KT / 4)) * 4, src[i] + (size_t)t * KT, true);
             }
         }
         cp_async_commit();
     };
-    for (int t = 0; t < SGS_STAGES - 1; ++t) fetch(t);
-    float acc = 0.0f;
+    for (int t = 0; t < NST - 1; ++t) fetch(t);
+    float acc[MR][MO];
+#pragma unroll
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < MO; ++j) acc[i][j] = 0.0f;
     for (int t = 0; t < nk; ++t) {
-        cp_async_wait<SGS_STAGES - 2>();
+        cp_async_wait<NST - 2>();
         __syncthreads();                           // tile t has landed for everyone; everyone is done with tile t - 1
-        fetch(t + SGS_STAGES - 1);                 // into the slot tile t - 1 used
-        const float* st = ring + (size_t)(t % SGS_STAGES) * 2 * 16 * SGS_ST;
-        const float* wr = st + tx * SGS_ST; const float* xr = st + (16 + ty) * SGS_ST;
-#pragma unroll 8
-        for (int kk = 0; kk < SGS_K; kk += 4) {
-            const float4 a = *(const float4*)(wr + kk), c = *(const float4*)(xr + kk);
-            if (FUSED) { acc = fmaf(a.x, c.x, acc); acc = fmaf(a.y, c.y, acc); acc = fmaf(a.z, c.z, acc); acc = fmaf(a.w, c.w, acc); }
-            else {
-                acc = __fadd_rn(acc, __fmul_rn(a.x, c.x)); acc = __fadd_rn(acc, __fmul_rn(a.y, c.y));
-                acc = __fadd_rn(acc, __fmul_rn(a.z, c.z)); acc = __fadd_rn(acc, __fmul_rn(a.w, c.w));
-            }
+        fetch(t + NST - 1);                        // into the slot tile t - 1 used
+        const float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
+        const float* wr = st + tx * ST; const float* xr = st + (TO + ty) * ST;
+#pragma unroll(MO * MR <= 2 ? KT / 4 : 4)
+        for (int kk = 0; kk < KT; kk += 4) {
+            float4 a[MO], c[MR];
+#pragma unroll
+            for (int j = 0; j < MO; ++j) a[j] = *(const float4*)(wr + j * NX * ST + kk);
+#pragma unroll
+            for (int i = 0; i < MR; ++i) c[i] = *(const float4*)(xr + i * NY * ST + kk);
+            auto step = [&](float (&acc)[MR][MO], auto get) {
+#pragma unroll
+                for (int i = 0; i < MR; ++i)
+#pragma unroll
+                    for (int j = 0; j < MO; ++j) acc[i][j] = FUSED ? fmaf(get(a[j]), get(c[i]), acc[i][j]) : __fadd_rn(acc[i][j], __fmul_rn(get(a[j]), get(c[i])));
+            };
+            step(acc, [](const float4& v) { return v.x; }); step(acc, [](const float4& v) { return v.y; });
+            step(acc, [](const float4& v) { return v.z; }); step(acc, [](const float4& v) { return v.w; });
         }
     }
     cp_async_wait<0>();
-    if (r0 + ty < n_rows && o0 + tx < w.n_out) out[(size_t)(r0 + ty) * w.n_out + o0 + tx] = acc;
+#pragma unroll
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < MO; ++j)
+            if (r0 + ty + i * NY < n_rows && o0 + tx + j * NX < w.n_out) out[(size_t)(r0 + ty + i * NY) * w.n_out + o0 + tx + j * NX] = acc[i][j];
+}
+constexpr int SGS_KT = 64, SGS_NST = 6, SGB_KT = 32, SGB_NST = 4;      // 16 x 16 tiles: 1,536 steps' bytes in flight hide HBM's latency behind 4 cycles a step
+constexpr size_t sgemm_small_smem() { return (size_t)SGS_NST * 32 * (SGS_KT + 4) * 4; }
+constexpr size_t sgemm_big_smem() { return (size_t)SGB_NST * 96 * (SGB_KT + 4) * 4; }
+inline bool sgemm_chain_ok(int n_in) { return n_in % SGS_KT == 0; }
+// One matrix, or two over the same rows. The wide tiles where they give every SM a block, else the small ones.
+template <bool FUSED>
+static void sgemm_chain(cudaStream_t st, int sms, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb = DevF32{}, float* ob = nullptr) {
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(k_sgemm_chain<FUSED, 16, 16, 1, 2, SGS_KT, SGS_NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sgemm_small_smem());
+        cudaFuncSetAttribute(k_sgemm_chain<FUSED, 32, 64, 4, 4, SGB_KT, SGB_NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sgemm_big_smem());
+        attr = true;
+    }
+    const int n_out = std::max(wa.n_out, wb.w ? wb.n_out : 0), nz = wb.w ? 2 : 1;
+    if (((wa.n_out + 31) / 32) * ((n_rows + 63) / 64) >= sms)
+        k_sgemm_chain<FUSED, 32, 64, 4, 4, SGB_KT, SGB_NST><<<dim3((n_out + 31) / 32, (n_rows + 63) / 64, nz), 128, sgemm_big_smem(), st>>>(wa, x, n_rows, oa, wb, ob);
+    else
+        k_sgemm_chain<FUSED, 16, 16, 1, 2, SGS_KT, SGS_NST><<<dim3((n_out + 15) / 16, (n_rows + 15) / 16, nz), 128, sgemm_small_smem(), st>>>(wa, x, n_rows, oa, wb, ob);
+}
+
+// A dense Q8_0 matrix against n_rows >= 1 quantised rows: out[row][n_out] = or += (mode). tc: the tensor-core forms the context's
+// options name may be used (eager many-token passes); same: xq / xs are what the previous call with tc read. False: a device error.
+static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool tc, bool same) {
+    const int k = w.n_in;
+    // many rows, dense=f16tc (tolerance class): both operands dequantised to f16, one tcgen05 GEMM with f32 accumulators
+    if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, xq, xs, n_rows, out, stride, mode, same);
+    // many rows, dense=q8tc: exact integer dots of 128 x 128 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
+    if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, xq, xs, n_rows, out, stride, mode, same);
+    static bool attr = false;
+    if (!attr) {
+        for (const void* f : {(const void*)k_tile_q8<1, 256, 4>, (const void*)k_tile_q8<4, 256, 2>}) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        attr = true;
+    }
+    const bool skinny = n_rows <= 32;
+    const int ns = std::min(k / 256, TILE_STAGES);
+    if (skinny && k % 256 == 0) k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, xq, xs, n_rows, out, stride, mode, ns);
+    else if (k % 256 == 0) k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, xq, xs, n_rows, out, stride, mode, ns);
+    else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st>>>(w, xq, xs, n_rows, out, stride, mode);
+    else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st>>>(w, xq, xs, n_rows, out, stride, mode);
+    return true;
 }
 
 // RMSNorm + Q8_0 quantisation of each row (src/ops/naive.rs:139-152, :653-675): normalised f32 row, int8 quants,

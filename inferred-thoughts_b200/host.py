@@ -70,8 +70,17 @@ def lib():
     return _LIB
 
 
+def _addr(a):
+    """The address of an array's first element. Through the buffer protocol: a third of what `a.ctypes.data` costs; read-only, empty or
+    strided arrays take the long way."""
+    try:
+        return C.addressof(C.c_char.from_buffer(a))
+    except (TypeError, ValueError, BufferError):
+        return a.ctypes.data
+
+
 def _p(a):
-    return C.c_void_p(a.ctypes.data) if a is not None else C.c_void_p(None)
+    return C.c_void_p(_addr(a) if a is not None else None)
 
 
 class Weights:
@@ -193,7 +202,7 @@ class B200Ops:
     def softmax(self, x, row): self.L.itb_softmax(self.h, _p(x), SZ(x.size), SZ(row))
 
     def attend(self, q, k_slab, v_slab, kv_dim, n_pos, head_dim, n_head, n_head_kv, scale, out):
-        a = _Attn(q.ctypes.data, q.size, k_slab.ctypes.data, v_slab.ctypes.data, k_slab.size, kv_dim, n_pos, head_dim,
+        a = _Attn(_addr(q), q.size, _addr(k_slab), _addr(v_slab), k_slab.size, kv_dim, n_pos, head_dim,
                   n_head, n_head_kv, scale)
         self.L.itb_attend(self.h, C.byref(a), _p(out), SZ(out.size))
 
@@ -224,8 +233,8 @@ class B200Ops:
 
     def delta_rule(self, q, k, v, alpha, beta, ssm_a, dt_bias, head_k_dim, head_v_dim, n_k_heads, n_v_heads, state, out):
         n_tok = v.size // (n_v_heads * head_v_dim)
-        d = _Delta(q.ctypes.data, k.ctypes.data, v.ctypes.data, alpha.ctypes.data, beta.ctypes.data, ssm_a.ctypes.data,
-                   dt_bias.ctypes.data, n_tok, head_k_dim, head_v_dim, n_k_heads, n_v_heads)
+        d = _Delta(_addr(q), _addr(k), _addr(v), _addr(alpha), _addr(beta), _addr(ssm_a),
+                   _addr(dt_bias), n_tok, head_k_dim, head_v_dim, n_k_heads, n_v_heads)
         self.L.itb_delta_rule(self.h, C.byref(d), _p(state), SZ(state.size), _p(out), SZ(out.size))
 
     def route(self, probs, n_expert, n_used):
@@ -425,7 +434,7 @@ class Engine:
     def prefill(self, tokens, want_logits=True):
         """tokens: [n_seq][n] (or [n] for one sequence); returns the last token's logits, [n_seq][n_vocab] (or [n_vocab])."""
         tokens = np.ascontiguousarray(tokens, np.uint32).reshape(self.n_seq, -1)
-        logits = np.zeros((self.n_seq, self.n_vocab), np.float32) if want_logits else None
+        logits = np.empty((self.n_seq, self.n_vocab), np.float32) if want_logits else None
         self._chk(self.L.itb_engine_prefill(self.h, _p(tokens), SZ(tokens.shape[1]), _p(logits)), "prefill")
         if logits is None:
             return None
@@ -434,7 +443,7 @@ class Engine:
     def decode(self, tokens, want_logits=True):
         tokens = np.ascontiguousarray(tokens, np.uint32).reshape(-1)
         assert tokens.size == self.n_seq
-        logits = np.zeros((self.n_seq, self.n_vocab), np.float32) if want_logits else None
+        logits = np.empty((self.n_seq, self.n_vocab), np.float32) if want_logits else None
         nxt = np.zeros(self.n_seq, np.uint32)
         self._chk(self.L.itb_engine_decode(self.h, _p(tokens), _p(logits), _p(nxt)), "decode")
         return logits, nxt

@@ -323,6 +323,37 @@ def test_grouped_expert_tiles_at_their_edges(ops, E, H, ff):
     exact(o, o_want, "matmul_experts(down)")
 
 
+@pytest.mark.parametrize("n_tok,n_in,n_out", [(1, 64, 1), (15, 384, 16), (17, 2048, 33), (33, 448, 129), (300, 64, 1000), (321, 2048, 993)])
+def test_f32_matmul_tiles_at_their_edges(ops, n_tok, n_in, n_out):
+    """Chains per output in 16 x 16 and 32 x 64 tiles: fewer k steps than the ring has stages, ragged rows and outputs; inputs and outputs
+    on both sides of the sizes at which the copies to and from the host change."""
+    from inferred_thoughts_b200 import host
+    w, x = keep(noise(n_in * n_out, 160)), keep(noise(n_tok * n_in, 161))
+    out = keep(np.zeros(n_tok * n_out, np.float32)); want = np.zeros_like(out)
+    for rep in range(3):                       # the same buffers again: staging memory is reused while copies may still run
+        x += np.float32(rep)
+        ops.begin_pass(n_tok)
+        ops.matmul(host.Weights(w, host.F32, n_in, n_out), x, out); ops.host_needs(out); ops.check()
+        L.orc_matmul(0, w.view(np.uint8), n_in, n_out, x, x.size, want, 0)
+        exact(out, want, "F32 matmul")
+
+
+@pytest.mark.parametrize("n,ff", [(1, 64), (5, 40), (15, 16)])
+def test_gated_experts_of_few_pairs(ops, n, ff):
+    """Fewer pairs than the grouped form takes: 16 gate and 16 up rows to a block, the last block ragged."""
+    from inferred_thoughts_b200 import host
+    E, H = 7, 192
+    (gb, gs), (ub, us) = nvfp4_weights(E, ff, H, 162), nvfp4_weights(E, ff, H, 163)
+    gs *= 300; us *= 300
+    ids = (np.arange(n) * 3 % E).astype(np.int32); x = noise(n * H, 164)
+    h = keep(np.zeros(n * ff, np.float32)); scratch = keep(np.zeros_like(h)); h_want = np.zeros_like(h)
+    ops.begin_pass(n)
+    ops.moe_glu(host.Experts(gb, host.NVFP4, H, ff, E, gs), host.Experts(ub, host.NVFP4, H, ff, E, us), host.Route.host(ids.astype(np.uint64), None, 1), x, h, scratch)
+    ops.host_needs(h); ops.check()
+    L.orc_moe_glu(gb, gs.ctypes.data, ub, us.ctypes.data, H, ff, E, ids, n, 1, x, x.size, h_want, 0)
+    close(h, h_want, 8 * EPS, "moe_glu (through silu)")
+
+
 def test_grouped_expert_matmuls_at_8192_tokens_repeat_the_small_case(ops, cfg2_experts):
     """At the microbenchmark's largest size the CPU check is too slow; instead 8,192 tokens made of 16 copies of 512 distinct
     ones must give 16 copies of the 512-token result (the tiles are 64 tokens wide there, 16 wide at 512 tokens)."""
