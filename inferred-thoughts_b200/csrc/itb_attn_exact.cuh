@@ -6,7 +6,9 @@
 // per softmax sum, n_pos multiply-adds per output) one thread each. Selected by exact=1; exact=0 keeps the split-K kernels,
 // which reassociate the sums (tolerance class) and are faster at long contexts.
 #pragma once
+#include <type_traits>
 #include "itb_kernels.cuh"
+#include "itb_tile.cuh"
 
 namespace {
 
@@ -173,6 +175,224 @@ __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
     __syncthreads();
     const float sum = s_sum;
     for (int s = tid; s < n_pos; s += 256) sc[s] = w[s] / sum;
+}
+// ---- many query rows of a sequence: the same folds as tiled products ----
+// A row of the product is a (token, head of the group) pair -- they all read the KV head's one key or value line -- and a thread owns
+// MR x 4 chains of a tile of 16 * MR such lines by 64 positions (scores) or 64 dimensions (outputs), walked in the CPU path's order
+// with product and sum rounded apart. What bounds them is the f32 pipe: two operations a step, 64 steps a cycle and SM; the tile
+// keeps shared-memory reads (12 of 16 bytes for 256 operations at MR = 8) and conversions below that, where one chain per thread
+// (above) waits on its own reads. Tiles of 32 k arrive through a 3-stage cp.async ring. Token tiles run from the last (most positions)
+// to the first, so that no long one starts late.
+// A 5,548-token prompt in passes of 2,048 rows (16 heads of 256 over 2 KV heads), all ten layers: scores 117 -> 47.5 ms, values
+// 374 -> 50.0 ms; the operations alone take 35 ms each at 1.9 GHz.
+constexpr int AT_KT = 32, AT_ST = AT_KT + 4, AT_NST = 3, AT_KST = 40;       // line strides: floats; 16-bit elements of a key line
+struct AtTile { int r0, nt, seq; };            // first row, tokens, sequence
+template <int MR>
+__device__ __forceinline__ AtTile at_tile(int rows_per_seq, int group, int* s_lim, const int* n_pos_dev, int n_pos_last, int n_q) {
+    const int tt = 16 * MR / group, per = (rows_per_seq + tt - 1) / tt, t = per - 1 - (int)blockIdx.z % per;
+    AtTile a;
+    a.seq = (int)blockIdx.z / per; a.r0 = a.seq * rows_per_seq + t * tt; a.nt = min(tt, rows_per_seq - t * tt);
+    if (threadIdx.x == 0) { s_lim[0] = 0; s_lim[1] = 0x7fffffff; }
+    __syncthreads();
+    if ((int)threadIdx.x < a.nt) {
+        const int np = n_pos_dev ? n_pos_dev[a.r0 + threadIdx.x] : n_pos_last - n_q + 1 + a.r0 + (int)threadIdx.x;
+        atomicMax(&s_lim[0], np); atomicMin(&s_lim[1], np);
+    }
+    __syncthreads();
+    return a;
+}
+template <int MR> constexpr size_t attn_scores_tile_smem() { return (size_t)AT_NST * (16 * MR * AT_ST * 4 + 64 * AT_KST * 2); }
+template <int MR> constexpr size_t attn_out_tile_smem() { return (size_t)AT_NST * (16 * MR * AT_ST * 4 + AT_KT * 64 * 2); }
+// grid (ceil(n_pos_max / 64), n_head_kv, sequences * token tiles), block 256; hd a multiple of 32.
+template <int MR, bool BF>
+__global__ void __launch_bounds__(256, 2) k_attn_scores_tile(AxScores p) {
+    constexpr int TL = 16 * MR, QB = TL * AT_ST * 4, STAGE = QB + 64 * AT_KST * 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_lim[2];
+    const int hk = blockIdx.y, hd = p.hd, group = p.n_head / p.n_head_kv, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, p0 = blockIdx.x * 64;
+    pdl_trigger(); pdl_wait();
+    const AtTile t = at_tile<MR>(p.rows_per_seq, group, s_lim, p.n_pos_dev, p.n_pos_last, p.n_q);
+    const int mx = s_lim[0], nl = t.nt * group, nk = hd / AT_KT;
+    if (p0 >= mx) return;
+    const float* qb = p.q + ((size_t)t.r0 * p.n_head + hk * group) * hd;
+    auto q_line = [&](int l) { l = min(l, nl - 1); return ((size_t)(l / group) * p.n_head + l % group) * hd; };
+    const float* qsrc[MR / 2];
+#pragma unroll
+    for (int i = 0; i < MR / 2; ++i) qsrc[i] = qb + q_line((tid + 256 * i) >> 3) + (tid & 7) * 4;
+    const uint16_t* ksrc = p.kslab + (size_t)t.seq * p.slab_stride + (size_t)min(p0 + (tid >> 2), mx - 1) * p.kv_dim + hk * hd + (tid & 3) * 8;
+    auto fetch = [&](int k) {
+        if (k < nk) {
+            unsigned char* st = smem + (k % AT_NST) * STAGE;
+#pragma unroll
+            for (int i = 0; i < MR / 2; ++i) cp_async16((float*)st + ((tid + 256 * i) >> 3) * AT_ST + (tid & 7) * 4, qsrc[i] + k * AT_KT, true);
+            cp_async16((uint16_t*)(st + QB) + (tid >> 2) * AT_KST + (tid & 3) * 8, ksrc + k * AT_KT, true);
+        }
+        cp_async_commit();
+    };
+    for (int k = 0; k < AT_NST - 1; ++k) fetch(k);
+    float acc[MR][4];
+#pragma unroll
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    for (int k = 0; k < nk; ++k) {
+        cp_async_wait<AT_NST - 2>();
+        __syncthreads();                           // tile k has landed for everyone; everyone is done with tile k - 1
+        fetch(k + AT_NST - 1);
+        const unsigned char* st = smem + (k % AT_NST) * STAGE;
+        const float* qs = (const float*)st + ty * AT_ST;
+        const uint16_t* ks = (const uint16_t*)(st + QB) + tx * AT_KST;
+#pragma unroll
+        for (int kk = 0; kk < AT_KT; kk += 8) {
+            uint4 kw[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) kw[j] = *(const uint4*)(ks + 16 * j * AT_KST + kk);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 q[MR];
+#pragma unroll
+                for (int i = 0; i < MR; ++i) q[i] = *(const float4*)(qs + 16 * i * AT_ST + kk + 4 * h);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float kv[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) kv[j] = kv_elem(h == 0 ? (u < 2 ? kw[j].x : kw[j].y) : (u < 2 ? kw[j].z : kw[j].w), u & 1, BF);
+#pragma unroll
+                    for (int i = 0; i < MR; ++i) {
+                        const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(qv, kv[j]));
+                    }
+                }
+            }
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < MR; ++i) {
+        const int l = ty + 16 * i, r = t.r0 + l / group;
+        if (l >= nl) break;
+        const int np = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
+        float* out = p.scores + ((size_t)r * p.n_head + hk * group + l % group) * p.s_stride + p0 + tx;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (p0 + tx + 16 * j < np) out[16 * j] = acc[i][j] * p.scale;
+    }
+}
+// The weighted values from the softmax weights (weights_ready), 64 dimensions of a head to a block; gate and Q8_0 as in k_attn_out_exact.
+// Positions past a row's own take no part in its chain: the tiles that all of a block's rows span go unguarded, the few after them by
+// a select. grid (hd / 64, n_head_kv, sequences * token tiles), block 256; s_stride a multiple of 4.
+template <int MR, bool BF>
+__global__ void __launch_bounds__(256, 2) k_attn_out_tile(AxOut p) {
+    constexpr int TL = 16 * MR, WB = TL * AT_ST * 4, STAGE = WB + AT_KT * 64 * 2;
+    static_assert(AT_NST * STAGE >= TL * 68 * 4, "the epilogue's tile fits the ring");
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_lim[2];
+    const int d0 = blockIdx.x * 64, hk = blockIdx.y, hd = p.hd, group = p.n_head / p.n_head_kv, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    pdl_trigger(); pdl_wait();
+    const AtTile t = at_tile<MR>(p.rows_per_seq, group, s_lim, p.n_pos_dev, p.n_pos_last, p.n_q);
+    const int mx = s_lim[0], full = s_lim[1] / AT_KT, nl = t.nt * group, nk = (mx + AT_KT - 1) / AT_KT;
+    const float* wb = p.scores + ((size_t)t.r0 * p.n_head + hk * group) * p.s_stride;
+    const float* wsrc[MR / 2];
+#pragma unroll
+    for (int i = 0; i < MR / 2; ++i) {
+        const int l = min((tid + 256 * i) >> 3, nl - 1);
+        wsrc[i] = wb + ((size_t)(l / group) * p.n_head + l % group) * p.s_stride + (tid & 7) * 4;
+    }
+    const uint16_t* vsrc = p.vslab + (size_t)t.seq * p.slab_stride + hk * hd + d0 + (tid & 7) * 8;
+    auto fetch = [&](int k) {
+        if (k < nk) {
+            unsigned char* st = smem + (k % AT_NST) * STAGE;
+            const bool in_w = k * AT_KT + (tid & 7) * 4 < mx, in_v = k * AT_KT + (tid >> 3) < mx;
+#pragma unroll
+            for (int i = 0; i < MR / 2; ++i) cp_async16((float*)st + ((tid + 256 * i) >> 3) * AT_ST + (tid & 7) * 4, wsrc[i] + (in_w ? k * AT_KT : 0), in_w);
+            cp_async16((uint16_t*)(st + WB) + (tid >> 3) * 64 + (tid & 7) * 8, vsrc + (size_t)(in_v ? k * AT_KT + (tid >> 3) : 0) * p.kv_dim, in_v);
+        }
+        cp_async_commit();
+    };
+    for (int k = 0; k < AT_NST - 1; ++k) fetch(k);
+    float acc[MR][4];
+    int np[MR];
+#pragma unroll
+    for (int i = 0; i < MR; ++i) {
+        const int r = t.r0 + min(ty + 16 * i, nl - 1) / group;
+        np[i] = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    }
+    auto tile = [&](int k, auto guarded) {
+        const unsigned char* st = smem + (k % AT_NST) * STAGE;
+        const float* ws = (const float*)st + ty * AT_ST;
+        const uint16_t* vs = (const uint16_t*)(st + WB) + tx * 4;
+#pragma unroll
+        for (int kk = 0; kk < AT_KT; kk += 4) {
+            float4 w[MR];
+#pragma unroll
+            for (int i = 0; i < MR; ++i) w[i] = *(const float4*)(ws + 16 * i * AT_ST + kk);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint2 vw = *(const uint2*)(vs + (kk + u) * 64);
+                const float v[4] = {kv_elem(vw.x, 0, BF), kv_elem(vw.x, 1, BF), kv_elem(vw.y, 0, BF), kv_elem(vw.y, 1, BF)};
+#pragma unroll
+                for (int i = 0; i < MR; ++i) {
+                    const float wv = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+                    const bool in = !decltype(guarded)::value || k * AT_KT + kk + u < np[i];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { const float n = __fadd_rn(acc[i][j], __fmul_rn(wv, v[j])); acc[i][j] = in ? n : acc[i][j]; }
+                }
+            }
+        }
+    };
+    for (int k = 0; k < nk; ++k) {
+        cp_async_wait<AT_NST - 2>();
+        __syncthreads();
+        fetch(k + AT_NST - 1);
+        if (k < full) tile(k, std::false_type{}); else tile(k, std::true_type{});
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    float* ot = (float*)smem;                      // [TL][68]
+#pragma unroll
+    for (int i = 0; i < MR; ++i) *(float4*)(ot + (ty + 16 * i) * 68 + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
+    const int wid = tid >> 5, lane = tid & 31;
+    for (int u = wid; u < 2 * nl; u += 8) {        // 32 dimensions of a line
+        const int l = u >> 1, r = t.r0 + l / group;
+        const size_t idx = ((size_t)r * p.n_head + hk * group + l % group) * hd + d0 + (u & 1) * 32 + lane;
+        float o = ot[l * 68 + (u & 1) * 32 + lane];
+        if (p.gate) o *= sigmoid_f(p.gate[idx]);
+        if (p.out_q) {
+            float dq;
+            const int8_t q = warp_quant_q8(o, &dq);
+            p.out_q[idx] = q;
+            if (lane == 0) p.out_s[idx / 32] = dq;
+        } else p.out[idx] = o;
+    }
+}
+// Lines (16 * MR) of a tile, 0: a chain per thread (k_attn_scores_exact / k_attn_out_exact). A tile pays from about half of its
+// smallest form's lines on; the large one where its blocks still give every SM two.
+inline int attn_tile_rows(int rows_per_seq, int n_seq, int hd, int n_head, int n_head_kv, int sms) {
+    const int group = n_head / n_head_kv;
+    if (hd % 64 || rows_per_seq * group < 32) return 0;
+    const long long blocks = (long long)(hd / 64) * n_head_kv * n_seq * ((rows_per_seq + 128 / group - 1) / (128 / group));
+    return blocks >= 2 * sms ? 8 : 4;
+}
+// Scores, softmax and weighted values of a pass in that form. launch(kernel, grid, block, shared memory, argument).
+template <class L>
+static void attn_exact_tiles(const AxScores& a, const AxSoft& sm, const AxOut& o, int mr, int n_seq, int rows, int n_pos_max, L&& launch) {
+    const int group = a.n_head / a.n_head_kv, tt = 16 * mr / group, z = n_seq * ((a.rows_per_seq + tt - 1) / tt);
+    const size_t soft = (size_t)((n_pos_max + 3) & ~3) * 4;
+    auto run = [&](auto scores, auto out, size_t scores_smem, size_t out_smem) {
+        cudaFuncSetAttribute(scores, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scores_smem);
+        cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
+        cudaFuncSetAttribute(k_attn_softmax_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        launch(scores, dim3((n_pos_max + 63) / 64, a.n_head_kv, z), dim3(256), scores_smem, a);
+        launch(k_attn_softmax_exact, dim3(a.n_head, rows), dim3(256), soft, sm);
+        launch(out, dim3(a.hd / 64, a.n_head_kv, z), dim3(256), out_smem, o);
+    };
+    if (mr == 8 && a.bf16) run(k_attn_scores_tile<8, true>, k_attn_out_tile<8, true>, attn_scores_tile_smem<8>(), attn_out_tile_smem<8>());
+    else if (mr == 8) run(k_attn_scores_tile<8, false>, k_attn_out_tile<8, false>, attn_scores_tile_smem<8>(), attn_out_tile_smem<8>());
+    else if (a.bf16) run(k_attn_scores_tile<4, true>, k_attn_out_tile<4, true>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
+    else run(k_attn_scores_tile<4, false>, k_attn_out_tile<4, false>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
 }
 inline size_t attn_out_exact_smem(int n_pos_max) { return (size_t)((n_pos_max + 3) & ~3) * 4 + 2 * AX_VT * 32 * 2; }
 inline size_t attn_scores_exact_smem(int hd, int group) { return (size_t)group * (hd + AX_QSTRIDE_PAD) * 4; }

@@ -718,8 +718,9 @@ constexpr size_t SMEM_BUDGET = 200 * 1024;   // dynamic shared memory the row-st
 // Q8_0 quantisation into e->aq / e->as. Needs a row stride of whole 16-byte spans; the scores buffer holds n_ctx per (row, head).
 static bool exact_attention_ok(const itb_engine* e) { return e->c->exact && (e->m->d.head_dim * e->m->d.n_head_kv) % 8 == 0 && e->m->d.n_head / e->m->d.n_head_kv <= 8; }
 static void drop_graph(itb_engine* e);
+static size_t scores_stride(const itb_engine* e) { return (e->n_ctx + 3) & ~(size_t)3; }
 static bool ensure_scores(itb_engine* e, size_t rows) {
-    const size_t need = rows * e->m->d.n_head * e->n_ctx;
+    const size_t need = rows * e->m->d.n_head * scores_stride(e);
     if (e->scores_cap >= need) return true;
     cudaStreamSynchronize(e->c->stream);
     drop_graph(e);        // a captured step holds the old pointer
@@ -736,19 +737,25 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
     if (!attr) { set_smem((const void*)k_attn_out_exact, 200 * 1024); attr = true; }
     AxScores a{};
     a.q = e->qn; a.kslab = kslab; a.slab_stride = slab_stride; a.rows_per_seq = rows_per_seq; a.n_pos_dev = e->npos; a.kv_dim = kvd; a.hd = hd;
-    a.n_head = d.n_head; a.n_head_kv = d.n_head_kv; a.scale = 1.0f / sqrtf((float)hd); a.bf16 = e->c->kv_bf16; a.scores = e->scores; a.s_stride = (int)e->n_ctx;
-    launch_k(pdl, k_attn_scores_exact, dim3((n_pos_max + AX_TP - 1) / AX_TP, d.n_head_kv, rows), dim3(AX_TP * group), attn_scores_exact_smem(hd, group), st, a);
+    a.n_head = d.n_head; a.n_head_kv = d.n_head_kv; a.scale = 1.0f / sqrtf((float)hd); a.bf16 = e->c->kv_bf16; a.scores = e->scores; a.s_stride = (int)scores_stride(e);
     AxOut o{};
+    AxSoft sm{e->scores, (int)scores_stride(e), e->npos, 0, 0, (int)d.n_head};
+    o.scores = e->scores; o.s_stride = (int)scores_stride(e); o.vslab = vslab; o.slab_stride = slab_stride; o.rows_per_seq = rows_per_seq; o.n_pos_dev = e->npos;
+    o.kv_dim = kvd; o.hd = hd; o.n_head = d.n_head; o.n_head_kv = d.n_head_kv; o.bf16 = e->c->kv_bf16; o.gate = e->gate; o.out_q = e->aq; o.out_s = e->as;
+    const int n_seq = rows / std::max(1, rows_per_seq);
+    if (const int mr = attn_tile_rows(rows_per_seq, n_seq, hd, d.n_head, d.n_head_kv, e->c->sm_count)) {
+        o.weights_ready = 1;
+        attn_exact_tiles(a, sm, o, mr, n_seq, rows, n_pos_max, [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { launch_k(pdl, k, g, b, smem, st, arg); });
+        return;
+    }
+    launch_k(pdl, k_attn_scores_exact, dim3((n_pos_max + AX_TP - 1) / AX_TP, d.n_head_kv, rows), dim3(AX_TP * group), attn_scores_exact_smem(hd, group), st, a);
     if (rows >= 8) {
         // many rows: the softmax once per (row, head), in place, instead of once per block of the weighted-value kernel
-        AxSoft sm{e->scores, (int)e->n_ctx, e->npos, 0, 0, (int)d.n_head};
         static bool attr2 = false;
         if (!attr2) { set_smem((const void*)k_attn_softmax_exact, 200 * 1024); attr2 = true; }
         launch_k(pdl, k_attn_softmax_exact, dim3(d.n_head, rows), dim3(256), (size_t)((n_pos_max + 3) & ~3) * 4, st, sm);
         o.weights_ready = 1;
     }
-    o.scores = e->scores; o.s_stride = (int)e->n_ctx; o.vslab = vslab; o.slab_stride = slab_stride; o.rows_per_seq = rows_per_seq; o.n_pos_dev = e->npos;
-    o.kv_dim = kvd; o.hd = hd; o.n_head = d.n_head; o.n_head_kv = d.n_head_kv; o.bf16 = e->c->kv_bf16; o.gate = e->gate; o.out_q = e->aq; o.out_s = e->as;
     launch_k(pdl, k_attn_out_exact, dim3(hd / 32, d.n_head, rows), dim3(256), attn_out_exact_smem(n_pos_max), st, o);
 }
 
@@ -1359,7 +1366,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
 #undef AM_CASE
                 launches++;
                 k_attn_combine_rows<<<R * d.n_head, d.head_dim, 0, st>>>(e->part_acc, e->part_ml, 1, d.head_dim, e->gate, e->npos, d.n_head, e->aq, e->as); launches++;
-            } else if (exact_attention_ok(e) && e->scores_cap >= (size_t)R * d.n_head * e->n_ctx) {
+            } else if (exact_attention_ok(e) && e->scores_cap >= (size_t)R * d.n_head * scores_stride(e)) {
                 uint32_t top = 0;
                 for (int sq = 0; sq < n_seq; ++sq) top = std::max(top, e->host_pos[sq] + (uint32_t)n_tok);
                 if (n_tok == 1) top = e->n_ctx;        // a decode pass is replayed from a graph: its launches must hold any length
@@ -2166,7 +2173,7 @@ extern "C" int itb_engine_prefill(itb_engine* e, const uint32_t* tokens, size_t 
     // exact mode: room for the scores of a whole pass (up to 2 GB; beyond that the pass keeps the split-K attention)
     if (ok && exact_attention_ok(e) && getenv("ITB_PREFILL_STEPWISE") == nullptr) {
         const size_t rows = e->B * std::min(std::max<size_t>(1, e->R / e->B), n);
-        if (rows * e->m->d.n_head * e->n_ctx * 4 <= ((size_t)2 << 30)) ok = ensure_scores(e, rows);
+        if (rows * e->m->d.n_head * scores_stride(e) * 4 <= ((size_t)2 << 30)) ok = ensure_scores(e, rows);
     }
     // chunk-parallel delta rule: room for what its first kernel hands its second, for the largest pass of this call
     if (ok && (c->gdn_chunk || !c->exact) && e->m->d.ssm_d_state == 128 && getenv("ITB_PREFILL_STEPWISE") == nullptr) {

@@ -480,6 +480,28 @@ def test_attend_in_exact_mode_equals_the_cpu_path_bit_for_bit(hd, nh, nkv, n_pos
     ops.close()
 
 
+@pytest.mark.parametrize("hd,nh,nkv,n_pos,n_q,kv", [(64, 6, 2, 65, 11, "f16"), (128, 8, 1, 131, 131, "bf16"), (256, 16, 2, 200, 33, "f16"), (128, 32, 16, 600, 580, "bf16")])
+def test_attend_of_many_rows_equals_the_cpu_path_bit_for_bit(hd, nh, nkv, n_pos, n_q, kv):
+    """The tiled form: head groups that do not divide a tile, a last tile of few tokens, rows from the first position on, and enough
+    rows for the large tile. Positions past a row's own hold infinities: no row may see the values of later ones."""
+    from inferred_thoughts_b200 import host
+    ops = host.B200Ops(0, "exact=1,kv=" + kv)
+    kvd = hd * nkv
+    q = noise(n_q * nh * hd, 170)
+    ks, vs = noise(n_pos * kvd, 171), noise(n_pos * kvd, 172)
+    enc = (lambda a: (a.view(np.uint32) >> 16).astype(np.uint16)) if kv == "bf16" else (lambda a: a.astype(np.float16).view(np.uint16))
+    ks, vs = enc(ks), enc(vs)
+    vs[(n_pos - 1) * kvd:] = enc(np.full(1, np.inf, np.float32))[0]
+    scale = np.float32(1.0 / np.sqrt(hd))
+    want = np.zeros(n_q * nh * hd, np.float32); got = np.zeros_like(want)
+    L.orc_attend(q, q.size, ks, vs, kvd, n_pos, hd, nh, nkv, scale, int(kv == "bf16"), want)
+    ops.begin_pass(n_q)
+    ops.attend(q, ks, vs, kvd, n_pos, hd, nh, nkv, float(scale), got); ops.host_needs(got); ops.check()
+    m = (n_q - 1) * nh * hd                        # the last row is the one that sees the infinities
+    assert np.isfinite(want[:m]).all() and got[:m].view(np.uint32).tolist() == want[:m].view(np.uint32).tolist()
+    ops.close()
+
+
 def test_fp4_tensor_core_ceiling_runs_and_verifies_its_accumulators():
     """tcgen05.mma kind::mxf4nvf4 with unchanging operands (every value 1.0, every scale 1.0): each accumulator must end at
     64 * iters exactly; the rate is the denominator of the expert GEMMs' roofline fraction."""
