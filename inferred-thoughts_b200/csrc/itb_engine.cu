@@ -1327,7 +1327,9 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             } else {
                 const dim3 gs(n_v, sk / 32, n_seq);
                 float* sst = e->ssm_state + (size_t)rs * e->B * state_stride;
-                if (sk == 128) k_gdn_scan<128><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);
+                if (n_tok == 1 && sk == 128) k_gdn_step<128><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
+                else if (n_tok == 1) k_gdn_step<64><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
+                else if (sk == 128) k_gdn_scan<128><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);
                 else k_gdn_scan<64><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);   // 64 or 128 only (checked at model creation)
             }
             launches++;

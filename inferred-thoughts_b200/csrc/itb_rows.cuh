@@ -5,6 +5,7 @@
 // CPU path's arithmetic order, so a prefill is bit-identical to feeding the tokens one at a time, which the
 // reference asserts of its own backends (tests/qwen35.rs:94-139 there).
 #pragma once
+#include <type_traits>
 #include "itb_kernels.cuh"
 #include "itb_tile.cuh"
 
@@ -288,93 +289,181 @@ __global__ void k_gdn_pre(const float* conv, int cd, const float* alpha, const f
 // the rows, FOUR lanes per row, each lane holding a quarter of the row's state in registers across the pass's tokens.
 // The CPU's serial sums over the 128 keys are kept to the bit: lane 0 of a row adds its quarter's products in order
 // and hands the running sum to lane 1, and so on, so the chain is the CPU's chain; what the split buys is four times
-// the warps (the chain's latency is hidden by other rows) and a quarter of the per-lane multiplies. The next token's
-// k, q, v, g, beta are fetched while the current one is computed.
+// the warps and a quarter of the per-lane multiplies.
+// Bound by that chain: 128 adds of 4 cycles a token, and a scheduler has about one warp, whose instructions go between them. So a
+// token's read-out sum goes along with the NEXT token's prediction sum as the other half of packed adds (one instruction for both);
+// the update, decay and products of a column are formed in the first quarter's steps, just ahead of the add that takes them; the
+// next token's operands come during the other quarters, in straight-line code. A 512-token pass of 32 heads: 429 -> 257 us a layer
+// (lines of a quarter are CW + 4 floats apart: the four lanes of a row read distinct banks, where they shared one).
 template <int SK>
 __global__ void __launch_bounds__(128) k_gdn_scan(const float* qh, const float* kh, const float* vh, const float* gb, int n_tok, int n_k, int n_v,
                                                   float* state, size_t state_stride, float* out) {
     constexpr int CW = SK / 4;             // state columns per lane
-    constexpr int DEPTH = 4;               // tokens whose operands are in flight (cp.async ring, one group per token)
-    constexpr int SLOT = 2 * SK + 8 + 4;   // floats per token and warp: k | q | v of the warp's 8 rows | g, beta, pad
+    constexpr int QS = CW + 4, VEC = 4 * QS;
+    constexpr int DEPTH = 5;               // tokens whose operands are in flight or in use (cp.async ring, one group per token)
+    constexpr int SLOT = 2 * VEC + 8 + 4;  // floats per token and warp: k | q | v of the warp's 8 rows | g, beta, pad
     __shared__ __align__(16) float ring_all[4][DEPTH][SLOT];
     const int h = blockIdx.x, s = blockIdx.z, khd = h % n_k, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int r = lane >> 2, part = lane & 3, j0 = blockIdx.y * 32 + wid * 8, j = j0 + r;      // j: value row of the head
     float* sg = state + (size_t)s * state_stride + ((size_t)h * SK + j) * SK + part * CW;
-    float S[CW];
-#pragma unroll
-    for (int i = 0; i < CW; i += 4) { const float4 v = *(const float4*)(sg + i); S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w; }
+    if (n_tok <= 0) return;
+    // Straight-line on purpose: a branch would end the block of instructions that the sums' adds are spread over. pk, pq: this lane's
+    // 16 bytes of k and q (two lanes copy the same at SK = 64); px: v's for lanes 0 and 1, g and beta for lane 2.
+    const size_t row0 = (size_t)s * n_tok;
+    const int e4 = lane * 4 % SK;
+    const float* pk = kh + (row0 * n_k + khd) * SK + e4; const float* pq = qh + (row0 * n_k + khd) * SK + e4;
+    const float* px = lane < 2 ? vh + (row0 * n_v + h) * SK + j0 + lane * 4 : gb + (row0 * n_v + h) * 2;
+    const int step_k = n_k * SK, step_x = lane < 2 ? n_v * SK : n_v * 2;
+    const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(ring_all[wid][0]), ring_z = ring0 + DEPTH * SLOT * 4;
+    const uint32_t o_k = (uint32_t)(e4 / CW * QS + e4 % CW) * 4, o_x = (uint32_t)(2 * VEC + (lane < 2 ? lane * 4 : 8)) * 4;
+    uint32_t put = ring0;
     auto fetch = [&](int t) {
-        if (t < n_tok) {
-            const size_t row = (size_t)s * n_tok + t;
-            float* slot = ring_all[wid][t % DEPTH];
-            if (lane * 4 < SK) {
-                cp_async16(slot + lane * 4, kh + (row * n_k + khd) * SK + lane * 4, true);
-                cp_async16(slot + SK + lane * 4, qh + (row * n_k + khd) * SK + lane * 4, true);
-            }
-            if (lane < 2) cp_async16(slot + 2 * SK + lane * 4, vh + (row * n_v + h) * SK + j0 + lane * 4, true);
-            if (lane == 2) {
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(slot + 2 * SK + 8);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(gb + (row * n_v + h) * 2));
-            }
-        }
-        cp_async_commit();
+        asm volatile("{.reg .pred p, a, b;\n setp.lt.s32 p, %0, %1;\n setp.lt.and.u32 a, %2, 2, p;\n setp.eq.and.u32 b, %2, 2, p;\n"
+                     "@p cp.async.cg.shared.global [%3], [%4], 16;\n @p cp.async.cg.shared.global [%5], [%6], 16;\n"
+                     "@a cp.async.cg.shared.global [%7], [%8], 16;\n @b cp.async.ca.shared.global [%7], [%8], 8;\n cp.async.commit_group;}"
+                     ::"r"(t), "r"(n_tok), "r"(lane), "r"(put + o_k), "l"(pk), "r"(put + VEC * 4 + o_k), "l"(pq), "r"(put + o_x), "l"(px) : "memory");
+        pk += step_k; pq += step_k; px += step_x;
+        put += SLOT * 4; put = put == ring_z ? ring0 : put;
+    };
+    auto quarter = [](float* to, const float* from) {
+#pragma unroll
+        for (int i = 0; i < CW; i += 4) { const float4 v = *(const float4*)(from + i); to[i] = v.x; to[i + 1] = v.y; to[i + 2] = v.z; to[i + 3] = v.w; }
     };
     for (int t = 0; t < DEPTH - 1; ++t) fetch(t);
-    float po[CW];
+    float S[CW], qp[CW], k0[CW], k1[CW];
+    uint64_t P[CW];                          // (prediction product, read-out product) of a column
+    quarter(S, sg);
 #pragma unroll
-    for (int i = 0; i < CW; ++i) po[i] = 0.0f;
-#pragma unroll 1
-    for (int t = 0; t < n_tok; ++t) {
-        cp_async_wait<DEPTH - 2>();
+    for (int i = 0; i < CW; ++i) qp[i] = 0.0f;
+    cp_async_wait<DEPTH - 2>();
+    __syncwarp();
+    const float* cur = ring_all[wid][0];
+    quarter(k0, cur + part * QS);
+    float v = cur[2 * VEC + r], g = cur[2 * VEC + 8], b = cur[2 * VEC + 9], d = 0.0f;
+    float* o = out + ((size_t)s * n_tok * n_v + h) * SK + j;          // the read-out that is written next
+    const int step_o = n_v * SK;
+    auto write = [&](int t, float x) {
+        asm volatile("{.reg .pred p;\n setp.ge.s32 p, %0, 0;\n setp.eq.and.s32 p, %1, 0, p;\n @p st.global.f32 [%2], %3;}" ::"r"(t), "r"(part), "l"(o), "f"(x) : "memory");
+        o = t >= 0 ? o + step_o : o;
+    };
+    auto pair = [](float lo, float hi) { uint64_t p; asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi)); return p; };
+    auto add2 = [](uint64_t& acc, uint64_t p) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(p)); };
+    auto hand = [&](uint64_t& acc, int ph) {             // lane ph of a row hands both sums to the row's other lanes
+        float lo, hi;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+        acc = pair(__shfl_sync(0xffffffffu, lo, (lane & ~3) | ph), __shfl_sync(0xffffffffu, hi, (lane & ~3) | ph));
+    };
+    auto add = [&](uint64_t& acc, int ph) {
+#pragma unroll
+        for (int i = 0; i < CW; ++i) add2(acc, P[i]);
+        hand(acc, ph);
+    };
+    // Token t, its keys in kk (the token before's in kp, which takes the next token's). first: there is no token before.
+    auto token = [&](int t, float* kk, float* kp, bool first) {
+        uint64_t acc = pair(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < CW; ++i) {
+            float po = 0.0f;
+            if (!first) { S[i] = S[i] + kp[i] * d; po = S[i] * qp[i]; }
+            S[i] = S[i] * g;
+            P[i] = pair(S[i] * kk[i], po);
+            add2(acc, P[i]);
+        }
+        hand(acc, 0);
+        fetch(t + DEPTH - 1);                // refills the slot token t - 1 used: every lane has its values (the shuffles)
+        add(acc, 1);
+        quarter(qp, cur + VEC + part * QS);
+        cp_async_wait<DEPTH - 2>();          // token t + 1 is there (after the last token: stale values nothing uses)
         __syncwarp();
-        fetch(t + DEPTH - 1);            // refills the slot token t-1 used: every lane is past it (the __syncwarp above)
-        const float* slot = ring_all[wid][t % DEPTH];
-        const float v = slot[2 * SK + r], g = slot[2 * SK + 8], b = slot[2 * SK + 9];
-        float kk[CW], pr[CW];
+        cur = cur == ring_all[wid][DEPTH - 1] ? ring_all[wid][0] : cur + SLOT;
+        const float vn = cur[2 * VEC + r], gn = cur[2 * VEC + 8], bn = cur[2 * VEC + 9];
+        add(acc, 2);
+        quarter(kp, cur + part * QS);
+        add(acc, 3);
+        float run, runo;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(run), "=f"(runo) : "l"(acc));
+        write(t - 1, runo);
+        d = b * (v - run);
+        v = vn; g = gn; b = bn;
+    };
+    token(0, k0, k1, true);
+    int t = 1;
+#pragma unroll 1
+    for (; t + 1 < n_tok; t += 2) { token(t, k1, k0, false); token(t + 1, k0, k1, false); }
+    if (t < n_tok) {
+        token(t, k1, k0, false);
 #pragma unroll
-        for (int i = 0; i < CW; i += 4) {
-            const float4 k4 = *(const float4*)(slot + part * CW + i);
-            kk[i] = k4.x; kk[i + 1] = k4.y; kk[i + 2] = k4.z; kk[i + 3] = k4.w;
-        }
-#pragma unroll
-        for (int i = 0; i < CW; ++i) { S[i] = S[i] * g; pr[i] = S[i] * kk[i]; }
-        // Two serial sums side by side: this token's prediction (needed before the state can move on) and the
-        // PREVIOUS token's read-out, whose products po were formed last trip. They do not depend on each other,
-        // so their adds interleave and the second chain's latency disappears behind the first.
-        float run = 0.0f, runo = 0.0f;
-#pragma unroll
-        for (int ph = 0; ph < 4; ++ph) {
-            float a = run, c = runo;
-#pragma unroll
-            for (int i = 0; i < CW; ++i) { a += pr[i]; c += po[i]; }
-            run = __shfl_sync(0xffffffffu, a, (lane & ~3) | ph);
-            runo = __shfl_sync(0xffffffffu, c, (lane & ~3) | ph);
-        }
-        if (part == 0 && t > 0) out[(((size_t)s * n_tok + t - 1) * n_v + h) * SK + j] = runo;
-        const float d = b * (v - run);
-#pragma unroll
-        for (int i = 0; i < CW; i += 4) {
-            const float4 q4 = *(const float4*)(slot + SK + part * CW + i);
-            S[i] = S[i] + kk[i] * d; po[i] = S[i] * q4.x;
-            S[i + 1] = S[i + 1] + kk[i + 1] * d; po[i + 1] = S[i + 1] * q4.y;
-            S[i + 2] = S[i + 2] + kk[i + 2] * d; po[i + 2] = S[i + 2] * q4.z;
-            S[i + 3] = S[i + 3] + kk[i + 3] * d; po[i + 3] = S[i + 3] * q4.w;
-        }
+        for (int i = 0; i < CW; ++i) k0[i] = k1[i];
     }
-    {
-        float runo = 0.0f;                  // read-out of the last token
+    float runo = 0.0f;                       // the last token's update and read-out
 #pragma unroll
-        for (int ph = 0; ph < 4; ++ph) {
-            float c = runo;
+    for (int i = 0; i < CW; ++i) { S[i] = S[i] + k0[i] * d; qp[i] = S[i] * qp[i]; }
+    for (int ph = 0; ph < 4; ++ph) {
 #pragma unroll
-            for (int i = 0; i < CW; ++i) c += po[i];
-            runo = __shfl_sync(0xffffffffu, c, (lane & ~3) | ph);
-        }
-        if (part == 0 && n_tok > 0) out[(((size_t)s * n_tok + n_tok - 1) * n_v + h) * SK + j] = runo;
+        for (int i = 0; i < CW; ++i) runo += qp[i];
+        runo = __shfl_sync(0xffffffffu, runo, (lane & ~3) | ph);
     }
+    write(n_tok - 1, runo);
     cp_async_wait<0>();
 #pragma unroll
     for (int i = 0; i < CW; i += 4) *(float4*)(sg + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+}
+// One token per sequence (a batched decode step): the state passes through once, 8 rows (4 KB in a piece) to a warp, and memory bounds
+// it -- so it moves as whole 16-byte spans in address order through shared memory (quarters CW + 4 floats apart, as above), with
+// registers for several blocks an SM; the scan above, at one block's registers and 16 bytes of every 128 to a lane, took 53 us for 32
+// sequences of 32 heads against 26 us here (134 MB: 20 us at copy speed). Same sums, same order.
+template <int SK>
+__global__ void __launch_bounds__(128, 4) k_gdn_step(const float* qh, const float* kh, const float* vh, const float* gb, int n_k, int n_v, float* state, size_t state_stride, float* out) {
+    constexpr int CW = SK / 4, QS = CW + 4, VEC = 4 * QS;
+    __shared__ __align__(16) float st_all[4][8 * VEC], kq_all[4][2 * VEC];
+    const int h = blockIdx.x, s = blockIdx.z, khd = h % n_k, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int r = lane >> 2, part = lane & 3, j0 = blockIdx.y * 32 + wid * 8;
+    float* st = st_all[wid]; float* kq = kq_all[wid];
+    float* sg = state + (size_t)s * state_stride + ((size_t)h * SK + j0) * SK;
+    auto at = [](int e) { return (e / CW) * QS + e % CW; };                // element e of a warp's rows, or of k or q
+#pragma unroll
+    for (int i = 0; i < SK / 16; ++i) cp_async16(st + at((i * 32 + lane) * 4), sg + (i * 32 + lane) * 4, true);
+    if (lane * 4 < SK) {
+        cp_async16(kq + at(lane * 4), kh + ((size_t)s * n_k + khd) * SK + lane * 4, true);
+        cp_async16(kq + VEC + at(lane * 4), qh + ((size_t)s * n_k + khd) * SK + lane * 4, true);
+    }
+    cp_async_commit();
+    const float v = vh[((size_t)s * n_v + h) * SK + j0 + r], g = gb[((size_t)s * n_v + h) * 2], b = gb[((size_t)s * n_v + h) * 2 + 1];
+    cp_async_wait<0>();
+    __syncwarp();
+    float S[CW], pr[CW];
+    float* mine = st + r * VEC + part * QS; const float* k = kq + part * QS; const float* q = k + VEC;
+#pragma unroll
+    for (int i = 0; i < CW; i += 4) {
+        const float4 x = *(const float4*)(mine + i), kv = *(const float4*)(k + i);
+        S[i] = x.x * g; S[i + 1] = x.y * g; S[i + 2] = x.z * g; S[i + 3] = x.w * g;
+        pr[i] = S[i] * kv.x; pr[i + 1] = S[i + 1] * kv.y; pr[i + 2] = S[i + 2] * kv.z; pr[i + 3] = S[i + 3] * kv.w;
+    }
+    auto fold = [&] {
+        float run = 0.0f;
+#pragma unroll
+        for (int ph = 0; ph < 4; ++ph) {
+            float a = run;
+#pragma unroll
+            for (int i = 0; i < CW; ++i) a += pr[i];
+            run = __shfl_sync(0xffffffffu, a, (lane & ~3) | ph);
+        }
+        return run;
+    };
+    const float d = b * (v - fold());
+#pragma unroll
+    for (int i = 0; i < CW; i += 4) {
+        const float4 kv = *(const float4*)(k + i), qv = *(const float4*)(q + i);
+        float4 x;
+        x.x = S[i] + kv.x * d; x.y = S[i + 1] + kv.y * d; x.z = S[i + 2] + kv.z * d; x.w = S[i + 3] + kv.w * d;
+        pr[i] = x.x * qv.x; pr[i + 1] = x.y * qv.y; pr[i + 2] = x.z * qv.z; pr[i + 3] = x.w * qv.w;
+        *(float4*)(mine + i) = x;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < SK / 16; ++i) *(float4*)(sg + (i * 32 + lane) * 4) = *(const float4*)(st + at((i * 32 + lane) * 4));
+    const float o = fold();
+    if (part == 0) out[((size_t)s * n_v + h) * SK + j0 + r] = o;
 }
 
 // Gated RMSNorm of the recurrence's output, the SiLU(z) gate and the Q8_0 quantisation of the result
