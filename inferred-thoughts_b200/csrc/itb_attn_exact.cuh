@@ -6,14 +6,16 @@
 // per softmax sum, n_pos multiply-adds per output) one thread each. Selected by exact=1; exact=0 keeps the split-K kernels,
 // which reassociate the sums (tolerance class) and are faster at long contexts.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 #include "itb_kernels.cuh"
 #include "itb_tile.cuh"
 
 namespace {
 
-constexpr int AX_TP = 64;          // positions per block of the scores kernel
+constexpr int AX_TP = 32;          // positions per tile of the scores kernel
 constexpr int AX_QSTRIDE_PAD = 4;  // q rows in shared memory are head_dim + 4 floats apart: the heads of a group hit different banks
+constexpr int AX_KPAD = 8;         // key rows in shared memory are head_dim + 8 elements apart: so do a warp's positions
 
 __device__ __forceinline__ float kv_elem(uint32_t word, int hi, int bf16) {
     const uint16_t h = (uint16_t)(word >> (hi * 16));
@@ -21,7 +23,10 @@ __device__ __forceinline__ float kv_elem(uint32_t word, int hi, int bf16) {
 }
 
 // scores[row][head][s] = (sum_i q[i] * k_s[i], i ascending) * scale for s < n_pos(row).
-// grid (ceil(n_pos_max / AX_TP), n_head_kv, rows); block AX_TP * group threads: thread = (position in tile, head of the group).
+// grid (blocks that share a row's position tiles, n_head_kv, rows); block AX_TP * group threads: thread = (position in tile, head of
+// the group). A tile's keys arrive in shared memory as one copy, the next tile's while this one's chains run (read by each chain as it
+// goes they cost a memory round trip per 16 dimensions), and a row has only as many blocks as fill the machine: a block per tile of the
+// whole context cost 24 us a layer at 32 sequences of 130 positions, most of it blocks that leave at once; now 8.9.
 struct AxScores {
     const float* q; const uint16_t* kslab; size_t slab_stride; int rows_per_seq;   // q [rows][n_head][hd]; row r reads the slab of sequence r / rows_per_seq
     const int* n_pos_dev; int n_pos_last, n_q;                                      // per-row positions, or n_pos_last - n_q + 1 + row
@@ -30,112 +35,197 @@ struct AxScores {
 };
 __global__ void k_attn_scores_exact(AxScores p) {
     extern __shared__ __align__(16) unsigned char smem[];
+    const int hk = blockIdx.y, r = blockIdx.z, hd = p.hd, group = p.n_head / p.n_head_kv, qst = hd + AX_QSTRIDE_PAD, kst = hd + AX_KPAD;
     float* qs = (float*)smem;                                    // [group][hd + pad]
-    const int hk = blockIdx.y, r = blockIdx.z, hd = p.hd, group = p.n_head / p.n_head_kv, qst = hd + AX_QSTRIDE_PAD;
+    uint16_t* ks = (uint16_t*)(qs + group * qst);                // [2][AX_TP][hd + pad]
     pdl_trigger(); pdl_wait();
     const int n_pos = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
-    const int p0 = blockIdx.x * AX_TP;
-    if (p0 >= n_pos) return;
+    const int n_tiles = (n_pos + AX_TP - 1) / AX_TP, cpr = hd / 8;
+    if ((int)blockIdx.x >= n_tiles) return;
+    const uint16_t* kbase = p.kslab + (size_t)(r / max(1, p.rows_per_seq)) * p.slab_stride + hk * hd;
+    auto fetch = [&](int t, int buf) {
+        if (t < n_tiles) {
+            const int p0 = t * AX_TP, np = min(AX_TP, n_pos - p0);
+            for (int i = threadIdx.x; i < np * cpr; i += blockDim.x)
+                cp_async16(ks + (buf * AX_TP + i / cpr) * kst + (i % cpr) * 8, kbase + (size_t)(p0 + i / cpr) * p.kv_dim + (i % cpr) * 8, true);
+        }
+        cp_async_commit();
+    };
+    fetch(blockIdx.x, 0);
     for (int i = threadIdx.x; i < group * hd; i += blockDim.x)
         qs[(i / hd) * qst + i % hd] = p.q[((size_t)r * p.n_head + hk * group) * hd + i];
-    __syncthreads();
-    const int g = threadIdx.x % group, s = p0 + threadIdx.x / group;
-    if (s >= n_pos) return;
-    const uint16_t* key = p.kslab + (size_t)(r / max(1, p.rows_per_seq)) * p.slab_stride + (size_t)s * p.kv_dim + hk * hd;
+    const int g = threadIdx.x % group, sl = threadIdx.x / group;
     const float* qg = qs + g * qst;
-    float dot = 0.0f;
-#pragma unroll 2
-    for (int i = 0; i < hd; i += 8) {
-        const uint4 kw = *(const uint4*)(key + i);
-        const float4 q0 = *(const float4*)(qg + i), q1 = *(const float4*)(qg + i + 4);
-        dot += q0.x * kv_elem(kw.x, 0, p.bf16); dot += q0.y * kv_elem(kw.x, 1, p.bf16);
-        dot += q0.z * kv_elem(kw.y, 0, p.bf16); dot += q0.w * kv_elem(kw.y, 1, p.bf16);
-        dot += q1.x * kv_elem(kw.z, 0, p.bf16); dot += q1.y * kv_elem(kw.z, 1, p.bf16);
-        dot += q1.z * kv_elem(kw.w, 0, p.bf16); dot += q1.w * kv_elem(kw.w, 1, p.bf16);
+    float* out = p.scores + ((size_t)r * p.n_head + hk * group + g) * p.s_stride;
+    int buf = 0;
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, buf ^= 1) {
+        fetch(t + gridDim.x, buf ^ 1);
+        cp_async_wait<1>();
+        __syncthreads();
+        const int s = t * AX_TP + sl;
+        if (s < n_pos) {
+            const uint16_t* key = ks + (buf * AX_TP + sl) * kst;
+            float dot = 0.0f;
+#pragma unroll 4
+            for (int i = 0; i < hd; i += 8) {
+                const uint4 kw = *(const uint4*)(key + i);
+                const float4 q0 = *(const float4*)(qg + i), q1 = *(const float4*)(qg + i + 4);
+                dot += q0.x * kv_elem(kw.x, 0, p.bf16); dot += q0.y * kv_elem(kw.x, 1, p.bf16);
+                dot += q0.z * kv_elem(kw.y, 0, p.bf16); dot += q0.w * kv_elem(kw.y, 1, p.bf16);
+                dot += q1.x * kv_elem(kw.z, 0, p.bf16); dot += q1.y * kv_elem(kw.z, 1, p.bf16);
+                dot += q1.z * kv_elem(kw.w, 0, p.bf16); dot += q1.w * kv_elem(kw.w, 1, p.bf16);
+            }
+            out[s] = dot * p.scale;
+        }
+        __syncthreads();                                         // the buffer is free for the tile after the next
     }
-    p.scores[((size_t)r * p.n_head + hk * group + g) * p.s_stride + s] = dot * p.scale;
+    cp_async_wait<0>();
+}
+// Blocks that share a row's tiles: two to an SM over all rows and KV heads.
+inline int attn_scores_blocks(int n_pos_max, int n_head_kv, int rows, int sms) {
+    const long long tiles = (n_pos_max + AX_TP - 1) / AX_TP, share = (2LL * sms + (long long)n_head_kv * rows - 1) / ((long long)n_head_kv * rows);
+    return (int)std::max(1LL, std::min(tiles, share));
 }
 
+// The serial sum of n floats of shared memory (16-byte aligned), by every lane of a warp alike. Read 32 ahead of the adds: the chain
+// of 4-cycle adds is all there is to wait for.
+__device__ __forceinline__ float serial_sum(const float* w, int n) {
+    float sum = 0.0f;
+    float4 a[8];
+    const int n32 = n & ~31;
+    if (n32 > 0)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = *(const float4*)(w + 4 * j);
+#pragma unroll 1
+    for (int s = 0; s < n32; s += 32) {
+        const float* nx = w + (s + 32 < n32 ? s + 32 : s);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 e = a[j];
+            a[j] = *(const float4*)(nx + 4 * j);
+            sum += e.x; sum += e.y; sum += e.z; sum += e.w;
+        }
+    }
+    for (int s = n32; s < n; ++s) sum += w[s];
+    return sum;
+}
 // Softmax of one (row, head)'s scores and the weighted sum of the values for 32 dimensions of that head.
-// grid (hd / 32, n_head, rows); block 256: everyone on the softmax, then warp 0 walks the positions (a lane per dimension, one
-// multiply-add chain each) over value tiles the other warps stage in shared memory one tile ahead.
+// grid (hd / 32, n_head, rows); block 288: everyone on the maximum, exponentials and divisions, warp 0 on the serial sums: of the
+// exponentials, then of the weighted values, a lane per dimension. Those two chains (n_pos adds of 4 cycles each) bound the kernel, so
+// the chain warp does nothing else: the other eight multiply a tile of AX_VT positions at a time into shared memory, a line per
+// dimension, one tile ahead of it and with the values of AX_AHEAD tiles in flight. With the chain warp converting and multiplying
+// too, and the sum read as it went, 6,500 positions took 124 us; now 46 (the chains alone: 31).
 // gate != null: times sigmoid(gate) (src/model/qwen35.rs:1216-1218); out_q != null: the result leaves quantised to Q8_0 (the
 // output projection's own quantisation), else as f32 in out.
-constexpr int AX_VT = 128;         // positions per staged value tile
+// READY (the scores already hold the softmax weights: many rows, where the blocks that share a head would each redo the softmax): no
+// weights in shared memory, so more blocks to an SM.
+// A value line's four 16-byte pieces go to neighbouring lanes (a lane per position touched 32 lines a load); the lines of each eight
+// dimensions start 8 floats further on, so that their products fall on distinct banks.
+constexpr int AX_VT = 128, AX_VLD = AX_VT + 4, AX_AHEAD = 4, AX_VBUF = 32 * AX_VLD + 32;
+constexpr int AX_OUT_SMEM = 226 * 1024;       // room for 49,408 positions
 struct AxOut {
     const float* scores; int s_stride;
     const uint16_t* vslab; size_t slab_stride; int rows_per_seq;
     const int* n_pos_dev; int n_pos_last, n_q;
     int kv_dim, hd, n_head, n_head_kv, bf16;
     const float* gate; float* out; int8_t* out_q; float* out_s;
-    int weights_ready;             // the scores buffer already holds the softmax weights (k_attn_softmax_exact ran): skip the softmax here
 };
-__global__ void __launch_bounds__(256) k_attn_out_exact(AxOut p) {
+template <bool READY>
+__global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float s_red[8];
+    __shared__ float s_red[9];
     __shared__ float s_sum;
     const int j = blockIdx.x, h = blockIdx.y, r = blockIdx.z, hd = p.hd, group = p.n_head / p.n_head_kv, hk = h / group;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     pdl_trigger(); pdl_wait();
     const int n_pos = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
-    float* w = (float*)smem;                                      // [n_pos] scores -> exponentials -> weights
-    uint16_t* vt = (uint16_t*)(w + ((n_pos + 3) & ~3));           // [2][AX_VT][32]
+    float* prod = (float*)smem;                                   // [2][32][AX_VLD]
+    float* w = prod + 2 * AX_VBUF;                                // [n_pos] scores -> exponentials -> weights
     const float* sc = p.scores + ((size_t)r * p.n_head + h) * p.s_stride;
-    const uint16_t* vbase = p.vslab + (size_t)(r / max(1, p.rows_per_seq)) * p.slab_stride + hk * hd + j * 32;
-    auto stage = [&](int tile) {                                  // warps 1..7: tile `tile` of the values into its buffer
-        const int s0 = tile * AX_VT, ns = min(AX_VT, n_pos - s0);
-        uint16_t* dst = vt + (tile & 1) * AX_VT * 32;
-        for (int i = tid - 32; i < ns * 4; i += 224) {            // 4 x 16 bytes per position
-            const int s = i >> 2, q = i & 3;
-            *(uint4*)(dst + s * 32 + q * 8) = *(const uint4*)(vbase + (size_t)(s0 + s) * p.kv_dim + q * 8);
+    const size_t idx = ((size_t)r * p.n_head + h) * hd + j * 32 + lane;
+    const float gate = p.gate && wid == 0 ? p.gate[idx] : 0.0f;
+    const int n_tiles = (n_pos + AX_VT - 1) / AX_VT;
+    // warps 1..8: 16 positions of each tile, a lane 8 dimensions of two of them
+    const int vs = (wid - 1) * 16 + (lane >> 2), q = lane & 3;
+    const uint16_t* vbase = p.vslab + (size_t)(r / max(1, p.rows_per_seq)) * p.slab_stride + hk * hd + j * 32 + q * 8;
+    uint4 v[AX_AHEAD][2];
+    float vw[AX_AHEAD][2];
+    auto load = [&](int t, uint4* to, float* wt) {
+        if (t < n_tiles) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int s = min(t * AX_VT + vs + 8 * i, n_pos - 1);
+                to[i] = *(const uint4*)(vbase + (size_t)s * p.kv_dim);
+                if (READY) wt[i] = sc[s];
+            }
         }
     };
-    if (wid > 0 && n_pos > 0) stage(0);
-    if (p.weights_ready) {
-        for (int s = tid; s < n_pos; s += 256) w[s] = sc[s];
-    } else {
+    auto multiply = [&](int t, const uint4* x, const float* wt) {
+        float* d = prod + (t & 1) * AX_VBUF + q * 8 * (AX_VLD + 1) + vs;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int s = t * AX_VT + vs + 8 * i;
+            if (s < n_pos) {
+                const float ws = READY ? wt[i] : w[s];
+                const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+                if (p.bf16)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) d[k * AX_VLD + 8 * i] = ws * kv_elem(u[k >> 1], k & 1, 1);
+                else
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) d[k * AX_VLD + 8 * i] = ws * kv_elem(u[k >> 1], k & 1, 0);
+            }
+        }
+    };
+    if (wid > 0)
+#pragma unroll
+        for (int t = 0; t < AX_AHEAD; ++t) load(t, v[t], vw[t]);
+    if (!READY) {
         float mx = -INFINITY;
-        for (int s = tid; s < n_pos; s += 256) { const float v = sc[s]; w[s] = v; mx = fmaxf(mx, v); }
+#pragma unroll 4
+        for (int s = tid; s < n_pos; s += 288) { const float x = sc[s]; w[s] = x; mx = fmaxf(mx, x); }
         mx = warp_max(mx);
         if (lane == 0) s_red[wid] = mx;
         __syncthreads();
         mx = s_red[0];
-        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_red[k]);
-        for (int s = tid; s < n_pos; s += 256) w[s] = exp_f(w[s] - mx);
+        for (int k = 1; k < 9; ++k) mx = fmaxf(mx, s_red[k]);
+#pragma unroll 2
+        for (int s = tid; s < n_pos; s += 288) w[s] = exp_f(w[s] - mx);
         __syncthreads();
-        if (tid == 0) {                                               // the sum in position order
-            float sum = 0.0f;
-            int s = 0;
-            for (; s + 4 <= n_pos; s += 4) { const float4 e = *(const float4*)(w + s); sum += e.x; sum += e.y; sum += e.z; sum += e.w; }
-            for (; s < n_pos; ++s) sum += w[s];
-            s_sum = sum;
+        if (wid == 0) {                                               // the sum in position order
+            const float sum = serial_sum(w, n_pos);
+            if (lane == 0) s_sum = sum;
         }
         __syncthreads();
-        {
-            const float sum = s_sum;
-            for (int s = tid; s < n_pos; s += 256) w[s] /= sum;
-        }
+        const float sum = s_sum;
+#pragma unroll 2
+        for (int s = tid; s < n_pos; s += 288) w[s] /= sum;
+        __syncthreads();
     }
-    __syncthreads();
     float o = 0.0f;
-    const int n_tiles = (n_pos + AX_VT - 1) / AX_VT;
-    for (int t = 0; t < n_tiles; ++t) {
-        if (wid > 0) { if (t + 1 < n_tiles) stage(t + 1); }
-        else {
-            const int s0 = t * AX_VT, ns = min(AX_VT, n_pos - s0);
-            const uint16_t* src = vt + (t & 1) * AX_VT * 32 + lane;
-            const float* ws = w + s0;
-#pragma unroll 8
-            for (int s = 0; s < ns; ++s) {
-                const uint16_t hb = src[s * 32];
-                o += ws[s] * (p.bf16 ? bf16_bits_to_f32(hb) : f16_bits_to_f32(hb));
+    if (wid > 0 && n_pos > 0) { multiply(0, v[0], vw[0]); load(AX_AHEAD, v[0], vw[0]); }
+    __syncthreads();
+    for (int t0 = 0; t0 < n_tiles; t0 += AX_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < AX_AHEAD; ++u) {
+            const int t = t0 + u;
+            if (t < n_tiles) {
+                if (wid > 0) {
+                    if (t + 1 < n_tiles) { multiply(t + 1, v[(u + 1) % AX_AHEAD], vw[(u + 1) % AX_AHEAD]); load(t + 1 + AX_AHEAD, v[(u + 1) % AX_AHEAD], vw[(u + 1) % AX_AHEAD]); }
+                } else {
+                    const float* x = prod + (t & 1) * AX_VBUF + lane * AX_VLD + (lane >> 3) * 8;
+                    const int ns = n_pos - t * AX_VT;
+                    if (ns >= AX_VT) {
+#pragma unroll
+                        for (int s = 0; s < AX_VT; s += 4) { const float4 e = *(const float4*)(x + s); o += e.x; o += e.y; o += e.z; o += e.w; }
+                    } else for (int s = 0; s < ns; ++s) o += x[s];
+                }
+                __syncthreads();
             }
         }
-        __syncthreads();
     }
     if (wid == 0) {
-        const size_t idx = ((size_t)r * p.n_head + h) * hd + j * 32 + lane;
-        if (p.gate) o *= sigmoid_f(p.gate[idx]);
+        if (p.gate) o *= sigmoid_f(gate);
         if (p.out_q) {
             float dq;
             const int8_t q = warp_quant_q8(o, &dq);
@@ -165,12 +255,9 @@ __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
     for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_red[k]);
     for (int s = tid; s < n_pos; s += 256) w[s] = exp_f(w[s] - mx);
     __syncthreads();
-    if (tid == 0) {
-        float sum = 0.0f;
-        int s = 0;
-        for (; s + 4 <= n_pos; s += 4) { const float4 e = *(const float4*)(w + s); sum += e.x; sum += e.y; sum += e.z; sum += e.w; }
-        for (; s < n_pos; ++s) sum += w[s];
-        s_sum = sum;
+    if (wid == 0) {
+        const float sum = serial_sum(w, n_pos);
+        if (lane == 0) s_sum = sum;
     }
     __syncthreads();
     const float sum = s_sum;
@@ -278,7 +365,7 @@ __global__ void __launch_bounds__(256, 2) k_attn_scores_tile(AxScores p) {
         for (int j = 0; j < 4; ++j) if (p0 + tx + 16 * j < np) out[16 * j] = acc[i][j] * p.scale;
     }
 }
-// The weighted values from the softmax weights (weights_ready), 64 dimensions of a head to a block; gate and Q8_0 as in k_attn_out_exact.
+// The weighted values from the softmax weights, 64 dimensions of a head to a block; gate and Q8_0 as in k_attn_out_exact.
 // Positions past a row's own take no part in its chain: the tiles that all of a block's rows span go unguarded, the few after them by
 // a select. grid (hd / 64, n_head_kv, sequences * token tiles), block 256; s_stride a multiple of 4.
 template <int MR, bool BF>
@@ -394,7 +481,7 @@ static void attn_exact_tiles(const AxScores& a, const AxSoft& sm, const AxOut& o
     else if (a.bf16) run(k_attn_scores_tile<4, true>, k_attn_out_tile<4, true>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
     else run(k_attn_scores_tile<4, false>, k_attn_out_tile<4, false>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
 }
-inline size_t attn_out_exact_smem(int n_pos_max) { return (size_t)((n_pos_max + 3) & ~3) * 4 + 2 * AX_VT * 32 * 2; }
-inline size_t attn_scores_exact_smem(int hd, int group) { return (size_t)group * (hd + AX_QSTRIDE_PAD) * 4; }
+inline size_t attn_out_exact_smem(int n_pos_max, bool ready = false) { return (ready ? 0 : (size_t)((n_pos_max + 3) & ~3) * 4) + 2 * AX_VBUF * 4; }
+inline size_t attn_scores_exact_smem(int hd, int group) { return (size_t)group * (hd + AX_QSTRIDE_PAD) * 4 + (size_t)2 * AX_TP * (hd + AX_KPAD) * 2; }
 
 }  // namespace

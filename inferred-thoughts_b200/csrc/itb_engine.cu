@@ -734,7 +734,7 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
     const itb_model_dims& d = e->m->d;
     const int hd = d.head_dim, group = d.n_head / d.n_head_kv, kvd = hd * d.n_head_kv;
     static bool attr = false;
-    if (!attr) { set_smem((const void*)k_attn_out_exact, 200 * 1024); attr = true; }
+    if (!attr) { set_smem((const void*)k_attn_out_exact<false>, AX_OUT_SMEM); set_smem((const void*)k_attn_scores_exact, 64 * 1024); attr = true; }
     AxScores a{};
     a.q = e->qn; a.kslab = kslab; a.slab_stride = slab_stride; a.rows_per_seq = rows_per_seq; a.n_pos_dev = e->npos; a.kv_dim = kvd; a.hd = hd;
     a.n_head = d.n_head; a.n_head_kv = d.n_head_kv; a.scale = 1.0f / sqrtf((float)hd); a.bf16 = e->c->kv_bf16; a.scores = e->scores; a.s_stride = (int)scores_stride(e);
@@ -744,19 +744,19 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
     o.kv_dim = kvd; o.hd = hd; o.n_head = d.n_head; o.n_head_kv = d.n_head_kv; o.bf16 = e->c->kv_bf16; o.gate = e->gate; o.out_q = e->aq; o.out_s = e->as;
     const int n_seq = rows / std::max(1, rows_per_seq);
     if (const int mr = attn_tile_rows(rows_per_seq, n_seq, hd, d.n_head, d.n_head_kv, e->c->sm_count)) {
-        o.weights_ready = 1;
         attn_exact_tiles(a, sm, o, mr, n_seq, rows, n_pos_max, [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { launch_k(pdl, k, g, b, smem, st, arg); });
         return;
     }
-    launch_k(pdl, k_attn_scores_exact, dim3((n_pos_max + AX_TP - 1) / AX_TP, d.n_head_kv, rows), dim3(AX_TP * group), attn_scores_exact_smem(hd, group), st, a);
+    launch_k(pdl, k_attn_scores_exact, dim3(attn_scores_blocks(n_pos_max, d.n_head_kv, rows, e->c->sm_count), d.n_head_kv, rows), dim3(AX_TP * group), attn_scores_exact_smem(hd, group), st, a);
     if (rows >= 8) {
         // many rows: the softmax once per (row, head), in place, instead of once per block of the weighted-value kernel
         static bool attr2 = false;
         if (!attr2) { set_smem((const void*)k_attn_softmax_exact, 200 * 1024); attr2 = true; }
         launch_k(pdl, k_attn_softmax_exact, dim3(d.n_head, rows), dim3(256), (size_t)((n_pos_max + 3) & ~3) * 4, st, sm);
-        o.weights_ready = 1;
+        launch_k(pdl, k_attn_out_exact<true>, dim3(hd / 32, d.n_head, rows), dim3(288), attn_out_exact_smem(n_pos_max, true), st, o);
+        return;
     }
-    launch_k(pdl, k_attn_out_exact, dim3(hd / 32, d.n_head, rows), dim3(256), attn_out_exact_smem(n_pos_max), st, o);
+    launch_k(pdl, k_attn_out_exact<false>, dim3(hd / 32, d.n_head, rows), dim3(288), attn_out_exact_smem(n_pos_max), st, o);
 }
 
 // One decode step for all B sequences, enqueued on `st`.

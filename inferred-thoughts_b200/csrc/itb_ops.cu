@@ -515,7 +515,7 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
         return;
     }
     if (c->exact && a->kv_dim % 8 == 0 && a->n_head / a->n_head_kv <= 8 && (a->head_dim == 64 || a->head_dim == 128 || a->head_dim == 256) &&
-        attn_out_exact_smem((int)a->n_pos) <= 200 * 1024) {
+        attn_out_exact_smem((int)a->n_pos) <= AX_OUT_SMEM) {
         // the CPU path's own order (src/ops/naive.rs:420-466): scores, then softmax and weighted values per 32 dimensions of a head
         const size_t s_stride = (a->n_pos + 3) & ~(size_t)3, need_s = n_q * a->n_head * s_stride;
         if (c->tmp_cap < need_s) {
@@ -533,17 +533,16 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
         op.n_pos_last = (int)a->n_pos; op.n_q = (int)n_q; op.kv_dim = (int)a->kv_dim; op.hd = (int)a->head_dim; op.n_head = (int)a->n_head;
         op.n_head_kv = (int)a->n_head_kv; op.bf16 = c->kv_bf16; op.gate = nullptr; op.out = od; op.out_q = nullptr; op.out_s = nullptr;
         if (const int mr = attn_tile_rows((int)n_q, 1, op.hd, op.n_head, op.n_head_kv, c->sm_count)) {
-            op.weights_ready = 1;
             attn_exact_tiles(sp, AxSoft{c->tmp_f32, (int)s_stride, nullptr, (int)a->n_pos, (int)n_q, (int)a->n_head}, op, mr, 1, (int)n_q, (int)a->n_pos,
                              [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { k<<<g, b, smem, c->stream>>>(arg); ITB_LAUNCHED(c); });
             return;
         }
-        k_attn_scores_exact<<<dim3((unsigned)((a->n_pos + AX_TP - 1) / AX_TP), (unsigned)a->n_head_kv, (unsigned)n_q), AX_TP * group,
+        k_attn_scores_exact<<<dim3((unsigned)attn_scores_blocks((int)a->n_pos, (int)a->n_head_kv, (int)n_q, c->sm_count), (unsigned)a->n_head_kv, (unsigned)n_q), AX_TP * group,
                               attn_scores_exact_smem((int)a->head_dim, group), c->stream>>>(sp);
         ITB_LAUNCHED(c);
         static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(k_attn_out_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr = true; }
-        k_attn_out_exact<<<dim3((unsigned)(a->head_dim / 32), (unsigned)a->n_head, (unsigned)n_q), 256, attn_out_exact_smem((int)a->n_pos), c->stream>>>(op);
+        if (!attr) { cudaFuncSetAttribute(k_attn_out_exact<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AX_OUT_SMEM); cudaFuncSetAttribute(k_attn_scores_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024); attr = true; }
+        k_attn_out_exact<false><<<dim3((unsigned)(a->head_dim / 32), (unsigned)a->n_head, (unsigned)n_q), 288, attn_out_exact_smem((int)a->n_pos), c->stream>>>(op);
         ITB_LAUNCHED(c);
         return;
     }
