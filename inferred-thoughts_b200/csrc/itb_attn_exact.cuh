@@ -87,15 +87,15 @@ inline int attn_scores_blocks(int n_pos_max, int n_head_kv, int rows, int sms) {
     return (int)std::max(1LL, std::min(tiles, share));
 }
 
-// The serial sum of n floats of shared memory (16-byte aligned), by every lane of a warp alike. Read 32 ahead of the adds: the chain
-// of 4-cycle adds is all there is to wait for.
+// The serial sum of n floats of shared memory (16-byte aligned, zeros up to a multiple of 32), by every lane of a warp alike. Read 32
+// ahead of the adds: the chain of 4-cycle adds is all there is to wait for.
+__host__ __device__ constexpr int ax_pad(int n) { return (n + 31) & ~31; }
 __device__ __forceinline__ float serial_sum(const float* w, int n) {
     float sum = 0.0f;
     float4 a[8];
-    const int n32 = n & ~31;
-    if (n32 > 0)
+    const int n32 = ax_pad(n);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = *(const float4*)(w + 4 * j);
+    for (int j = 0; j < 8; ++j) a[j] = *(const float4*)(w + 4 * j);
 #pragma unroll 1
     for (int s = 0; s < n32; s += 32) {
         const float* nx = w + (s + 32 < n32 ? s + 32 : s);
@@ -106,7 +106,6 @@ __device__ __forceinline__ float serial_sum(const float* w, int n) {
             sum += e.x; sum += e.y; sum += e.z; sum += e.w;
         }
     }
-    for (int s = n32; s < n; ++s) sum += w[s];
     return sum;
 }
 // Softmax of one (row, head)'s scores and the weighted sum of the values for 32 dimensions of that head.
@@ -165,15 +164,12 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int s = t * AX_VT + vs + 8 * i;
-            if (s < n_pos) {
-                const float ws = READY ? wt[i] : w[s];
-                const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-                if (p.bf16)
+            const float ws = s >= n_pos ? 0.0f : READY ? wt[i] : w[s];
+            const uint32_t u[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) d[k * AX_VLD + 8 * i] = ws * kv_elem(u[k >> 1], k & 1, 1);
-                else
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) d[k * AX_VLD + 8 * i] = ws * kv_elem(u[k >> 1], k & 1, 0);
+            for (int k = 0; k < 8; ++k) {
+                const float y = p.bf16 ? kv_elem(u[k >> 1], k & 1, 1) : kv_elem(u[k >> 1], k & 1, 0);
+                d[k * AX_VLD + 8 * i] = s < n_pos ? ws * y : -0.0f;      // past the end: a term that changes no sum
             }
         }
     };
@@ -190,7 +186,7 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
         mx = s_red[0];
         for (int k = 1; k < 9; ++k) mx = fmaxf(mx, s_red[k]);
 #pragma unroll 2
-        for (int s = tid; s < n_pos; s += 288) w[s] = exp_f(w[s] - mx);
+        for (int s = tid; s < ax_pad(n_pos); s += 288) w[s] = s < n_pos ? exp_f(w[s] - mx) : 0.0f;
         __syncthreads();
         if (wid == 0) {                                               // the sum in position order
             const float sum = serial_sum(w, n_pos);
@@ -214,11 +210,14 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
                     if (t + 1 < n_tiles) { multiply(t + 1, v[(u + 1) % AX_AHEAD], vw[(u + 1) % AX_AHEAD]); load(t + 1 + AX_AHEAD, v[(u + 1) % AX_AHEAD], vw[(u + 1) % AX_AHEAD]); }
                 } else {
                     const float* x = prod + (t & 1) * AX_VBUF + lane * AX_VLD + (lane >> 3) * 8;
-                    const int ns = n_pos - t * AX_VT;
-                    if (ns >= AX_VT) {
+                    if (n_pos - t * AX_VT > AX_VT - 32) {
 #pragma unroll
                         for (int s = 0; s < AX_VT; s += 4) { const float4 e = *(const float4*)(x + s); o += e.x; o += e.y; o += e.z; o += e.w; }
-                    } else for (int s = 0; s < ns; ++s) o += x[s];
+                    } else
+#pragma unroll 1
+                        for (int s0 = 0; s0 < n_pos - t * AX_VT; s0 += 32)
+#pragma unroll
+                            for (int s = s0; s < s0 + 32; s += 4) { const float4 e = *(const float4*)(x + s); o += e.x; o += e.y; o += e.z; o += e.w; }
                 }
                 __syncthreads();
             }
@@ -253,7 +252,7 @@ __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
     __syncthreads();
     mx = s_red[0];
     for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_red[k]);
-    for (int s = tid; s < n_pos; s += 256) w[s] = exp_f(w[s] - mx);
+    for (int s = tid; s < ax_pad(n_pos); s += 256) w[s] = s < n_pos ? exp_f(w[s] - mx) : 0.0f;
     __syncthreads();
     if (wid == 0) {
         const float sum = serial_sum(w, n_pos);
@@ -467,7 +466,7 @@ inline int attn_tile_rows(int rows_per_seq, int n_seq, int hd, int n_head, int n
 template <class L>
 static void attn_exact_tiles(const AxScores& a, const AxSoft& sm, const AxOut& o, int mr, int n_seq, int rows, int n_pos_max, L&& launch) {
     const int group = a.n_head / a.n_head_kv, tt = 16 * mr / group, z = n_seq * ((a.rows_per_seq + tt - 1) / tt);
-    const size_t soft = (size_t)((n_pos_max + 3) & ~3) * 4;
+    const size_t soft = (size_t)ax_pad(n_pos_max) * 4;
     auto run = [&](auto scores, auto out, size_t scores_smem, size_t out_smem) {
         cudaFuncSetAttribute(scores, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scores_smem);
         cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
@@ -481,7 +480,7 @@ static void attn_exact_tiles(const AxScores& a, const AxSoft& sm, const AxOut& o
     else if (a.bf16) run(k_attn_scores_tile<4, true>, k_attn_out_tile<4, true>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
     else run(k_attn_scores_tile<4, false>, k_attn_out_tile<4, false>, attn_scores_tile_smem<4>(), attn_out_tile_smem<4>());
 }
-inline size_t attn_out_exact_smem(int n_pos_max, bool ready = false) { return (ready ? 0 : (size_t)((n_pos_max + 3) & ~3) * 4) + 2 * AX_VBUF * 4; }
+inline size_t attn_out_exact_smem(int n_pos_max, bool ready = false) { return (ready ? 0 : (size_t)ax_pad(n_pos_max) * 4) + 2 * AX_VBUF * 4; }
 inline size_t attn_scores_exact_smem(int hd, int group) { return (size_t)group * (hd + AX_QSTRIDE_PAD) * 4 + (size_t)2 * AX_TP * (hd + AX_KPAD) * 2; }
 
 }  // namespace

@@ -272,11 +272,12 @@ extern "C" int itb_model_synth_read(itb_model* m, uint64_t seed, const char* nam
     return 0;
 }
 
-// w[n_out][n_in] -> units of 32 rows, k-major inside a unit: wt[(u * n_in + k) * 32 + r] = w[u * 32 + r][k] (zero past n_out).
-__global__ void k_f32_kmajor(const float* w, int n_in, int n_out, float* wt) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)((n_out + 31) / 32) * n_in * 32;
+// w[n_out][n_in] -> units of F32S_ROWS rows, four k of a row together: wt[((u * n_in + k) / 4) * 4 * F32S_ROWS + r * 4 + k % 4] =
+// w[u * F32S_ROWS + r][k], n_in a multiple of 4 (zero past n_out).
+__global__ void k_f32_units(const float* w, int n_in, int n_out, float* wt) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)((n_out + F32S_ROWS - 1) / F32S_ROWS) * n_in * F32S_ROWS;
     if (i >= total) return;
-    const int r = (int)(i % 32); const size_t uk = i / 32; const int k = (int)(uk % n_in), u = (int)(uk / n_in), row = u * 32 + r;
+    const int r = (int)(i / 4 % F32S_ROWS), k = (int)(i / (4 * F32S_ROWS) * 4 % n_in + i % 4), row = (int)(i / F32S_ROWS / n_in) * F32S_ROWS + r;
     wt[i] = row < n_out ? w[(size_t)row * n_in + k] : 0.0f;
 }
 static bool finalize(itb_model* m) {
@@ -291,14 +292,14 @@ static bool finalize(itb_model* m) {
     };
     auto q8 = [&](const std::string& n) { const DevTensor* t = get(n); return t ? DevQ8{(const int8_t*)t->a, (const uint16_t*)t->b, (int)t->n_in, (int)t->n_out} : DevQ8{}; };
     auto f32 = [&](const std::string& n) { const DevTensor* t = get(n); return t ? DevF32{(const float*)t->a, (int)t->n_in, (int)t->n_out} : DevF32{}; };
-    // the small F32 matrices of the one-token step (router, shared-expert gate, alpha, beta) also k-major, for the serial-k fold
+    // the small F32 matrices of the one-token step (router, shared-expert gate, alpha, beta) also in the serial-k fold's order
     auto f32k = [&](const std::string& n) {
         DevF32 w = f32(n);
-        if (!w.w || !c->exact) return w;
-        const size_t total = (size_t)((w.n_out + 31) / 32) * w.n_in * 32;
+        if (!w.w || !c->exact || w.n_in % 4) return w;
+        const size_t total = (size_t)((w.n_out + F32S_ROWS - 1) / F32S_ROWS) * w.n_in * F32S_ROWS;
         float* wt = nullptr;
         if (cudaMalloc(&wt, total * 4) != cudaSuccess) { cudaGetLastError(); return w; }      // without the copy the row-per-warp path serves
-        k_f32_kmajor<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(w.w, w.n_in, w.n_out, wt);
+        k_f32_units<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(w.w, w.n_in, w.n_out, wt);
         m->extra.push_back(wt); m->bytes += total * 4;
         w.wt = wt;
         return w;
@@ -752,7 +753,7 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
         // many rows: the softmax once per (row, head), in place, instead of once per block of the weighted-value kernel
         static bool attr2 = false;
         if (!attr2) { set_smem((const void*)k_attn_softmax_exact, 200 * 1024); attr2 = true; }
-        launch_k(pdl, k_attn_softmax_exact, dim3(d.n_head, rows), dim3(256), (size_t)((n_pos_max + 3) & ~3) * 4, st, sm);
+        launch_k(pdl, k_attn_softmax_exact, dim3(d.n_head, rows), dim3(256), (size_t)ax_pad(n_pos_max) * 4, st, sm);
         launch_k(pdl, k_attn_out_exact<true>, dim3(hd / 32, d.n_head, rows), dim3(288), attn_out_exact_smem(n_pos_max, true), st, o);
         return;
     }
@@ -787,13 +788,13 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
         p.br = std::max(pass_in, std::min(p.br, cap / pass_in * pass_in));
         p.f32_ring = 0; p.err = e->err;
         if (c->exact && p.nf) {
-            // serial-k F32 rows: 32 to a warp (a lane per row) through the block's ring, when every unit gets a block of its own
+            // serial-k F32 rows: F32S_ROWS to a unit (a lane per row) through the block's ring, when every unit gets a block of its own
             // and the ring fits; otherwise a row per warp, staged in the warp's term scratch (make it hold the whole row)
             int units = 0;
-            for (int m = 0; m < p.nf; ++m) units += (p.f[m].n_out + 31) / 32;
-            bool kmajor = true;
-            for (int m = 0; m < p.nf; ++m) kmajor = kmajor && p.f[m].wt;
-            if (kmajor && units <= gx && NWG >= 4 && H % F32S_K == 0 && H / F32S_K >= F32S_STAGES && in_proj_smem(H, 1, p.br, 1) <= SMEM_BUDGET) p.f32_ring = units;
+            for (int m = 0; m < p.nf; ++m) units += (p.f[m].n_out + F32S_ROWS - 1) / F32S_ROWS;
+            bool has_units = true;
+            for (int m = 0; m < p.nf; ++m) has_units = has_units && p.f[m].wt;
+            if (has_units && units <= gx && NWG > 2 + F32S_MULT && H % F32S_K == 0 && H / F32S_K >= 4 && in_proj_smem(H, 1, p.br, 1) <= SMEM_BUDGET) p.f32_ring = units;
             else {
                 const int want = (H + H / 32) / (H / 32 + 1) + 1;
                 p.br = std::max(p.br, std::min((want + pass_in - 1) / pass_in * pass_in, cap / pass_in * pass_in));
@@ -826,7 +827,7 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
         hint_add(h, w.q, (size_t)w.n_in * w.n_out); hint_add(h, w.s, (size_t)(w.n_in / 32) * w.n_out * 2);
     };
     auto hint_f32 = [&](L2Hint& h, const DevF32& w) {
-        if (c->exact && w.wt) hint_add(h, w.wt, (size_t)((w.n_out + 31) / 32) * 32 * w.n_in * 4);
+        if (c->exact && w.wt) hint_add(h, w.wt, (size_t)((w.n_out + F32S_ROWS - 1) / F32S_ROWS) * F32S_ROWS * w.n_in * 4);
         else hint_add(h, w.w, (size_t)w.n_in * w.n_out * 4);
     };
     // the input projections of layer `il` (what its first kernel streams)

@@ -23,7 +23,7 @@ struct InProj {
     const float* conv_w; float* conv_state; int conv_kernel; size_t conv_state_stride;
     int8_t* xq_out; float* xs_out;                // optional copy of the quantised normed row, [B][n_embd]
     int exact; int br;                             // br: rows whose terms a warp collects before folding them together
-    int f32_ring; int* err;                        // serial-k F32 rows through the block's ring (in_proj_smem counts it): the number of 32-row units, 0 = off; status word of its bounded waits
+    int f32_ring; int* err;                        // serial-k F32 rows through the block's ring (in_proj_smem counts it): the number of units, 0 = off; status word of its bounded waits
     int tl_slot;                                   // phase-timeline slot of this launch (-1: none)
     L2Hint hint;                                   // what the kernels after this one will stream
 };
@@ -47,19 +47,19 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
     const size_t ring_off = ((size_t)((const unsigned char*)(tile + (p.exact ? 32 * 33 : 0) + nw * (tfl + CONV_CAP * 8)) - smem) + 127) & ~(size_t)127;
     float* ring = (float*)(smem + ring_off);
     unsigned long long* ring_full = (unsigned long long*)(ring + F32S_FLOATS);
-    unsigned long long* ring_empty = ring_full + F32S_STAGES;
-    // serial-k F32 units: unit u belongs to block gridDim.x - 1 - u; there the last warp folds and the one before it feeds the
-    // ring, and neither takes Q8_0 rows (the fold is the longest thing in the kernel)
+    unsigned long long* ring_empty = ring_full + F32S_STAGES; unsigned long long* ring_ready = ring_empty + F32S_STAGES;
+    // serial-k F32 units: unit u belongs to block gridDim.x - 1 - u; there the last warp folds, the one before it feeds the
+    // ring, F32S_MULT more multiply, and none of them takes Q8_0 rows (the fold is the longest thing in the kernel)
     const int my_unit = p.f32_ring ? (int)gridDim.x - 1 - (int)blockIdx.x : -1;
     const bool unit_block = my_unit >= 0 && my_unit < p.f32_ring;
     const float* unit_w = nullptr; float* unit_out = nullptr; int unit_r0 = 0, unit_nr = 0;
     if (unit_block) {
         int u = my_unit;
         for (int m = 0; m < p.nf; ++m) {
-            const int units = (p.f[m].n_out + 31) / 32;
+            const int units = (p.f[m].n_out + F32S_ROWS - 1) / F32S_ROWS;
             if (u < units) {
-                unit_w = p.f[m].wt + (size_t)u * 32 * n; unit_out = p.fout[m] + (size_t)b * p.fstride[m];
-                unit_r0 = u * 32; unit_nr = min(32, p.f[m].n_out - u * 32);
+                unit_w = p.f[m].wt + (size_t)u * F32S_ROWS * n; unit_out = p.fout[m] + (size_t)b * p.fstride[m];
+                unit_r0 = u * F32S_ROWS; unit_nr = min(F32S_ROWS, p.f[m].n_out - u * F32S_ROWS);
                 break;
             }
             u -= units;
@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
             for (int i = 0; i < F32S_STAGES; ++i) {
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(ring_full + i)) : "memory");
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(ring_empty + i)) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(ring_ready + i)), "r"(F32S_MULT) : "memory");
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
     // itself from the start (its fold is the longest thing in the kernel, and four warps to a scheduler slow its chain)
     const bool spare_units = p.f32_ring > 0 && 2 * p.f32_ring <= (int)gridDim.x;
     const int gq = spare_units ? (int)gridDim.x - p.f32_ring : (int)gridDim.x;
-    const int nwq = unit_block ? nw - 2 : nw;                     // warps that take Q8_0 rows
+    const int nwq = unit_block ? nw - 2 - F32S_MULT : nw;         // warps that take Q8_0 rows
     // this warp's share of the concatenated Q8_0 rows
     int total = 0;
     for (int m = 0; m < p.nq; ++m) total += p.q[m].n_out;
@@ -115,9 +116,11 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
     // Otherwise a row per warp handed out from the far end of the grid's warps: serial fold over staged products, or shuffle tree.
     if (p.f32_ring) {
         if (unit_block && wid == nw - 1)
-            f32_rows32_serial(n, unit_r0, unit_nr, xn, ring, ring_full, ring_empty, p.err, [&](int row, float v) { unit_out[row] = v; });
+            f32_rows_serial(n, unit_r0, unit_nr, ring, ring_ready, ring_empty, p.err, [&](int row, float v) { unit_out[row] = v; });
         else if (unit_block && wid == nw - 2 && lane == 0)
             f32_unit_feed(unit_w, n, ring, ring_full, ring_empty, p.err);
+        else if (unit_block && wid >= nwq && wid < nw - 2)
+            f32_unit_multiply(n, wid - nwq, xn, ring, ring_full, ring_ready, p.err);
     } else {
         const int ngw = gridDim.x * nw, gw = ngw - 1 - (wid * (int)gridDim.x + (int)blockIdx.x);
         int ubase = 0;
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
 size_t in_proj_smem(int n, int exact, int br, int f32_ring = 0) {
     int nb = n / 32;
     return 256 + (size_t)n * 5 + (size_t)nb * 4 + (exact ? 32 * 33 * 4 : 0) + (size_t)NWG * (br * (nb + 1) + CONV_CAP * 8) * 4 + 64 +
-           (f32_ring ? (size_t)F32S_FLOATS * 4 + 2 * F32S_STAGES * 8 + 128 : 0);
+           (f32_ring ? (size_t)F32S_FLOATS * 4 + 3 * F32S_STAGES * 8 + 128 : 0);
 }
 
 // ------------------------------------------------------------------------------------------------------

@@ -387,15 +387,17 @@ __device__ __forceinline__ void f32_rows(const float* __restrict__ w, int n_in, 
     }
 }
 
-// Serial-k F32 rows, 32 rows per warp: lane = row, every lane folds ITS row in k order (product and sum rounded separately,
-// src/ops/naive.rs:49-56), so 32 chains run side by side at one add latency per k for all of them. The unit's weights come
-// from the k-major copy (DevF32::wt): a stage of 256 k is 32 KB in one piece, fetched by ONE bulk asynchronous copy that
-// signals the stage's `full` mbarrier; in shared memory lane r reads word k * 32 + r, no conflicts. The copies are issued
-// by ANOTHER warp (f32_unit_feed): the folding warp does nothing but wait for a stage, fold it and hand the slot back
-// (`empty` mbarrier), so the chain of adds is the only thing on its critical path. Four stages keep enough bytes in flight
-// for one warp to stream at the pace of the chain. Waits are bounded: one that runs out stores `F32S_FAIL` in *err and the
+// Serial-k F32 rows, F32S_ROWS rows to a block: lane = row, every lane folds ITS row in k order (product and sum rounded separately,
+// src/ops/naive.rs:49-56), so the chains run side by side at one add latency per k for all of them. The unit's weights come
+// from the device copy DevF32::wt (four k of a row together, rows next to each other): a stage of 256 k is 8 KB in one piece, fetched
+// by ONE bulk asynchronous copy that signals the stage's `full` mbarrier; eight stages hold a whole unit of 2,048 k, requested before
+// the norm. The chain of adds bounds the unit, so the folding warp does nothing else: F32S_MULT warps multiply a stage in place by the
+// activation and signal `ready`, a feeding warp issues the copies of longer rows (f32_unit_feed), and the folding warp reads 16 k ahead of
+// its adds and hands slots back (`empty`). Few rows to a unit, because a stage passes through shared memory three times: at 32 that took
+// as long as the adds. From norm to result, 2,048 k: 32 rows with the folding warp multiplying 11.0 cycles a k, with multiplying warps
+// 7.2, 8 rows 5.7 (the adds: 4). Waits are bounded: one that runs out stores `F32S_FAIL` in *err and the
 // fold goes on over whatever the slot holds (the host reads *err after the step). n_in a multiple of 256.
-constexpr int F32S_K = 256, F32S_STAGES = 4, F32S_STAGE_FLOATS = 32 * F32S_K, F32S_FLOATS = F32S_STAGES * F32S_STAGE_FLOATS;
+constexpr int F32S_ROWS = 8, F32S_K = 256, F32S_STAGES = 8, F32S_STAGE_FLOATS = F32S_ROWS * F32S_K, F32S_FLOATS = F32S_STAGES * F32S_STAGE_FLOATS, F32S_MULT = 8;
 constexpr int F32S_FAIL = 0x7001;
 __device__ __forceinline__ bool f32s_wait(unsigned long long* bar, uint32_t parity, int* err) {
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
@@ -424,39 +426,57 @@ __device__ __forceinline__ void f32_unit_feed(const float* wt_unit, int n_in, fl
         f32_unit_issue(wt_unit, t, ring, full);
     }
 }
-template <class Epi>
-__device__ __forceinline__ void f32_rows32_serial(int n_in, int r0, int nr, const float* x, const float* ring, unsigned long long* full,
-                                                  unsigned long long* empty, int* err, Epi epi) {
+// Warp `part` of F32S_MULT: its share of every stage's products, in place.
+__device__ __forceinline__ void f32_unit_multiply(int n_in, int part, const float* x, float* ring, unsigned long long* full, unsigned long long* ready, int* err) {
     const int lane = threadIdx.x & 31, nst = n_in / F32S_K;
-    float sum = 0.0f;
 #pragma unroll 1
     for (int t = 0; t < nst; ++t) {
         const int slot = t % F32S_STAGES;
         f32s_wait(full + slot, (uint32_t)(t / F32S_STAGES) & 1u, err);
-        const float* col = ring + slot * F32S_STAGE_FLOATS + lane;
-        const float* xs = x + t * F32S_K;
-        // the products of the next 16 k are formed while the current 16 are added: the adds are the only chain
-        float pa[16], pb[16];
-        auto prod = [&](float (&pr)[16], int k0) {
+        float4* w = (float4*)(ring + slot * F32S_STAGE_FLOATS);
+        const float4* xs = (const float4*)(x + t * F32S_K);
+        constexpr int N = F32S_STAGE_FLOATS / 4 / (F32S_MULT * 32);
+        float4 a[N], b[N];                          // all read first: the writes go where they came from
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-                const float4 xv = *(const float4*)(xs + k0 + i);
-                pr[i] = __fmul_rn(col[(k0 + i) * 32], xv.x); pr[i + 1] = __fmul_rn(col[(k0 + i + 1) * 32], xv.y);
-                pr[i + 2] = __fmul_rn(col[(k0 + i + 2) * 32], xv.z); pr[i + 3] = __fmul_rn(col[(k0 + i + 3) * 32], xv.w);
-            }
-        };
-        prod(pa, 0);
-#pragma unroll 2
-        for (int k0 = 0; k0 < F32S_K; k0 += 32) {
-            prod(pb, k0 + 16);
+        for (int i = 0; i < N; ++i) { const int e = (i * F32S_MULT + part) * 32 + lane; a[i] = w[e]; b[i] = xs[e / F32S_ROWS]; }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) sum = __fadd_rn(sum, pa[i]);
-            if (k0 + 32 < F32S_K) prod(pa, k0 + 32);
+        for (int i = 0; i < N; ++i)
+            w[(i * F32S_MULT + part) * 32 + lane] = make_float4(__fmul_rn(a[i].x, b[i].x), __fmul_rn(a[i].y, b[i].y), __fmul_rn(a[i].z, b[i].z), __fmul_rn(a[i].w, b[i].w));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // these writes come before the copy that refills the slot
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(ready + slot)) : "memory");
+    }
+}
+template <class Epi>
+__device__ __forceinline__ void f32_rows_serial(int n_in, int r0, int nr, const float* ring, unsigned long long* ready,
+                                                  unsigned long long* empty, int* err, Epi epi) {
+    const int lane = threadIdx.x & 31, nst = n_in / F32S_K;
+    const float4* at = (const float4*)ring + lane % F32S_ROWS;
+    float sum = 0.0f;
+    float4 a[4], b[4];                             // the 16 k being added and the 16 after them
+    auto add = [&](const float4 (&v)[4]) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) sum = __fadd_rn(sum, pb[i]);
+        for (int i = 0; i < 4; ++i) { sum = __fadd_rn(sum, v[i].x); sum = __fadd_rn(sum, v[i].y); sum = __fadd_rn(sum, v[i].z); sum = __fadd_rn(sum, v[i].w); }
+    };
+    f32s_wait(ready, 0, err);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = at[i * F32S_ROWS];
+#pragma unroll 1
+    for (int t = 0; t < nst; ++t) {
+        const int nx = t + 1 < nst ? t + 1 : t;
+        const float4* p = at + (t % F32S_STAGES) * (F32S_STAGE_FLOATS / 4); const float4* q = at + (nx % F32S_STAGES) * (F32S_STAGE_FLOATS / 4);
+#pragma unroll
+        for (int j = 0; j < F32S_K / 4; j += 8) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) b[i] = p[(j + 4 + i) * F32S_ROWS];
+            add(a);
+            if (j + 8 == F32S_K / 4) f32s_wait(ready + nx % F32S_STAGES, (uint32_t)(nx / F32S_STAGES) & 1u, err);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = j + 8 < F32S_K / 4 ? p[(j + 8 + i) * F32S_ROWS] : q[i * F32S_ROWS];
+            add(b);
         }
-        __syncwarp();                           // every lane has read the slot: hand it back
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(empty + slot)) : "memory");
+        __syncwarp();                               // every lane has this stage's products: its slot goes back
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(empty + t % F32S_STAGES)) : "memory");
     }
     if (lane < nr) epi(r0 + lane, sum);
 }

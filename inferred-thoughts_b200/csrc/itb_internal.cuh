@@ -49,8 +49,8 @@ __device__ __forceinline__ int fp4_slot(const DevFp4& w, int e) {
 struct DevF32 {
     const float* w = nullptr;
     int n_in = 0, n_out = 0;
-    // optional second copy for the serial-k one-token path: units of 32 rows, k-major inside a unit ([unit][k][32 rows], rows
-    // past n_out zero), so that 128 k of a unit are 16 KB in one piece and a lane per row reads them without bank conflicts
+    // optional second copy for the serial-k one-token path: units of F32S_ROWS rows, [unit][k / 4][rows][4 k] (rows past n_out
+    // zero), so that a unit's k range is one piece and a lane per row reads four k at a time without bank conflicts
     const float* wt = nullptr;
 };
 
