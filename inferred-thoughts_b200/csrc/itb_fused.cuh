@@ -102,6 +102,13 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
         if (wid == nw - 2 && lane == 0)
             for (int t = 0; t < F32S_STAGES && t < n / F32S_K; ++t) f32_unit_issue(unit_w, t, ring, ring_full);
     }
+    // the first rows' weights are requested before the row they will meet is there
+    RowTrip<2, 2> trip;
+    {
+        int base = 0, m = 0;
+        while (m + 1 < p.nq && r0 >= base + p.q[m].n_out) base += p.q[m++].n_out;
+        if (r0 < r1) trip_load(trip, (const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, r0 - base, min(r1 - base, p.q[m].n_out), lane & ((1 << gsh) - 1), gsh);
+    }
     pdl_wait();
     TL(TLK_IN_PROJ, 1);
     const bool quantised = block_rms_norm(p.x + (size_t)b * p.x_stride, p.norm_w, n, p.eps, xn, red, xq, xs);
@@ -140,12 +147,13 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
     for (int m = 0; m < p.nq; ++m) {
         const int lo = max(r0, base) - base, hi = min(r1, base + p.q[m].n_out) - base;
         if (lo < hi) {
+            if (r0 < base) trip_load(trip, (const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, lane & ((1 << gsh) - 1), gsh);     // the rows go on into another matrix
             float* o = p.qout[m] + (size_t)b * p.qstride[m];
             if (m == 0 && p.conv_w) {
                 float* cs = p.conv_state + (size_t)b * p.conv_state_stride;
                 const float* cw = p.conv_w;
                 const int kernel = p.conv_kernel;
-                rows_batched<2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh, [&](int row, float v) {
+                rows_batched<2, 2>(trip, (const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh, [&](int row, float v) {
                     float* past = cs + (size_t)row * keep;
                     const bool pre = row - conv_lo < CONV_CAP;
                     const float* pin = pre ? cpre + (row - conv_lo) * 8 : past;
@@ -158,7 +166,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
                     past[keep - 1] = v;
                 });
             } else {
-                rows_batched<2, 2>((const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh,
+                rows_batched<2, 2>(trip, (const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, lo, hi, xq, xs, terms, p.br, gsh,
                                           [&](int row, float v) { o[row] = v; });
             }
         }
@@ -192,15 +200,19 @@ __global__ void __launch_bounds__(NWG * 32) k_out_proj(OutProj p) {
     share(b1 - b0, nw, wid, r0, r1);
     TL(TLK_OUT_PROJ, 0);
     pdl_trigger();
+    const int lane = threadIdx.x & 31, lo = b0 + r0, hi = b0 + r1;
+    RowTrip<1, 4> trip;                            // requested before the activation is there: a warp has a row or two in all
+    if (lo < hi) trip_load(trip, (const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, lo, hi, lane & ((1 << gsh) - 1), gsh);
     pdl_wait();
     TL(TLK_OUT_PROJ, 1);
+    float* x = p.x + (size_t)b * p.x_stride;
+    const float old = lo + lane < hi ? x[lo + lane] : 0.0f;
     for (int i = threadIdx.x; i < n / 16; i += blockDim.x) ((uint4*)aq)[i] = ((const uint4*)(p.aq + (size_t)b * n))[i];
     for (int i = threadIdx.x; i < nb; i += blockDim.x) as[i] = p.as[(size_t)b * nb + i];
     __syncthreads();
     TL(TLK_OUT_PROJ, 2);
-    float* x = p.x + (size_t)b * p.x_stride;
-    rows_batched<1, 4>((const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, b0 + r0, b0 + r1, aq, as, terms, p.br, gsh,
-                              [&](int row, float v) { x[row] += v; });
+    rows_batched<1, 4>(trip, (const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, lo, hi, aq, as, terms, p.br, gsh,
+                              [&](int row, float v) { x[row] = (row == lo + lane ? old : x[row]) + v; });
     if (wid == 0) l2_hint(p.hint, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, threadIdx.x & 31);
     TL(TLK_OUT_PROJ, 3);
 }

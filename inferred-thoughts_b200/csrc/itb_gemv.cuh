@@ -256,16 +256,33 @@ __device__ __forceinline__ void rows_direct_ub(const uint8_t* __restrict__ pa, c
     }
 }
 
+// One trip's weights: units u0, u0 + G, .. (UB of them) of the rows r + slot, r + slot + SLOTS, .. (RP of them) below r1.
+template <int RP, int UB> struct RowTrip { UnitW w[UB][RP]; };
+template <int RP, int UB>
+__device__ __forceinline__ void trip_load(RowTrip<RP, UB>& t, const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r, int r1, int u0, int gsh) {
+    const int G = 1 << gsh, slot = (threadIdx.x & 31) >> gsh, SLOTS = 32 >> gsh, nunits = n_in >> 5;
+#pragma unroll
+    for (int i = 0; i < RP; ++i) {
+        const int row = r + i * SLOTS + slot;
+        if (row < r1) {
+#pragma unroll
+            for (int h = 0; h < UB; ++h)
+                if (u0 + h * G < nunits) unit_load(t.w[h][i], pa + (size_t)row * n_in, pb + (size_t)row * (n_in / 16), u0 + h * G);
+        }
+    }
+}
 // As rows_direct_ub, but the terms of up to `br` rows are collected first and then folded by `br` lanes at
 // once: the fold is a serial chain per row, so folding one or two rows at a time leaves most lanes idle and
 // costs as many instructions as the dots themselves. terms: br * (row_terms + 1) floats, warp-private.
+// A warp has a handful of trips, each a round trip to memory: the first one's weights (cur, trip_load of r0 and the lane's first unit)
+// come from the caller, who can request them before the activation is there. (A second set of registers for the next trip's as well
+// took the room of the next kernel's blocks and slowed the LM head from 92 to 126 us.)
 template <int RP, int UB, class Epi>
-__device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r0, int r1,
+__device__ __forceinline__ void rows_batched(RowTrip<RP, UB>& cur, const uint8_t* __restrict__ pa, const uint8_t* __restrict__ pb, int n_in, int r0, int r1,
                                              const int8_t* xq, const float* xs, float* terms, int br, int gsh, Epi epi) {
     const int G = 1 << gsh, lane = threadIdx.x & 31, sub = lane & (G - 1), slot = lane >> gsh;
     const int SLOTS = 32 >> gsh, ROWS = RP * SLOTS;
     const int nunits = n_in >> 5, nt = n_in >> 5, stride = nt + 1;
-    const int arb = n_in, brb = n_in / 16;
     br = min(br, 32) / ROWS * ROWS;   // whole passes per batch (the caller sizes terms for at least one pass)
 #pragma unroll 1
     for (int rb = r0; rb < r1; rb += br) {
@@ -274,16 +291,7 @@ __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, con
         for (int r = rb; r < rend; r += ROWS) {
 #pragma unroll 1
             for (int u0 = sub; u0 < nunits; u0 += UB * G) {
-                UnitW w[UB][RP];
-#pragma unroll
-                for (int i = 0; i < RP; ++i) {
-                    const int row = r + i * SLOTS + slot;
-                    if (row < rend) {
-#pragma unroll
-                        for (int h = 0; h < UB; ++h)
-                            if (u0 + h * G < nunits) unit_load(w[h][i], pa + (size_t)row * arb, pb + (size_t)row * brb, u0 + h * G);
-                    }
-                }
+                if (r > r0 || u0 > sub) trip_load(cur, pa, pb, n_in, r, rend, u0, gsh);
 #pragma unroll
                 for (int h = 0; h < UB; ++h) {
                     if (u0 + h * G < nunits) {
@@ -293,7 +301,7 @@ __device__ __forceinline__ void rows_batched(const uint8_t* __restrict__ pa, con
 #pragma unroll
                         for (int i = 0; i < RP; ++i) {
                             const int row = r + i * SLOTS + slot;
-                            if (row < rend) unit_terms(w[h][i], xa, xb, dx, terms + (row - rb) * stride, u);
+                            if (row < rend) unit_terms(cur.w[h][i], xa, xb, dx, terms + (row - rb) * stride, u);
                         }
                     }
                 }
