@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     float* kq = S + sv * (sk + 1);           // k[sk] | q[sk]
     float* o = kq + 2 * sk;                  // [sv]
     __shared__ double red2[8];
-    __shared__ float s_gb[2];
+    __shared__ float s_gb[2], s_z[SK];
     const int key_dim = p.n_k * sk;
     const float* cv = p.conv + (size_t)b * p.conv_stride;
     float* sg = p.state + (size_t)b * p.state_stride + (size_t)h * sv * sk;
@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     TL(TLK_GDN_CORE, 1);
     // every other global operand is requested now too, so the kernel has one memory round trip
     const float r_alpha = p.alpha[(size_t)b * p.n_v + h], r_beta = p.beta[(size_t)b * p.n_v + h];
-    const size_t oidx = (size_t)b * p.n_v * sv + (size_t)h * sv + (tid < sv ? tid : 0);
-    const float r_z = p.z[oidx];
+    const size_t obase = (size_t)b * p.n_v * sv + (size_t)h * sv;
+    const float r_z = tid >= sv && tid < 2 * sv ? p.z[obase + tid - sv] : 0.0f;      // the output gate, by threads that have no state row
     // SiLU of this head's conv sums: threads [0, 2*sk) take k then q, threads [0, sv) their v element later
     if (tid < 2 * sk) kq[tid] = silu_f(cv[(tid < sk ? key_dim : 0) + kh * sk + (tid < sk ? tid : tid - sk)]);
     float vj = 0.0f;
@@ -326,35 +326,32 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
 #pragma unroll
         for (int i = 0; i < SK; ++i) row[i] = R[i];
         o[tid] = acc;
-    }
+    } else if (tid < 2 * sv) s_z[tid - sv] = silu_f(r_z);
     __syncthreads();
     TL(TLK_GDN_CORE, 4);
-    {
-        double acc = 0.0;
-        for (int i = tid; i < sv; i += blockDim.x) acc += (double)(o[i] * o[i]);
-        acc = warp_sum_d(acc);
+    if (tid < sv) {   // whole warps: sv is a multiple of 32; the others write the state meanwhile
+        const double acc = warp_sum_d((double)(o[tid] * o[tid]));
         if (lane == 0) red2[wid] = acc;
-        __syncthreads();
+        asm volatile("bar.sync 1, %0;" ::"n"(SK) : "memory");
         double tot = 0.0;
-        if (lane == 0) for (int w = 0; w < 8; ++w) tot += red2[w];      // one lane per warp adds (slow f64 unit), the rest get it by shuffle
+        if (lane == 0) for (int w = 0; w < sv / 32; ++w) tot += red2[w];      // one lane per warp adds (slow f64 unit), the rest get it by shuffle
         tot = __shfl_sync(0xffffffffu, tot, 0);
         float mean = (float)(tot / (double)sv);
         float sc = 1.0f / sqrtf(mean + p.eps);
-        if (tid < sv) {   // whole warps: sv is a multiple of 32
-            float core = o[tid] * sc * r_nw;
-            size_t idx = oidx;
-            float val = silu_f(r_z) * core;
-            float dq;
-            int8_t q = warp_quant_q8(val, &dq);
-            p.out_q[idx] = q;
-            if (lane == 0) p.out_s[idx / 32] = dq;
+        float core = o[tid] * sc * r_nw;
+        float val = s_z[tid] * core;
+        float dq;
+        int8_t q = warp_quant_q8(val, &dq);
+        const size_t idx = obase + tid;
+        p.out_q[idx] = q;
+        if (lane == 0) p.out_s[idx / 32] = dq;
+    } else {
+#pragma unroll 8
+        for (int i = tid - sv; i < sv * sk / 4; i += 256 - sv) {
+            const int e = i * 4, r = e / sk, c0 = e % sk;
+            const float* s = S + r * (sk + 1) + c0;
+            __stcs((float4*)sg + i, make_float4(s[0], s[1], s[2], s[3]));
         }
-    }
-#pragma unroll
-    for (int i = 0; i < LD; ++i) {
-        int e = (tid + i * 256) * 4, r = e / sk, c0 = e % sk;
-        const float* s = S + r * (sk + 1) + c0;
-        __stcs((float4*)sg + tid + i * 256, make_float4(s[0], s[1], s[2], s[3]));
     }
     TL(TLK_GDN_CORE, 5);
 }
@@ -722,6 +719,17 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_down(MoeDown p) {
     if (su_in) unit_load(su, (const uint8_t*)p.shared_down.q + (size_t)su_row * sff, (const uint8_t*)p.shared_down.s + (size_t)su_row * (sff / 16), su_u);
     pdl_wait();
     TL(TLK_MOE_DOWN, 1);
+    // one-GPU form: a warp's first piece (with 16 warps and 8 picks of 512, its only one) is on its way as soon as its expert's id is here,
+    // under the activation's loads: 6.1 -> 5.5 us after the wait
+    const int slices = (kgs + DOWN_KG - 1) / DOWN_KG;
+    Fp4Trips<DOWN_KG / 2> first;
+    if (!pairs && wid < K * slices) {
+        const int el = p.ids[(size_t)b * K + wid / slices] - p.down.expert_lo, g0 = wid % slices * DOWN_KG;
+        if (el >= 0 && el < p.down.n_expert) {
+            const size_t ro = (size_t)el * n_out + row0;
+            fp4_trips_load(first, p.down.nib + ro * (ff / 2), p.down.sc + ro * nsb, g0 + (lane >> 4), min(kgs, g0 + DOWN_KG));
+        }
+    }
     if (tid < K) {
         int el = p.ids[(size_t)b * K + tid] - p.down.expert_lo;
         s_el[tid] = (el < 0 || el >= p.down.n_expert) ? -1 : el;
@@ -744,11 +752,12 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_down(MoeDown p) {
     // lane k keeps pick k's second scale; the load is issued here and first used after the row dots, so it costs no round trip
     const int ck = tid % K, cr = tid / K;                 // the (pick, row) chain this thread folds
     const float s2k = (has_s && cr < 16 && s_el[ck] >= 0) ? p.down.scale2[s_el[ck]] : 1.0f;
-    const int slices = (kgs + DOWN_KG - 1) / DOWN_KG, n_items = (pairs ? s_nloc : K) * slices;
+    const int n_items = (pairs ? s_nloc : K) * slices;
 #pragma unroll 1
     for (int it = wid; it < n_items; it += nw) {
         const int pk = pairs ? s_loc[it / slices] : it / slices, g0 = (it % slices) * DOWN_KG, el = s_el[pk];
         if (el < 0) continue;
+        if (!pairs && it == wid) { fp4_trips_terms(first, g0 + (lane >> 4), min(kgs, g0 + DOWN_KG), hq + pk * ff, hs + pk * nbf, terms + pk * 16 * (nsb + 1), nsb + 1); continue; }
         const size_t ro = (size_t)el * n_out + row0;
         fp4_tile_terms<DOWN_KG / 2>(p.down.nib + ro * (ff / 2), p.down.sc + ro * nsb, g0, min(kgs, g0 + DOWN_KG), hq + pk * ff, hs + pk * nbf, terms + pk * 16 * (nsb + 1), nsb + 1);
     }

@@ -188,22 +188,32 @@ __device__ __forceinline__ void fp4_group_terms(const uint4& v0, const uint4& v1
 }
 // A warp on one 16-row tile of an NVFP4 matrix (nib, sc: the tile), groups [g0, g1) of 64 elements: lane = (row, group parity), so a
 // trip reads two groups, 1 KB in one piece. UB trips are loaded before the first dot. Terms go to t[row * stride + term].
+template <int UB> struct Fp4Trips { uint4 v[UB][2]; uint32_t s[UB]; };
+template <int UB>
+__device__ __forceinline__ void fp4_trips_load(Fp4Trips<UB>& w, const uint8_t* __restrict__ nib, const uint8_t* __restrict__ sc, int k0, int g1) {
+    const int r = threadIdx.x & 15;
+#pragma unroll
+    for (int i = 0; i < UB; ++i)
+        if (k0 + 2 * i < g1) {
+            const uint8_t* p = nib + (size_t)(k0 + 2 * i) * 512 + r * 32;
+            w.v[i][0] = ld_stream16(p); w.v[i][1] = ld_stream16(p + 16);
+            w.s[i] = __ldg((const uint32_t*)(sc + (size_t)(k0 + 2 * i) * 64 + r * 4));
+        }
+}
+template <int UB>
+__device__ __forceinline__ void fp4_trips_terms(const Fp4Trips<UB>& w, int k0, int g1, const int8_t* xq, const float* xs, float* t, int stride) {
+    const int r = threadIdx.x & 15;
+#pragma unroll
+    for (int i = 0; i < UB; ++i)
+        if (k0 + 2 * i < g1) { const int k = k0 + 2 * i; fp4_group_terms(w.v[i][0], w.v[i][1], w.s[i], xq + k * 64, xs + k * 2, t + r * stride + k * 4); }
+}
 template <int UB>
 __device__ __forceinline__ void fp4_tile_terms(const uint8_t* __restrict__ nib, const uint8_t* __restrict__ sc, int g0, int g1, const int8_t* xq, const float* xs, float* t, int stride) {
-    const int lane = threadIdx.x & 31, r = lane & 15, par = lane >> 4;
 #pragma unroll 1
-    for (int k0 = g0 + par; k0 < g1; k0 += 2 * UB) {
-        uint4 v[UB][2]; uint32_t s[UB];
-#pragma unroll
-        for (int i = 0; i < UB; ++i)
-            if (k0 + 2 * i < g1) {
-                const uint8_t* p = nib + (size_t)(k0 + 2 * i) * 512 + r * 32;
-                v[i][0] = ld_stream16(p); v[i][1] = ld_stream16(p + 16);
-                s[i] = __ldg((const uint32_t*)(sc + (size_t)(k0 + 2 * i) * 64 + r * 4));
-            }
-#pragma unroll
-        for (int i = 0; i < UB; ++i)
-            if (k0 + 2 * i < g1) { const int k = k0 + 2 * i; fp4_group_terms(v[i][0], v[i][1], s[i], xq + k * 64, xs + k * 2, t + r * stride + k * 4); }
+    for (int k0 = g0 + ((threadIdx.x >> 4) & 1); k0 < g1; k0 += 2 * UB) {
+        Fp4Trips<UB> w;
+        fp4_trips_load(w, nib, sc, k0, g1);
+        fp4_trips_terms(w, k0, g1, xq, xs, t, stride);
     }
 }
 // Ascending fold of one row's terms.
@@ -409,11 +419,15 @@ constexpr int F32S_ROWS = 8, F32S_K = 256, F32S_STAGES = 8, F32S_STAGE_FLOATS = 
 constexpr int F32S_FAIL = 0x7001;
 __device__ __forceinline__ bool f32s_wait(unsigned long long* bar, uint32_t parity, int* err) {
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
-    const long long t0 = clock64();
-    for (;;) {
+    auto arrived = [&] {
         uint32_t ok;
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(b), "r"(parity) : "memory");
-        if (ok) return true;
+        return ok != 0;
+    };
+    if (arrived()) return true;
+    const long long t0 = clock64();
+    for (;;) {
+        if (arrived()) return true;
         if (clock64() - t0 > 2000000000ll) { if (err) atomicExch(err, F32S_FAIL); return false; }
     }
 }
@@ -450,7 +464,7 @@ __device__ __forceinline__ void f32_unit_multiply(int n_in, int part, const floa
 #pragma unroll
         for (int i = 0; i < N; ++i)
             w[(i * F32S_MULT + part) * 32 + lane] = make_float4(__fmul_rn(a[i].x, b[i].x), __fmul_rn(a[i].y, b[i].y), __fmul_rn(a[i].z, b[i].z), __fmul_rn(a[i].w, b[i].w));
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // these writes come before the copy that refills the slot
+        if (t + F32S_STAGES < nst) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // these writes come before the copy that refills the slot
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(ready + slot)) : "memory");
     }
@@ -483,6 +497,7 @@ __device__ __forceinline__ void f32_rows_serial(int n_in, int r0, int nr, const 
             for (int i = 0; i < 4; ++i) a[i] = j + 8 < F32S_K / 4 ? p[(j + 8 + i) * F32S_ROWS] : q[i * F32S_ROWS];
             add(b);
         }
+        if (t + F32S_STAGES >= nst) continue;       // nobody waits for this slot any more
         __syncwarp();                               // every lane has this stage's products: its slot goes back
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(empty + t % F32S_STAGES)) : "memory");
     }
