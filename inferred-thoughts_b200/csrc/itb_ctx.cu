@@ -120,6 +120,7 @@ static void free_map(std::unordered_map<const void*, Mirror>& m) {
     m.clear();
 }
 
+static void itb_pipe_free(itb_ctx* c);
 extern "C" void itb_destroy(itb_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
@@ -129,7 +130,7 @@ extern "C" void itb_destroy(itb_ctx* c) {
     cudaFree(c->pair_off); cudaFree(c->pair_list); cudaFree(c->pair_tiles);
     itb_tc_free(c);
     cudaFree(c->route_ids); cudaFree(c->route_w); cudaFree(c->xq); cudaFree(c->xs); cudaFree(c->tmp_f32);
-    delete c->pipe;
+    itb_pipe_free(c);
     cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -219,6 +220,7 @@ struct HostPipe {
         cudaFreeHost(ring); cudaFreeHost(chunk[0]);
     }
 };
+static void itb_pipe_free(itb_ctx* c) { delete c->pipe; c->pipe = nullptr; }
 bool itb_upload(itb_ctx* c, void* dev, const void* host, size_t bytes) {
     if (!c->pipe) c->pipe = new HostPipe();
     HostPipe& p = *c->pipe;
