@@ -38,7 +38,7 @@ __global__ void k_attn_scores_exact(AxScores p) {
     const int hk = blockIdx.y, r = blockIdx.z, hd = p.hd, group = p.n_head / p.n_head_kv, qst = hd + AX_QSTRIDE_PAD, kst = hd + AX_KPAD;
     float* qs = (float*)smem;                                    // [group][hd + pad]
     uint16_t* ks = (uint16_t*)(qs + group * qst);                // [2][AX_TP][hd + pad]
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const int n_pos = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
     const int n_tiles = (n_pos + AX_TP - 1) / AX_TP, cpr = hd / 8;
     if ((int)blockIdx.x >= n_tiles) return;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
     __shared__ float s_sum;
     const int j = blockIdx.x, h = blockIdx.y, r = blockIdx.z, hd = p.hd, group = p.n_head / p.n_head_kv, hk = h / group;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const int n_pos = p.n_pos_dev ? p.n_pos_dev[r] : p.n_pos_last - p.n_q + 1 + r;
     float* prod = (float*)smem;                                   // [2][32][AX_VLD]
     float* w = prod + 2 * AX_VBUF;                                // [n_pos] scores -> exponentials -> weights
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256, 2) k_attn_scores_tile(AxScores p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_lim[2];
     const int hk = blockIdx.y, hd = p.hd, group = p.n_head / p.n_head_kv, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, p0 = blockIdx.x * 64;
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const AtTile t = at_tile<MR>(p.rows_per_seq, group, s_lim, p.n_pos_dev, p.n_pos_last, p.n_q);
     const int mx = s_lim[0], nl = t.nt * group, nk = hd / AT_KT;
     if (p0 >= mx) return;
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(256, 2) k_attn_out_tile(AxOut p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_lim[2];
     const int d0 = blockIdx.x * 64, hk = blockIdx.y, hd = p.hd, group = p.n_head / p.n_head_kv, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const AtTile t = at_tile<MR>(p.rows_per_seq, group, s_lim, p.n_pos_dev, p.n_pos_last, p.n_q);
     const int mx = s_lim[0], full = s_lim[1] / AT_KT, nl = t.nt * group, nk = (mx + AT_KT - 1) / AT_KT;
     const float* wb = p.scores + ((size_t)t.r0 * p.n_head + hk * group) * p.s_stride;

@@ -33,7 +33,6 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
     const int n = p.n_embd, nb = n / 32, gsh = lanes_shift(nb);
     const int b = blockIdx.y, wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     TL(TLK_IN_PROJ, 0);
-    pdl_trigger();
     double* red = (double*)smem;
     float* xn = (float*)(red + 32);
     int8_t* xq = (int8_t*)(xn + n);
@@ -110,6 +109,7 @@ __global__ void __launch_bounds__(NWG * 32) k_in_proj(InProj p) {
         if (r0 < r1) trip_load(trip, (const uint8_t*)p.q[m].q, (const uint8_t*)p.q[m].s, n, r0 - base, min(r1 - base, p.q[m].n_out), lane & ((1 << gsh) - 1), gsh);
     }
     pdl_wait();
+    pdl_trigger();
     TL(TLK_IN_PROJ, 1);
     const bool quantised = block_rms_norm(p.x + (size_t)b * p.x_stride, p.norm_w, n, p.eps, xn, red, xq, xs);
     TL(TLK_IN_PROJ, 2);
@@ -199,11 +199,11 @@ __global__ void __launch_bounds__(NWG * 32) k_out_proj(OutProj p) {
     share(p.w.n_out, gridDim.x, blockIdx.x, b0, b1);
     share(b1 - b0, nw, wid, r0, r1);
     TL(TLK_OUT_PROJ, 0);
-    pdl_trigger();
     const int lane = threadIdx.x & 31, lo = b0 + r0, hi = b0 + r1;
     RowTrip<1, 4> trip;                            // requested before the activation is there: a warp has a row or two in all
     if (lo < hi) trip_load(trip, (const uint8_t*)p.w.q, (const uint8_t*)p.w.s, n, lo, hi, lane & ((1 << gsh) - 1), gsh);
     pdl_wait();
+    pdl_trigger();
     TL(TLK_OUT_PROJ, 1);
     float* x = p.x + (size_t)b * p.x_stride;
     const float old = lo + lane < hi ? x[lo + lane] : 0.0f;
@@ -250,13 +250,13 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     const float* cv = p.conv + (size_t)b * p.conv_stride;
     float* sg = p.state + (size_t)b * p.state_stride + (size_t)h * sv * sk;
     TL(TLK_GDN_CORE, 0);
-    pdl_trigger();
     // the state belongs to this layer alone: its loads are in flight while the predecessor kernel finishes
     float4 ld[LD];
 #pragma unroll
     for (int i = 0; i < LD; ++i) ld[i] = __ldcs((const float4*)sg + tid + i * 256);
     const float r_dt = p.dt_bias[h], r_a = p.ssm_a[h], r_nw = p.ssm_norm[tid < sv ? tid : 0];
     pdl_wait();
+    pdl_trigger();
     TL(TLK_GDN_CORE, 1);
     // every other global operand is requested now too, so the kernel has one memory round trip
     const float r_alpha = p.alpha[(size_t)b * p.n_v + h], r_beta = p.beta[(size_t)b * p.n_v + h];
@@ -374,7 +374,7 @@ __global__ void k_attn_prep(AttnPrep p) {
     __shared__ double red[8];
     const int job = blockIdx.x, b = blockIdx.y, d = threadIdx.x, hd = p.hd, kvd = p.n_head_kv * hd;
     TL(TLK_ATTN_PREP, 0);
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     TL(TLK_ATTN_PREP, 1);
     const int pos = p.pos[b];
     if (job == 0 && d == 0) p.npos_out[b] = pos + 1;
@@ -425,7 +425,7 @@ __global__ void k_attn_combine_q(const float* part_acc, const float* part_ml, in
                                  const int* n_pos_dev, int n_head, int8_t* out_q, float* out_s) {
     const size_t th = blockIdx.x;
     const int d = threadIdx.x, b = (int)(th / n_head);
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const int n_pos = n_pos_dev[b], per = max(ATTN_MIN_SPLIT, (n_pos + n_split - 1) / n_split), n_act = (n_pos + per - 1) / per;
     // splits in trips of 8 with every load of a trip in flight; the combine itself keeps ascending split order
     const float gt = gate[th * hd + d];
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     const int b = blockIdx.y, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int unit = blockIdx.x, n_units = p.n_used * upp;
     TL(TLK_MOE_GLU, 0);
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     TL(TLK_MOE_GLU, 1);
     if (unit >= n_units) {
         // shared expert: silu(gate) * up for 32 elements, quantised (src/model/qwen35.rs:1669-1678)
@@ -711,13 +711,13 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_down(MoeDown p) {
     constexpr bool pairs = PAIRS;            // compile-time: the one-GPU kernel carries none of the expert-parallel branches
     const bool shared_here = pairs ? b == p.own_row : !p.local_only;
     TL(TLK_MOE_DOWN, 0);
-    pdl_trigger();
     // the shared expert's weights do not depend on the routing: this thread's first 32-element unit is on its way before the wait
     UnitW su{};
     const int su_row = row0 + tid / nbs, su_u = tid % nbs;
     const bool su_in = shared_here && tid < 16 * nbs;
     if (su_in) unit_load(su, (const uint8_t*)p.shared_down.q + (size_t)su_row * sff, (const uint8_t*)p.shared_down.s + (size_t)su_row * (sff / 16), su_u);
     pdl_wait();
+    pdl_trigger();
     TL(TLK_MOE_DOWN, 1);
     // one-GPU form: a warp's first piece (with 16 warps and 8 picks of 512, its only one) is on its way as soon as its expert's id is here,
     // under the activation's loads: 6.1 -> 5.5 us after the wait
@@ -805,7 +805,7 @@ size_t moe_down_smem(int n_used, int ff, int sff) {
 // ------------------------------------------------------------------------------------------------------
 __global__ void k_embed(const float* table, int n_embd, const int32_t* tokens, float* x) {
     int b = blockIdx.x;
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const float* row = table + (size_t)tokens[b] * n_embd;
     if ((n_embd & 3) == 0) {
         const int nv = n_embd >> 2;
@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(256) k_argmax_partial(const float* logits, int
     int part = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int lo, hi;
     share(n_vocab, gridDim.x, part, lo, hi);
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     const float* l = logits + (size_t)b * n_vocab;
     float bv = -INFINITY; int bi = 0x7fffffff;
     for (int i0 = lo + tid; i0 < hi; i0 += 8 * blockDim.x) {
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(256) k_argmax_partial(const float* logits, int
 __global__ void k_argmax_advance(const float* pv, const int* pi, int n_part, int32_t* tokens, int* pos, int32_t* next_out,
                                  int32_t* history, int history_cap, int* step_counter, int n_seq) {
     int b = blockIdx.x, lane = threadIdx.x;
-    pdl_trigger(); pdl_wait();
+    pdl_wait(); pdl_trigger();
     float bv = -INFINITY; int bi = 0x7fffffff;
     for (int i = lane; i < n_part; i += 32) argmax_merge(bv, bi, pv[(size_t)b * n_part + i], pi[(size_t)b * n_part + i]);
     for (int o = 16; o > 0; o >>= 1) argmax_merge(bv, bi, __shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
