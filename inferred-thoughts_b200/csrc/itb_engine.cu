@@ -638,6 +638,7 @@ struct itb_engine {
     float *x = nullptr, *qkvc = nullptr, *z = nullptr, *alpha = nullptr, *beta = nullptr, *zc = nullptr;
     float *qg = nullptr, *kbuf = nullptr, *vbuf = nullptr, *qn = nullptr, *gate = nullptr, *att = nullptr;
     float *part_acc = nullptr, *part_ml = nullptr;
+    uint32_t* words = nullptr;                         // pinned: a step's tokens, next tokens and status word
     float* scores = nullptr; size_t scores_cap = 0;    // exact attention: [rows][n_head][n_ctx] scores (grown on demand)
     float *router = nullptr, *shlogit = nullptr, *sg = nullptr, *su = nullptr, *h = nullptr, *logits = nullptr;
     int8_t* xq = nullptr; float* xs = nullptr;
@@ -1793,7 +1794,7 @@ extern "C" void itb_engine_destroy(itb_engine* e) {
         delete t->g; delete t; e->tier = nullptr;
     }
     for (void* p : e->allocs) cudaFree(p);
-    cudaFree(e->history); cudaFree(e->prompt); cudaFree(e->scores); cudaFree(e->gdn_scratch);
+    cudaFreeHost(e->words); cudaFree(e->history); cudaFree(e->prompt); cudaFree(e->scores); cudaFree(e->gdn_scratch);
     cudaEventDestroy(e->ev0); cudaEventDestroy(e->ev1);
     delete e;
 }
@@ -2026,10 +2027,11 @@ static bool ensure_graph(itb_engine* e) {
 
 // The one-kernel step's waits are bounded: a wait that ran out stores (stage << 8) | reason in the status word and every
 // block returns. Turn it into the sticky error and put the grid barrier's counters back.
-static bool check_flag(itb_engine* e) {
+// known: the word, where the caller has brought it home with its results.
+static bool check_flag(itb_engine* e, const uint32_t* known = nullptr) {
     if (e->mega != 1 && !e->c->exact && !(e->ep && (e->ep->p2p || e->ep->p2p_rows))) return true;
-    int f = 0;
-    if (cudaMemcpy(&f, e->err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return itb_fail_msg(e->c, "engine: cannot read the device status word");
+    int f = known ? (int)*known : 0;
+    if (!known && cudaMemcpy(&f, e->err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return itb_fail_msg(e->c, "engine: cannot read the device status word");
     if (f == EP_WAIT_FAIL) {
         cudaMemset(e->err, 0, 4);
         return itb_fail_msg(e->c, "expert-parallel engine: a peer's rows never arrived in this rank's memory (bounded wait ran out)");
@@ -2120,17 +2122,27 @@ static bool run_steps(itb_engine* e, uint32_t steps, bool timed) {
     return true;
 }
 
+// A step's few words go through pinned memory, so that nothing but the one wait at its end blocks: tokens in, next tokens and the status
+// word out. words: a step's tokens (B), next tokens (B), status.
+static uint32_t* step_words(itb_engine* e) {
+    if (!e->words && cudaMallocHost((void**)&e->words, (2 * (size_t)e->B + 1) * 4) != cudaSuccess) { e->words = nullptr; cudaGetLastError(); itb_fail_msg(e->c, "engine: out of pinned host memory"); }
+    return e->words;
+}
 extern "C" int itb_engine_decode(itb_engine* e, const uint32_t* tokens, float* logits_out, uint32_t* next_out) {
     itb_ctx* c = e->c;
     cudaStream_t st = c->stream;
-    if (!ep_agree(e, tokens_in_range(e, tokens, e->B) && steps_ready(e, 1))) return 1;
-    ITB_CUDA_RET(c, cudaMemcpyAsync(e->tokens, tokens, e->B * 4, cudaMemcpyHostToDevice, st), 1);
+    uint32_t* w = nullptr;
+    if (!ep_agree(e, tokens_in_range(e, tokens, e->B) && steps_ready(e, 1) && (w = step_words(e)))) return 1;
+    memcpy(w, tokens, e->B * 4);
+    ITB_CUDA_RET(c, cudaMemcpyAsync(e->tokens, w, e->B * 4, cudaMemcpyHostToDevice, st), 1);
     if (!run_steps(e, 1, true)) return 1;
-    if (next_out) cudaMemcpyAsync(next_out, e->next, e->B * 4, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(w + e->B, e->next, e->B * 4, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(w + 2 * e->B, e->err, 4, cudaMemcpyDeviceToHost, st);
     if (logits_out && !itb_download(c, logits_out, e->logits, (size_t)e->B * e->m->d.n_vocab * 4)) return 1;
     ITB_CUDA_RET(c, cudaStreamSynchronize(st), 1);
+    if (next_out) memcpy(next_out, w + e->B, e->B * 4);
     cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1);
-    return check_flag(e) ? 0 : 1;
+    return check_flag(e, w + 2 * e->B) ? 0 : 1;
 }
 
 extern "C" int itb_engine_decode_loop(itb_engine* e, const uint32_t* first, uint32_t steps, uint32_t* tokens_out) {
@@ -2142,17 +2154,21 @@ extern "C" int itb_engine_decode_loop(itb_engine* e, const uint32_t* first, uint
         cudaStreamSynchronize(st);
         drop_graph(e);  // the graph holds the history pointer
         cudaFree(e->history); e->history = nullptr; e->history_cap = 0;
-        if (cudaMalloc(&e->history, (size_t)steps * e->B * 4) != cudaSuccess) { e->history = nullptr; ok = itb_fail_msg(c, "decode_loop: out of device memory for the token history"); }
-        else e->history_cap = steps;
+        const uint32_t cap = std::max<uint32_t>(steps, 1024);      // a longer loop than the last drops the captured step
+        if (cudaMalloc(&e->history, (size_t)cap * e->B * 4) != cudaSuccess) { e->history = nullptr; ok = itb_fail_msg(c, "decode_loop: out of device memory for the token history"); }
+        else e->history_cap = cap;
     }
-    if (!ep_agree(e, ok && steps_ready(e, steps))) return 1;
-    ITB_CUDA_RET(c, cudaMemcpyAsync(e->tokens, first, e->B * 4, cudaMemcpyHostToDevice, st), 1);
+    uint32_t* w = nullptr;
+    if (!ep_agree(e, ok && steps_ready(e, steps) && (w = step_words(e)))) return 1;
+    memcpy(w, first, e->B * 4);
+    ITB_CUDA_RET(c, cudaMemcpyAsync(e->tokens, w, e->B * 4, cudaMemcpyHostToDevice, st), 1);
     cudaMemsetAsync(e->step_counter, 0, e->B * 4, st);
     if (!run_steps(e, steps, true)) return 1;
+    cudaMemcpyAsync(w + 2 * e->B, e->err, 4, cudaMemcpyDeviceToHost, st);
     if (tokens_out) cudaMemcpyAsync(tokens_out, e->history, (size_t)steps * e->B * 4, cudaMemcpyDeviceToHost, st);
     ITB_CUDA_RET(c, cudaStreamSynchronize(st), 1);
     cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1);
-    return check_flag(e) ? 0 : 1;
+    return check_flag(e, w + 2 * e->B) ? 0 : 1;
 }
 
 // Prefill in multi-row passes: every sequence advances `chunk` tokens per pass (rows = n_seq * chunk <= R), each
@@ -2233,15 +2249,13 @@ extern "C" long itb_engine_generate(itb_engine* e, const uint32_t* prompt, size_
     if (itb_engine_prefill(e, prompt, n_prompt, nullptr)) return -1;
     uint32_t next = 0;
     ITB_CUDA_RET(c, cudaMemcpy(&next, e->next, 4, cudaMemcpyDeviceToHost), -1);
-    size_t produced = 0;
-    for (size_t i = 0; i < max_new; ++i) {
-        out[produced++] = next;
-        if (produced == max_new) break;
-        if (e->host_pos[0] + 1 >= e->n_ctx) break;  // StopReason::ContextFull
-        uint32_t tok = next;
-        if (itb_engine_decode(e, &tok, nullptr, &next)) return -1;
-    }
-    return (long)produced;
+    if (max_new == 0) return 0;
+    out[0] = next;
+    // up to the limit or the last position (StopReason::ContextFull); each step's pick is the next one's token on the device, so the
+    // steps are queued behind each other
+    const size_t room = (size_t)e->n_ctx - 1 > e->host_pos[0] ? (size_t)e->n_ctx - 1 - e->host_pos[0] : 0, steps = std::min(max_new - 1, room);
+    if (steps && itb_engine_decode_loop(e, &next, (uint32_t)steps, out + 1)) return -1;
+    return (long)(1 + steps);
 }
 
 extern "C" int itb_engine_read_routes(itb_engine* e, int32_t* ids, size_t cap) {
