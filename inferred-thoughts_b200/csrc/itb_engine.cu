@@ -1317,8 +1317,8 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             else k_conv_rows<<<dim3((cd + 127) / 128, R), 128, 0, st>>>(cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d, d.ssm_d_conv);
             launches++;
             k_conv_state<<<dim3((cd + 127) / 128, n_seq), 128, 0, st>>>(cst, conv_stride, e->qkvc, n_tok, cd, d.ssm_d_conv); launches++;
-            k_gdn_pre<<<dim3(R, 2 * n_k + n_v), sk, 0, st>>>(e->qkvc2, cd, e->alpha, e->beta, L.ssm_a, L.dt_bias, sk, n_k, n_v, d.rms_eps,
-                                                            e->qh, e->kh, e->vh, e->gb); launches++;
+            (sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>)<<<dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st>>>(
+                e->qkvc2, cd, e->alpha, e->beta, L.ssm_a, L.dt_bias, n_k, n_v, d.rms_eps, e->qh, e->kh, e->vh, e->gb); launches++;
             const size_t chunk_need = (size_t)n_seq * ((n_tok + GC - 1) / GC) * n_v * gdn_chunk_floats<128>();
             if ((c->gdn_chunk || !c->exact) && n_tok >= 32 && sk == 128 && e->gdn_scratch_cap >= chunk_need) {
                 // many tokens: everything that does not touch the state for all chunks at once, then three small products per chunk
@@ -1335,7 +1335,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                 else k_gdn_scan<64><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);   // 64 or 128 only (checked at model creation)
             }
             launches++;
-            k_gdn_post<<<dim3(R, n_v), sk, 0, st>>>(e->core, e->z, L.ssm_norm, sk, n_v, d.rms_eps, e->aq, e->as); launches++;
+            (sk == 128 ? k_gdn_post<4> : k_gdn_post<2>)<<<dim3(R, row_share(R, n_v, sms)), 256, 0, st>>>(e->core, e->z, L.ssm_norm, n_v, d.rms_eps, e->aq, e->as); launches++;
             gemm(L.ssm_out, e->aq, e->as, e->x, H, 1);
         } else {
             const int as = e->slot_of[il];
@@ -1349,7 +1349,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             a.kslab = e->kslab + (size_t)as * e->B * a.slab_stride; a.vslab = e->vslab + (size_t)as * e->B * a.slab_stride;
             a.pos = e->pos; a.npos_out = e->npos; a.n_tok = n_tok; a.hd = d.head_dim; a.n_head = d.n_head; a.n_head_kv = d.n_head_kv;
             a.n_rot = d.n_rot; a.theta = d.rope_theta; a.eps = d.rms_eps; a.bf16 = c->kv_bf16;
-            k_attn_prep_rows<<<dim3(d.n_head + 2 * d.n_head_kv, R), d.head_dim, d.head_dim * 4, st>>>(a); launches++;
+            k_attn_prep_rows<<<dim3(R, row_share(R, d.n_head + 2 * d.n_head_kv, sms)), 256, (d.n_rot + 8 * d.head_dim) * 4, st>>>(a); launches++;
             const float scale = 1.0f / sqrtf((float)d.head_dim);
             const int nwa = 8, ns = n_tok > 1 ? e->n_split_rows : e->n_split;
             const size_t smem_a = (size_t)nwa * 8 * 2 * 4 + (size_t)nwa * 8 * d.head_dim * 4;

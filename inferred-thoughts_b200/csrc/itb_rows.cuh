@@ -59,14 +59,13 @@ __global__ void __launch_bounds__(256) k_matmul_f32_rows(DevF32 w, const float* 
 // apart, so the 16-byte reads of a warp fall on distinct banks. FUSED (tolerance class): the same walk with one fused multiply-add
 // per step. Two matrices over the same rows in one launch (blockIdx.z picks; w1.w null: one): the router and the shared expert's
 // gate, or alpha and beta -- each alone is a handful of blocks walking a 2,048-long chain.
-// grid (ceil(n_out / TO), ceil(n_rows / TR), 1 or 2), block 128; n_in a multiple of KT.
-// What bounds the two shapes: 16 x 16 (2 chains to a thread, a warp to a scheduler) the chain itself, 4 cycles a step, which the
-// shared-memory reads just keep up with (a thread per output at 256 threads read twice as much per step and took twice as long);
-// 32 x 64 the f32 pipe (16 chains, 32 operations for 8 reads of 4 steps).
+// grid (ceil(n_out / TO), ceil(n_rows / TR), 1 or 2), block (TO / MO) * (TR / MR); n_in a multiple of KT.
+// What bounds the shapes: 8 x 8, a chain to a thread, the chain itself: 4 cycles a step, and with up to four such blocks an SM a
+// scheduler has the slots for its warps' reads, products and sums between them; the larger ones the f32 pipe and the reads.
 template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
-__global__ void __launch_bounds__(128) k_sgemm_chain(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
-    static_assert((TO / MO) * (TR / MR) == 128, "a thread per MO x MR outputs");
-    constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, PIECES = (TO + TR) * (KT / 4) / 128;
+__global__ void __launch_bounds__((TO / MO) * (TR / MR)) k_sgemm_chain(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
+    constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, NT = NX * NY, PIECES = (TO + TR) * (KT / 4) / NT;      // a thread per MO x MR outputs
+    static_assert((TO + TR) * (KT / 4) % NT == 0, "whole pieces");
     extern __shared__ __align__(16) unsigned char smem[];
     float* ring = (float*)smem;                    // [stage][TO weight lines | TR activation lines][ST]
     const DevF32 w = blockIdx.z ? w1 : w0;
@@ -77,7 +76,7 @@ __global__ void __launch_bounds__(128) k_sgemm_chain(DevF32 w0, const float* __r
     const float* src[PIECES];
 #pragma unroll
     for (int i = 0; i < PIECES; ++i) {
-        const int c = threadIdx.x + 128 * i, line = c / (KT / 4), k4 = (c % (KT / 4)) * 4;
+        const int c = threadIdx.x + NT * i, line = c / (KT / 4), k4 = (c % (KT / 4)) * 4;
         src[i] = (line < TO ? w.w + (size_t)min(o0 + line, w.n_out - 1) * n : x + (size_t)min(r0 + line - TO, n_rows - 1) * n) + k4;
     }
     auto fetch = [&](int t) {
@@ -85,7 +84,7 @@ __global__ void __launch_bounds__(128) k_sgemm_chain(DevF32 w0, const float* __r
             float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
 #pragma unroll
             for (int i = 0; i < PIECES; ++i) {
-                const int c = threadIdx.x + 128 * i;
+                const int c = threadIdx.x + NT * i;
                 cp_async16(st + (c / (KT / 4)) * ST + (c % (KT / 4)) * 4, src[i] + (size_t)t * KT, true);
             }
         }
@@ -127,24 +126,25 @@ __global__ void __launch_bounds__(128) k_sgemm_chain(DevF32 w0, const float* __r
         for (int j = 0; j < MO; ++j)
             if (r0 + ty + i * NY < n_rows && o0 + tx + j * NX < w.n_out) out[(size_t)(r0 + ty + i * NY) * w.n_out + o0 + tx + j * NX] = acc[i][j];
 }
-constexpr int SGS_KT = 64, SGS_NST = 6, SGB_KT = 32, SGB_NST = 4;      // 16 x 16 tiles: 1,536 steps' bytes in flight hide HBM's latency behind 4 cycles a step
-constexpr size_t sgemm_small_smem() { return (size_t)SGS_NST * 32 * (SGS_KT + 4) * 4; }
-constexpr size_t sgemm_big_smem() { return (size_t)SGB_NST * 96 * (SGB_KT + 4) * 4; }
-inline bool sgemm_chain_ok(int n_in) { return n_in % SGS_KT == 0; }
-// One matrix, or two over the same rows. The wide tiles where they give every SM a block, else the small ones.
+constexpr int SG_KT = 64;
+inline bool sgemm_chain_ok(int n_in) { return n_in % SG_KT == 0; }
+template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
+static void sgemm_tiles(cudaStream_t st, int n_out, int nz, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb, float* ob) {
+    constexpr size_t smem = (size_t)NST * (TO + TR) * (KT + 4) * 4;
+    cudaFuncSetAttribute(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST><<<dim3((n_out + TO - 1) / TO, (n_rows + TR - 1) / TR, nz), (TO / MO) * (TR / MR), smem, st>>>(wa, x, n_rows, oa, wb, ob);
+}
+// One matrix, or two over the same rows. 8 x 8, a chain to a thread, is fastest as long as an SM has no more than four such blocks (32 rows
+// of 257 outputs, 2,048 k: 11.8 us, at 16 x 16 18.5), but it reads every line once per 8 of the others. Large passes: unfused, where a
+// step is two operations, 2 x 2 chains and twice the warps (2,048 rows: 145 us, at 4 x 4 173); fused, fewer reads (119, at 2 x 2 149).
 template <bool FUSED>
 static void sgemm_chain(cudaStream_t st, int sms, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb = DevF32{}, float* ob = nullptr) {
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_sgemm_chain<FUSED, 16, 16, 1, 2, SGS_KT, SGS_NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sgemm_small_smem());
-        cudaFuncSetAttribute(k_sgemm_chain<FUSED, 32, 64, 4, 4, SGB_KT, SGB_NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sgemm_big_smem());
-        attr = true;
-    }
-    const int n_out = std::max(wa.n_out, wb.w ? wb.n_out : 0), nz = wb.w ? 2 : 1;
-    if (((wa.n_out + 31) / 32) * ((n_rows + 63) / 64) >= sms)
-        k_sgemm_chain<FUSED, 32, 64, 4, 4, SGB_KT, SGB_NST><<<dim3((n_out + 31) / 32, (n_rows + 63) / 64, nz), 128, sgemm_big_smem(), st>>>(wa, x, n_rows, oa, wb, ob);
-    else
-        k_sgemm_chain<FUSED, 16, 16, 1, 2, SGS_KT, SGS_NST><<<dim3((n_out + 15) / 16, (n_rows + 15) / 16, nz), 128, sgemm_small_smem(), st>>>(wa, x, n_rows, oa, wb, ob);
+    const int n_out = std::max(wa.n_out, wb.w ? wb.n_out : 0), nz = wb.w ? 2 : 1, n_all = wa.n_out + (wb.w ? wb.n_out : 0);
+    auto blocks = [&](int to, int tr) { return (long long)((n_all + to - 1) / to) * ((n_rows + tr - 1) / tr); };
+    if (blocks(8, 8) <= 4 * sms) sgemm_tiles<FUSED, 8, 8, 1, 1, 64, 8>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (FUSED && blocks(32, 64) >= sms) sgemm_tiles<FUSED, 32, 64, 4, 4, 32, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (!FUSED && blocks(32, 32) >= 2 * sms) sgemm_tiles<FUSED, 32, 32, 2, 2, 32, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else sgemm_tiles<FUSED, 16, 16, 1, 2, 64, 6>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
 }
 
 // A dense Q8_0 matrix against n_rows >= 1 quantised rows: out[row][n_out] = or += (mode). tc: the tensor-core forms the context's
@@ -253,34 +253,49 @@ __global__ void k_conv_state(float* state, size_t state_stride, const float* x, 
 
 // Everything of the GatedDeltaNet block that does not depend on the state, per row: SiLU of the conv sums,
 // l2-norm of q and k (q also scaled by 1/sqrt(sk)), the decay g and the write strength beta
-// (src/model/qwen35.rs:1280-1316, src/ops/naive.rs:101-107, :254-273). grid (rows, 2*n_k + n_v), block sk.
-__global__ void k_gdn_pre(const float* conv, int cd, const float* alpha, const float* beta, const float* ssm_a, const float* dt_bias,
-                          int sk, int n_k, int n_v, float eps, float* qh, float* kh, float* vh, float* gb) {
-    __shared__ double red[8];
+// (src/model/qwen35.rs:1280-1316, src/ops/naive.rs:101-107, :254-273).
+// Blocks (row, share of its jobs; row_share), a warp per head of q or k (NJ = sk / 32 elements a lane, the sum of squares in the same order
+// as a warp per 32 of them), then per 128 elements of v, then per 32 heads' decays. Memory would bound it (131 MB at 2,048 rows of
+// 8,192: 20 us); a block of 128 threads per head, with a block-wide sum and the decays by one lane, took 97 us, this 58: the
+// library-exact exponential's f64 steps.
+// Blocks that share a row's jobs (8 warps each): enough rows fill the machine on their own, few rows take a warp per job.
+inline unsigned row_share(int rows, int jobs, int sms) { return (unsigned)std::max(1, std::min((jobs + 7) / 8, (8 * sms + rows - 1) / rows)); }
+template <int NJ>
+__global__ void __launch_bounds__(256) k_gdn_pre(const float* conv, int cd, const float* alpha, const float* beta, const float* ssm_a, const float* dt_bias,
+                          int n_k, int n_v, float eps, float* qh, float* kh, float* vh, float* gb) {
+    constexpr int sk = NJ * 32;
     const size_t r = blockIdx.x;
-    const int u = blockIdx.y, d = threadIdx.x, key_dim = n_k * sk;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, key_dim = n_k * sk, vd = n_v * sk, vjobs = (vd + 127) / 128, jobs = 2 * n_k + vjobs + (n_v + 31) / 32;
     const float* cv = conv + r * cd;
-    if (u < 2 * n_k) {
-        const bool is_q = u < n_k;
-        const int h = is_q ? u : u - n_k;
-        float v = silu_f(cv[(is_q ? 0 : key_dim) + h * sk + d]);
-        double acc = warp_sum_d((double)(v * v));
-        if ((d & 31) == 0) red[d >> 5] = acc;
-        __syncthreads();
-        double tot = 0.0;
-        for (int w = 0; w < sk / 32; ++w) tot += red[w];
-        float sc = 1.0f / fmaxf(sqrtf((float)tot), eps);
-        v = v * sc;
-        if (is_q) v = v * (1.0f / sqrtf((float)sk));
-        (is_q ? qh : kh)[(r * n_k + h) * sk + d] = v;
-    } else {
-        const int h = u - 2 * n_k;
-        vh[(r * n_v + h) * sk + d] = silu_f(cv[2 * key_dim + h * sk + d]);
-        if (d == 0) {
-            float a = alpha[r * n_v + h] + dt_bias[h];
-            float sp = a > 20.0f ? a : log_f(1.0f + exp_f(a));
-            gb[(r * n_v + h) * 2] = exp_f(sp * ssm_a[h]);
-            gb[(r * n_v + h) * 2 + 1] = sigmoid_f(beta[r * n_v + h]);
+    for (int u = blockIdx.y * 8 + wid; u < jobs; u += 8 * gridDim.y) {
+        if (u < 2 * n_k) {
+            const bool is_q = u < n_k;
+            const int h = is_q ? u : u - n_k;
+            const float* src = cv + (is_q ? 0 : key_dim) + h * sk + lane;
+            float v[NJ];
+            double tot = 0.0;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) v[j] = silu_f(src[32 * j]);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) tot += warp_sum_d((double)(v[j] * v[j]));
+            const float sc = 1.0f / fmaxf(sqrtf((float)tot), eps), qs = 1.0f / sqrtf((float)sk);
+            float* dst = (is_q ? qh : kh) + (r * n_k + h) * sk + lane;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) { float x = v[j] * sc; if (is_q) x = x * qs; dst[32 * j] = x; }
+        } else if (u < 2 * n_k + vjobs) {
+            const int i = (u - 2 * n_k) * 128 + lane * 4;
+            if (i < vd) {
+                const float4 x = *(const float4*)(cv + 2 * key_dim + i);
+                *(float4*)(vh + r * vd + i) = make_float4(silu_f(x.x), silu_f(x.y), silu_f(x.z), silu_f(x.w));
+            }
+        } else {
+            const int h = (u - 2 * n_k - vjobs) * 32 + lane;
+            if (h < n_v) {
+                const float a = alpha[r * n_v + h] + dt_bias[h];
+                const float sp = a > 20.0f ? a : log_f(1.0f + exp_f(a));
+                gb[(r * n_v + h) * 2] = exp_f(sp * ssm_a[h]);
+                gb[(r * n_v + h) * 2 + 1] = sigmoid_f(beta[r * n_v + h]);
+            }
         }
     }
 }
@@ -467,30 +482,39 @@ __global__ void __launch_bounds__(128, 4) k_gdn_step(const float* qh, const floa
 }
 
 // Gated RMSNorm of the recurrence's output, the SiLU(z) gate and the Q8_0 quantisation of the result
-// (src/model/qwen35.rs:1319-1325). grid (rows, n_v), block sv.
-__global__ void k_gdn_post(const float* o, const float* z, const float* norm_w, int sv, int n_v, float eps, int8_t* out_q, float* out_s) {
-    __shared__ double red[8];
+// (src/model/qwen35.rs:1319-1325). Blocks and warps as in k_gdn_pre (75 MB at 2,048 rows of 4,096, 11 us; a block per head 65 us, this 42).
+template <int NJ>
+__global__ void __launch_bounds__(256) k_gdn_post(const float* o, const float* z, const float* norm_w, int n_v, float eps, int8_t* out_q, float* out_s) {
+    constexpr int sv = NJ * 32;
     const size_t r = blockIdx.x;
-    const int h = blockIdx.y, d = threadIdx.x;
-    const size_t idx = (r * n_v + h) * sv + d;
-    const float v = o[idx];
-    double acc = warp_sum_d((double)(v * v));
-    if ((d & 31) == 0) red[d >> 5] = acc;
-    __syncthreads();
-    double tot = 0.0;
-    for (int w = 0; w < sv / 32; ++w) tot += red[w];
-    const float mean = (float)(tot / (double)sv);
-    const float sc = 1.0f / sqrtf(mean + eps);
-    const float core = v * sc * norm_w[d];
-    const float val = silu_f(z[idx]) * core;
-    float dq;
-    const int8_t q = warp_quant_q8(val, &dq);
-    out_q[idx] = q;
-    if ((d & 31) == 0) out_s[idx / 32] = dq;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float nw[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) nw[j] = norm_w[lane + 32 * j];
+    for (int h = blockIdx.y * 8 + wid; h < n_v; h += 8 * gridDim.y) {
+        const size_t idx = (r * n_v + h) * sv + lane;
+        float v[NJ], g[NJ];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) { v[j] = o[idx + 32 * j]; g[j] = z[idx + 32 * j]; }
+        double tot = 0.0;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) tot += warp_sum_d((double)(v[j] * v[j]));
+        const float mean = (float)(tot / (double)sv);
+        const float sc = 1.0f / sqrtf(mean + eps);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const float core = v[j] * sc * nw[j];
+            const float val = silu_f(g[j]) * core;
+            float dq;
+            const int8_t q = warp_quant_q8(val, &dq);
+            out_q[idx + 32 * j] = q;
+            if (lane == 0) out_s[idx / 32 + j] = dq;
+        }
+    }
 }
 
 // Attention prologue per (row, head): as k_attn_prep, the row's sequence and position derived from the pass
-// shape: sequence = row / n_tok, position = pos[sequence] + row % n_tok. grid (n_head + 2*n_head_kv, rows).
+// shape: sequence = row / n_tok, position = pos[sequence] + row % n_tok.
 struct AttnPrepRows {
     const float* qg; const float* k; const float* v;
     const float* q_norm; const float* k_norm;
@@ -499,50 +523,55 @@ struct AttnPrepRows {
     const int* pos; int* npos_out; int n_tok;
     int hd, n_head, n_head_kv, n_rot; float theta, eps; int bf16;
 };
-__global__ void k_attn_prep_rows(AttnPrepRows p) {
+// Blocks and warps as in k_gdn_pre: the row's rotations once, in double as the CPU takes them, then a warp per head (a block per (row,
+// head) took each rotation 18 times: 116 us at 2,048 rows of 16 + 2 + 2 heads of 256, this 63). Dynamic shared memory: n_rot + 8 * hd floats.
+__global__ void __launch_bounds__(256) k_attn_prep_rows(AttnPrepRows p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float* val = (float*)smem;
-    __shared__ double red[8];
-    const int job = blockIdx.x, d = threadIdx.x, hd = p.hd, kvd = p.n_head_kv * hd;
-    const size_t r = blockIdx.y;
+    const int hd = p.hd, nj = hd / 32, half = p.n_rot / 2, kvd = p.n_head_kv * hd, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    float* cs = (float*)smem; float* sn = cs + half; float* val = sn + half + wid * hd;
+    const size_t r = blockIdx.x;
     const int s = (int)(r / p.n_tok), pos = p.pos[s] + (int)(r % p.n_tok);
-    if (job == 0 && d == 0) p.npos_out[r] = pos + 1;
-    const bool is_q = job < p.n_head, is_k = !is_q && job < p.n_head + p.n_head_kv;
-    const int hk = is_q ? job : is_k ? job - p.n_head : job - p.n_head - p.n_head_kv;
-    float v;
-    if (is_q) {
-        v = p.qg[r * 2 * hd * p.n_head + (size_t)hk * 2 * hd + d];
-        p.g_out[(r * p.n_head + hk) * hd + d] = p.qg[r * 2 * hd * p.n_head + (size_t)hk * 2 * hd + hd + d];
-    } else {
-        v = (is_k ? p.k : p.v)[r * kvd + hk * hd + d];
+    if (tid == 0 && blockIdx.y == 0) p.npos_out[r] = pos + 1;
+    for (int d = tid; d < half; d += 256) {
+        const double freq = pow((double)p.theta, -2.0 * (double)d / (double)p.n_rot), th = (double)pos * freq;
+        sn[d] = (float)sin(th); cs[d] = (float)cos(th);
     }
-    if (is_q || is_k) {
-        double acc = warp_sum_d((double)(v * v));
-        if ((d & 31) == 0) red[d >> 5] = acc;
-        __syncthreads();
-        double tot = 0.0;
-        for (int w = 0; w < hd / 32; ++w) tot += red[w];
-        float mean = (float)(tot / (double)hd);
-        float sc = 1.0f / sqrtf(mean + p.eps);
-        v = v * sc * (is_q ? p.q_norm : p.k_norm)[d];
-        val[d] = v;
-        __syncthreads();
-        const int half = p.n_rot / 2;
-        if (d < half) {
-            double freq = pow((double)p.theta, -2.0 * (double)d / (double)p.n_rot);
-            double th = (double)pos * freq;
-            float sn = (float)sin(th), cs = (float)cos(th);
-            float x0 = val[d], x1 = val[d + half];
-            val[d] = x0 * cs - x1 * sn;
-            val[d + half] = x0 * sn + x1 * cs;
+    __syncthreads();
+    for (int job = blockIdx.y * 8 + wid; job < p.n_head + 2 * p.n_head_kv; job += 8 * gridDim.y) {
+        const bool is_q = job < p.n_head, is_k = !is_q && job < p.n_head + p.n_head_kv;
+        const int hk = is_q ? job : is_k ? job - p.n_head : job - p.n_head - p.n_head_kv;
+        const float* src = is_q ? p.qg + r * 2 * hd * p.n_head + (size_t)hk * 2 * hd : (is_k ? p.k : p.v) + r * kvd + hk * hd;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) if (j < nj) v[j] = src[lane + 32 * j];
+        if (is_q)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (j < nj) p.g_out[(r * p.n_head + hk) * hd + lane + 32 * j] = src[hd + lane + 32 * j];
+        if (is_q || is_k) {
+            double tot = 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (j < nj) tot += warp_sum_d((double)(v[j] * v[j]));
+            const float mean = (float)(tot / (double)hd);
+            const float sc = 1.0f / sqrtf(mean + p.eps);
+            const float* nw = is_q ? p.q_norm : p.k_norm;
+            __syncwarp();                              // everyone has the job before's values
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (j < nj) { v[j] = v[j] * sc * nw[lane + 32 * j]; val[lane + 32 * j] = v[j]; }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int d = lane + 32 * j;
+                if (j < nj && d < half) v[j] = v[j] * cs[d] - val[d + half] * sn[d];
+                else if (j < nj && d < 2 * half) v[j] = val[d - half] * sn[d - half] + v[j] * cs[d - half];
+            }
         }
-        __syncthreads();
-        v = val[d];
-    }
-    if (is_q) p.q_out[(r * p.n_head + hk) * hd + d] = v;
-    else {
-        uint16_t* slab = (is_k ? p.kslab : p.vslab) + (size_t)s * p.slab_stride + (size_t)pos * kvd + hk * hd + d;
-        *slab = p.bf16 ? f32_to_bf16_bits(v) : f32_to_f16_bits(v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j >= nj) continue;
+            const int d = lane + 32 * j;
+            if (is_q) p.q_out[(r * p.n_head + hk) * hd + d] = v[j];
+            else (is_k ? p.kslab : p.vslab)[(size_t)s * p.slab_stride + (size_t)pos * kvd + hk * hd + d] = p.bf16 ? f32_to_bf16_bits(v[j]) : f32_to_f16_bits(v[j]);
+        }
     }
 }
 
