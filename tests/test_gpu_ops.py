@@ -101,6 +101,20 @@ def test_matmul_q8_0_as_f16_tensor_core_gemm(n_in, n_out, n_tok):
     o2.close()
 
 
+@pytest.mark.parametrize("n_in,n_out,n_tok", [(128, 128, 64), (384, 256, 65), (2048, 128, 191), (640, 1280, 1000), (1536, 2432, 515)])
+def test_matmul_q8_0_on_the_tensor_cores_exact(n_in, n_out, n_tok):
+    """dense=q8tc: tiles of 64 tokens (few blocks) and of 128, a last tile of 1, 3 or 63 rows, fewer stages of k than the ring holds and more."""
+    from inferred_thoughts_b200 import host
+    o2 = host.B200Ops(0, "exact=1,dense=q8tc")
+    wb = q8_weights(n_out, n_in, 22 + n_in)
+    x = noise(n_tok * n_in, 23); out = np.zeros(n_tok * n_out, np.float32); want = np.zeros_like(out)
+    o2.begin_pass(n_tok)
+    o2.matmul(host.Weights(wb, host.Q8_0, n_in, n_out), x, out); o2.host_needs(out); o2.check()
+    L.orc_matmul(8, wb, n_in, n_out, x, x.size, want, 0)
+    exact(out, want, "Q8_0 matmul on the tensor cores")
+    o2.close()
+
+
 @pytest.mark.parametrize("n_in,n_out,n_tok", [(2048, 64, 1), (512, 48, 2), (256, 16, 1), (128, 9, 3), (768, 8, 1), (2048, 200, 40), (512, 130, 33)])
 def test_matmul_nvfp4_dense_exact(ops, n_in, n_out, n_tok):
     from inferred_thoughts_b200 import host
