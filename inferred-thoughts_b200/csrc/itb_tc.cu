@@ -16,14 +16,17 @@ __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__
 // Bounded wait on an mbarrier phase: polls (the try_wait itself suspends for a short, hardware-chosen time) and gives up after
 // `limit_cycles` of this SM's clock (the cheap clock: reading the global timer in the polling loop costs microseconds).
 __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit_cycles) {
+    auto arrived = [&] {
+        uint32_t ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        return ok != 0;
+    };
+    if (arrived()) return true;
     const long long t0 = clock64();
     for (;;) {
-        uint32_t ok;
 #pragma unroll 1
-        for (int i = 0; i < 64; ++i) {
-            asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-            if (ok) return true;
-        }
+        for (int i = 0; i < 64; ++i)
+            if (arrived()) return true;
         if ((unsigned long long)(clock64() - t0) > limit_cycles) return false;
     }
 }
@@ -686,10 +689,11 @@ extern "C" int itb_fp4_quantize(itb_ctx* c, const float* x, size_t n, uint8_t* s
 // times (weight scale * activation scale), added to the row's sum in block order. The dot of 128 weight rows against NT activation
 // rows is two tcgen05.mma kind::f16 (M 128, N NT, K 16 each, f32 accumulators in tensor memory, the second accumulating): int8 values
 // are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. Four accumulator
-// buffers rotate, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
+// buffers rotate in pairs, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
 // scales and the addition in the CPU's own order and rounding. The result equals the CPU path to the bit; what bounds the kernel is
 // those three f32 instructions per (output, block): 384 cycles a block of 128 x 128. kind::i8 with eight warps, whose s32 accumulators
-// took two more instructions to convert and which had two warps a scheduler to hide the read-back, took 1,407; this Q8_CYC.
+// took two more instructions to convert and which had two warps a scheduler to hide the read-back, took 1,407; with waits and releases
+// per block this took 1,241, per pair of blocks 911 (128 x 64: 576).
 // Operand images ("K32 block": two K16 blocks of rows x 16 f16 = rows x 32 B as [2 chunks of 16 B][rows / 8][8 rows][16 B], K-major, no
 // swizzle; descriptor leading offset rows * 16, stride offset 128) are made once per weight matrix and once per pass for the activations.
 namespace {
@@ -745,7 +749,7 @@ template <int NT>
 __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int STAGES = q8_stages<NT>(), STAGE = q8_stage_bytes<NT>(), CW = NT / 4, H = CW / 16, B_BLK = NT * 64;
-    __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[4], s_dfree[4];
+    __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[2], s_dfree[2];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int rt = blockIdx.x, tt = blockIdx.y, kbs = p.kbs, n_stage = kbs / Q8_KB;
@@ -755,7 +759,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&s_full[s])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&s_empty[s])), "r"(1 + Q8_EPW) : "memory");      // the MMAs' commit + the warps done with the scales
         }
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 2; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&s_dfull[i])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&s_dfree[i])), "r"(Q8_EPW) : "memory");
         }
@@ -790,26 +794,21 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     } else if (wid == Q8_EPW + 1 && lane == 0) {
         const uint32_t idesc = tc_idesc_f16(128, NT);
         const uint64_t dA = tc_desc(sbase, 2048, 128), dB = tc_desc(sbase + O_B, NT * 16, 128);
-        for (int b = 0; b < kbs && ok; ++b) {
-            const int s = (b / Q8_KB) % STAGES, k = b % Q8_KB, db = b & 3;
-            if (k == 0) {
-                ok = tc_mbar_wait(tc_smem(&s_full[s]), ((b / Q8_KB) / STAGES) & 1, 2000000000ull);
-                if (!ok) break;
-            }
-            if (b >= 4) {
-                ok = tc_mbar_wait(tc_smem(&s_dfree[db]), ((b >> 2) - 1) & 1, 2000000000ull);
-                if (!ok) break;
-            }
+        for (int st = 0; st < n_stage && ok; ++st) {
+            const int s = st % STAGES, dp = st & 1;
+            ok = tc_mbar_wait(tc_smem(&s_full[s]), (st / STAGES) & 1, 2000000000ull);
+            if (ok && st >= 2) ok = tc_mbar_wait(tc_smem(&s_dfree[dp]), ((st >> 1) - 1) & 1, 2000000000ull);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t so = (uint32_t)s * (STAGE >> 4);
 #pragma unroll
-            for (uint32_t i = 0; i < 2; ++i)
+            for (uint32_t i = 0; i < 2 * Q8_KB; ++i)
                 asm volatile(
                     "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }\n"
-                    ::"r"(tm + (uint32_t)NT * db), "l"(dA + so + (Q8_A_BLK / 16) * k + (Q8_A_BLK / 32) * i), "l"(dB + so + (B_BLK / 16) * k + (B_BLK / 32) * i), "r"(idesc), "r"(i) : "memory");
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_dfull[db])) : "memory");
-            if (k == Q8_KB - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
+                    ::"r"(tm + (uint32_t)NT * (Q8_KB * dp + i / 2)), "l"(dA + so + (Q8_A_BLK / 32) * i), "l"(dB + so + (B_BLK / 32) * i), "r"(idesc), "r"(i & 1) : "memory");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_dfull[dp])) : "memory");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
         }
         if (!ok) atomicCAS(p.status, 0, 4);
     } else if (wid < Q8_EPW) {
@@ -818,53 +817,59 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
 #pragma unroll
         for (int j = 0; j < CW; ++j) acc[j] = 0.0f;
         uint32_t d0[16], d1[16];
-        // unit u: 16 of this warp's columns of block u / H. Start reading its accumulators (asynchronous: tcgen05.wait::ld ends it); a
-        // block's first unit also waits for the block's MMAs (and, at a stage's first block, for the stage's scales)
-        auto fetch = [&](int u, uint32_t (&d)[16]) {
-            const int b = u / H, h = u % H, s = (b / Q8_KB) % STAGES, k = b % Q8_KB, db = b & 3;
-            if (h == 0) {
-                if (k == 0) ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_full[s]), ((b / Q8_KB) / STAGES) & 1, 2000000000ull));
-                ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_dfull[db]), (b >> 2) & 1, 2000000000ull));
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            if (!ok) return;
-            const uint32_t ta = tm + (uint32_t)(NT * db + col0 + 16 * h) + ((uint32_t)(quarter * 32) << 16);
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        // A stage's two blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
+        // it: 16 of this warp's columns of block i / H; load starts reading them (asynchronous: tcgen05.wait::ld ends it).
+        auto open = [&](int st, int s, uint32_t phase) {
+            ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_full[s]), phase, 2000000000ull));
+            ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_dfull[st & 1]), (st >> 1) & 1, 2000000000ull));
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        };
+        auto load = [&](int st, int i, uint32_t (&d)[16]) {
+            const uint32_t ta = tm + (uint32_t)(NT * (Q8_KB * (st & 1) + i / H) + col0 + 16 * (i % H)) + ((uint32_t)(quarter * 32) << 16);
+            if (ok)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]),
                            "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]) : "r"(ta) : "memory");
         };
         // scale and add a unit in the CPU's order: sum += dot * (dw * dx)
-        auto scale_add = [&](int u, int h, const uint32_t (&d)[16]) {
-            const int b = u / H, s = (b / Q8_KB) % STAGES, k = b % Q8_KB;
-            const float* sa = (const float*)(smem + (size_t)s * STAGE + O_SA) + k * 128;
-            const float* sb = (const float*)(smem + (size_t)s * STAGE + O_SB) + k * NT + col0 + 16 * h;
-            const float dw = sa[row];
+        auto scale_add = [&](const unsigned char* stage, int i, const uint32_t (&d)[16]) {
+            const float* sb = (const float*)(stage + O_SB) + i / H * NT + col0 + 16 * (i % H);
+            const float dw = ((const float*)(stage + O_SA))[i / H * 128 + row];
 #pragma unroll
             for (int j = 0; j < 16; j += 4) {
                 const float4 dx = *(const float4*)(sb + j);
                 const float dxs[4] = {dx.x, dx.y, dx.z, dx.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    acc[16 * h + j + i] = __fadd_rn(acc[16 * h + j + i], __fmul_rn(__uint_as_float(d[j + i]), __fmul_rn(dw, dxs[i])));
+                for (int c = 0; c < 4; ++c) {
+                    float& a = acc[16 * (i % H) + j + c];
+                    a = __fadd_rn(a, __fmul_rn(__uint_as_float(d[j + c]), __fmul_rn(dw, dxs[c])));
+                }
             }
         };
         long long* pf = p.prof ? p.prof + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 : nullptr;
         const long long t_begin = clock64();
-        const int units = kbs * H;                 // even: kbs is
         auto arrive = [&](unsigned long long* bar) { if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory"); };
-        fetch(0, d0); fetch(1, d1);
+        open(0, 0, 0); load(0, 0, d0); load(0, 1, d1);
+        int s = 0; uint32_t phase = 0;
 #pragma unroll 1
-        for (int u = 0; u < units && ok; u += 2) {
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");      // both units are in registers
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            arrive(&s_dfree[u / H & 3]);
-            if (H == 1) arrive(&s_dfree[(u + 1) & 3]);
-            scale_add(u, 0, d0);
-            if (u + 2 < units) fetch(u + 2, d0);                              // lands while the second unit is being added
-            scale_add(u + 1, H - 1, d1);
-            if (u + 3 < units) fetch(u + 3, d1);
-            const int b = (u + 1) / H;
-            if (b % Q8_KB == Q8_KB - 1) { __syncwarp(); arrive(&s_empty[(b / Q8_KB) % STAGES]); }
+        for (int st = 0; st < n_stage && ok; ++st) {
+            const unsigned char* stage = smem + (size_t)s * STAGE;
+            const int s_next = s + 1 == STAGES ? 0 : s + 1; const uint32_t p_next = s_next ? phase : phase ^ 1u;
+            const bool more = st + 1 < n_stage;
+#pragma unroll
+            for (int g = 0; g < H; ++g) {
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");      // both units are in registers
+                if (g == H - 1) { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); arrive(&s_dfree[st & 1]); }
+                scale_add(stage, 2 * g, d0);
+                if (g < H - 1) load(st, 2 * g + 2, d0);                           // lands while the second unit is being added
+                else if (more) { open(st + 1, s_next, p_next); load(st + 1, 0, d0); }
+                scale_add(stage, 2 * g + 1, d1);
+                if (g < H - 1) load(st, 2 * g + 3, d1);
+                else if (more) load(st + 1, 1, d1);
+            }
+            __syncwarp();
+            arrive(&s_empty[s]);
+            s = s_next; phase = p_next;
         }
         if (pf && tid == 0) { pf[0] = clock64() - t_begin; }
         if (ok && __shfl_sync(0xffffffffu, *(volatile int*)p.status, 0) == 0) {
