@@ -688,20 +688,20 @@ extern "C" int itb_fp4_quantize(itb_ctx* c, const float* x, size_t n, uint8_t* s
 // The CPU path's Q8_0 dot (src/ops/naive.rs:676-712) is, per 32-element block, an integer dot product, converted to f32,
 // times (weight scale * activation scale), added to the row's sum in block order. The dot of 128 weight rows against NT activation
 // rows is two tcgen05.mma kind::f16 (M 128, N NT, K 16 each, f32 accumulators in tensor memory, the second accumulating): int8 values
-// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. Four accumulator
-// buffers rotate in pairs, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
+// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. Two stages'
+// accumulators fill tensor memory, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
 // scales and the addition in the CPU's own order and rounding. The result equals the CPU path to the bit; what bounds the kernel is
 // those three f32 instructions per (output, block): 384 cycles a block of 128 x 128. kind::i8 with eight warps, whose s32 accumulators
 // took two more instructions to convert and which had two warps a scheduler to hide the read-back, took 1,407; with waits and releases
-// per block this took 1,241, per pair of blocks 911 (128 x 64: 576).
+// per block this took 1,241, per stage of two 911 (128 x 64: 880, per stage of two 576, of four 457).
 // Operand images ("K32 block": two K16 blocks of rows x 16 f16 = rows x 32 B as [2 chunks of 16 B][rows / 8][8 rows][16 B], K-major, no
 // swizzle; descriptor leading offset rows * 16, stride offset 128) are made once per weight matrix and once per pass for the activations.
 namespace {
 
-constexpr int Q8_KB = 2;           // K32 blocks per pipeline stage
+template <int NT> __host__ __device__ constexpr int q8_kb() { return 256 / NT; }      // K32 blocks per pipeline stage: two stages' accumulators fill tensor memory
 constexpr int Q8_EPW = 16;         // warps that read accumulators back
 constexpr int Q8_A_BLK = 128 * 64;                                         // bytes of a weight K32 block
-template <int NT> __host__ __device__ constexpr int q8_stage_bytes() { return Q8_KB * (Q8_A_BLK + NT * 64 + (128 + NT) * 4); }     // A | B | weight scales | activation scales
+template <int NT> __host__ __device__ constexpr int q8_stage_bytes() { return q8_kb<NT>() * (Q8_A_BLK + NT * 64 + (128 + NT) * 4); }     // A | B | weight scales | activation scales
 template <int NT> __host__ __device__ constexpr int q8_stages() { return 200 * 1024 / q8_stage_bytes<NT>(); }
 
 // kind::f16: f32 accumulators (1 at bit 4), f16 operands (0 at bits 7 and 10), both K-major, M x N
@@ -748,11 +748,11 @@ struct TcQ8 {
 template <int NT>
 __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int STAGES = q8_stages<NT>(), STAGE = q8_stage_bytes<NT>(), CW = NT / 4, H = CW / 16, B_BLK = NT * 64;
+    constexpr int STAGES = q8_stages<NT>(), STAGE = q8_stage_bytes<NT>(), CW = NT / 4, H = CW / 16, B_BLK = NT * 64, KB = q8_kb<NT>(), PAIRS = KB * H / 2;
     __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[2], s_dfree[2];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int rt = blockIdx.x, tt = blockIdx.y, kbs = p.kbs, n_stage = kbs / Q8_KB;
+    const int rt = blockIdx.x, tt = blockIdx.y, kbs = p.kbs, n_stage = kbs / KB;
     const uint32_t sbase = tc_smem(smem);
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tm = s_tmem;
-    constexpr uint32_t O_B = Q8_KB * Q8_A_BLK, O_SA = O_B + Q8_KB * B_BLK, O_SB = O_SA + Q8_KB * 128 * 4;
+    constexpr uint32_t O_B = KB * Q8_A_BLK, O_SA = O_B + KB * B_BLK, O_SB = O_SA + KB * 128 * 4;
     bool ok = true;
     if (wid == Q8_EPW && lane == 0) {
         const size_t a0 = (size_t)rt * kbs, b0 = (size_t)tt * kbs;
@@ -784,11 +784,11 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             if (!ok) break;
             const uint32_t full = tc_smem(&s_full[s]), dst = sbase + s * STAGE;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)STAGE) : "memory");
-            const size_t kb0 = (size_t)st * Q8_KB;
-            tc_bulk(dst, p.a_img + (a0 + kb0) * Q8_A_BLK, Q8_KB * Q8_A_BLK, full);
-            tc_bulk(dst + O_B, p.b_img + (b0 + kb0) * B_BLK, Q8_KB * B_BLK, full);
-            tc_bulk(dst + O_SA, p.a_sc + (a0 + kb0) * 128, Q8_KB * 128 * 4, full);
-            tc_bulk(dst + O_SB, p.b_sc + (b0 + kb0) * NT, Q8_KB * NT * 4, full);
+            const size_t kb0 = (size_t)st * KB;
+            tc_bulk(dst, p.a_img + (a0 + kb0) * Q8_A_BLK, KB * Q8_A_BLK, full);
+            tc_bulk(dst + O_B, p.b_img + (b0 + kb0) * B_BLK, KB * B_BLK, full);
+            tc_bulk(dst + O_SA, p.a_sc + (a0 + kb0) * 128, KB * 128 * 4, full);
+            tc_bulk(dst + O_SB, p.b_sc + (b0 + kb0) * NT, KB * NT * 4, full);
         }
         if (!ok) atomicCAS(p.status, 0, 3);
     } else if (wid == Q8_EPW + 1 && lane == 0) {
@@ -802,11 +802,11 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t so = (uint32_t)s * (STAGE >> 4);
 #pragma unroll
-            for (uint32_t i = 0; i < 2 * Q8_KB; ++i)
+            for (uint32_t i = 0; i < 2 * KB; ++i)
                 asm volatile(
                     "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }\n"
-                    ::"r"(tm + (uint32_t)NT * (Q8_KB * dp + i / 2)), "l"(dA + so + (Q8_A_BLK / 32) * i), "l"(dB + so + (B_BLK / 32) * i), "r"(idesc), "r"(i & 1) : "memory");
+                    ::"r"(tm + (uint32_t)NT * (KB * dp + i / 2)), "l"(dA + so + (Q8_A_BLK / 32) * i), "l"(dB + so + (B_BLK / 32) * i), "r"(idesc), "r"(i & 1) : "memory");
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_dfull[dp])) : "memory");
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
         }
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
 #pragma unroll
         for (int j = 0; j < CW; ++j) acc[j] = 0.0f;
         uint32_t d0[16], d1[16];
-        // A stage's two blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
+        // A stage's blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
         // it: 16 of this warp's columns of block i / H; load starts reading them (asynchronous: tcgen05.wait::ld ends it).
         auto open = [&](int st, int s, uint32_t phase) {
             ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_full[s]), phase, 2000000000ull));
@@ -825,7 +825,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         };
         auto load = [&](int st, int i, uint32_t (&d)[16]) {
-            const uint32_t ta = tm + (uint32_t)(NT * (Q8_KB * (st & 1) + i / H) + col0 + 16 * (i % H)) + ((uint32_t)(quarter * 32) << 16);
+            const uint32_t ta = tm + (uint32_t)(NT * (KB * (st & 1) + i / H) + col0 + 16 * (i % H)) + ((uint32_t)(quarter * 32) << 16);
             if (ok)
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]),
@@ -857,14 +857,14 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             const int s_next = s + 1 == STAGES ? 0 : s + 1; const uint32_t p_next = s_next ? phase : phase ^ 1u;
             const bool more = st + 1 < n_stage;
 #pragma unroll
-            for (int g = 0; g < H; ++g) {
+            for (int g = 0; g < PAIRS; ++g) {
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");      // both units are in registers
-                if (g == H - 1) { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); arrive(&s_dfree[st & 1]); }
+                if (g == PAIRS - 1) { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); arrive(&s_dfree[st & 1]); }
                 scale_add(stage, 2 * g, d0);
-                if (g < H - 1) load(st, 2 * g + 2, d0);                           // lands while the second unit is being added
+                if (g < PAIRS - 1) load(st, 2 * g + 2, d0);                           // lands while the second unit is being added
                 else if (more) { open(st + 1, s_next, p_next); load(st + 1, 0, d0); }
                 scale_add(stage, 2 * g + 1, d1);
-                if (g < H - 1) load(st, 2 * g + 3, d1);
+                if (g < PAIRS - 1) load(st, 2 * g + 3, d1);
                 else if (more) load(st + 1, 1, d1);
             }
             __syncwarp();
