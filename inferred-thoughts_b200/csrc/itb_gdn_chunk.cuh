@@ -167,39 +167,28 @@ __global__ void __launch_bounds__(256) k_gdn_chunk_scan(const float* scratch, in
 #pragma unroll 1
     for (int ch = 0; ch < n_ch; ++ch) {
         const int t0 = ch * GC, nv = min(GC, n_tok - t0);
-        cp_async_wait<2>();                    // W of this chunk (the groups behind it: its Q/P and K/U)
+        cp_async_wait<1>();                    // W, Q, P and U of this chunk (behind them: its K)
         __syncthreads();                       // ... and the state as the previous chunk left it
-        float acc[4][2];
-        // D = U - W S^T
+        // D = U - W S^T and the first half of O = Qg S^T + P D in one walk over the keys: the state is read once for both, and sixteen
+        // sums a thread hide the reads' latency (one after the other, eight each: 317 us a layer at 2,048 tokens; now 301. Shared
+        // memory bounds it: half the work to each of 512 threads reads more and took 338)
+        float acc[4][2], oc[4][2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) { acc[a][0] = 0.f; acc[a][1] = 0.f; }
+        for (int a = 0; a < 4; ++a) { acc[a][0] = 0.f; acc[a][1] = 0.f; oc[a][0] = 0.f; oc[a][1] = 0.f; }
+#pragma unroll 2
         for (int i = 0; i < SK; i += 4) {
             const float4 s0 = ld4(S + jq * ST + i), s1 = ld4(S + (jq + 16) * ST + i);
+            auto add = [&](float& sum, const float4& w, const float4& v) { sum = __fmaf_rn(w.x, v.x, sum); sum = __fmaf_rn(w.y, v.y, sum); sum = __fmaf_rn(w.z, v.z, sum); sum = __fmaf_rn(w.w, v.w, sum); };
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const float4 w = ld4(Ws + (tq + a) * ST + i);
-                acc[a][0] = __fmaf_rn(w.x, s0.x, acc[a][0]); acc[a][0] = __fmaf_rn(w.y, s0.y, acc[a][0]); acc[a][0] = __fmaf_rn(w.z, s0.z, acc[a][0]); acc[a][0] = __fmaf_rn(w.w, s0.w, acc[a][0]);
-                acc[a][1] = __fmaf_rn(w.x, s1.x, acc[a][1]); acc[a][1] = __fmaf_rn(w.y, s1.y, acc[a][1]); acc[a][1] = __fmaf_rn(w.z, s1.z, acc[a][1]); acc[a][1] = __fmaf_rn(w.w, s1.w, acc[a][1]);
+                const float4 w = ld4(Ws + (tq + a) * ST + i), q = ld4(Qs + (tq + a) * ST + i);
+                add(acc[a][0], w, s0); add(acc[a][1], w, s1); add(oc[a][0], q, s0); add(oc[a][1], q, s1);
             }
         }
         __syncthreads();                       // every thread is done with W
         load_w(ch + 1);
-        cp_async_wait<2>();                    // Q, P and U of this chunk (behind them: K, the next W)
-        __syncthreads();
 #pragma unroll
         for (int a = 0; a < 4; ++a) { D[(tq + a) * DS + jq] = Us[(tq + a) * DS + jq] - acc[a][0]; D[(tq + a) * DS + jq + 16] = Us[(tq + a) * DS + jq + 16] - acc[a][1]; }
-        // O = Qg S^T + P D
-#pragma unroll
-        for (int a = 0; a < 4; ++a) { acc[a][0] = 0.f; acc[a][1] = 0.f; }
-        for (int i = 0; i < SK; i += 4) {
-            const float4 s0 = ld4(S + jq * ST + i), s1 = ld4(S + (jq + 16) * ST + i);
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float4 w = ld4(Qs + (tq + a) * ST + i);
-                acc[a][0] = __fmaf_rn(w.x, s0.x, acc[a][0]); acc[a][0] = __fmaf_rn(w.y, s0.y, acc[a][0]); acc[a][0] = __fmaf_rn(w.z, s0.z, acc[a][0]); acc[a][0] = __fmaf_rn(w.w, s0.w, acc[a][0]);
-                acc[a][1] = __fmaf_rn(w.x, s1.x, acc[a][1]); acc[a][1] = __fmaf_rn(w.y, s1.y, acc[a][1]); acc[a][1] = __fmaf_rn(w.z, s1.z, acc[a][1]); acc[a][1] = __fmaf_rn(w.w, s1.w, acc[a][1]);
-            }
-        }
         __syncthreads();                       // D is complete
         for (int s = 0; s < GC; s += 4) {
             float d0[4], d1[4];
@@ -208,15 +197,15 @@ __global__ void __launch_bounds__(256) k_gdn_chunk_scan(const float* scratch, in
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 const float4 pr = ld4(Ps + (tq + a) * PS + s);
-                acc[a][0] = __fmaf_rn(pr.x, d0[0], acc[a][0]); acc[a][0] = __fmaf_rn(pr.y, d0[1], acc[a][0]); acc[a][0] = __fmaf_rn(pr.z, d0[2], acc[a][0]); acc[a][0] = __fmaf_rn(pr.w, d0[3], acc[a][0]);
-                acc[a][1] = __fmaf_rn(pr.x, d1[0], acc[a][1]); acc[a][1] = __fmaf_rn(pr.y, d1[1], acc[a][1]); acc[a][1] = __fmaf_rn(pr.z, d1[2], acc[a][1]); acc[a][1] = __fmaf_rn(pr.w, d1[3], acc[a][1]);
+                oc[a][0] = __fmaf_rn(pr.x, d0[0], oc[a][0]); oc[a][0] = __fmaf_rn(pr.y, d0[1], oc[a][0]); oc[a][0] = __fmaf_rn(pr.z, d0[2], oc[a][0]); oc[a][0] = __fmaf_rn(pr.w, d0[3], oc[a][0]);
+                oc[a][1] = __fmaf_rn(pr.x, d1[0], oc[a][1]); oc[a][1] = __fmaf_rn(pr.y, d1[1], oc[a][1]); oc[a][1] = __fmaf_rn(pr.z, d1[2], oc[a][1]); oc[a][1] = __fmaf_rn(pr.w, d1[3], oc[a][1]);
             }
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a)
             if (tq + a < nv) {
                 float* o = out + (((size_t)seq * n_tok + t0 + tq + a) * n_v + h) * SK + vs0;
-                o[jq] = acc[a][0]; o[jq + 16] = acc[a][1];
+                o[jq] = oc[a][0]; o[jq + 16] = oc[a][1];
             }
         // S = G_C S + D^T Kd
         float up[4][4];
