@@ -1227,15 +1227,14 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     cudaStreamCaptureStatus cap_rows = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cap_rows);
     const bool f16tc = c->f16tc && n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone;
-    // same: this matmul reads the quantised rows the previous one read (their tensor-core images are still current)
-    auto gemm_n = [&](const DevQ8& w, const int8_t* xq, const float* xs, float* out, size_t stride, int mode, int R, bool same = false) {
-        dense_q8(c, st, w, xq, xs, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone, same);
+    auto gemm_n = [&](const DevQ8& w, const QRows& x, float* out, size_t stride, int mode, int R) {
+        dense_q8(c, st, w, x, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone);
         launches++;
     };
-    auto gemm = [&](const DevQ8& w, const int8_t* xq, const float* xs, float* out, size_t stride, int mode, bool same = false) { gemm_n(w, xq, xs, out, stride, mode, R, same); };
+    auto gemm = [&](const DevQ8& w, const QRows& x, float* out, size_t stride, int mode) { gemm_n(w, x, out, stride, mode, R); };
     // two or three dense matrices over the same quantised rows (mode 0): with few rows (batched decode) one launch for all of
-    // them; otherwise one after the other, the later ones told that the rows' tensor-core images are current
-    auto gemm_multi = [&](int n, const DevQ8* const* w, float* const* out, const size_t* stride, const int8_t* xq, const float* xs) {
+    // them; otherwise one after the other, the later ones reading the tensor-core image the first one made of the rows
+    auto gemm_multi = [&](int n, const DevQ8* const* w, float* const* out, const size_t* stride, const QRows& x) {
         bool one = R <= 32 && n <= 3;
         for (int i = 0; i < n; ++i) one = one && w[i]->q && w[i]->n_in == w[0]->n_in && w[i]->n_in % 256 == 0;
         if (one) {
@@ -1244,11 +1243,11 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             int tiles = 0;
             for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; p.tiles[i] = (w[i]->n_out + 31) / 32; tiles += p.tiles[i]; }
             const int k = w[0]->n_in, ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8_multi<1, 256, 4><<<dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(p, xq, xs, R, ns);
+            k_tile_q8_multi<1, 256, 4><<<dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(p, x.q, x.s, R, ns);
             launches++;
             return;
         }
-        for (int i = 0; i < n; ++i) gemm(*w[i], xq, xs, out[i], stride[i], 0, i > 0);
+        for (int i = 0; i < n; ++i) gemm(*w[i], x, out[i], stride[i], 0);
     };
     // A dense matrix stored as NVFP4 (shared experts, LM head of an NVFP4 file): int8 activations x E2M1 weights in the CPU
     // order (src/ops/naive.rs:714-734), then the tensor's second scale on the result (src/model/qwen35.rs:1668-1682).
@@ -1304,12 +1303,13 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     for (uint32_t il = 0; il < d.n_layer; ++il) {
         const DevLayer& L = m->layers[il];
         k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.attn_norm, H, d.rms_eps, e->xn, e->xq, e->xs); launches++;
+        const QRows xa = c->quantised(e->xq, e->xs);
         if (L.recurrent) {
             const int rs = e->slot_of[il];
             const size_t state_stride = (size_t)n_v * sk * sk, conv_stride = (size_t)cd * (d.ssm_d_conv - 1);
             {
                 const DevQ8* ws[2] = {&L.wqkv, &L.wgate}; float* os[2] = {e->qkvc, e->z}; const size_t ss[2] = {(size_t)cd, (size_t)vd};
-                gemm_multi(2, ws, os, ss, e->xq, e->xs);
+                gemm_multi(2, ws, os, ss, xa);
             }
             f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn);
             float* cst = e->conv_state + (size_t)rs * e->B * conv_stride;
@@ -1336,12 +1336,12 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             }
             launches++;
             (sk == 128 ? k_gdn_post<4> : k_gdn_post<2>)<<<dim3(R, row_share(R, n_v, sms)), 256, 0, st>>>(e->core, e->z, L.ssm_norm, n_v, d.rms_eps, e->aq, e->as); launches++;
-            gemm(L.ssm_out, e->aq, e->as, e->x, H, 1);
+            gemm(L.ssm_out, c->quantised(e->aq, e->as), e->x, H, 1);
         } else {
             const int as = e->slot_of[il];
             {
                 const DevQ8* ws[3] = {&L.wq, &L.wk, &L.wv}; float* os[3] = {e->qg, e->kbuf, e->vbuf}; const size_t ss[3] = {(size_t)2 * qd, (size_t)kvd, (size_t)kvd};
-                gemm_multi(3, ws, os, ss, e->xq, e->xs);
+                gemm_multi(3, ws, os, ss, xa);
             }
             AttnPrepRows a{};
             a.qg = e->qg; a.k = e->kbuf; a.v = e->vbuf; a.q_norm = L.q_norm; a.k_norm = L.k_norm; a.q_out = e->qn; a.g_out = e->gate;
@@ -1392,18 +1392,19 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             k_attn_combine_rows<<<R * d.n_head, d.head_dim, 0, st>>>(e->part_acc, e->part_ml, ns, d.head_dim, e->gate, e->npos, d.n_head,
                                                                     e->aq, e->as); launches++;
             }
-            gemm(L.wo, e->aq, e->as, e->x, H, 1);
+            gemm(L.wo, c->quantised(e->aq, e->as), e->x, H, 1);
         }
         // routed FFN
         k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, e->ep ? nullptr : e->xh); launches++;
+        const QRows xf = c->quantised(e->xq, e->xs);
         if (!L.shared4[0].nib && !L.shared4[1].nib) {
             const DevQ8* ws[2] = {&L.shared_gate, &L.shared_up}; float* os[2] = {e->sg, e->su}; const size_t ss[2] = {(size_t)d.shared_ff, (size_t)d.shared_ff};
-            gemm_multi(2, ws, os, ss, e->xq, e->xs);
+            gemm_multi(2, ws, os, ss, xf);
         } else {
             if (L.shared4[0].nib) gemm_fp4d(L.shared4[0], e->xq, e->xs, e->sg, R, L.has_shared_s[0], L.shared_s[0]);
-            else gemm(L.shared_gate, e->xq, e->xs, e->sg, d.shared_ff, 0);
+            else gemm(L.shared_gate, xf, e->sg, d.shared_ff, 0);
             if (L.shared4[1].nib) gemm_fp4d(L.shared4[1], e->xq, e->xs, e->su, R, L.has_shared_s[1], L.shared_s[1]);
-            else gemm(L.shared_up, e->xq, e->xs, e->su, d.shared_ff, 0, !L.shared4[0].nib);
+            else gemm(L.shared_up, xf, e->su, d.shared_ff, 0);
         }
         f32mm2(L.gate_inp, e->router, L.shared_gate_inp, e->shlogit, e->xn);
         {
@@ -1552,7 +1553,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             }
             k_shared_act_rows<<<R, 128, 0, st>>>(e->sg, e->su, d.shared_ff, e->sq, e->ss); launches++;
             if (L.shared4[2].nib) gemm_fp4d(L.shared4[2], e->sq, e->ss, e->shd, R, L.has_shared_s[2], L.shared_s[2]);
-            else gemm(L.shared_down, e->sq, e->ss, e->shd, H, 0);
+            else gemm(L.shared_down, c->quantised(e->sq, e->ss), e->shd, H, 0);
             const size_t total = (size_t)R * H;
             k_moe_finish_rows<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
         }
@@ -1564,7 +1565,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         // several sequences: one pass over the output matrix for all of them
         k_norm_quant<<<n_seq, 256, smem_nq, st>>>(xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs); launches++;
         if (m->output4.nib) gemm_fp4d(m->output4, e->xq, e->xs, e->logits, n_seq, m->has_output_s, m->output_s);
-        else gemm_n(m->output, e->xq, e->xs, e->logits, d.n_vocab, 0, n_seq);
+        else gemm_n(m->output, c->quantised(e->xq, e->xs), e->logits, d.n_vocab, 0, n_seq);
     } else if (m->output4.nib) {
         k_norm_quant<<<1, 256, smem_nq, st>>>(xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs); launches++;
         gemm_fp4d(m->output4, e->xq, e->xs, e->logits, 1, m->has_output_s, m->output_s);

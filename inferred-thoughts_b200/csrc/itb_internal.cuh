@@ -69,6 +69,14 @@ struct WeightEntry {
     size_t bytes = 0;
 };
 
+// Q8_0-quantised activation rows as the matmuls read them. id: which quantisation wrote them, a number no other one of the context
+// has (itb_ctx::quantised; 0: none). What is derived from the rows and kept is kept under it: the buffer is the same in every call.
+struct QRows {
+    const int8_t* q = nullptr;   // [rows][n_in]
+    const float* s = nullptr;    // [rows][n_in / 32]
+    uint64_t id = 0;
+};
+
 struct HostPipe;                 // pinned staging and copy threads of one context (itb_ctx.cu)
 struct itb_ctx {
     int device = 0;
@@ -93,6 +101,8 @@ struct itb_ctx {
     size_t route_grouped = 0; int route_tile_cap = 0;      // expert count and tile size pair_off / pair_list / pair_tiles were made for (0: not for this route)
     // scratch for activation quantisation
     int8_t* xq = nullptr; float* xs = nullptr; size_t xq_cap = 0;
+    uint64_t n_quantised = 0;
+    QRows quantised(const int8_t* q, const float* s) { return QRows{q, s, ++n_quantised}; }     // to be called where a kernel that writes them is launched
     float* tmp_f32 = nullptr; size_t tmp_cap = 0;
     const void* last_state_key = nullptr;
     size_t mirror_bytes = 0, weight_bytes = 0;
@@ -104,9 +114,9 @@ struct itb_ctx {
     size_t tc_cap_tiles = 0, tc_cap_slots = 0, tc_cap_b = 0, tc_cap_sf = 0, tc_cap_codes = 0, tc_cap_scales = 0;
     // Q8_0 tensor path: the pass's activation rows as K32 block images (kept for a following matmul over the same rows)
     uint8_t* tc_q8_b = nullptr; float* tc_q8_sx = nullptr; size_t tc_cap_q8b = 0, tc_cap_q8sx = 0;
-    const void* tc_q8_src = nullptr; int tc_q8_src_rows = 0, tc_q8_src_in = 0, tc_q8_src_tile = 0;
+    uint64_t tc_q8_src = 0; int tc_q8_src_rows = 0, tc_q8_src_in = 0, tc_q8_src_tile = 0;      // the quantisation (QRows::id) they were made from
     uint8_t* tc_hf_b = nullptr; size_t tc_cap_hfb = 0;                 // dense=f16tc: the pass's activation rows as f16 operand tiles
-    const void* tc_hf_src = nullptr; int tc_hf_src_rows = 0, tc_hf_src_in = 0;
+    uint64_t tc_hf_src = 0; int tc_hf_src_rows = 0, tc_hf_src_in = 0;
     bool f16tc = false;     // opts dense=f16tc: many-row passes run the dense Q8_0 matmuls as f16 tcgen05 GEMMs over dequantised operands (tolerance class)
     bool q8tc = false;       // opts dense=q8tc: many-row passes run the dense Q8_0 matmuls as tcgen05 int8 MMAs (bit-identical results)
     bool fp4tc = false;      // opts experts=fp4tc: many-row passes multiply FP4 activations on the tensor cores
@@ -120,8 +130,8 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
 bool itb_tc_shape_ok(const DevFp4& w);
 bool itb_tc_q8_shape_ok(const DevQ8& w);
 bool itb_tc_f16_shape_ok(const DevQ8& w);
-bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool same_acts);
-bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool same_acts);
+bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode);
+bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode);
 void itb_tc_free(itb_ctx* c);
 
 bool itb_fail(itb_ctx* c, const char* what, cudaError_t e);

@@ -195,17 +195,19 @@ static void once_smem(const void* fn, size_t bytes) {
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     h = bytes;
 }
-static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in) {
+// Into the context's buffer, over what the call before left there. False: out of memory.
+static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in, QRows* rows) {
     if (!itb_ensure_xq(c, n_rows * n_in)) return false;
     k_quant_q8<<<(unsigned)n_rows, 256, 0, c->stream>>>(xd, (int)n_in, c->xq, c->xs);
     ITB_LAUNCHED(c);
+    *rows = c->quantised(c->xq, c->xs);
     return true;
 }
 
-static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od, bool same) {
+static void launch_q8(itb_ctx* c, const WeightEntry* w, const QRows& x, size_t n_tok, float* od) {
     DevQ8 dw{(const int8_t*)w->a, (const uint16_t*)w->b, (int)w->n_in, (int)w->n_out};
     if (n_tok >= 2 && w->n_in % 32 == 0 && gemm_smem((int)w->n_in) <= 200 * 1024) {
-        dense_q8(c, c->stream, dw, c->xq, c->xs, (int)n_tok, od, w->n_out, 0, true, same);       // every weight row read once per token tile
+        dense_q8(c, c->stream, dw, x, (int)n_tok, od, w->n_out, 0, true);       // every weight row read once per token tile
         ITB_LAUNCHED(c);
         return;
     }
@@ -215,7 +217,7 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, size_t n_tok, float* od,
     size_t smem = w->n_in + nb * 4 + (size_t)nw * terms_floats(4, gsh, nb) * 4;
     dim3 grid(gx, (unsigned)n_tok);
     once_smem((const void*)k_matmul_q8, smem);
-    k_matmul_q8<<<grid, nw * 32, smem, c->stream>>>(dw, c->xq, c->xs, od);
+    k_matmul_q8<<<grid, nw * 32, smem, c->stream>>>(dw, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
 
@@ -253,12 +255,12 @@ static bool experts_tc(itb_ctx* c, const itb_experts* g, const itb_experts* u, c
     return true;
 }
 // ids==nullptr: dense NVFP4 matrix, one "pair" per token reading its own row.
-static void launch_fp4(itb_ctx* c, const WeightEntry* w, const int32_t* ids, size_t n_pairs, int n_used, int rows_mode, float* od) {
+static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const int32_t* ids, size_t n_pairs, int n_used, int rows_mode, float* od) {
     if (!ids && n_pairs >= 2 && gemm_smem((int)w->n_in) <= 200 * 1024) {
         size_t sm = gemm_smem((int)w->n_in);
         once_smem((const void*)k_gemm_fp4, sm);
         dim3 g((unsigned)((w->n_out + MMA_ROWS - 1) / MMA_ROWS), (unsigned)((n_pairs + MMA_TOK - 1) / MMA_TOK));
-        k_gemm_fp4<<<g, 256, sm, c->stream>>>((const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, c->xq, c->xs,
+        k_gemm_fp4<<<g, 256, sm, c->stream>>>((const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, x.q, x.s,
                                              (int)n_pairs, od, w->n_out, 1.0f, 0);
         ITB_LAUNCHED(c);
         return;
@@ -268,7 +270,7 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const int32_t* ids, siz
     if (gx < 1) gx = 1;
     const size_t smem = matmul_fp4_smem((int)w->n_in);
     once_smem((const void*)k_matmul_fp4, smem);
-    k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, c->xq, c->xs, od);
+    k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
 
@@ -295,20 +297,21 @@ static void launch_f32(itb_ctx* c, const WeightEntry* w, const float* xd, size_t
     ITB_LAUNCHED(c);
 }
 
-// same: c->xq / c->xs already hold these rows (the second matrix of a pair).
-static void matmul_dev(itb_ctx* c, const itb_weights* w, const float* xd, size_t n_tok, float* od, bool same = false) {
+// rows: the same rows' quantisation if a matrix before needed one (id 0: none did), which the matrices of a pair share.
+static void matmul_dev(itb_ctx* c, const itb_weights* w, const float* xd, size_t n_tok, float* od, QRows* rows) {
     const WeightEntry* we = itb_weight(c, w->data, w->bytes, w->ggml_type, w->n_in, w->n_out, 1, nullptr, 0);
     if (!we) return;
     if (we->ty != ITB_Q8_0 && we->ty != ITB_NVFP4) { launch_f32(c, we, xd, n_tok, od); return; }
-    if (!same && !quantize_rows(c, xd, n_tok, w->n_in)) return;
-    if (we->ty == ITB_Q8_0) launch_q8(c, we, n_tok, od, same); else launch_fp4(c, we, nullptr, n_tok, 1, 0, od);
+    if (rows->id == 0 && !quantize_rows(c, xd, n_tok, w->n_in, rows)) return;
+    if (we->ty == ITB_Q8_0) launch_q8(c, we, *rows, n_tok, od); else launch_fp4(c, we, *rows, nullptr, n_tok, 1, 0, od);
 }
 
 extern "C" void itb_matmul(itb_ctx* c, const itb_weights* w, const float* x, size_t x_len, float* out, size_t out_len) {
     if (w->n_in == 0 || x_len % w->n_in || out_len != x_len / w->n_in * w->n_out) { itb_fail_msg(c, "matmul: bad shape"); return; }
     const float* xd = itb_mirror_in(c, x, x_len); float* od = itb_mirror_out(c, out, out_len);
     if (!xd || !od) return;
-    matmul_dev(c, w, xd, x_len / w->n_in, od);
+    QRows rows;
+    matmul_dev(c, w, xd, x_len / w->n_in, od, &rows);
 }
 extern "C" void itb_matmul_pair(itb_ctx* c, const itb_weights* a, const itb_weights* b, const float* x, size_t x_len,
                                 float* out_a, size_t out_a_len, float* out_b, size_t out_b_len) {
@@ -318,10 +321,10 @@ extern "C" void itb_matmul_pair(itb_ctx* c, const itb_weights* a, const itb_weig
     const float* xd = itb_mirror_in(c, x, x_len);
     float* oa = itb_mirror_out(c, out_a, out_a_len); float* ob = itb_mirror_out(c, out_b, out_b_len);
     if (!xd || !oa || !ob) return;
-    auto quantised = [](const itb_weights* w) { return w->ggml_type == ITB_Q8_0 || w->ggml_type == ITB_NVFP4; };
-    matmul_dev(c, a, xd, nt, oa);
+    QRows rows;
+    matmul_dev(c, a, xd, nt, oa, &rows);
     if (!c->error.empty()) return;
-    matmul_dev(c, b, xd, nt, ob, quantised(a) && quantised(b));
+    matmul_dev(c, b, xd, nt, ob, &rows);
 }
 
 // ------------------------------------------------------------------ routing and experts
@@ -394,8 +397,9 @@ static void experts_dev(itb_ctx* c, const itb_experts* w, const itb_route_t* r, 
     if (!we) return;
     size_t n_pairs = r->n_tok * r->n_used, rows = x_len / w->n_in;
     int mode = rows == n_pairs ? 0 : rows > 1 ? 1 : 2;
-    if (!quantize_rows(c, xd, rows, w->n_in)) return;
-    launch_fp4(c, we, c->route_ids, n_pairs, (int)r->n_used, mode, od);
+    QRows x;
+    if (!quantize_rows(c, xd, rows, w->n_in, &x)) return;
+    launch_fp4(c, we, x, c->route_ids, n_pairs, (int)r->n_used, mode, od);
 }
 extern "C" void itb_matmul_experts(itb_ctx* c, const itb_experts* w, const itb_route_t* r, const float* x, size_t x_len,
                                    float* out, size_t out_len) {
@@ -422,13 +426,14 @@ extern "C" void itb_moe_glu(itb_ctx* c, const itb_experts* gate, const itb_exper
         const WeightEntry* wg = itb_weight(c, gate->data, gate->bytes, gate->ggml_type, gate->n_in, gate->n_out, gate->n_expert, gate->scale, gate->scale_bytes);
         const WeightEntry* wu = itb_weight(c, up->data, up->bytes, up->ggml_type, up->n_in, up->n_out, up->n_expert, up->scale, up->scale_bytes);
         const size_t n_pairs = r->n_tok * r->n_used, rows = x_len / gate->n_in;
-        if (!wg || !wu || !quantize_rows(c, xd, rows, gate->n_in)) return;
+        QRows xr;
+        if (!wg || !wu || !quantize_rows(c, xd, rows, gate->n_in, &xr)) return;
         const size_t smem = matmul_fp4_smem((int)gate->n_in);
         once_smem((const void*)k_matmul_fp4_glu, smem);
         k_matmul_fp4_glu<<<dim3((unsigned)((gate->n_out + 15) / 16), (unsigned)n_pairs), 256, smem, c->stream>>>(
             DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0},
             DevFp4{(const uint8_t*)wu->a, (const uint8_t*)wu->b, wu->scale2, (int)wu->n_in, (int)wu->n_out, (int)wu->n_expert, 0}, c->route_ids, (int)r->n_used,
-            rows == n_pairs ? 0 : rows > 1 ? 1 : 2, c->xq, c->xs, od);
+            rows == n_pairs ? 0 : rows > 1 ? 1 : 2, xr.q, xr.s, od);
         ITB_LAUNCHED(c);
         return;
     }

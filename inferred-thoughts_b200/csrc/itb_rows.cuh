@@ -148,13 +148,13 @@ static void sgemm_chain(cudaStream_t st, int sms, const DevF32& wa, const float*
 }
 
 // A dense Q8_0 matrix against n_rows >= 1 quantised rows: out[row][n_out] = or += (mode). tc: the tensor-core forms the context's
-// options name may be used (eager many-token passes); same: xq / xs are what the previous call with tc read. False: a device error.
-static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool tc, bool same) {
+// options name may be used (eager many-token passes). False: a device error.
+static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode, bool tc) {
     const int k = w.n_in;
     // many rows, dense=f16tc (tolerance class): both operands dequantised to f16, one tcgen05 GEMM with f32 accumulators
-    if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, xq, xs, n_rows, out, stride, mode, same);
+    if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, x, n_rows, out, stride, mode);
     // many rows, dense=q8tc: exact integer dots of 128 x 128 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
-    if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, xq, xs, n_rows, out, stride, mode, same);
+    if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, x, n_rows, out, stride, mode);
     static bool attr = false;
     if (!attr) {
         for (const void* f : {(const void*)k_tile_q8<1, 256, 4>, (const void*)k_tile_q8<4, 256, 2>}) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
@@ -163,10 +163,10 @@ static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* 
     }
     const bool skinny = n_rows <= 32;
     const int ns = std::min(k / 256, TILE_STAGES);
-    if (skinny && k % 256 == 0) k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, xq, xs, n_rows, out, stride, mode, ns);
-    else if (k % 256 == 0) k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, xq, xs, n_rows, out, stride, mode, ns);
-    else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st>>>(w, xq, xs, n_rows, out, stride, mode);
-    else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st>>>(w, xq, xs, n_rows, out, stride, mode);
+    if (skinny && k % 256 == 0) k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode, ns);
+    else if (k % 256 == 0) k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode, ns);
+    else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode);
+    else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode);
     return true;
 }
 

@@ -563,8 +563,8 @@ void itb_tc_free(itb_ctx* c) {
     for (auto& kv : c->tc_weights) { cudaFree(kv.second.img); cudaFree(kv.second.sf); }
     c->tc_weights.clear();
     cudaFree(c->tc_tiles); cudaFree(c->tc_n_tiles); cudaFree(c->tc_slot_tile); cudaFree(c->tc_b_img); cudaFree(c->tc_b_sf); cudaFree(c->tc_status); cudaFree(c->tc_codes); cudaFree(c->tc_scales); cudaFree(c->tc_q8_b); cudaFree(c->tc_q8_sx); cudaFree(c->tc_hf_b);
-    c->tc_hf_b = nullptr; c->tc_cap_hfb = 0; c->tc_hf_src = nullptr;
-    c->tc_q8_b = nullptr; c->tc_q8_sx = nullptr; c->tc_cap_q8b = c->tc_cap_q8sx = 0; c->tc_q8_src = nullptr;
+    c->tc_hf_b = nullptr; c->tc_cap_hfb = 0; c->tc_hf_src = 0;
+    c->tc_q8_b = nullptr; c->tc_q8_sx = nullptr; c->tc_cap_q8b = c->tc_cap_q8sx = 0; c->tc_q8_src = 0;
     c->tc_tiles = nullptr; c->tc_n_tiles = nullptr; c->tc_slot_tile = nullptr; c->tc_b_img = nullptr; c->tc_b_sf = nullptr; c->tc_status = nullptr; c->tc_codes = nullptr; c->tc_scales = nullptr; c->tc_cap_codes = c->tc_cap_scales = 0;
     c->tc_cap_tiles = c->tc_cap_slots = c->tc_cap_b = c->tc_cap_sf = 0;
 }
@@ -902,8 +902,8 @@ template <int NT> constexpr size_t tc_q8_smem() { return (size_t)q8_stages<NT>()
 }  // namespace
 
 bool itb_tc_q8_shape_ok(const DevQ8& w) { return w.n_in % 128 == 0 && w.n_out % 128 == 0 && w.q && w.s; }
-// out[token][row] (+)= W x for n_rows quantised activation rows (xq int8 [n_rows][n_in], xs f32 [n_rows][n_in / 32]). False: not run.
-bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool same_acts) {
+// out[token][row] (+)= W x for n_rows quantised activation rows. False: not run.
+bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode) {
     if (!itb_tc_q8_shape_ok(w) || n_rows <= 0) return false;
     // 64 tokens to a tile where 128 would leave half of the SMs without a block (an output projection over 512 rows)
     const size_t kbs = w.n_in / 32, rts = w.n_out / 128, nt = 2 * rts * (((size_t)n_rows + 127) / 128) <= (size_t)c->sm_count ? 64 : 128, tts = ((size_t)n_rows + nt - 1) / nt;
@@ -921,12 +921,12 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* x
     size_t cap1 = c->tc_status ? 1 : 0;
     bool ok = tc_grow(&c->tc_status, &cap1, 1, st) && tc_grow(&c->tc_q8_b, &c->tc_cap_q8b, tts * nt * kbs * 64, st) && tc_grow(&c->tc_q8_sx, &c->tc_cap_q8sx, tts * nt * kbs, st);
     if (!ok) return itb_fail_msg(c, "Q8_0 tensor path: out of device memory for the pass");
-    // same_acts: the caller vouches that xq/xs hold what the previous call's did (consecutive matmuls over one quantised row set)
-    if (!same_acts || c->tc_q8_src != xq || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in || c->tc_q8_src_tile != (int)nt) {
+    // consecutive matmuls over one quantised row set share its image
+    if (x.id == 0 || c->tc_q8_src != x.id || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in || c->tc_q8_src_tile != (int)nt) {
         const size_t n = tts * nt * kbs;
-        k_q8_tile<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(xq, nullptr, xs, n_rows, w.n_in, (int)nt, c->tc_q8_b, c->tc_q8_sx);
+        k_q8_tile<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x.q, nullptr, x.s, n_rows, w.n_in, (int)nt, c->tc_q8_b, c->tc_q8_sx);
         c->launches++;
-        c->tc_q8_src = xq; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in; c->tc_q8_src_tile = (int)nt;
+        c->tc_q8_src = x.id; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in; c->tc_q8_src_tile = (int)nt;
     }
     cudaMemsetAsync(c->tc_status, 0, 4, st);
     TcQ8 g{};
@@ -1163,8 +1163,8 @@ constexpr size_t tc_f16_smem() { return (size_t)HF_STAGES * HF_STAGE_BYTES + 128
 }  // namespace
 
 bool itb_tc_f16_shape_ok(const DevQ8& w) { return w.n_in % (16 * HF_KB) == 0 && w.n_out % 128 == 0 && w.q && w.s; }
-// out[token][row] (+)= W x for n_rows quantised activation rows (xq int8 [n_rows][n_in], xs f32 [n_rows][n_in / 32]). False: not run.
-bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* xq, const float* xs, int n_rows, float* out, size_t stride, int mode, bool same_acts) {
+// out[token][row] (+)= W x for n_rows quantised activation rows. False: not run.
+bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode) {
     if (!itb_tc_f16_shape_ok(w) || n_rows <= 0) return false;
     const size_t kbs = w.n_in / 16, rts = w.n_out / 128, tts = ((size_t)n_rows + HF_N - 1) / HF_N;
     auto it = c->tc_weights.find(w.s);                       // keyed by the scale array: the int8 images of dense=q8tc are keyed by w.q
@@ -1180,12 +1180,12 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const int8_t* 
     size_t cap1 = c->tc_status ? 1 : 0;
     bool ok = tc_grow(&c->tc_status, &cap1, 1, st) && tc_grow(&c->tc_hf_b, &c->tc_cap_hfb, tts * kbs * HF_B_BLK, st);
     if (!ok) return itb_fail_msg(c, "f16 tensor path: out of device memory for the pass");
-    // same_acts: the caller vouches that xq/xs hold what the previous call's did (consecutive matmuls over one quantised row set)
-    if (!same_acts || c->tc_hf_src != xq || c->tc_hf_src_rows != n_rows || c->tc_hf_src_in != w.n_in) {
+    // consecutive matmuls over one quantised row set share its image
+    if (x.id == 0 || c->tc_hf_src != x.id || c->tc_hf_src_rows != n_rows || c->tc_hf_src_in != w.n_in) {
         const size_t n = tts * HF_N * kbs;
-        k_f16_tile<HF_N><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(xq, nullptr, xs, n_rows, w.n_in, c->tc_hf_b);
+        k_f16_tile<HF_N><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x.q, nullptr, x.s, n_rows, w.n_in, c->tc_hf_b);
         c->launches++;
-        c->tc_hf_src = xq; c->tc_hf_src_rows = n_rows; c->tc_hf_src_in = w.n_in;
+        c->tc_hf_src = x.id; c->tc_hf_src_rows = n_rows; c->tc_hf_src_in = w.n_in;
     }
     cudaMemsetAsync(c->tc_status, 0, 4, st);
     TcHf g{};

@@ -163,6 +163,40 @@ def test_matmul_pair_and_f16(ops):
     exact(oa, wa_, "pair a"); exact(ob, wb_, "pair b (F16)")
 
 
+@pytest.mark.parametrize("opts", ["exact=1,dense=q8tc", "exact=0,dense=f16tc"])
+@pytest.mark.parametrize("first", ["Q8_0", "NVFP4", "F32"])
+@pytest.mark.parametrize("n_tok", [64, 70])
+def test_matmul_pair_multiplies_this_calls_rows(opts, first, n_tok):
+    """The second matrix of a pair takes the tensor cores, the first does not (96 outputs, or another type). The image of the rows is
+    kept for matmuls over the same rows; a later call's rows lie in the same buffer with the same shape and must not meet it. Every
+    result equals, bit for bit, the one of a context that has seen nothing else."""
+    from inferred_thoughts_b200 import host
+    n_in, na, nb = 256, 96, 128
+    wb = host.Weights(q8_weights(nb, n_in, 401), host.Q8_0, n_in, nb)
+    wa = {"Q8_0": lambda: host.Weights(q8_weights(na, n_in, 400), host.Q8_0, n_in, na),
+          "NVFP4": lambda: host.Weights(nvfp4_weights(1, na, n_in, 400)[0], host.NVFP4, n_in, na),
+          "F32": lambda: host.Weights(keep(noise(na * n_in, 400, 0.02)), host.F32, n_in, na)}[first]()
+
+    def pair(o, x):
+        oa = np.zeros(n_tok * na, np.float32); ob = np.zeros(n_tok * nb, np.float32)
+        o.begin_pass(n_tok)
+        o.matmul_pair(wa, wb, x, oa, ob); o.host_needs(oa); o.host_needs(ob); o.check()
+        return oa, ob
+    o = host.B200Ops(0, opts)
+    for seed in (402, 403, 402):
+        x = noise(n_tok * n_in, seed)
+        got = pair(o, x)
+        fresh = host.B200Ops(0, opts)
+        want = pair(fresh, x)
+        fresh.close()
+        exact(got[0], want[0], f"first matrix, rows {seed}"); exact(got[1], want[1], f"second matrix, rows {seed}")
+        if opts.startswith("exact=1"):
+            ref = np.zeros(n_tok * nb, np.float32)
+            L.orc_matmul(8, wb.data, n_in, nb, x, x.size, ref, 0)
+            exact(got[1], ref, f"second matrix against the CPU path, rows {seed}")
+    o.close()
+
+
 def test_norms_exact(ops):
     x = noise(3 * 2048, 50); w = 1 + noise(2048, 51, 0.02); out = np.zeros_like(x); want = np.zeros_like(x)
     ops.begin_pass(3)
