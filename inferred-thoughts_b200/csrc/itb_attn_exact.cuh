@@ -468,9 +468,9 @@ static void attn_exact_tiles(const AxScores& a, const AxSoft& sm, const AxOut& o
     const int group = a.n_head / a.n_head_kv, tt = 16 * mr / group, z = n_seq * ((a.rows_per_seq + tt - 1) / tt);
     const size_t soft = (size_t)ax_pad(n_pos_max) * 4;
     auto run = [&](auto scores, auto out, size_t scores_smem, size_t out_smem) {
-        cudaFuncSetAttribute(scores, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scores_smem);
-        cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
-        cudaFuncSetAttribute(k_attn_softmax_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        itb_raise_smem(scores, scores_smem);
+        itb_raise_smem(out, out_smem);
+        itb_raise_smem(k_attn_softmax_exact, 200 * 1024);
         launch(scores, dim3((n_pos_max + 63) / 64, a.n_head_kv, z), dim3(256), scores_smem, a);
         launch(k_attn_softmax_exact, dim3(a.n_head, rows), dim3(256), soft, sm);
         launch(out, dim3(a.hd / 64, a.n_head_kv, z), dim3(256), out_smem, o);

@@ -9,6 +9,7 @@
 #include <thread>
 
 #include "itb_internal.cuh"
+#include "itb_smem.h"
 
 void itb_ops_use_logf_fix(const uint32_t* dev_tab, uint32_t n);      // itb_ops.cu: points that unit's log_f at the table
 void itb_engine_use_logf_fix(const uint32_t* dev_tab, uint32_t n);   // itb_engine.cu
@@ -21,6 +22,14 @@ bool itb_fail_msg(itb_ctx* c, const std::string& msg) {
 }
 bool itb_fail(itb_ctx* c, const char* what, cudaError_t e) {
     return itb_fail_msg(c, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+cudaError_t itb_raise_smem(const void* fn, size_t bytes) {
+    static SmemLimits limits;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return limits.raise(dev, fn, bytes, [&] { return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 extern "C" const char* itb_last_create_error(void) { return g_create_error.empty() ? nullptr : g_create_error.c_str(); }

@@ -696,8 +696,8 @@ static bool dalloc(itb_engine* e, T** p, size_t count) {
 }
 
 static void set_smem(const void* fn, size_t bytes) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) fprintf(stderr, "[itb] cudaFuncSetAttribute(%zu bytes) failed: %s\n", bytes, cudaGetErrorString(e));
+    cudaError_t e = itb_raise_smem(fn, bytes);
+    if (e != cudaSuccess) fprintf(stderr, "[itb] shared-memory limit (%zu bytes) failed: %s\n", bytes, cudaGetErrorString(e));
 }
 
 // Launch with (pdl) or without the programmatic-serialization attribute: with it the kernel may be scheduled
@@ -735,8 +735,7 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
                                     int rows, int rows_per_seq, int n_pos_max) {
     const itb_model_dims& d = e->m->d;
     const int hd = d.head_dim, group = d.n_head / d.n_head_kv, kvd = hd * d.n_head_kv;
-    static bool attr = false;
-    if (!attr) { set_smem((const void*)k_attn_out_exact<false>, AX_OUT_SMEM); set_smem((const void*)k_attn_scores_exact, 64 * 1024); attr = true; }
+    set_smem((const void*)k_attn_out_exact<false>, AX_OUT_SMEM); set_smem((const void*)k_attn_scores_exact, 64 * 1024);
     AxScores a{};
     a.q = e->qn; a.kslab = kslab; a.slab_stride = slab_stride; a.rows_per_seq = rows_per_seq; a.n_pos_dev = e->npos; a.kv_dim = kvd; a.hd = hd;
     a.n_head = d.n_head; a.n_head_kv = d.n_head_kv; a.scale = 1.0f / sqrtf((float)hd); a.bf16 = e->c->kv_bf16; a.scores = e->scores; a.s_stride = (int)scores_stride(e);
@@ -752,8 +751,7 @@ static void enqueue_exact_attention(itb_engine* e, cudaStream_t st, bool pdl, co
     launch_k(pdl, k_attn_scores_exact, dim3(attn_scores_blocks(n_pos_max, d.n_head_kv, rows, e->c->sm_count), d.n_head_kv, rows), dim3(AX_TP * group), attn_scores_exact_smem(hd, group), st, a);
     if (rows >= 8) {
         // many rows: the softmax once per (row, head), in place, instead of once per block of the weighted-value kernel
-        static bool attr2 = false;
-        if (!attr2) { set_smem((const void*)k_attn_softmax_exact, 200 * 1024); attr2 = true; }
+        set_smem((const void*)k_attn_softmax_exact, 200 * 1024);
         launch_k(pdl, k_attn_softmax_exact, dim3(d.n_head, rows), dim3(256), (size_t)ax_pad(n_pos_max) * 4, st, sm);
         launch_k(pdl, k_attn_out_exact<true>, dim3(hd / 32, d.n_head, rows), dim3(288), attn_out_exact_smem(n_pos_max, true), st, o);
         return;
@@ -838,14 +836,10 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
         if (L.recurrent) { hint_q8(h, L.wqkv); hint_q8(h, L.wgate); hint_f32(h, L.ssm_alpha); hint_f32(h, L.ssm_beta); }
         else { hint_q8(h, L.wq); hint_q8(h, L.wk); hint_q8(h, L.wv); }
     };
-    static bool attrs_set = false;
-    if (!attrs_set) {
-        set_smem((const void*)k_in_proj, 200 * 1024); set_smem((const void*)k_out_proj, 200 * 1024);
-        set_smem((const void*)k_moe_glu, 100 * 1024);
-        set_smem((const void*)k_moe_down<false>, 200 * 1024); set_smem((const void*)k_moe_down<true>, 200 * 1024);
-        set_smem((const void*)k_gdn_core<128>, 100 * 1024); set_smem((const void*)k_gdn_core<64>, 100 * 1024);
-        attrs_set = true;
-    }
+    set_smem((const void*)k_in_proj, 200 * 1024); set_smem((const void*)k_out_proj, 200 * 1024);
+    set_smem((const void*)k_moe_glu, 100 * 1024);
+    set_smem((const void*)k_moe_down<false>, 200 * 1024); set_smem((const void*)k_moe_down<true>, 200 * 1024);
+    set_smem((const void*)k_gdn_core<128>, 100 * 1024); set_smem((const void*)k_gdn_core<64>, 100 * 1024);
     if (prof) prof->mark(-1, 0, st);
     const bool p2p = e->ep && e->ep->p2p;
     if (p2p) { k_ep_tick<<<1, 32, 0, st>>>(e->ep->seq); launches++; }    // the step number the peers' flags will carry
@@ -1213,15 +1207,11 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     const int qd = d.head_dim * d.n_head, kvd = d.head_dim * d.n_head_kv;
     const int TPB = NWG * 32;
     uint64_t launches = 0;
-    static bool attrs_set = false;
-    if (!attrs_set) {
-        set_smem((const void*)k_matmul_f32_rows<20>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<24>, 64 * 1024);
-        set_smem((const void*)k_matmul_f32_rows<28>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<32>, 64 * 1024);
-        set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
-        set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
-        set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
-        attrs_set = true;
-    }
+    set_smem((const void*)k_matmul_f32_rows<20>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<24>, 64 * 1024);
+    set_smem((const void*)k_matmul_f32_rows<28>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<32>, 64 * 1024);
+    set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
+    set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
+    set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
     // Pipelined tile kernels when k is a multiple of the chunk (every matrix of the 35B and 177B shapes); the
     // direct-load MMA kernels otherwise.
     cudaStreamCaptureStatus cap_rows = cudaStreamCaptureStatusNone;
@@ -1908,7 +1898,7 @@ static bool mega_prepare(itb_engine* e) {
     if (left <= 0 || ns_a < 2) return no("not enough shared memory for the rings");
     ns_a = std::min(ns_a, MG_MAX_SLOTS);
     const size_t smem = act + terms + ns_a * slot_a + ns_b * slot_b;
-    if (cudaFuncSetAttribute((const void*)k_mega, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { cudaGetLastError(); return no("cannot raise the shared-memory limit"); }
+    if (itb_raise_smem(k_mega, smem) != cudaSuccess) { cudaGetLastError(); return no("cannot raise the shared-memory limit"); }
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mega, MG_THREADS, smem) != cudaSuccess || occ < 1) { cudaGetLastError(); return no("the kernel does not fit an SM"); }
     // buffers the step needs beyond the engine's

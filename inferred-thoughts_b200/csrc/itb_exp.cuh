@@ -277,8 +277,7 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
 }
 template <int NJ, bool GLU>
 static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(k_exp<NJ, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); attr = true; }
+    itb_raise_smem(k_exp<NJ, GLU>, 224 * 1024);
     k_exp<NJ, GLU><<<dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st>>>(a);
 }
 // Pairs per tile. Up to 4 per expert on average nearly every expert holds at most 16: tiles of 16, whose kernel keeps three stages

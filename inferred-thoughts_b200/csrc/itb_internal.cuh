@@ -135,6 +135,10 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
 void itb_tc_free(itb_ctx* c);
 
 bool itb_fail(itb_ctx* c, const char* what, cudaError_t e);
+// Before a launch of `fn` with that much dynamic shared memory on the current device (itb_smem.h: a table lookup once it has been
+// seen there, where the runtime's own call costs a microsecond). An error also stays as the runtime's last one.
+cudaError_t itb_raise_smem(const void* fn, size_t bytes);
+template <class... A> static inline cudaError_t itb_raise_smem(void (*fn)(A...), size_t bytes) { return itb_raise_smem((const void*)fn, bytes); }
 bool itb_fail_msg(itb_ctx* c, const std::string& msg);
 #define ITB_CUDA(c, call)                                              \
     do {                                                               \

@@ -63,8 +63,8 @@ extern "C" int itb_attend_decode_noalloc(void* stream, const float* q_dev, const
         float* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress((void**)&p, g_attn_scratch);
         if (e != cudaSuccess || !p) return fail(err, err_cap, cudaGetErrorString(e));
-        e = cudaFuncSetAttribute(k_attn_partial<256, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 8 * 2 * 4 + 8 * 8 * 256 * 4);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_partial<128, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 8 * 2 * 4 + 8 * 8 * 128 * 4);
+        e = itb_raise_smem(k_attn_partial<256, 8>, 8 * 8 * 2 * 4 + 8 * 8 * 256 * 4);
+        if (e == cudaSuccess) e = itb_raise_smem(k_attn_partial<128, 8>, 8 * 8 * 2 * 4 + 8 * 8 * 128 * 4);
         if (e != cudaSuccess) return fail(err, err_cap, cudaGetErrorString(e));
         g_scratch_dev[dev] = p;
         g_ready[dev] = true;

@@ -169,12 +169,8 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
         }
         float* qs = c->tmp_f32; float* gbd = qs + nt * kper; float* scr = gbd + nt * n_v * 2;
         k_gdn_op_pre<<<(unsigned)((nt * kper + 255) / 256), 256, 0, c->stream>>>(q, al, be, sa, dt, nt, n_k * sk, n_v, 1.0f / sqrtf((float)sk), qs, gbd);
-        static bool attr = false;
-        if (!attr) {
-            cudaFuncSetAttribute(k_gdn_chunk_prep<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gdn_chunk_prep_smem<128>());
-            cudaFuncSetAttribute(k_gdn_chunk_scan<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gdn_chunk_scan_smem<128>());
-            attr = true;
-        }
+        itb_raise_smem(k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>());
+        itb_raise_smem(k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
         k_gdn_chunk_prep<128><<<dim3(n_ch, n_v, 1), 256, gdn_chunk_prep_smem<128>(), c->stream>>>(qs, k, v, gbd, (int)nt, n_k, n_v, scr);
         k_gdn_chunk_scan<128><<<dim3(n_v, sk / GC_VS, 1), 256, gdn_chunk_scan_smem<128>(), c->stream>>>(scr, (int)nt, n_v, sd, (size_t)n_v * sk * sk, od);
         ITB_LAUNCHED(c);
@@ -187,14 +183,6 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
 }
 
 // ------------------------------------------------------------------ matmuls
-// Raises a kernel's shared-memory limit when a launch needs more than any before it (the call costs a microsecond of host time).
-static void once_smem(const void* fn, size_t bytes) {
-    static thread_local std::unordered_map<const void*, size_t> have;
-    size_t& h = have[fn];
-    if (bytes <= h || bytes <= 48 * 1024) return;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    h = bytes;
-}
 // Into the context's buffer, over what the call before left there. False: out of memory.
 static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in, QRows* rows) {
     if (!itb_ensure_xq(c, n_rows * n_in)) return false;
@@ -216,7 +204,7 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, const QRows& x, size_t n
     if (gx < 1) gx = 1;
     size_t smem = w->n_in + nb * 4 + (size_t)nw * terms_floats(4, gsh, nb) * 4;
     dim3 grid(gx, (unsigned)n_tok);
-    once_smem((const void*)k_matmul_q8, smem);
+    itb_raise_smem(k_matmul_q8, smem);
     k_matmul_q8<<<grid, nw * 32, smem, c->stream>>>(dw, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
@@ -258,7 +246,7 @@ static bool experts_tc(itb_ctx* c, const itb_experts* g, const itb_experts* u, c
 static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const int32_t* ids, size_t n_pairs, int n_used, int rows_mode, float* od) {
     if (!ids && n_pairs >= 2 && gemm_smem((int)w->n_in) <= 200 * 1024) {
         size_t sm = gemm_smem((int)w->n_in);
-        once_smem((const void*)k_gemm_fp4, sm);
+        itb_raise_smem(k_gemm_fp4, sm);
         dim3 g((unsigned)((w->n_out + MMA_ROWS - 1) / MMA_ROWS), (unsigned)((n_pairs + MMA_TOK - 1) / MMA_TOK));
         k_gemm_fp4<<<g, 256, sm, c->stream>>>((const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, x.q, x.s,
                                              (int)n_pairs, od, w->n_out, 1.0f, 0);
@@ -269,7 +257,7 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const i
     int gx = (int)std::min<size_t>((w->n_out + 31) / 32, (size_t)c->sm_count * 2);
     if (gx < 1) gx = 1;
     const size_t smem = matmul_fp4_smem((int)w->n_in);
-    once_smem((const void*)k_matmul_fp4, smem);
+    itb_raise_smem(k_matmul_fp4, smem);
     k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
@@ -288,10 +276,10 @@ static void launch_f32(itb_ctx* c, const WeightEntry* w, const float* xd, size_t
     size_t smem = w->n_in * 4 + (size_t)nw * 32 * 33 * 4;
     dim3 grid(gx, (unsigned)n_tok);
     if (c->exact) {
-        once_smem((const void*)k_matmul_f32<true>, smem);
+        itb_raise_smem(k_matmul_f32<true>, smem);
         k_matmul_f32<true><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
     } else {
-        once_smem((const void*)k_matmul_f32<false>, smem);
+        itb_raise_smem(k_matmul_f32<false>, smem);
         k_matmul_f32<false><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
     }
     ITB_LAUNCHED(c);
@@ -429,7 +417,7 @@ extern "C" void itb_moe_glu(itb_ctx* c, const itb_experts* gate, const itb_exper
         QRows xr;
         if (!wg || !wu || !quantize_rows(c, xd, rows, gate->n_in, &xr)) return;
         const size_t smem = matmul_fp4_smem((int)gate->n_in);
-        once_smem((const void*)k_matmul_fp4_glu, smem);
+        itb_raise_smem(k_matmul_fp4_glu, smem);
         k_matmul_fp4_glu<<<dim3((unsigned)((gate->n_out + 15) / 16), (unsigned)n_pairs), 256, smem, c->stream>>>(
             DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0},
             DevFp4{(const uint8_t*)wu->a, (const uint8_t*)wu->b, wu->scale2, (int)wu->n_in, (int)wu->n_out, (int)wu->n_expert, 0}, c->route_ids, (int)r->n_used,
@@ -462,7 +450,7 @@ void itb_attend_dev(itb_ctx* c, cudaStream_t st, const float* q, const uint16_t*
     size_t smem = (size_t)nw * 8 * 2 * 4 + (size_t)nw * 8 * hd * 4;
 #define ATT_CASE(H)                                                                                                   \
     case H:                                                                                                           \
-        cudaFuncSetAttribute(k_attn_partial<H, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+        itb_raise_smem(k_attn_partial<H, 8>, smem);                                                                   \
         k_attn_partial<H, 8><<<grid, nw * 32, smem, st>>>(q, k, v, kv_dim, n_pos, n_q, n_head, n_head_kv, scale, bf16, \
                                                           n_pos_dev, part_acc, part_ml);                              \
         break;
@@ -508,8 +496,8 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
         const dim3 ga((unsigned)((n_q + AM_ROWS / group - 1) / (AM_ROWS / group)), (unsigned)a->n_head_kv, 1);
 #define AM_CASE(HD)                                                                                                                        \
     case HD:                                                                                                                                \
-        cudaFuncSetAttribute(k_attn_mma<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_mma_smem<HD>());                  \
-        cudaFuncSetAttribute(k_attn_mma<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_mma_smem<HD>());                 \
+        itb_raise_smem(k_attn_mma<HD, true>, attn_mma_smem<HD>());                                                                          \
+        itb_raise_smem(k_attn_mma<HD, false>, attn_mma_smem<HD>());                                                                         \
         if (c->kv_bf16) k_attn_mma<HD, true><<<ga, 256, attn_mma_smem<HD>(), c->stream>>>(ap);                                              \
         else k_attn_mma<HD, false><<<ga, 256, attn_mma_smem<HD>(), c->stream>>>(ap);                                                        \
         break;
@@ -542,11 +530,11 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
                              [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { k<<<g, b, smem, c->stream>>>(arg); ITB_LAUNCHED(c); });
             return;
         }
+        itb_raise_smem(k_attn_scores_exact, attn_scores_exact_smem((int)a->head_dim, group));
         k_attn_scores_exact<<<dim3((unsigned)attn_scores_blocks((int)a->n_pos, (int)a->n_head_kv, (int)n_q, c->sm_count), (unsigned)a->n_head_kv, (unsigned)n_q), AX_TP * group,
                               attn_scores_exact_smem((int)a->head_dim, group), c->stream>>>(sp);
         ITB_LAUNCHED(c);
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(k_attn_out_exact<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AX_OUT_SMEM); cudaFuncSetAttribute(k_attn_scores_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024); attr = true; }
+        itb_raise_smem(k_attn_out_exact<false>, AX_OUT_SMEM);
         k_attn_out_exact<false><<<dim3((unsigned)(a->head_dim / 32), (unsigned)a->n_head, (unsigned)n_q), 288, attn_out_exact_smem((int)a->n_pos), c->stream>>>(op);
         ITB_LAUNCHED(c);
         return;

@@ -131,7 +131,7 @@ inline bool sgemm_chain_ok(int n_in) { return n_in % SG_KT == 0; }
 template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
 static void sgemm_tiles(cudaStream_t st, int n_out, int nz, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb, float* ob) {
     constexpr size_t smem = (size_t)NST * (TO + TR) * (KT + 4) * 4;
-    cudaFuncSetAttribute(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    itb_raise_smem(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, smem);
     k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST><<<dim3((n_out + TO - 1) / TO, (n_rows + TR - 1) / TR, nz), (TO / MO) * (TR / MR), smem, st>>>(wa, x, n_rows, oa, wb, ob);
 }
 // One matrix, or two over the same rows. 8 x 8, a chain to a thread, is fastest as long as an SM has no more than four such blocks (32 rows
@@ -155,12 +155,8 @@ static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, x, n_rows, out, stride, mode);
     // many rows, dense=q8tc: exact integer dots of 128 x 128 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
     if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, x, n_rows, out, stride, mode);
-    static bool attr = false;
-    if (!attr) {
-        for (const void* f : {(const void*)k_tile_q8<1, 256, 4>, (const void*)k_tile_q8<4, 256, 2>}) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-        for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr = true;
-    }
+    for (const void* f : {(const void*)k_tile_q8<1, 256, 4>, (const void*)k_tile_q8<4, 256, 2>}) itb_raise_smem(f, 226 * 1024);
+    for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) itb_raise_smem(f, 200 * 1024);
     const bool skinny = n_rows <= 32;
     const int ns = std::min(k / 256, TILE_STAGES);
     if (skinny && k % 256 == 0) k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode, ns);

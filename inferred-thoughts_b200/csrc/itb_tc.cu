@@ -619,13 +619,9 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     g.s2g = wg.scale2; g.s2u = wu ? wu->scale2 : nullptr; g.expert_lo = wg.expert_lo;
     g.b_img = c->tc_b_img; g.b_sf = c->tc_b_sf; g.tiles = tiles; g.n_tiles = c->tc_n_tiles; g.pair_list = pair_list;
     g.n_out = wg.n_out; g.n_in = wg.n_in; g.out = out; g.out_stride = wg.n_out; g.status = c->tc_status;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_tc_gemm<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_gemm_smem(true));
-        cudaFuncSetAttribute(k_tc_gemm<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_gemm_smem(true));
-        cudaFuncSetAttribute(k_tc_gemm<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_gemm_smem(false));
-        attr = true;
-    }
+    itb_raise_smem(k_tc_gemm<true, true>, tc_gemm_smem(true));
+    itb_raise_smem(k_tc_gemm<true, false>, tc_gemm_smem(true));
+    itb_raise_smem(k_tc_gemm<false, false>, tc_gemm_smem(false));
     const size_t n_blocks = std::min<size_t>((size_t)c->sm_count, max_tiles * (size_t)(wg.n_out / TC_M));
     const dim3 grid((unsigned)n_blocks);
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
@@ -934,7 +930,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     g.out = out; g.stride = stride; g.mode = mode; g.status = c->tc_status;
     auto kernel = nt == 64 ? k_tc_q8<64> : k_tc_q8<128>;
     const size_t smem = nt == 64 ? tc_q8_smem<64>() : tc_q8_smem<128>();
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    itb_raise_smem(kernel, smem);
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = rts * tts;
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
@@ -1191,8 +1187,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     TcHf g{};
     g.a_img = it->second.img; g.b_img = c->tc_hf_b; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_rt = (int)rts; g.n_tt = (int)tts;
     g.out = out; g.stride = stride; g.mode = mode; g.status = c->tc_status;
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(k_tc_f16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_f16_smem()); attr = true; }
+    itb_raise_smem(k_tc_f16, tc_f16_smem());
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = std::min<size_t>((size_t)c->sm_count, rts * tts);
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
