@@ -2,13 +2,13 @@
 // Mirrors the reference's device-backend host layer (src/ops/cuda/ops/residency.rs:23-100,
 // src/ops/cuda/ops/mod.rs:91-110, :559-633) with a plain CUDA-runtime implementation.
 #include <math.h>
-#include <semaphore.h>
 #include <string.h>
 
-#include <atomic>
+#include <new>
 #include <thread>
 
 #include "itb_internal.cuh"
+#include "itb_pipe.h"
 #include "itb_smem.h"
 
 void itb_ops_use_logf_fix(const uint32_t* dev_tab, uint32_t n);      // itb_ops.cu: points that unit's log_f at the table
@@ -160,130 +160,19 @@ extern "C" const char* itb_take_error(itb_ctx* c) {
 extern "C" uint64_t itb_launch_count(itb_ctx* c) { return c->launches; }
 
 // ------------------------------------------------------------------ host transfers
-// A copy from or to pageable memory goes through a staging buffer somewhere: the driver's does it on one thread, at 6 GB/s up and 21
-// down on this pool's hosts, and asks for a stream synchronise to be sure of it. Here: a small copy is one memcpy into a pinned ring
-// and an asynchronous copy behind it (no synchronise); a large one runs in chunks, the chunk in flight on the bus while the next is
-// copied by four threads (16.8 MB up: 2.7 ms -> see the measured figures beside the callers). The threads start with the first large
-// copy and end with the context.
-struct HostPipe {
-    static constexpr size_t RING = 1 << 20, SMALL = 128 << 10, CHUNK = 2 << 20;
-    static constexpr int N_CHUNK = 3, N_THREAD = 3;
-    uint8_t* ring = nullptr; size_t ring_at = 0; int ring_half = 0; cudaEvent_t half_ev[2] = {nullptr, nullptr}; bool half_used[2] = {false, false};
-    uint8_t* chunk[N_CHUNK] = {nullptr, nullptr, nullptr}; cudaEvent_t chunk_ev[N_CHUNK] = {nullptr, nullptr, nullptr}; bool chunk_used[N_CHUNK] = {false, false, false};
-    // Copy threads. A copy is cut into PARTS; whoever is free takes the next one, the caller included, so a thread that wakes late costs
-    // nothing but its help. turn = (copy number << 8) | next part: a part is taken by raising it from the value under which the
-    // copy's arguments were read, and the arguments change only after every part of the copy before is done.
-    static constexpr uint64_t PARTS = 8;
-    std::vector<std::thread> threads; sem_t wake; std::atomic<bool> quit{false};
-    std::atomic<uint64_t> turn{PARTS}, done{0};
-    std::atomic<uint8_t*> jd{nullptr}; std::atomic<const uint8_t*> js{nullptr}; std::atomic<size_t> jn{0};
-    void take_parts() {
-        for (;;) {
-            uint64_t t = turn.load(std::memory_order_acquire);
-            if ((t & 255) >= PARTS) return;
-            uint8_t* d = jd.load(std::memory_order_relaxed); const uint8_t* s = js.load(std::memory_order_relaxed); const size_t n = jn.load(std::memory_order_relaxed);
-            if (!turn.compare_exchange_strong(t, t + 1, std::memory_order_acq_rel)) continue;
-            const size_t per = ((n + PARTS - 1) / PARTS + 4095) & ~(size_t)4095, a = std::min(n, per * (t & 255)), z = std::min(n, a + per);
-            if (z > a) memcpy(d + a, s + a, z - a);
-            done.fetch_add(1, std::memory_order_release);
-        }
-    }
-    void copy(void* d, const void* s, size_t n) {
-        if (n < (512 << 10)) { memcpy(d, s, n); return; }
-        if (threads.empty())
-            for (int i = 0; i < N_THREAD; ++i)
-                threads.emplace_back([this] {
-                    for (;;) {
-                        while (sem_wait(&wake) != 0) {}
-                        if (quit.load(std::memory_order_acquire)) return;
-                        take_parts();
-                    }
-                });
-        jd.store((uint8_t*)d, std::memory_order_relaxed); js.store((const uint8_t*)s, std::memory_order_relaxed); jn.store(n, std::memory_order_relaxed);
-        done.store(0, std::memory_order_relaxed);
-        turn.store(((turn.load(std::memory_order_relaxed) >> 8) + 1) << 8, std::memory_order_release);
-        for (int i = 0; i < N_THREAD; ++i) sem_post(&wake);
-        take_parts();
-        while (done.load(std::memory_order_acquire) < PARTS) std::this_thread::yield();
-    }
-    HostPipe() { sem_init(&wake, 0, 0); }
-    bool ready_small() {
-        if (ring) return true;
-        if (cudaMallocHost(&ring, RING) != cudaSuccess) { ring = nullptr; cudaGetLastError(); return false; }
-        for (auto& e : half_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-        return true;
-    }
-    bool ready_large() {
-        if (chunk[0]) return true;
-        if (cudaMallocHost(&chunk[0], CHUNK * N_CHUNK) != cudaSuccess) { chunk[0] = nullptr; cudaGetLastError(); return false; }
-        for (int i = 0; i < N_CHUNK; ++i) { chunk[i] = chunk[0] + i * CHUNK; cudaEventCreateWithFlags(&chunk_ev[i], cudaEventDisableTiming); }
-        return true;
-    }
-    ~HostPipe() {
-        quit.store(true, std::memory_order_release);
-        for (size_t i = 0; i < threads.size(); ++i) sem_post(&wake);
-        for (auto& t : threads) t.join();
-        sem_destroy(&wake);
-        for (auto& e : half_ev) if (e) cudaEventDestroy(e);
-        for (auto& e : chunk_ev) if (e) cudaEventDestroy(e);
-        cudaFreeHost(ring); cudaFreeHost(chunk[0]);
-    }
-};
 static void itb_pipe_free(itb_ctx* c) { delete c->pipe; c->pipe = nullptr; }
+static HostPipe* pipe_of(itb_ctx* c) {
+    if (!c->pipe) c->pipe = new (std::nothrow) HostPipe();
+    return c->pipe;
+}
 bool itb_upload(itb_ctx* c, void* dev, const void* host, size_t bytes) {
-    if (!c->pipe) c->pipe = new HostPipe();
-    HostPipe& p = *c->pipe;
-    cudaError_t e = cudaSuccess;
-    if (bytes <= HostPipe::SMALL && p.ready_small()) {
-        // the ring's halves alternate: a half is written again only after the copies out of it have run
-        const size_t need = (bytes + 255) & ~(size_t)255, half = HostPipe::RING / 2;
-        if (p.ring_at + need > half) {
-            cudaEventRecord(p.half_ev[p.ring_half], c->stream); p.half_used[p.ring_half] = true;
-            p.ring_half ^= 1; p.ring_at = 0;
-            if (p.half_used[p.ring_half]) cudaEventSynchronize(p.half_ev[p.ring_half]);
-        }
-        const size_t at = half * p.ring_half + p.ring_at;
-        memcpy(p.ring + at, host, bytes);
-        e = cudaMemcpyAsync(dev, p.ring + at, bytes, cudaMemcpyHostToDevice, c->stream);
-        p.ring_at += need;
-    } else if (p.ready_large()) {
-        int i = 0;
-        for (size_t at = 0; at < bytes && e == cudaSuccess; at += HostPipe::CHUNK, i = (i + 1) % HostPipe::N_CHUNK) {
-            const size_t n = std::min(HostPipe::CHUNK, bytes - at);
-            if (p.chunk_used[i]) cudaEventSynchronize(p.chunk_ev[i]);
-            p.copy(p.chunk[i], (const uint8_t*)host + at, n);
-            e = cudaMemcpyAsync((uint8_t*)dev + at, p.chunk[i], n, cudaMemcpyHostToDevice, c->stream);
-            cudaEventRecord(p.chunk_ev[i], c->stream); p.chunk_used[i] = true;
-        }
-    } else {
-        e = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    }
+    HostPipe* p = pipe_of(c);
+    const cudaError_t e = p ? p->up(c->stream, dev, host, bytes) : HostPipe::plain(c->stream, dev, host, bytes, cudaMemcpyHostToDevice);
     return e == cudaSuccess || itb_fail(c, "h2d", e);
 }
 bool itb_download(itb_ctx* c, void* host, const void* dev, size_t bytes) {
-    if (!c->pipe) c->pipe = new HostPipe();
-    HostPipe& p = *c->pipe;
-    cudaError_t e = cudaSuccess;
-    if (bytes > (64 << 10) && p.ready_large()) {
-        const size_t step = bytes >= 4 * HostPipe::CHUNK ? HostPipe::CHUNK : std::min(HostPipe::CHUNK, (bytes / 3 + 65535) & ~(size_t)65535), n_step = (bytes + step - 1) / step;
-        auto issue = [&](size_t s) {
-            const int i = (int)(s % HostPipe::N_CHUNK);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(p.chunk[i], (const uint8_t*)dev + s * step, std::min(step, bytes - s * step), cudaMemcpyDeviceToHost, c->stream);
-            cudaEventRecord(p.chunk_ev[i], c->stream); p.chunk_used[i] = true;
-        };
-        for (int i = 0; i < HostPipe::N_CHUNK; ++i) if (p.chunk_used[i]) cudaEventSynchronize(p.chunk_ev[i]);
-        for (size_t s = 0; s < n_step && s < (size_t)HostPipe::N_CHUNK; ++s) issue(s);
-        for (size_t s = 0; s < n_step && e == cudaSuccess; ++s) {
-            const int i = (int)(s % HostPipe::N_CHUNK);
-            e = cudaEventSynchronize(p.chunk_ev[i]);
-            if (e == cudaSuccess) p.copy((uint8_t*)host + s * step, p.chunk[i], std::min(step, bytes - s * step));
-            if (s + HostPipe::N_CHUNK < n_step) issue(s + HostPipe::N_CHUNK);
-        }
-    } else {
-        e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    }
+    HostPipe* p = pipe_of(c);
+    const cudaError_t e = p ? p->down(c->stream, host, dev, bytes) : HostPipe::plain(c->stream, host, dev, bytes, cudaMemcpyDeviceToHost);
     return e == cudaSuccess || itb_fail(c, "d2h", e);
 }
 

@@ -12,7 +12,7 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 def run(tmp_path, source):
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
     src.write_text(source)
-    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-g", "-Wall", f"-I{CSRC}", f"-I{CUDA}/include", str(src), "-o", str(exe), "-pthread"], check=True, timeout=120)
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-g", "-Wall", f"-I{CSRC}", f"-I{CUDA}/include", str(src), "-o", str(exe), "-pthread", "-ldl"], check=True, timeout=120)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stdout}{r.stderr}"
 
@@ -65,3 +65,83 @@ def test_every_kernel_limit_goes_through_that_table():
     for p in CSRC.iterdir():
         if p.suffix in (".cu", ".cuh"):
             assert not re.search(r"static (thread_local )?bool attr", p.read_text()), p.name
+
+
+# The runtime calls that itb_pipe.h makes, with a stream whose copies run only when something waits for them -- so a staging buffer that is
+# written again too early is seen in the data -- and switches that make one kind of call fail.
+FAKE_RUNTIME = CHECK + r"""
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
+#include <deque>
+#include <vector>
+#include "itb_pipe.h"
+struct CUevent_st { size_t at = 0; };
+struct Copy { void* d; const void* s; size_t n; };
+static std::deque<Copy> queue;
+static size_t issued = 0, ran = 0;
+static int events = 0;                       // alive
+static bool no_pinned = false, no_event = false, no_record = false, no_wait = false, no_thread = false;
+static int event_after = 1 << 30;            // with no_event: that many are still made
+static void run_to(size_t at) { for (; ran < at; ++ran) { memcpy(queue.front().d, queue.front().s, queue.front().n); queue.pop_front(); } }
+extern "C" {
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { if (no_pinned) return cudaErrorMemoryAllocation; *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { if (no_event && event_after-- <= 0) return cudaErrorMemoryAllocation; *e = new CUevent_st; ++events; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { delete e; --events; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { if (!e || no_record) return cudaErrorInvalidResourceHandle; e->at = issued; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { if (!e || no_wait) return cudaErrorInvalidResourceHandle; run_to(e->at); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { run_to(issued); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { queue.push_back({d, s, n}); ++issued; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) noexcept {
+    if (no_thread) return EAGAIN;
+    return ((int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*))dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, x);
+}
+}
+static void transfers() {
+    {
+        HostPipe p;
+        unsigned seed = 1;
+        std::vector<std::vector<uint8_t>> dev, want;
+        for (int round = 0; round < 3; ++round)
+            for (size_t n : {(size_t)1, (size_t)4096, (size_t)131072, (size_t)131072, (size_t)131072, (size_t)131072, (size_t)131072, (size_t)131073, (size_t)3000001, (size_t)9000000, (size_t)524288}) {
+                std::vector<uint8_t> h(n);
+                for (auto& b : h) b = (uint8_t)((seed = seed * 1664525u + 1013904223u) >> 24);
+                dev.emplace_back(n); want.push_back(h);
+                CHECK(p.up(nullptr, dev.back().data(), h.data(), n) == cudaSuccess);
+                memset(h.data(), 0, n);                    // the caller may change its bytes once the call is back
+            }
+        run_to(issued);
+        for (size_t i = 0; i < dev.size(); ++i) CHECK(dev[i] == want[i]);
+        for (size_t i = 0; i < dev.size(); ++i) {
+            std::vector<uint8_t> h(dev[i].size());
+            CHECK(p.down(nullptr, h.data(), dev[i].data(), h.size()) == cudaSuccess);
+            CHECK(h == want[i]);
+        }
+    }
+    CHECK(events == 0);
+}
+"""
+
+
+def test_transfers_come_through(tmp_path):
+    run(tmp_path, FAKE_RUNTIME + "int main() { transfers(); return 0; }")
+
+
+def test_transfers_without_copy_threads(tmp_path):
+    """The system refuses a thread: the caller copies alone, and nothing is thrown out of the C interface."""
+    run(tmp_path, FAKE_RUNTIME + "int main() { no_thread = true; transfers(); return 0; }")
+
+
+def test_transfers_without_pinned_memory_or_events(tmp_path):
+    run(tmp_path, FAKE_RUNTIME + """int main() {
+        no_pinned = true; transfers(); no_pinned = false;
+        for (int made = 0; made < 6; ++made) { no_event = true; event_after = made; transfers(); }
+        return 0;
+    }""")
+
+
+def test_transfers_whose_events_cannot_be_recorded_or_waited_for(tmp_path):
+    """A staging buffer is not written again while a copy may still read it, whichever call fails."""
+    run(tmp_path, FAKE_RUNTIME + "int main() { no_record = true; transfers(); no_record = false; no_wait = true; transfers(); return 0; }")
