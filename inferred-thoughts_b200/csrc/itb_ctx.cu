@@ -372,8 +372,7 @@ const WeightEntry* itb_weight(itb_ctx* c, const uint8_t* data, size_t bytes, uin
         const WeightEntry& h = it->second;
         if (h.ty == ty && h.n_in == n_in && h.n_out == n_out && h.n_expert == n_expert) return &it->second;
         // The address now names a different tensor (the caller freed and reallocated): drop the old upload.
-        cudaStreamSynchronize(c->stream);
-        cudaFree(h.a); cudaFree(h.b); cudaFree(h.scale2);
+        itb_free_weight(c, h.a, h.b, h.scale2);
         c->weight_bytes -= h.bytes;
         c->weights.erase(it);
     }

@@ -105,7 +105,7 @@ extern "C" void itb_model_dims_of(itb_model* m, itb_model_dims* out) { *out = m-
 extern "C" void itb_model_destroy(itb_model* m) {
     if (!m) return;
     cudaStreamSynchronize(m->c->stream);
-    for (auto& kv : m->t) { cudaFree(kv.second.a); cudaFree(kv.second.b); cudaFree(kv.second.scale2); }
+    for (auto& kv : m->t) itb_free_weight(m->c, kv.second.a, kv.second.b, kv.second.scale2);
     for (auto& l : m->host_experts) for (auto& h : l) { cudaFreeHost(h.nib); cudaFreeHost(h.sc); }
     for (void* p : m->extra) cudaFree(p);
     delete m;
@@ -137,7 +137,7 @@ static int adopt_raw(itb_model* m, const std::string& name, uint32_t ty, size_t 
     } else return 1;
     c->launches++;
     auto it = m->t.find(name);
-    if (it != m->t.end()) { cudaFree(it->second.a); cudaFree(it->second.b); cudaFree(it->second.scale2); m->bytes -= it->second.bytes; }
+    if (it != m->t.end()) { itb_free_weight(c, it->second.a, it->second.b, it->second.scale2); m->bytes -= it->second.bytes; }
     m->t[name] = t;
     m->bytes += t.bytes;
     m->finalized = false;
@@ -178,7 +178,7 @@ extern "C" int itb_model_set_tensor(itb_model* m, const char* name, uint32_t ty,
         ITB_CUDA_RET(c, cudaMemcpyAsync(t.a, data, bytes, cudaMemcpyHostToDevice, c->stream), 1);
         ITB_CUDA_RET(c, cudaStreamSynchronize(c->stream), 1);
         auto it = m->t.find(name);
-        if (it != m->t.end()) { cudaFree(it->second.a); m->bytes -= it->second.bytes; }
+        if (it != m->t.end()) { itb_free_weight(c, it->second.a, it->second.b, it->second.scale2); m->bytes -= it->second.bytes; }
         m->t[name] = t; m->bytes += bytes; m->finalized = false;
         return 0;
     }
@@ -227,7 +227,7 @@ extern "C" int itb_model_synth(itb_model* m, uint64_t seed, uint32_t e_lo, uint3
             itb_synth_f32(c->stream, key, s.elems(), s.dist, s.std_, (float*)t.a);
             c->launches++;
             auto it = m->t.find(s.name);
-            if (it != m->t.end()) { cudaFree(it->second.a); m->bytes -= it->second.bytes; }
+            if (it != m->t.end()) { itb_free_weight(c, it->second.a, it->second.b, it->second.scale2); m->bytes -= it->second.bytes; }
             m->t[s.name] = t; m->bytes += t.bytes;
         } else if (s.ty == synth::TY_Q8_0) {
             itb_synth_q8_raw(c->stream, key, s.elems() / 32, s.dist, s.std_, raw);
@@ -375,7 +375,7 @@ extern "C" int itb_model_offload_experts(itb_model* m) {
             h.has_s2 = t.scale2 != nullptr;
             h.s2.assign(t.n_expert, 1.0f);
             if (h.has_s2) ITB_CUDA_RET(c, cudaMemcpy(h.s2.data(), t.scale2, t.n_expert * 4, cudaMemcpyDeviceToHost), 1);
-            cudaFree(t.a); cudaFree(t.b); cudaFree(t.scale2);
+            itb_free_weight(c, t.a, t.b, t.scale2);
             m->bytes -= nb + sb;
             t.a = nullptr; t.b = nullptr; t.scale2 = nullptr;
         }

@@ -133,6 +133,9 @@ bool itb_tc_f16_shape_ok(const DevQ8& w);
 bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode);
 bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode);
 void itb_tc_free(itb_ctx* c);
+// Gives device planes of a weight back, and the tensor-core images made of them: those are found by the planes' addresses, which the next
+// weight may get. What the stream still does with them is waited for. Null planes are fine.
+void itb_free_weight(itb_ctx* c, void* a, void* b, void* scale2);
 
 bool itb_fail(itb_ctx* c, const char* what, cudaError_t e);
 // Before a launch of `fn` with that much dynamic shared memory on the current device (itb_smem.h: a table lookup once it has been

@@ -568,6 +568,16 @@ void itb_tc_free(itb_ctx* c) {
     c->tc_tiles = nullptr; c->tc_n_tiles = nullptr; c->tc_slot_tile = nullptr; c->tc_b_img = nullptr; c->tc_b_sf = nullptr; c->tc_status = nullptr; c->tc_codes = nullptr; c->tc_scales = nullptr; c->tc_cap_codes = c->tc_cap_scales = 0;
     c->tc_cap_tiles = c->tc_cap_slots = c->tc_cap_b = c->tc_cap_sf = 0;
 }
+void itb_free_weight(itb_ctx* c, void* a, void* b, void* scale2) {
+    cudaStreamSynchronize(c->stream);
+    for (const void* plane : {a, b}) {
+        auto it = plane ? c->tc_weights.find(plane) : c->tc_weights.end();
+        if (it == c->tc_weights.end()) continue;
+        cudaFree(it->second.img); cudaFree(it->second.sf);
+        c->tc_weights.erase(it);
+    }
+    cudaFree(a); cudaFree(b); cudaFree(scale2);
+}
 static const itb_ctx::TcWeights* tc_weights_of(itb_ctx* c, cudaStream_t st, const DevFp4& w) {
     auto it = c->tc_weights.find(w.nib);
     if (it != c->tc_weights.end()) return &it->second;

@@ -268,3 +268,63 @@ def test_dense_q8_0_matmuls_on_the_int8_tensor_cores_are_bit_identical(shape):
     o = om.forward([t]); lg, _ = eng.decode([t])
     assert (o.view(np.uint32) == lg[0].view(np.uint32)).all(), "decode step"
     ops.check(); eng.close(); model.close(); ops.close()
+
+
+@pytest.mark.parametrize("opts", ["exact=1,dense=q8tc", "exact=0,dense=f16tc,experts=fp4tc"])
+def test_tensor_core_images_end_with_their_weights(opts):
+    """The tensor paths keep re-tiled images of weights, found by the device address of the weight's planes. A model made after another
+    was destroyed gets its addresses back, a tensor set again frees its old planes: neither may meet the image of what was there
+    before. Logits equal, bit for bit, those of a context that has seen no other weights."""
+    from inferred_thoughts_b200 import host
+    dims = configs.MID
+    prompt = prompt_ids(81, 200, dims["n_vocab"])
+
+    def logits(model):
+        eng = host.Engine(model, 208, 1)
+        out = eng.prefill(prompt).copy()
+        eng.close()
+        return out
+
+    def made(ops, seed):
+        model = host.Model(ops, host_dims(dims)); model.synth(seed)
+        return model
+    fresh = host.B200Ops(0, opts)
+    model = made(fresh, 7)
+    want = logits(model)
+    fresh.check(); model.close(); fresh.close()
+    ops = host.B200Ops(0, opts)
+    first = made(ops, 0)
+    assert (logits(first) != want).any()
+    first.close()
+    second = made(ops, 7)
+    assert (logits(second).view(np.uint32) == want.view(np.uint32)).all(), "a second model in one context"
+    second.synth(0)                                             # every tensor generated again, in place of the other
+    second.synth(7)
+    assert (logits(second).view(np.uint32) == want.view(np.uint32)).all(), "tensors replaced"
+    ops.check(); second.close(); ops.close()
+
+
+@pytest.mark.parametrize("opts", ["exact=1,dense=q8tc", "exact=0,dense=f16tc"])
+def test_tensor_core_image_of_a_dropped_upload(opts):
+    """The op seam drops an upload when its host address names a tensor of another shape: its image goes with it."""
+    from inferred_thoughts_b200 import host
+    rng = np.random.default_rng(82)
+    blocks = np.frombuffer(rng.bytes(128 * 256 // 32 * 34), np.uint8).reshape(-1, 34).copy()
+    blocks[:, :2] = (0.0002 + 0.0002 * rng.random(len(blocks))).astype(np.float16).view(np.uint8).reshape(-1, 2)
+    data = blocks.reshape(-1)
+    x = {n: rng.standard_normal(64 * n).astype(np.float32) for n in (128, 256)}
+
+    def product(ops, n_in):
+        out = np.zeros(64 * (128 * 256 // n_in), np.float32)
+        ops.begin_pass(64)
+        ops.matmul(host.Weights(data, host.Q8_0, n_in, 128 * 256 // n_in), x[n_in], out); ops.host_needs(out); ops.check()
+        return out
+    want = {}
+    for n_in in (128, 256):
+        fresh = host.B200Ops(0, opts)
+        want[n_in] = product(fresh, n_in)
+        fresh.close()
+    ops = host.B200Ops(0, opts)
+    for n_in in (128, 256, 128, 256):
+        assert (product(ops, n_in).view(np.uint32) == want[n_in].view(np.uint32)).all(), n_in
+    ops.close()
