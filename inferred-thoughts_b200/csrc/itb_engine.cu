@@ -1207,8 +1207,6 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     const int qd = d.head_dim * d.n_head, kvd = d.head_dim * d.n_head_kv;
     const int TPB = NWG * 32;
     uint64_t launches = 0;
-    set_smem((const void*)k_matmul_f32_rows<20>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<24>, 64 * 1024);
-    set_smem((const void*)k_matmul_f32_rows<28>, 64 * 1024); set_smem((const void*)k_matmul_f32_rows<32>, 64 * 1024);
     set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
     set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
     set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
@@ -1258,17 +1256,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     };
     auto f32mm = [&](const DevF32& w, const float* x, float* out) {
         if (!c->exact && f16tc && sgemm_chain_ok(w.n_in) && R >= 64) { sgemm_chain<true>(st, sms, w, x, R, out); launches++; return; }   // tolerance-class passes: fused multiply-adds
-        if (!c->exact && w.n_in % 512 == 0 && w.n_in <= 4096) {
-            const dim3 g((w.n_out + 7) / 8, (R + F32_TOK - 1) / F32_TOK);
-            const size_t sm = (size_t)F32_TOK * w.n_in * 4;
-            switch (w.n_in / 128) {
-#define F32_CASE(NV) case NV: k_matmul_f32_rows<NV><<<g, 256, sm, st>>>(w, x, R, out); break;
-                F32_CASE(4) F32_CASE(8) F32_CASE(12) F32_CASE(16) F32_CASE(20) F32_CASE(24) F32_CASE(28) F32_CASE(32)
-#undef F32_CASE
-            }
-            launches++;
-            return;
-        }
+        if (!c->exact && f32_tree_ok(w.n_in)) { f32_tree(st, sms, w, x, R, out); launches++; return; }
         if (c->exact && sgemm_chain_ok(w.n_in)) { sgemm_chain<false>(st, sms, w, x, R, out); launches++; return; }   // also for a few rows: the tile's k loop is as long as a row's chain either way
         const int nw = 4;
         dim3 g(std::max(1, std::min(2 * sms, (w.n_out + 31) / 32)), R);

@@ -264,9 +264,13 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const i
 
 static void launch_f32(itb_ctx* c, const WeightEntry* w, const float* xd, size_t n_tok, float* od) {
     DevF32 dw{(const float*)w->a, (int)w->n_in, (int)w->n_out};
-    if (sgemm_chain_ok(dw.n_in) && (c->exact || (c->f16tc && n_tok >= 64))) {
-        // a chain per (token, output); fused multiply-adds in the tolerance-class mode of many-token passes
-        if (c->exact) sgemm_chain<false>(c->stream, c->sm_count, dw, xd, (int)n_tok, od); else sgemm_chain<true>(c->stream, c->sm_count, dw, xd, (int)n_tok, od);
+    if (c->exact && sgemm_chain_ok(dw.n_in)) {              // a chain per (token, output)
+        sgemm_chain<false>(c->stream, c->sm_count, dw, xd, (int)n_tok, od);
+        ITB_LAUNCHED(c);
+        return;
+    }
+    if (!c->exact && n_tok >= 64 && f32_tree_ok(dw.n_in)) {  // the sums of k_matmul_f32<false>, a weight row read once for four tokens
+        f32_tree(c->stream, c->sm_count, dw, xd, (int)n_tok, od);
         ITB_LAUNCHED(c);
         return;
     }

@@ -11,44 +11,102 @@
 
 namespace {
 
-// F32 matrix against many rows (router logits, alpha/beta, shared-expert gate), tree mode. A block takes 8 weight rows
-// (one per warp, held in registers) and F32_TOK token rows (staged in shared memory with every load in flight at once):
-// two memory round trips per block, blocks for every (row group, token group). Per lane the products are summed in the
-// order of f32_rows<false> (the one-token path), then the same shuffle tree, so a row gets the bits it gets alone.
-// grid (ceil(n_out/8), ceil(n_rows/F32_TOK)), block 256, dynamic smem F32_TOK * n_in floats; n_in = 128 * NV.
+// Sums of N values (4 or 8) over a warp's lanes, each with the additions of warp_sum: at every step a lane adds its partner's value to its
+// own, but hands half of the values over and keeps the other half while there is more than one. The lane gets the sum of value warp_sums_of().
+template <int N>
+__device__ __forceinline__ int warp_sums_of(int lane) { return N == 8 ? (lane >> 2) & 7 : (lane >> 3) & 3; }
+template <int N>
+__device__ __forceinline__ float warp_sums(const float (&a)[N], int lane) {
+    float v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = a[i];
+    int o = 16;
+#pragma unroll
+    for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = hi ? v[i] : v[i + n], mine = hi ? v[i + n] : v[i];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+// F32 matrix against many rows (router logits, alpha/beta, shared-expert gate), tree mode. A block takes 8 * MR weight rows (MR per
+// warp, held in registers) and tok_blk token rows, F32_TOK at a time through shared memory, the next ones on their way meanwhile.
+// Per lane the products are summed in the order of f32_rows<false> (the one-token path), then the same shuffle tree, so a row gets
+// the bits it gets alone.
+// What bounds it: the 16-byte reads of the token rows from shared memory, one for four products of each weight row that a warp holds (2,048
+// rows, 256 outputs, 2,048 k: 60 us with two rows a warp, as much as the products and sums take, 120 with one), and, with a block for
+// every F32_TOK rows, the weights, 1.07 GB from L2. That size takes 117 us; a block per token row and 32 outputs (k_matmul_f32) 307.
+// grid (ceil(n_out / (8 MR)), ceil(n_rows / tok_blk)), block 256, dynamic smem (tok_blk > F32_TOK ? 2 : 1) * F32_TOK * n_in floats; n_in = 128 * NV.
 constexpr int F32_TOK = 4;
-template <int NV>
-__global__ void __launch_bounds__(256) k_matmul_f32_rows(DevF32 w, const float* x, int n_rows, float* out) {
+template <int NV, int MR>
+__global__ void __launch_bounds__(256) k_matmul_f32_rows(DevF32 w, const float* __restrict__ x, int n_rows, float* out, int tok_blk) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* xs = (float*)smem;
-    constexpr int n = 128 * NV;
+    constexpr int n = 128 * NV, N = F32_TOK * MR, PER = F32_TOK * n / 4 / 256;   // PER: float4 per thread of the token tile
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 8 + wid, t0 = blockIdx.y * F32_TOK, nt = min(n_rows - t0, F32_TOK);
-    float4 wv[NV];
-    const float* wr = w.w + (size_t)min(row, w.n_out - 1) * n;
+    const int row0 = (blockIdx.x * 8 + wid) * MR, t_lo = blockIdx.y * tok_blk, t_hi = min(t_lo + tok_blk, n_rows), ng = (t_hi - t_lo + F32_TOK - 1) / F32_TOK;
+    auto fetch = [&](int g) {
+        if (g < ng) {
+            float* to = xs + (size_t)(g & 1) * F32_TOK * n;
 #pragma unroll
-    for (int j = 0; j < NV; ++j) wv[j] = __ldg((const float4*)(wr + lane * 4 + 128 * j));
-    constexpr int PER = F32_TOK * n / 4 / 256;   // float4 per thread of the token tile
-    float4 xv[PER];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int e = threadIdx.x + 256 * i, t = e / (n / 4);
-        xv[i] = t < nt ? __ldg((const float4*)(x + (size_t)t0 * n) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int i = 0; i < PER; ++i) ((float4*)xs)[threadIdx.x + 256 * i] = xv[i];
-    __syncthreads();
-    if (row >= w.n_out) return;
-    for (int t = 0; t < nt; ++t) {
-        const float* xr = xs + (size_t)t * n + lane * 4;
-        float s = 0.0f;
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const float4 v = *(const float4*)(xr + 128 * j);
-            s += wv[j].x * v.x + wv[j].y * v.y + wv[j].z * v.z + wv[j].w * v.w;
+            for (int i = 0; i < PER; ++i) {
+                const int e = threadIdx.x + 256 * i, t = min(t_lo + g * F32_TOK + e / (n / 4), n_rows - 1);
+                cp_async16(to + e * 4, x + (size_t)t * n + (e % (n / 4)) * 4, true);
+            }
         }
-        s = warp_sum(s);
-        if (lane == 0) out[(size_t)(t0 + t) * w.n_out + row] = s;
+        cp_async_commit();
+    };
+    fetch(0);
+    float4 wv[MR][NV];
+#pragma unroll
+    for (int r = 0; r < MR; ++r) {
+        const float* wr = w.w + (size_t)min(row0 + r, w.n_out - 1) * n;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) wv[r][j] = __ldg((const float4*)(wr + lane * 4 + 128 * j));
+    }
+    for (int g = 0; g < ng; ++g) {
+        fetch(g + 1);
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* xr = xs + (size_t)(g & 1) * F32_TOK * n + lane * 4;
+        float s[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) s[i] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+#pragma unroll
+            for (int t = 0; t < F32_TOK; ++t) {
+                const float4 v = *(const float4*)(xr + t * n + 128 * j);
+#pragma unroll
+                for (int r = 0; r < MR; ++r) s[t * MR + r] += wv[r][j].x * v.x + wv[r][j].y * v.y + wv[r][j].z * v.z + wv[r][j].w * v.w;
+            }
+        const float sum = warp_sums<N>(s, lane);
+        const int i = warp_sums_of<N>(lane), t = t_lo + g * F32_TOK + i / MR, row = row0 + i % MR;
+        if ((lane & (32 / N - 1)) == 0 && t < t_hi && row < w.n_out) out[(size_t)t * w.n_out + row] = sum;
+        __syncthreads();                           // everyone is done with these rows before the ones after the next take their place
+    }
+}
+inline bool f32_tree_ok(int n_in) { return n_in % 512 == 0 && n_in <= 4096; }
+// Two weight rows to a warp where their registers allow and the blocks still give every SM two; then as many tokens to a block as
+// leave it two.
+static void f32_tree(cudaStream_t st, int sms, const DevF32& w, const float* x, int n_rows, float* out) {
+    auto blocks = [&](int mr, int tok) { return (long long)((w.n_out + 8 * mr - 1) / (8 * mr)) * ((n_rows + tok - 1) / tok); };
+    const int mr = w.n_in <= 2048 && blocks(2, F32_TOK) >= 2 * sms ? 2 : 1;
+    int tok = F32_TOK;
+    while (tok < 32 && blocks(mr, 2 * tok) >= 2 * sms) tok *= 2;
+    const dim3 g((w.n_out + 8 * mr - 1) / (8 * mr), (n_rows + tok - 1) / tok);
+    const size_t sm = (size_t)(tok > F32_TOK ? 2 : 1) * F32_TOK * w.n_in * 4;
+    auto run = [&](auto k) { itb_raise_smem(k, sm); k<<<g, 256, sm, st>>>(w, x, n_rows, out, tok); };
+    switch (w.n_in / 128) {
+#define F32_CASE(NV) case NV: if (mr == 2) run(k_matmul_f32_rows<NV, 2>); else run(k_matmul_f32_rows<NV, 1>); break;
+#define F32_CASE1(NV) case NV: run(k_matmul_f32_rows<NV, 1>); break;
+        F32_CASE(4) F32_CASE(8) F32_CASE(12) F32_CASE(16) F32_CASE1(20) F32_CASE1(24) F32_CASE1(28) F32_CASE1(32)
+#undef F32_CASE
+#undef F32_CASE1
     }
 }
 

@@ -386,6 +386,29 @@ def test_f32_matmul_tiles_at_their_edges(ops, n_tok, n_in, n_out):
         exact(out, want, "F32 matmul")
 
 
+@pytest.mark.parametrize("n_tok,n_in,n_out", [(64, 512, 1), (65, 2048, 257), (300, 2048, 257), (3001, 1536, 9), (127, 4096, 33),
+                                              (2000, 2560, 17), (70, 384, 20), (66, 4608, 8)])
+def test_f32_matmul_of_many_rows_sums_like_one_row_in_tolerance_mode(n_tok, n_in, n_out):
+    """exact=0: a row gets the partial sums and the tree it gets alone, bit for bit -- not one long chain, whose rounding is seven times
+    theirs at 2,048 terms. Against 64 bits: n/32 + 5 additions and one product on any path, each within eps/2 of the terms' magnitudes."""
+    from inferred_thoughts_b200 import host
+    o = host.B200Ops(0, "exact=0,dense=f16tc")
+    w, x = noise(n_in * n_out, 162, 0.02), noise(n_tok * n_in, 163)
+    wt = host.Weights(w, host.F32, n_in, n_out)
+    out = np.zeros(n_tok * n_out, np.float32)
+    o.begin_pass(n_tok)
+    o.matmul(wt, x, out); o.host_needs(out); o.check()
+    rows = [(np.ascontiguousarray(x[t * n_in:(t + 1) * n_in]), np.zeros(n_out, np.float32)) for t in range(n_tok)]
+    for xr, one in rows[::max(1, n_tok // 200)]:
+        o.matmul(wt, xr, one); o.host_needs(one)
+    o.check()
+    exact(out.reshape(n_tok, n_out)[::max(1, n_tok // 200)].ravel(), np.concatenate([one for _, one in rows[::max(1, n_tok // 200)]]), "rows together and alone")
+    x64, w64 = x.reshape(n_tok, n_in).astype(np.float64), w.reshape(n_out, n_in).astype(np.float64)
+    err = np.abs(out.reshape(n_tok, n_out) - x64 @ w64.T)
+    assert (err <= (n_in / 32 + 6) * EPS / 2 * (np.abs(x64) @ np.abs(w64).T)).all()
+    o.close()
+
+
 @pytest.mark.parametrize("n,ff", [(1, 64), (5, 40), (15, 16)])
 def test_gated_experts_of_few_pairs(ops, n, ff):
     """Fewer pairs than the grouped form takes: 16 gate and 16 up rows to a block, the last block ragged."""
