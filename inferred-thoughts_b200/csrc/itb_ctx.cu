@@ -10,6 +10,7 @@
 #include "itb_internal.cuh"
 #include "itb_pipe.h"
 #include "itb_smem.h"
+#include "itb_threads.h"
 
 void itb_ops_use_logf_fix(const uint32_t* dev_tab, uint32_t n);      // itb_ops.cu: points that unit's log_f at the table
 void itb_engine_use_logf_fix(const uint32_t* dev_tab, uint32_t n);   // itb_engine.cu
@@ -46,28 +47,25 @@ static void build_logf_fix() {
     if (!g_logf_fix_host.empty()) return;
     g_logf_fix_host.assign(LOGF_FIX_N / 16, 0u);
     const unsigned nt = std::max(1u, std::thread::hardware_concurrency());
-    std::vector<std::thread> th;
     std::vector<uint64_t> odd(nt, 0);
     const uint32_t words = LOGF_FIX_N / 16;
-    for (unsigned t = 0; t < nt; ++t)
-        th.emplace_back([=, &odd] {
-            const uint32_t w0 = (uint32_t)((uint64_t)words * t / nt), w1 = (uint32_t)((uint64_t)words * (t + 1) / nt);
-            for (uint32_t w = w0; w < w1; ++w) {
-                uint32_t word = 0;
-                for (uint32_t j = 0; j < 16; ++j) {
-                    const uint32_t bits = 0x3f800000u + w * 16 + j;
-                    float x; memcpy(&x, &bits, 4);
-                    const float lib = logf(x), cr = (float)log((double)x);
-                    uint32_t a, b; memcpy(&a, &lib, 4); memcpy(&b, &cr, 4);
-                    const int32_t d = (int32_t)(a - b);
-                    if (d == 1) word |= 1u << (2 * j);
-                    else if (d == -1) word |= 2u << (2 * j);
-                    else if (d != 0) odd[t]++;
-                }
-                g_logf_fix_host[w] = word;
+    on_threads(nt, [&](unsigned t) {
+        const uint32_t w0 = (uint32_t)((uint64_t)words * t / nt), w1 = (uint32_t)((uint64_t)words * (t + 1) / nt);
+        for (uint32_t w = w0; w < w1; ++w) {
+            uint32_t word = 0;
+            for (uint32_t j = 0; j < 16; ++j) {
+                const uint32_t bits = 0x3f800000u + w * 16 + j;
+                float x; memcpy(&x, &bits, 4);
+                const float lib = logf(x), cr = (float)log((double)x);
+                uint32_t a, b; memcpy(&a, &lib, 4); memcpy(&b, &cr, 4);
+                const int32_t d = (int32_t)(a - b);
+                if (d == 1) word |= 1u << (2 * j);
+                else if (d == -1) word |= 2u << (2 * j);
+                else if (d != 0) odd[t]++;
             }
-        });
-    for (auto& t : th) t.join();
+            g_logf_fix_host[w] = word;
+        }
+    });
     for (uint64_t o : odd) g_logf_fix_odd += o;
 }
 static const uint32_t* logf_fix_on_device(int dev) {

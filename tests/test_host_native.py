@@ -145,3 +145,21 @@ def test_transfers_without_pinned_memory_or_events(tmp_path):
 def test_transfers_whose_events_cannot_be_recorded_or_waited_for(tmp_path):
     """A staging buffer is not written again while a copy may still read it, whichever call fails."""
     run(tmp_path, FAKE_RUNTIME + "int main() { no_record = true; transfers(); no_record = false; no_wait = true; transfers(); return 0; }")
+
+
+def test_shares_whose_thread_is_refused_run_on_the_caller(tmp_path):
+    """The correction table of log is built on all host threads inside a C entry point: a refused thread must not end the program."""
+    run(tmp_path, FAKE_RUNTIME + r"""
+#include "itb_threads.h"
+int main() {
+    for (int refused : {0, 1}) {
+        no_thread = refused;
+        for (unsigned n : {1u, 2u, 33u}) {
+            std::vector<int> seen(n, 0);
+            on_threads(n, [&](unsigned t) { seen[t]++; });
+            for (int s : seen) CHECK(s == 1);
+        }
+    }
+    return 0;
+}
+""")
