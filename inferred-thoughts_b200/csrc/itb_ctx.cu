@@ -7,6 +7,7 @@
 #include <new>
 #include <thread>
 
+#include "itb_grow.h"
 #include "itb_internal.cuh"
 #include "itb_pipe.h"
 #include "itb_smem.h"
@@ -293,20 +294,10 @@ extern "C" void itb_device_report(itb_ctx* c) {
 }
 
 bool itb_ensure_route(itb_ctx* c, size_t n_pairs) {
-    if (c->route_cap >= n_pairs) return true;
-    cudaFree(c->route_ids); cudaFree(c->route_w);
-    if (cudaMalloc(&c->route_ids, n_pairs * 4) != cudaSuccess || cudaMalloc(&c->route_w, n_pairs * 4) != cudaSuccess)
-        return itb_fail_msg(c, "cudaMalloc(route)");
-    c->route_cap = n_pairs;
-    return true;
+    return grow_scratch(&c->route_cap, n_pairs, {{(void**)&c->route_ids, n_pairs * 4}, {(void**)&c->route_w, n_pairs * 4}}) || itb_fail_msg(c, "cudaMalloc(route)");
 }
 bool itb_ensure_xq(itb_ctx* c, size_t n) {
-    if (c->xq_cap >= n) return true;
-    cudaFree(c->xq); cudaFree(c->xs);
-    if (cudaMalloc(&c->xq, n) != cudaSuccess || cudaMalloc(&c->xs, (n / 16 + 1) * 4) != cudaSuccess)
-        return itb_fail_msg(c, "cudaMalloc(xq)");
-    c->xq_cap = n;
-    return true;
+    return grow_scratch(&c->xq_cap, n, {{(void**)&c->xq, n}, {(void**)&c->xs, (n / 16 + 1) * 4}}) || itb_fail_msg(c, "cudaMalloc(xq)");
 }
 
 // ------------------------------------------------------------------ repack kernels

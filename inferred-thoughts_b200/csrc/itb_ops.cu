@@ -6,6 +6,7 @@
 #include "itb_attn_mma.cuh"
 #include "itb_rows.cuh"
 #include "itb_exp.cuh"
+#include "itb_grow.h"
 
 static inline unsigned blocks_for(size_t n, int per = 256) { return (unsigned)((n + per - 1) / per); }
 
@@ -545,11 +546,7 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
     }
     int n_split = (int)std::max<size_t>(1, std::min<size_t>((a->n_pos + 63) / 64, (size_t)(2 * c->sm_count) / (a->n_head_kv * n_q) + 1));
     size_t need = n_q * a->n_head * n_split * (a->head_dim + 2);
-    if (c->tmp_cap < need) {
-        cudaFree(c->tmp_f32);
-        if (cudaMalloc(&c->tmp_f32, need * 4) != cudaSuccess) { itb_fail_msg(c, "cudaMalloc(attention partials)"); return; }
-        c->tmp_cap = need;
-    }
+    if (!grow_scratch(&c->tmp_cap, need, {{(void**)&c->tmp_f32, need * 4}})) { itb_fail_msg(c, "cudaMalloc(attention partials)"); return; }
     float* pa = c->tmp_f32; float* pm = pa + n_q * a->n_head * n_split * a->head_dim;
     itb_attend_dev(c, c->stream, qd, kd, vd, (int)a->kv_dim, (int)a->n_pos, (int)n_q, (int)a->head_dim, (int)a->n_head,
                    (int)a->n_head_kv, a->scale, (int)c->kv_bf16, nullptr, nullptr, pa, pm, n_split, od);

@@ -163,3 +163,32 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_scratch_that_cannot_grow_leaves_no_stale_pointer(tmp_path):
+    """One of two buffers cannot be had: both are gone and the capacity says so; a later call that needs less makes them again."""
+    run(tmp_path, CHECK + r"""
+#include <set>
+#include "itb_grow.h"
+static std::set<void*> alive;
+static int made = 0, fail_at = -1;
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) { if (made++ == fail_at) return cudaErrorMemoryAllocation; *p = malloc(n); alive.insert(*p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { if (p) { CHECK(alive.erase(p) == 1); free(p); } return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+}
+int main() {
+    for (int f : {-1, 2, 3}) {
+        made = 0; fail_at = f;
+        void *a = nullptr, *b = nullptr; size_t cap = 0;
+        CHECK(grow_scratch(&cap, 100, {{&a, 100}, {&b, 400}}) && cap == 100 && alive.count(a) && alive.count(b) && alive.size() == 2);
+        CHECK(grow_scratch(&cap, 60, {{&a, 60}, {&b, 240}}) && cap == 100 && made == 2);
+        const bool ok = grow_scratch(&cap, 1000, {{&a, 1000}, {&b, 4000}});
+        CHECK(ok == (f < 0));
+        if (!ok) CHECK(!a && !b && cap == 0 && alive.empty());
+        CHECK(grow_scratch(&cap, 50, {{&a, 50}, {&b, 200}}) && alive.count(a) && alive.count(b) && alive.size() == 2);
+        cudaFree(a); cudaFree(b);
+    }
+    return 0;
+}
+""")
