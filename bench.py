@@ -32,8 +32,8 @@ PROMPT, N_CTX = 512, 8192
 FALLBACK_HBM = 6650.0
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from the ncu capture summarised in
 # profiles/decode_step_bs1_kernels_4layer_ncu_full.md (per-launch traffic does not depend on the layer count)
-NCU_TRAFFIC = {"k_moe_glu": 9503000, "k_moe_down": 5881000, "k_in_proj[gdn]": 27570000, "k_in_proj[ffn]": 4413000,
-               "k_out_proj": 8943000, "k_gdn_core": 2192000}
+NCU_TRAFFIC = {"k_moe_glu": 9507000, "k_moe_down": 5887000, "k_in_proj[gdn]": 27597000, "k_in_proj[ffn]": 4485000,
+               "k_out_proj": 8951000, "k_gdn_core": 2196000}
 
 
 def peaks():
@@ -316,8 +316,8 @@ def other_configs(host, model, dims, seed, hbm, args, mode):
     try:
         ms = timed_prefill(host, model, n_vocab, seed)
         out["prefill_5548_exact"] = {"value": 5548 / (ms / 1e3), "unit": "tok/s", "ms": ms, "rows_per_pass": PREFILL_ROWS, "ops": mode,
-                                     "note": "bit-identical to the CPU path: dense Q8_0 matmuls as tcgen05 int8 MMAs with the block scales applied in CPU order, "
-                                             "expert-grouped NVFP4 x int8 tiles, CPU-order attention and delta-rule scan"}
+                                     "note": "bit-identical to the CPU path: exact dense Q8_0 matmuls on tcgen05 with the block scales applied in CPU order, "
+                                             "expert-grouped NVFP4 x int8-valued f16 tiles, CPU-order attention and delta-rule scan"}
     except Exception as ex:
         out["prefill_5548_exact"] = {"error": str(ex)}
     try:
@@ -370,14 +370,14 @@ def other_configs(host, model, dims, seed, hbm, args, mode):
             fast_model.close()
         if fast_ops is not None:
             fast_ops.close()
-    # the same tolerance-class pass with the dense matmuls kept bit-exact (int8 MMAs, scales in CPU order)
+    # the same tolerance-class pass with the dense matmuls kept bit-exact (exact dots, scales in CPU order)
     fast_ops = fast_model = None
     try:
         fast_ops = host.B200Ops(0, FAST_MODE_Q8)
         fast_model = host.Model(fast_ops, host.ModelDims(**dims)); fast_model.synth(configs.SEEDS[args.model])
         ms = timed_prefill(host, fast_model, n_vocab, seed)
         out["prefill_5548_exact_dense"] = {"value": 5548 / (ms / 1e3), "unit": "tok/s", "ms": ms, "rows_per_pass": PREFILL_ROWS, "ops": FAST_MODE_Q8,
-                                           "note": "as prefill_5548, but the dense Q8_0 matmuls as tcgen05 int8 MMAs per 32-element block with the scales applied in CPU "
+                                           "note": "as prefill_5548, but the dense Q8_0 matmuls as exact tcgen05 dots per 32-element block with the scales applied in CPU "
                                                    "order (bit-identical dense results)"}
     except Exception as ex:
         out["prefill_5548_exact_dense"] = {"error": str(ex)}

@@ -50,7 +50,7 @@ typedef struct { const float *q, *k, *v, *alpha, *beta, *ssm_a, *dt_bias; size_t
  * exact=0|1 (1, default: every sum in the CPU path's order -- F32 dots fold serially, attention walks positions in order --
  *   so results equal the CPU path bit for bit; 0: tree-summed F32 dots, split-K attention, and the many-token kernels below),
  * many-token passes (each also selectable on its own under exact=1; all tolerance class except dense=q8tc):
- *   dense=q8tc     dense Q8_0 matmuls as tcgen05 int8 MMAs per 32-element block, scales applied in CPU order (bit-identical),
+ *   dense=q8tc     dense Q8_0 matmuls as exact tcgen05 dots per 32-element block, scales applied in CPU order (bit-identical),
  *   dense=f16tc    dense Q8_0 matmuls as f16 tcgen05 GEMMs: weights and the Q8_0-quantised activation rows dequantised to f16
  *                  (int8 * block scale, rounded to nearest), f32 accumulators; 2 more bytes of device memory per dense weight;
  *                  wins over dense=q8tc where both are given; with exact=0 the small F32 matrices run as fused-multiply-add tiles,

@@ -1,4 +1,4 @@
-"""The synthetic model shapes BASELINE.json names (qwen35moe structure, src/model/qwen35.rs:193-249)."""
+"""The synthetic model shapes (qwen35moe structure, src/model/qwen35.rs:193-249)."""
 
 # cfg 1: tiny hybrid MoE, layers GDN, GDN, GDN, full attention. n_rot is hd/4, the 35B's 64/256 ratio.
 TINY = dict(n_layer=4, n_embd=256, n_head=4, n_head_kv=1, head_dim=64, n_vocab=1024, rope_theta=1e7, rms_eps=1e-6,

@@ -121,7 +121,7 @@ __device__ __forceinline__ float serial_sum(const float* w, int n) {
 // A value line's four 16-byte pieces go to neighbouring lanes (a lane per position touched 32 lines a load); the lines of each eight
 // dimensions start 8 floats further on, so that their products fall on distinct banks.
 constexpr int AX_VT = 128, AX_VLD = AX_VT + 4, AX_AHEAD = 4, AX_VBUF = 32 * AX_VLD + 32;
-constexpr int AX_OUT_SMEM = 226 * 1024;       // room for 49,408 positions
+constexpr int AX_OUT_SMEM = 226 * 1024;       // room for 49,344 positions beside the two tiles of products
 struct AxOut {
     const float* scores; int s_stride;
     const uint16_t* vslab; size_t slab_stride; int rows_per_seq;

@@ -9,8 +9,8 @@
 // d * sum is exact whatever order it adds in, and dy times it rounds once: the CPU's term to the bit, for two f32 operations per
 // (row, token, sub-block) instead of the five an integer MMA needs (convert twice, two scales, add). tests compare bits.
 //
-// Rates measured on this GPU: m16n8k16 f16 with its accumulators used, one per 2.8 cycles per SM (int8 m16n8k16: 1.3, but then
-// five f32 operations on 128 outputs are 5 cycles of the f32 pipe); f32 pipe 128 lanes per cycle, so mul + add are 2.0 cycles.
+// Rates measured on this GPU: m16n8k16, f16 or int8, one per 2.0 cycles and SM; f32 pipe 128 lanes per cycle, so mul + add on the 128
+// outputs of one are 2.0 cycles too, where the five operations behind an int8 dot would be 5.
 //
 // Two f32 operations go out as fma.rn.f32x2 / add.rn.f32x2 (two tokens per instruction: half the issue slots). The product is
 // fma(c, dy, 0) and not mul.rn.f32x2: the assembler contracts a packed multiply and the packed add behind it into one fma
@@ -122,9 +122,10 @@ __device__ __forceinline__ void exp_stage(const unsigned char* w0, const unsigne
 // grid (tiles, ceil(n_out / (GLU ? 128 : 256))), block 256: a block is one tile of an expert's pairs; a warp owns 16 gate rows and the same 16 up rows, or 32 rows of the
 // down matrix, and all tokens of the tile (up to 8 * NJ); groups of 8 tokens past the tile's last pair are
 // skipped, so a tile costs what it holds. k in stages of 128 through a cp.async ring. Any n_in that is a multiple of 64.
-// What bounds it: with 1-2 pairs per expert (batched decode) HBM -- each expert's weights once -- and the E2M1 decode (44 of 77
-// instructions per 32-element block); with many pairs the MMAs and the f32 operations behind them, which overlap only in part
-// (3.8 cycles per MMA and SM in the loop alone, against 2.1 for the MMAs and 2.2 for the f32 pipe).
+// What bounds it: with 1-2 pairs per expert (batched decode) the start of a tile -- a block serves one and begins with an empty ring:
+// at 32 rows gate + up stream their 197 MB at 42 % of DRAM's peak with 64 % of the issue slots and 20 % of the tensor pipe busy, down
+// its 98 MB at 34 %; with many pairs the MMAs and the f32 operations behind them, which overlap only in part (3.8 cycles per MMA
+// and SM in the loop alone, against 2.0 for the MMAs and as much for the f32 pipe; 2,048 rows: tensor pipe 34 %, f32 pipe 45 %).
 // Feeding the stages by bulk copies from a ninth warp was slower (1 KB and 128-byte pieces: 102 us against 63 at 32 tokens).
 template <int NJ, bool GLU>
 __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {

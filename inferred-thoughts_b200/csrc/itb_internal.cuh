@@ -118,7 +118,7 @@ struct itb_ctx {
     uint8_t* tc_hf_b = nullptr; size_t tc_cap_hfb = 0;                 // dense=f16tc: the pass's activation rows as f16 operand tiles
     uint64_t tc_hf_src = 0; int tc_hf_src_rows = 0, tc_hf_src_in = 0;
     bool f16tc = false;     // opts dense=f16tc: many-row passes run the dense Q8_0 matmuls as f16 tcgen05 GEMMs over dequantised operands (tolerance class)
-    bool q8tc = false;       // opts dense=q8tc: many-row passes run the dense Q8_0 matmuls as tcgen05 int8 MMAs (bit-identical results)
+    bool q8tc = false;       // opts dense=q8tc: many-row passes run the dense Q8_0 matmuls on tcgen05 (bit-identical results)
     bool fp4tc = false;      // opts experts=fp4tc: many-row passes multiply FP4 activations on the tensor cores
     bool gdn_chunk = false;  // opts gdn=chunk: many-token passes run the delta rule chunk-parallel even under exact=1 (exact=0 always does)
     bool attn_mma = false;   // opts attn=mma: many-token passes run attention as 16-bit matrix products even under exact=1 (exact=0 always does)

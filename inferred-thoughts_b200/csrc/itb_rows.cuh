@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(256) k_gdn_pre(const float* conv, int cd, cons
 // Bound by that chain: 128 adds of 4 cycles a token, and a scheduler has about one warp, whose instructions go between them. So a
 // token's read-out sum goes along with the NEXT token's prediction sum as the other half of packed adds (one instruction for both);
 // the update, decay and products of a column are formed in the first quarter's steps, just ahead of the add that takes them; the
-// next token's operands come during the other quarters, in straight-line code. A 512-token pass of 32 heads: 429 -> 257 us a layer
+// next token's operands come during the other quarters, in straight-line code. A 512-token pass of 32 heads: 429 -> 256 us a layer
 // (lines of a quarter are CW + 4 floats apart: the four lanes of a row read distinct banks, where they shared one).
 template <int SK>
 __global__ void __launch_bounds__(128) k_gdn_scan(const float* qh, const float* kh, const float* vh, const float* gb, int n_tok, int n_k, int n_v,

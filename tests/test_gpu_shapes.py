@@ -243,9 +243,9 @@ def test_three_sequences_with_tensor_core_attention():
 
 
 @pytest.mark.parametrize("shape", ["mid", "m35b", "l177b"])
-def test_dense_q8_0_matmuls_on_the_int8_tensor_cores_are_bit_identical(shape):
-    """dense=q8tc: many-row passes run every dense Q8_0 matmul as tcgen05 int8 MMAs (one per 32-element block, s32 accumulators
-    in tensor memory), the block scales and the sum applied afterwards in the CPU path's order and rounding. Nothing is
+def test_dense_q8_0_matmuls_on_the_tensor_cores_are_bit_identical(shape):
+    """dense=q8tc: many-row passes run every dense Q8_0 matmul as tcgen05 MMAs (two of kind::f16 per 32-element block: int8 values are
+    exact in f16 and the block's dot in the f32 accumulator), the block scales and the sum applied afterwards in the CPU path's order and rounding. Nothing is
     reassociated, so under exact=1 the logits of a 200-token prompt pass (a ragged second token tile), of 70 more tokens and
     of a decode step must equal the oracle's bit for bit."""
     from inferred_thoughts_b200 import host

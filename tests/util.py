@@ -1,4 +1,4 @@
-"""Shared test helpers: configurations named in BASELINE.json and seeded inputs."""
+"""Shared test helpers: the synthetic model shapes and seeded inputs."""
 import numpy as np
 
 from inferred_thoughts_b200.configs import TINY, MID, ODD, M35B, L177B  # noqa: F401
