@@ -34,6 +34,7 @@ template <int NJ> struct ExpCfg {
     static constexpr int NST = NJ >= 8 ? 2 : 3;          // stages
 };
 constexpr int EX_VS = 132;                               // floats per token of the gate and up tiles (they reuse the ring: 2 x 64 x 132 x 4 bytes fit two stages)
+constexpr size_t EX_SMEM = 224 * 1024;
 template <int NJ> static inline size_t exp_smem(int k) { return (size_t)ExpCfg<NJ>::NST * ExpCfg<NJ>::STAGE + (size_t)(k / 32) * ExpCfg<NJ>::TOK * 4; }
 
 // Two E2M1 codes (low byte of w >> 8 * B, low nibble first) to two f16, times the scale pair: exact.
@@ -278,9 +279,11 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
 }
 template <int NJ, bool GLU>
 static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) {
-    itb_raise_smem(k_exp<NJ, GLU>, 224 * 1024);
+    itb_raise_smem(k_exp<NJ, GLU>, EX_SMEM);
     k_exp<NJ, GLU><<<dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st>>>(a);
 }
+// The activation scales of a tile's whole rows lie beside the ring: up to 18,944 elements of k with 64 tokens.
+static inline bool exp_k_ok(int k) { return exp_smem<8>(k) <= EX_SMEM; }
 // Pairs per tile. Up to 4 per expert on average nearly every expert holds at most 16: tiles of 16, whose kernel keeps three stages
 // of the weight stream in flight in each of three blocks to an SM. More: 64, so that an expert's weights are decoded once for
 // most of its pairs -- unless that leaves SMs without a block (few experts or short rows): then as many as give every SM four.

@@ -363,10 +363,10 @@ static bool stage_route(itb_ctx* c, const itb_route_t* r, size_t n_expert) {
 }
 // Many pairs: grouped by expert, an expert's rows through the tensor-core form of the CPU arithmetic (itb_exp.cuh), so its weights
 // are read once (the reference groups the same way, kernels/moe.cuh:62-133 there). u: the up stack of a gated pair, or null.
-// False: too few pairs, or a stack it does not take.
+// False: too few pairs, or a stack it does not take (rows too long for the tiles' shared memory among them).
 static bool experts_grouped(itb_ctx* c, const itb_experts* g, const itb_experts* u, const itb_route_t* r, const float* xd, size_t x_len, float* od) {
     const size_t n_pairs = r->n_tok * r->n_used, rows = x_len / g->n_in, k = g->n_in;
-    if (g->ggml_type != ITB_NVFP4 || (u && u->ggml_type != ITB_NVFP4) || n_pairs < 16 || g->n_expert > 1024 || g->n_out % 32) return false;
+    if (g->ggml_type != ITB_NVFP4 || (u && u->ggml_type != ITB_NVFP4) || n_pairs < 16 || g->n_expert > 1024 || g->n_out % 32 || !exp_k_ok((int)k)) return false;
     const WeightEntry* wg = itb_weight(c, g->data, g->bytes, g->ggml_type, g->n_in, g->n_out, g->n_expert, g->scale, g->scale_bytes);
     const WeightEntry* wu = u ? itb_weight(c, u->data, u->bytes, u->ggml_type, u->n_in, u->n_out, u->n_expert, u->scale, u->scale_bytes) : nullptr;
     if (!wg || (u && !wu)) return true;                       // failed loudly

@@ -371,6 +371,21 @@ def test_grouped_expert_tiles_at_their_edges(ops, E, H, ff):
     exact(o, o_want, "matmul_experts(down)")
 
 
+@pytest.mark.parametrize("n_in", [18944, 19008])
+def test_grouped_experts_with_rows_as_long_as_the_tiles_hold_and_longer(ops, n_in):
+    """The grouped form keeps a tile's activation scales in shared memory; longer rows take the form without tiles."""
+    from inferred_thoughts_b200 import host
+    E, n_out, n = 3, 32, 16
+    wb, sc = nvfp4_weights(E, n_out, n_in, 171)
+    x = noise(n * n_in, 172); ids = np.random.default_rng(173).integers(0, E, n).astype(np.int32)
+    out = keep(np.zeros(n * n_out, np.float32)); want = np.zeros_like(out)
+    ops.begin_pass(n)
+    ops.matmul_experts(host.Experts(wb, host.NVFP4, n_in, n_out, E, sc), host.Route.host(ids.astype(np.uint64), None, 1), x, out)
+    ops.host_needs(out); ops.check()
+    L.orc_matmul_experts(wb, n_in, n_out, E, sc.ctypes.data, ids, n, 1, x, x.size, want, 0)
+    exact(out, want, "experts of long rows")
+
+
 @pytest.mark.parametrize("n_tok,n_in,n_out", [(1, 64, 1), (15, 384, 16), (17, 2048, 33), (33, 448, 129), (300, 64, 1000), (321, 2048, 993)])
 def test_f32_matmul_tiles_at_their_edges(ops, n_tok, n_in, n_out):
     """Chains per output in 16 x 16 and 32 x 64 tiles: fewer k steps than the ring has stages, ragged rows and outputs; inputs and outputs
