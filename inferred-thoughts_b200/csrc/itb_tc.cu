@@ -9,32 +9,10 @@
 // Every wait is bounded; a kernel that gives up frees its tensor memory and reports through its status word.
 #include "itb_internal.cuh"
 #include "itb_gemv.cuh"
+#include "itb_tcgen.cuh"
 
 namespace {
 
-__device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// Bounded wait on an mbarrier phase: polls (the try_wait itself suspends for a short, hardware-chosen time) and gives up after
-// `limit_cycles` of this SM's clock (the cheap clock: reading the global timer in the polling loop costs microseconds).
-__device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit_cycles) {
-    auto arrived = [&] {
-        uint32_t ok;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        return ok != 0;
-    };
-    if (arrived()) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 64; ++i)
-            if (arrived()) return true;
-        if ((unsigned long long)(clock64() - t0) > limit_cycles) return false;
-    }
-}
-// Shared-memory matrix descriptor, K-major, no swizzle: 8-row x 16-byte core matrices; `lbo` = bytes between the two 16-byte
-// K chunks of a row, `sbo` = bytes between 8-row groups; version 1 (this architecture) in bits 46-47.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((smem_addr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) | ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | (1ull << 46);
-}
 // Instruction descriptor of kind::mxf4nvf4: E2M1 x E2M1 (format code 1), UE4M3 scales (0), both operands K-major, M x N.
 __host__ __device__ constexpr uint32_t tc_idesc_fp4(int m, int n) { return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
 
@@ -694,24 +672,27 @@ extern "C" int itb_fp4_quantize(itb_ctx* c, const float* x, size_t n, uint8_t* s
 // The CPU path's Q8_0 dot (src/ops/naive.rs:676-712) is, per 32-element block, an integer dot product, converted to f32,
 // times (weight scale * activation scale), added to the row's sum in block order. The dot of 128 weight rows against NT activation
 // rows is two tcgen05.mma kind::f16 (M 128, N NT, K 16 each, f32 accumulators in tensor memory, the second accumulating): int8 values
-// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. Two stages'
-// accumulators fill tensor memory, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
-// scales and the addition in the CPU's own order and rounding. The result equals the CPU path to the bit; what bounds the kernel is
-// those three f32 instructions per (output, block): 384 cycles a block of 128 x 128. kind::i8 with eight warps, whose s32 accumulators
-// took two more instructions to convert and which had two warps a scheduler to hide the read-back, took 1,407; with waits and releases
-// per block this took 1,241, per stage of two 911 (128 x 64: 880, per stage of two 576, of four 457).
+// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. The accumulators of two to four
+// stages fill tensor memory, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
+// scales and the addition in the CPU's own order and rounding, two columns to an instruction (the products as fma with a zero the compiler
+// cannot see: the assembler fuses a packed multiply into the packed add behind it). The result equals the CPU path to the bit. What bounds it:
+// three f32 operations per (output, block), 384 cycles for the 16,384 outputs of 256 x 64, and their latencies with four warps to a scheduler
+// (f32 pipe 52 %). Measured per 16,384 outputs: 750 cycles (128 x 128 tiles with a value's scale read for each: 911; scalar instructions did
+// not change that, the reads of shared memory did); 128 x 64, for grids that would leave SMs idle, 380 per 8,192 (457). Waits and releases per
+// block instead of per stage of two cost 330 more.
 // Operand images ("K32 block": two K16 blocks of rows x 16 f16 = rows x 32 B as [2 chunks of 16 B][rows / 8][8 rows][16 B], K-major, no
 // swizzle; descriptor leading offset rows * 16, stride offset 128) are made once per weight matrix and once per pass for the activations.
 namespace {
 
-template <int NT> __host__ __device__ constexpr int q8_kb() { return 256 / NT; }      // K32 blocks per pipeline stage: two stages' accumulators fill tensor memory
 constexpr int Q8_EPW = 16;         // warps that read accumulators back
 constexpr int Q8_A_BLK = 128 * 64;                                         // bytes of a weight K32 block
-template <int NT> __host__ __device__ constexpr int q8_stage_bytes() { return q8_kb<NT>() * (Q8_A_BLK + NT * 64 + (128 + NT) * 4); }     // A | B | weight scales | activation scales
-template <int NT> __host__ __device__ constexpr int q8_stages() { return 200 * 1024 / q8_stage_bytes<NT>(); }
-
-// kind::f16: f32 accumulators (1 at bit 4), f16 operands (0 at bits 7 and 10), both K-major, M x N
-__host__ __device__ constexpr uint32_t tc_idesc_f16(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+template <int NT, int MT> struct Q8Cfg {                                  // tokens and 128-row weight tiles of a block
+    static constexpr int KB = MT == 1 ? 256 / NT : 2;                     // K32 blocks per pipeline stage
+    static constexpr int ND = 512 / (MT * NT * KB);                       // stages whose accumulators tensor memory holds
+    static constexpr int B_BLK = NT * 64, O_B = MT * KB * Q8_A_BLK, O_SA = O_B + KB * B_BLK, O_SB = O_SA + MT * KB * 512, STAGE = O_SB + KB * NT * 4;      // A | B | weight scales | activation scales
+    static constexpr int STAGES = 200 * 1024 / STAGE;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE + 128;
+};
 
 // int8 rows -> K32 block images of tiles of `tile` rows, scales -> f32 per (row tile, block, row). One thread per (row, block); rows
 // past n_rows are zeros. scales16 (f16, per weight row and block) or scales32 (f32, per activation row and block): whichever is not null.
@@ -747,163 +728,182 @@ struct TcQ8 {
     int kbs, n_rows, n_out;
     float* out; size_t stride; int mode;          // out[token][row]; mode 1: += (the residual add of an output projection)
     int* status;
+    unsigned long long zero2;                     // two f32 zeros the compiler knows nothing about
     long long* prof;                              // optional: 8 words per block, the first its cycles (ITB_TC_PROF=1)
 };
-// grid (n_out / 128, token tiles of NT); block 576: warps 0-15 read accumulators back and scale (lane quarter = warp % 4, NT / 4 columns by
-// warp / 4), warp 16 fetches operands, warp 17 issues the MMAs.
-template <int NT>
+// grid (weight rows / (128 MT), token tiles of NT); block 576: warps 0-15 read accumulators back and scale (lane quarter = warp % 4, NT / 4 columns of
+// every row tile by warp / 4), warp 16 fetches operands, warp 17 issues the MMAs.
+template <int NT, int MT>
 __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int STAGES = q8_stages<NT>(), STAGE = q8_stage_bytes<NT>(), CW = NT / 4, H = CW / 16, B_BLK = NT * 64, KB = q8_kb<NT>(), PAIRS = KB * H / 2;
-    __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[2], s_dfree[2];
+    using C = Q8Cfg<NT, MT>;
+    constexpr int STAGES = C::STAGES, STAGE = C::STAGE, KB = C::KB, ND = C::ND, CW = NT / 4, UW = CW < 16 ? CW : 16, UC = CW / UW, UNITS = KB * MT * UC;     // a unit: UW columns of a block's row tile
+    __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[ND], s_dfree[ND];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int rt = blockIdx.x, tt = blockIdx.y, kbs = p.kbs, n_stage = kbs / KB;
     const uint32_t sbase = tc_smem(smem);
     if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&s_full[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&s_empty[s])), "r"(1 + Q8_EPW) : "memory");      // the MMAs' commit + the warps done with the scales
-        }
-        for (int i = 0; i < 2; ++i) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&s_dfull[i])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&s_dfree[i])), "r"(Q8_EPW) : "memory");
-        }
+        for (int s = 0; s < STAGES; ++s) { tc_mbar_init(&s_full[s], 1); tc_mbar_init(&s_empty[s], 1 + Q8_EPW); }      // empty: the MMAs' commit + the warps done with the scales
+        for (int i = 0; i < ND; ++i) { tc_mbar_init(&s_dfull[i], 1); tc_mbar_init(&s_dfree[i], Q8_EPW); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (wid == Q8_EPW + 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc_smem(&s_tmem)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (wid == Q8_EPW + 1) tc_alloc(&s_tmem, 512);
+    tc_fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tc_fence_after();
     const uint32_t tm = s_tmem;
-    constexpr uint32_t O_B = KB * Q8_A_BLK, O_SA = O_B + KB * B_BLK, O_SB = O_SA + KB * 128 * 4;
     bool ok = true;
-    if (wid == Q8_EPW && lane == 0) {
-        const size_t a0 = (size_t)rt * kbs, b0 = (size_t)tt * kbs;
-        for (int st = 0; st < n_stage && ok; ++st) {
-            const int s = st % STAGES;
-            if (st >= STAGES) ok = tc_mbar_wait(tc_smem(&s_empty[s]), ((st / STAGES) - 1) & 1, 2000000000ull);
+    // Waits of a whole warp for two barriers at once (b1 0: one): a look at one that is ready takes 80 cycles, and the looks overlap.
+    auto wait = [&](uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1) {
+        bool r = tc_mbar_try(b0, p0);
+        if (b1) r &= tc_mbar_try(b1, p1);
+        if (__all_sync(0xffffffffu, r)) return;
+        r = ok && tc_mbar_wait(b0, p0, 2000000000ull);
+        if (b1) r = r && tc_mbar_wait(b1, p1, 2000000000ull);
+        ok = __all_sync(0xffffffffu, r);
+    };
+    if (wid == Q8_EPW) {
+        const size_t a0 = (size_t)rt * MT * kbs, b0 = (size_t)tt * kbs;
+        int s = 0; uint32_t phase = 1;
+        for (int st = 0; st < n_stage; ++st) {
+            if (st >= STAGES) wait(tc_smem(&s_empty[s]), phase, 0, 0);
             if (!ok) break;
             const uint32_t full = tc_smem(&s_full[s]), dst = sbase + s * STAGE;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)STAGE) : "memory");
             const size_t kb0 = (size_t)st * KB;
-            tc_bulk(dst, p.a_img + (a0 + kb0) * Q8_A_BLK, KB * Q8_A_BLK, full);
-            tc_bulk(dst + O_B, p.b_img + (b0 + kb0) * B_BLK, KB * B_BLK, full);
-            tc_bulk(dst + O_SA, p.a_sc + (a0 + kb0) * 128, KB * 128 * 4, full);
-            tc_bulk(dst + O_SB, p.b_sc + (b0 + kb0) * NT, KB * NT * 4, full);
-        }
-        if (!ok) atomicCAS(p.status, 0, 3);
-    } else if (wid == Q8_EPW + 1 && lane == 0) {
-        const uint32_t idesc = tc_idesc_f16(128, NT);
-        const uint64_t dA = tc_desc(sbase, 2048, 128), dB = tc_desc(sbase + O_B, NT * 16, 128);
-        for (int st = 0; st < n_stage && ok; ++st) {
-            const int s = st % STAGES, dp = st & 1;
-            ok = tc_mbar_wait(tc_smem(&s_full[s]), (st / STAGES) & 1, 2000000000ull);
-            if (ok && st >= 2) ok = tc_mbar_wait(tc_smem(&s_dfree[dp]), ((st >> 1) - 1) & 1, 2000000000ull);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t so = (uint32_t)s * (STAGE >> 4);
+            if (tc_elect()) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)STAGE) : "memory");
 #pragma unroll
-            for (uint32_t i = 0; i < 2 * KB; ++i)
-                asm volatile(
-                    "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }\n"
-                    ::"r"(tm + (uint32_t)NT * (KB * dp + i / 2)), "l"(dA + so + (Q8_A_BLK / 32) * i), "l"(dB + so + (B_BLK / 32) * i), "r"(idesc), "r"(i & 1) : "memory");
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_dfull[dp])) : "memory");
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
-        }
-        if (!ok) atomicCAS(p.status, 0, 4);
-    } else if (wid < Q8_EPW) {
-        const int quarter = wid & 3, col0 = (wid >> 2) * CW, row = quarter * 32 + lane;
-        float acc[CW];
+                for (int m = 0; m < MT; ++m) tc_bulk(dst + m * KB * Q8_A_BLK, p.a_img + (a0 + (size_t)m * kbs + kb0) * Q8_A_BLK, KB * Q8_A_BLK, full);
+                tc_bulk(dst + C::O_B, p.b_img + (b0 + kb0) * C::B_BLK, KB * C::B_BLK, full);
 #pragma unroll
-        for (int j = 0; j < CW; ++j) acc[j] = 0.0f;
-        uint32_t d0[16], d1[16];
-        // A stage's blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
-        // it: 16 of this warp's columns of block i / H; load starts reading them (asynchronous: tcgen05.wait::ld ends it).
-        auto open = [&](int st, int s, uint32_t phase) {
-            ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_full[s]), phase, 2000000000ull));
-            ok = ok && __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_dfull[st & 1]), (st >> 1) & 1, 2000000000ull));
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        };
-        auto load = [&](int st, int i, uint32_t (&d)[16]) {
-            const uint32_t ta = tm + (uint32_t)(NT * (KB * (st & 1) + i / H) + col0 + 16 * (i % H)) + ((uint32_t)(quarter * 32) << 16);
-            if (ok)
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]),
-                           "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]) : "r"(ta) : "memory");
-        };
-        // scale and add a unit in the CPU's order: sum += dot * (dw * dx)
-        auto scale_add = [&](const unsigned char* stage, int i, const uint32_t (&d)[16]) {
-            const float* sb = (const float*)(stage + O_SB) + i / H * NT + col0 + 16 * (i % H);
-            const float dw = ((const float*)(stage + O_SA))[i / H * 128 + row];
-#pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-                const float4 dx = *(const float4*)(sb + j);
-                const float dxs[4] = {dx.x, dx.y, dx.z, dx.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float& a = acc[16 * (i % H) + j + c];
-                    a = __fadd_rn(a, __fmul_rn(__uint_as_float(d[j + c]), __fmul_rn(dw, dxs[c])));
-                }
+                for (int m = 0; m < MT; ++m) tc_bulk(dst + C::O_SA + m * KB * 512, p.a_sc + (a0 + (size_t)m * kbs + kb0) * 128, KB * 512, full);
+                tc_bulk(dst + C::O_SB, p.b_sc + (b0 + kb0) * NT, KB * NT * 4, full);
             }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; phase ^= 1u; }
+        }
+        if (!ok && lane == 0) atomicCAS(p.status, 0, 3);
+    } else if (wid == Q8_EPW + 1) {
+        const uint32_t idesc = tc_idesc_f16(128, NT);
+        const uint64_t dA = tc_desc(sbase, 2048, 128), dB = tc_desc(sbase + C::O_B, NT * 16, 128);
+        int s = 0, dp = 0; uint32_t phase = 0, dphase = 1;
+        for (int st = 0; st < n_stage; ++st) {
+            wait(tc_smem(&s_full[s]), phase, st >= ND ? tc_smem(&s_dfree[dp]) : 0, dphase);
+            if (!ok) break;
+            tc_fence_after();
+            if (tc_elect()) {
+                const uint32_t so = (uint32_t)s * (STAGE >> 4), d0 = tm + (uint32_t)(MT * NT * KB) * dp;
+#pragma unroll
+                for (uint32_t i = 0; i < KB; ++i)
+#pragma unroll
+                    for (uint32_t m = 0; m < MT; ++m)
+#pragma unroll
+                        for (uint32_t k = 0; k < 2; ++k)
+                            tc_mma_f16(d0 + (i * MT + m) * NT, dA + so + (Q8_A_BLK / 32) * (2 * (m * KB + i) + k), dB + so + (C::B_BLK / 32) * (2 * i + k), idesc, k);
+                tc_commit(tc_smem(&s_dfull[dp]));
+                tc_commit(tc_smem(&s_empty[s]));
+            }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; phase ^= 1u; }
+            if (++dp == ND) { dp = 0; dphase ^= 1u; }
+        }
+        if (!ok && lane == 0) atomicCAS(p.status, 0, 4);
+    } else {
+        const int quarter = wid & 3, col0 = (wid >> 2) * CW, row = quarter * 32 + lane;
+        unsigned long long acc[MT * UC][UW / 2];     // f32 pairs: two columns to an instruction
+#pragma unroll
+        for (int m = 0; m < MT * UC; ++m)
+#pragma unroll
+            for (int j = 0; j < UW / 2; ++j) acc[m][j] = 0;
+        uint32_t d0[UW], d1[UW];
+        // A stage's blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
+        // it: UW of this warp's columns of row tile i / UC % MT of block i / (UC MT); load starts reading them (asynchronous: tc_wait_ld ends it).
+        int s_next = 0, dp = 0, dp_cur = 0, s_cur = 0; uint32_t p_next = 0, dphase = 0;
+        auto open = [&] {
+            wait(tc_smem(&s_dfull[dp]), dphase, tc_smem(&s_full[s_next]), p_next);
+            tc_fence_after();
+            s_cur = s_next; dp_cur = dp;
+            if (++s_next == STAGES) { s_next = 0; p_next ^= 1u; }
+            if (++dp == ND) { dp = 0; dphase ^= 1u; }
+        };
+        auto load = [&](int i, uint32_t (&d)[UW]) {
+            tc_ld(d, tm + (uint32_t)(MT * NT * KB * dp_cur + i / UC * NT + col0 + UW * (i % UC)) + ((uint32_t)(quarter * 32) << 16));
+        };
+        // the scales of a unit's columns: read once for a block's row tiles (a value for every lane: 32 lanes x 16 bytes are four cycles of the
+        // block's shared memory, 512 for 128 x 128 outputs, more than their f32 operations)
+        ulonglong2 dx[UC][UW / 4];
+        // scale and add a unit in the CPU's order: sum += dot * (dw * dx)
+        auto scale_add = [&](const unsigned char* stage, int i, const uint32_t (&d)[UW]) {
+            const int blk = i / (UC * MT), m = i / UC % MT, u = i % UC;
+            if (m == 0)
+#pragma unroll
+                for (int j = 0; j < UW / 4; ++j) dx[u][j] = *(const ulonglong2*)(stage + C::O_SB + (blk * NT + col0 + UW * u + 4 * j) * 4);
+            const float dw = ((const float*)(stage + C::O_SA))[(m * KB + blk) * 128 + row];
+            unsigned long long dw2;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(dw2) : "f"(dw));
+#pragma unroll
+            for (int j = 0; j < UW / 2; ++j)
+                asm volatile("{ .reg .b64 s, q;\n"
+                    "mov.b64 q, {%1, %2};\n"
+                    "fma.rn.f32x2 s, %3, %4, %5; fma.rn.f32x2 q, q, s, %5;\n"
+                    "add.rn.f32x2 %0, %0, q; }"
+                    : "+l"(acc[m * UC + u][j]) : "r"(d[2 * j]), "r"(d[2 * j + 1]), "l"(dw2), "l"(j & 1 ? dx[u][j / 2].y : dx[u][j / 2].x), "l"(p.zero2));
         };
         long long* pf = p.prof ? p.prof + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 : nullptr;
         const long long t_begin = clock64();
-        auto arrive = [&](unsigned long long* bar) { if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory"); };
-        open(0, 0, 0); load(0, 0, d0); load(0, 1, d1);
-        int s = 0; uint32_t phase = 0;
+        auto arrive = [&](unsigned long long* bar) { if (lane == 0) tc_mbar_arrive(tc_smem(bar)); };
+        open(); load(0, d0); load(1, d1);
 #pragma unroll 1
         for (int st = 0; st < n_stage && ok; ++st) {
+            const int s = s_cur;
             const unsigned char* stage = smem + (size_t)s * STAGE;
-            const int s_next = s + 1 == STAGES ? 0 : s + 1; const uint32_t p_next = s_next ? phase : phase ^ 1u;
-            const bool more = st + 1 < n_stage;
 #pragma unroll
-            for (int g = 0; g < PAIRS; ++g) {
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");      // both units are in registers
-                if (g == PAIRS - 1) { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); arrive(&s_dfree[st & 1]); }
+            for (int g = 0; g < UNITS / 2; ++g) {
+                const bool last = g == UNITS / 2 - 1;
+                tc_wait_ld();                                          // both units are in registers
+                if (last) { tc_fence_before(); arrive(&s_dfree[dp_cur]); }
                 scale_add(stage, 2 * g, d0);
-                if (g < PAIRS - 1) load(st, 2 * g + 2, d0);                           // lands while the second unit is being added
-                else if (more) { open(st + 1, s_next, p_next); load(st + 1, 0, d0); }
+                if (last && st + 1 < n_stage) open();
+                load(last ? 0 : 2 * g + 2, d0);                        // lands while the second unit is being added (behind the last stage: read again, for nobody)
                 scale_add(stage, 2 * g + 1, d1);
-                if (g < PAIRS - 1) load(st, 2 * g + 3, d1);
-                else if (more) load(st + 1, 1, d1);
+                load(last ? 1 : 2 * g + 3, d1);
             }
             __syncwarp();
             arrive(&s_empty[s]);
-            s = s_next; phase = p_next;
         }
+        tc_wait_ld();
         if (pf && tid == 0) { pf[0] = clock64() - t_begin; }
-        if (ok && __shfl_sync(0xffffffffu, *(volatile int*)p.status, 0) == 0) {
-            const size_t orow = (size_t)rt * 128 + row;
-            // mode 1 reads what it adds to: all of a batch's reads first, then the stores (a read placed after a store that may
-            // alias it waits for nothing, but the compiler keeps their order, and one read-add-store at a time is a memory round
-            // trip per column)
+        if (ok) {
 #pragma unroll
-            for (int j0 = 0; j0 < CW; j0 += 16) {
-                float old[16];
+            for (int m = 0; m < MT; ++m) {
+                const size_t orow = ((size_t)rt * MT + m) * 128 + row;
+                auto column = [&](int j) { const unsigned long long v = acc[m * UC + j / UW][j % UW / 2]; return __uint_as_float((uint32_t)(j & 1 ? v >> 32 : v)); };
+                // mode 1 reads what it adds to: all of a batch's reads first, then the stores (a read placed after a store that may
+                // alias it waits for nothing, but the compiler keeps their order, and one read-add-store at a time is a memory round
+                // trip per column)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int tok = tt * NT + col0 + j0 + j;
-                    old[j] = (p.mode && tok < p.n_rows) ? p.out[(size_t)tok * p.stride + orow] : 0.0f;
-                }
+                for (int j0 = 0; j0 < CW; j0 += UW) {
+                    float old[UW];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int tok = tt * NT + col0 + j0 + j;
-                    if (tok < p.n_rows) p.out[(size_t)tok * p.stride + orow] = p.mode ? __fadd_rn(old[j], acc[j0 + j]) : acc[j0 + j];
+                    for (int j = 0; j < UW; ++j) {
+                        const int tok = tt * NT + col0 + j0 + j;
+                        old[j] = (p.mode && tok < p.n_rows) ? p.out[(size_t)tok * p.stride + orow] : 0.0f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < UW; ++j) {
+                        const int tok = tt * NT + col0 + j0 + j;
+                        if (tok < p.n_rows) p.out[(size_t)tok * p.stride + orow] = p.mode ? __fadd_rn(old[j], column(j0 + j)) : column(j0 + j);
+                    }
                 }
             }
-        } else if (!ok) atomicCAS(p.status, 0, 5);
+        } else if (lane == 0) atomicCAS(p.status, 0, 5);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    tc_fence_before();
     __syncthreads();
-    if (wid == Q8_EPW + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm) : "memory");
+    if (wid == Q8_EPW + 1) tc_dealloc(tm, 512);
 }
-template <int NT> constexpr size_t tc_q8_smem() { return (size_t)q8_stages<NT>() * q8_stage_bytes<NT>() + 128; }
 
 }  // namespace
 
@@ -911,8 +911,8 @@ bool itb_tc_q8_shape_ok(const DevQ8& w) { return w.n_in % 128 == 0 && w.n_out % 
 // out[token][row] (+)= W x for n_rows quantised activation rows. False: not run.
 bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode) {
     if (!itb_tc_q8_shape_ok(w) || n_rows <= 0) return false;
-    // 64 tokens to a tile where 128 would leave half of the SMs without a block (an output projection over 512 rows)
-    const size_t kbs = w.n_in / 32, rts = w.n_out / 128, nt = 2 * rts * (((size_t)n_rows + 127) / 128) <= (size_t)c->sm_count ? 64 : 128, tts = ((size_t)n_rows + nt - 1) / nt;
+    // 256 rows x 64 tokens to a block; half as much where that would leave half of the SMs without one (an output projection over 512 rows)
+    const size_t kbs = w.n_in / 32, rts = w.n_out / 128, nt = 64, tts = ((size_t)n_rows + nt - 1) / nt, mt = rts % 2 == 0 && rts / 2 * tts > (size_t)c->sm_count / 2 ? 2 : 1;
     auto it = c->tc_weights.find(w.q);
     if (it == c->tc_weights.end()) {
         itb_ctx::TcWeights t;
@@ -938,13 +938,13 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     TcQ8 g{};
     g.a_img = it->second.img; g.a_sc = (const float*)it->second.sf; g.b_img = c->tc_q8_b; g.b_sc = c->tc_q8_sx; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_out = w.n_out;
     g.out = out; g.stride = stride; g.mode = mode; g.status = c->tc_status;
-    auto kernel = nt == 64 ? k_tc_q8<64> : k_tc_q8<128>;
-    const size_t smem = nt == 64 ? tc_q8_smem<64>() : tc_q8_smem<128>();
+    auto kernel = mt == 2 ? k_tc_q8<64, 2> : k_tc_q8<64, 1>;
+    const size_t smem = mt == 2 ? Q8Cfg<64, 2>::SMEM : Q8Cfg<64, 1>::SMEM;
     itb_raise_smem(kernel, smem);
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
-    const size_t n_blocks = rts * tts;
+    const size_t n_blocks = rts / mt * tts;
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
-    kernel<<<dim3((unsigned)rts, (unsigned)tts), Q8_EPW * 32 + 64, smem, st>>>(g);
+    kernel<<<dim3((unsigned)(rts / mt), (unsigned)tts), Q8_EPW * 32 + 64, smem, st>>>(g);
     c->launches++;
     if (prof_on && g.prof) {
         std::vector<long long> h(n_blocks * 8);
@@ -953,7 +953,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
         cudaFree(g.prof);
         double a = 0; size_t n = 0;
         for (size_t b = 0; b < n_blocks; ++b) if (h[b * 8]) { a += (double)h[b * 8]; ++n; }
-        if (n) fprintf(stderr, "tc_q8 %d x %d, %zu K32 blocks, %zu blocks of 128 x %zu: cycles per K32 block %.0f\n", w.n_out, n_rows, kbs, n, nt, a / n / kbs);
+        if (n) fprintf(stderr, "tc_q8 %d x %d, %zu K32 blocks, %zu blocks of %zu x %zu: cycles per K32 block %.0f\n", w.n_out, n_rows, kbs, n, 128 * mt, nt, a / n / kbs);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return itb_fail(c, "Q8_0 tensor path: launch", e);

@@ -115,6 +115,12 @@ def test_matmul_q8_0_on_the_tensor_cores_exact(n_in, n_out, n_tok):
     o2.close()
 
 
+@pytest.mark.parametrize("n_in,n_out,n_tok", [(128, 4864, 321), (1536, 4096, 515), (256, 19200, 65), (2048, 2560, 511)])
+def test_matmul_q8_0_on_the_tensor_cores_in_blocks_of_256_rows_exact(n_in, n_out, n_tok):
+    """dense=q8tc where a block takes two row tiles: a last tile of 1, 3 or 63 rows, two stages of k and more than the ring holds."""
+    test_matmul_q8_0_on_the_tensor_cores_exact(n_in, n_out, n_tok)
+
+
 @pytest.mark.parametrize("n_in,n_out,n_tok", [(2048, 64, 1), (512, 48, 2), (256, 16, 1), (128, 9, 3), (768, 8, 1), (2048, 200, 40), (512, 130, 33)])
 def test_matmul_nvfp4_dense_exact(ops, n_in, n_out, n_tok):
     from inferred_thoughts_b200 import host
