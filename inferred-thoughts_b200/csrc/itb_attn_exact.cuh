@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
 // the sum in position order by one thread, the division. grid (n_head, rows), block 256; dynamic shared memory n_pos_max floats.
 struct AxSoft { float* scores; int s_stride; const int* n_pos_dev; int n_pos_last, n_q, n_head; };
 __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float s_red[8];
     __shared__ float s_sum;

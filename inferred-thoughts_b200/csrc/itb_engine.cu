@@ -1005,7 +1005,7 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
             // gated shared expert and the residual add, as k_moe_down does them on one GPU
             const size_t KH = (size_t)d.n_expert_used * H;
             nccl_api().ReduceScatter(e->o_all, e->ep->o_mine, KH, NcclApi::Float32, NcclApi::Sum, e->ep->comm, st);
-            k_moe_finish_rows<<<(unsigned)((H + 255) / 256), 256, 0, st>>>(e->x, H, e->ep->o_mine, e->ep->gw + (size_t)e->ep->rank * d.n_expert_used,
+            launch_k(false, k_moe_finish_rows, (unsigned)((H + 255) / 256), 256, 0, st, e->x, H, e->ep->o_mine, e->ep->gw + (size_t)e->ep->rank * d.n_expert_used,
                                                                           d.n_expert_used, e->shd, e->shlogit, (size_t)H);
             launches += 2;
             // the routing this rank's token got, where read_routes looks for it
@@ -1207,6 +1207,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     const int qd = d.head_dim * d.n_head, kvd = d.head_dim * d.n_head_kv;
     const int TPB = NWG * 32;
     uint64_t launches = 0;
+    const bool chain = !e->ep && !e->tier;       // with them, copies, events and collectives come between the kernels: the first one behind such orders itself as ever
     set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
     set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
     set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
@@ -1231,7 +1232,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             int tiles = 0;
             for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; p.tiles[i] = (w[i]->n_out + 31) / 32; tiles += p.tiles[i]; }
             const int k = w[0]->n_in, ns = std::min(k / 256, TILE_STAGES);
-            k_tile_q8_multi<1, 256, 4><<<dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(p, x.q, x.s, R, ns);
+            itb_chain(k_tile_q8_multi<1, 256, 4>, dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st, p, x.q, x.s, R, ns);
             launches++;
             return;
         }
@@ -1242,7 +1243,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     auto gemm_fp4d = [&](const DevFp4& w, const int8_t* xq, const float* xs, float* out, int rows, bool has_s, float sc) {
         if (rows >= 2 && gemm_smem(w.n_in) <= 200 * 1024) {
             set_smem((const void*)k_gemm_fp4, gemm_smem(w.n_in));
-            k_gemm_fp4<<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), st>>>(
+            itb_chain(k_gemm_fp4, dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), st, 
                 w.nib, w.sc, w.n_in, w.n_out, xq, xs, rows, out, (size_t)w.n_out, sc, has_s ? 1 : 0);
             launches++;
             return;
@@ -1250,7 +1251,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         const int gx = std::max(1, std::min((w.n_out + 31) / 32, 2 * sms));
         const size_t smem = matmul_fp4_smem(w.n_in);
         set_smem((const void*)k_matmul_fp4, smem);
-        k_matmul_fp4<<<dim3(gx, rows), 256, smem, st>>>(w, nullptr, 1, 0, xq, xs, out);
+        itb_chain(k_matmul_fp4, dim3(gx, rows), 256, smem, st, w, nullptr, 1, 0, xq, xs, out);
         launches++;
         if (has_s) { const size_t n = (size_t)rows * w.n_out; k_scale<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, sc); launches++; }
     };
@@ -1261,8 +1262,8 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         const int nw = 4;
         dim3 g(std::max(1, std::min(2 * sms, (w.n_out + 31) / 32)), R);
         size_t sm = (size_t)w.n_in * 4 + (size_t)nw * 32 * 33 * 4;
-        if (c->exact) k_matmul_f32<true><<<g, nw * 32, sm, st>>>(w, x, out);
-        else k_matmul_f32<false><<<g, nw * 32, sm, st>>>(w, x, out);
+        if (c->exact) itb_chain(k_matmul_f32<true>, g, nw * 32, sm, st, w, x, out);
+        else itb_chain(k_matmul_f32<false>, g, nw * 32, sm, st, w, x, out);
         launches++;
     };
     // two F32 matrices over the same rows: one launch where both take the serial-order tiles, else one after the other
@@ -1277,10 +1278,10 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     };
     const size_t smem_nq = 256 + (size_t)H * 4;
     if (e->ep && e->ep->p2p_rows && n_tok == 1 && R == (int)e->B) { k_ep_tick<<<1, 32, 0, st>>>(e->ep->seq); launches++; }    // the step number the peers' flags will carry
-    k_embed<<<R, 256, 0, st>>>(m->tok_embd.w, H, tok_rows, e->x); launches++;
+    launch_k(chain, k_embed, R, 256, 0, st, m->tok_embd.w, H, tok_rows, e->x); launches++;
     for (uint32_t il = 0; il < d.n_layer; ++il) {
         const DevLayer& L = m->layers[il];
-        k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.attn_norm, H, d.rms_eps, e->xn, e->xq, e->xs); launches++;
+        itb_chain(k_norm_quant, R, 256, smem_nq, st, e->x, L.attn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, nullptr); launches++;
         const QRows xa = c->quantised(e->xq, e->xs);
         if (L.recurrent) {
             const int rs = e->slot_of[il];
@@ -1291,29 +1292,29 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             }
             f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn);
             float* cst = e->conv_state + (size_t)rs * e->B * conv_stride;
-            if (d.ssm_d_conv == 4 && n_tok >= CONV_T) k_conv_rows4<<<dim3((cd + 127) / 128, n_seq * ((n_tok + CONV_T - 1) / CONV_T)), 128, 0, st>>>(cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d);
-            else k_conv_rows<<<dim3((cd + 127) / 128, R), 128, 0, st>>>(cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d, d.ssm_d_conv);
+            if (d.ssm_d_conv == 4 && n_tok >= CONV_T) itb_chain(k_conv_rows4, dim3((cd + 127) / 128, n_seq * ((n_tok + CONV_T - 1) / CONV_T)), 128, 0, st, cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d);
+            else itb_chain(k_conv_rows, dim3((cd + 127) / 128, R), 128, 0, st, cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d, d.ssm_d_conv);
             launches++;
-            k_conv_state<<<dim3((cd + 127) / 128, n_seq), 128, 0, st>>>(cst, conv_stride, e->qkvc, n_tok, cd, d.ssm_d_conv); launches++;
-            (sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>)<<<dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st>>>(
+            itb_chain(k_conv_state, dim3((cd + 127) / 128, n_seq), 128, 0, st, cst, conv_stride, e->qkvc, n_tok, cd, d.ssm_d_conv); launches++;
+            itb_chain((sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>), dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st, 
                 e->qkvc2, cd, e->alpha, e->beta, L.ssm_a, L.dt_bias, n_k, n_v, d.rms_eps, e->qh, e->kh, e->vh, e->gb); launches++;
             const size_t chunk_need = (size_t)n_seq * ((n_tok + GC - 1) / GC) * n_v * gdn_chunk_floats<128>();
             if ((c->gdn_chunk || !c->exact) && n_tok >= 32 && sk == 128 && e->gdn_scratch_cap >= chunk_need) {
                 // many tokens: everything that does not touch the state for all chunks at once, then three small products per chunk
                 float* sst = e->ssm_state + (size_t)rs * e->B * state_stride;
-                k_gdn_chunk_prep<128><<<dim3((n_tok + GC - 1) / GC, n_v, n_seq), 256, gdn_chunk_prep_smem<128>(), st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, e->gdn_scratch);
-                k_gdn_chunk_scan<128><<<dim3(n_v, sk / GC_VS, n_seq), 256, gdn_chunk_scan_smem<128>(), st>>>(e->gdn_scratch, n_tok, n_v, sst, state_stride, e->core);
+                itb_chain(k_gdn_chunk_prep<128>, dim3((n_tok + GC - 1) / GC, n_v, n_seq), 256, gdn_chunk_prep_smem<128>(), st, e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, e->gdn_scratch);
+                itb_chain(k_gdn_chunk_scan<128>, dim3(n_v, sk / GC_VS, n_seq), 256, gdn_chunk_scan_smem<128>(), st, e->gdn_scratch, n_tok, n_v, sst, state_stride, e->core);
                 launches++;
             } else {
                 const dim3 gs(n_v, sk / 32, n_seq);
                 float* sst = e->ssm_state + (size_t)rs * e->B * state_stride;
-                if (n_tok == 1 && sk == 128) k_gdn_step<128><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
-                else if (n_tok == 1) k_gdn_step<64><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
-                else if (sk == 128) k_gdn_scan<128><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);
-                else k_gdn_scan<64><<<gs, 128, 0, st>>>(e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);   // 64 or 128 only (checked at model creation)
+                if (n_tok == 1 && sk == 128) itb_chain(k_gdn_step<128>, gs, 128, 0, st, e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
+                else if (n_tok == 1) itb_chain(k_gdn_step<64>, gs, 128, 0, st, e->qh, e->kh, e->vh, e->gb, n_k, n_v, sst, state_stride, e->core);
+                else if (sk == 128) itb_chain(k_gdn_scan<128>, gs, 128, 0, st, e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);
+                else itb_chain(k_gdn_scan<64>, gs, 128, 0, st, e->qh, e->kh, e->vh, e->gb, n_tok, n_k, n_v, sst, state_stride, e->core);   // 64 or 128 only (checked at model creation)
             }
             launches++;
-            (sk == 128 ? k_gdn_post<4> : k_gdn_post<2>)<<<dim3(R, row_share(R, n_v, sms)), 256, 0, st>>>(e->core, e->z, L.ssm_norm, n_v, d.rms_eps, e->aq, e->as); launches++;
+            itb_chain((sk == 128 ? k_gdn_post<4> : k_gdn_post<2>), dim3(R, row_share(R, n_v, sms)), 256, 0, st, e->core, e->z, L.ssm_norm, n_v, d.rms_eps, e->aq, e->as); launches++;
             gemm(L.ssm_out, c->quantised(e->aq, e->as), e->x, H, 1);
         } else {
             const int as = e->slot_of[il];
@@ -1327,7 +1328,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             a.kslab = e->kslab + (size_t)as * e->B * a.slab_stride; a.vslab = e->vslab + (size_t)as * e->B * a.slab_stride;
             a.pos = e->pos; a.npos_out = e->npos; a.n_tok = n_tok; a.hd = d.head_dim; a.n_head = d.n_head; a.n_head_kv = d.n_head_kv;
             a.n_rot = d.n_rot; a.theta = d.rope_theta; a.eps = d.rms_eps; a.bf16 = c->kv_bf16;
-            k_attn_prep_rows<<<dim3(R, row_share(R, d.n_head + 2 * d.n_head_kv, sms)), 256, (d.n_rot + 8 * d.head_dim) * 4, st>>>(a); launches++;
+            itb_chain(k_attn_prep_rows, dim3(R, row_share(R, d.n_head + 2 * d.n_head_kv, sms)), 256, (d.n_rot + 8 * d.head_dim) * 4, st, a); launches++;
             const float scale = 1.0f / sqrtf((float)d.head_dim);
             const int nwa = 8, ns = n_tok > 1 ? e->n_split_rows : e->n_split;
             const size_t smem_a = (size_t)nwa * 8 * 2 * 4 + (size_t)nwa * 8 * d.head_dim * 4;
@@ -1341,18 +1342,18 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
 #define AM_CASE(HD)                                                                                                      \
     case HD:                                                                                                              \
         set_smem((const void*)k_attn_mma<HD, true>, attn_mma_smem<HD>()); set_smem((const void*)k_attn_mma<HD, false>, attn_mma_smem<HD>()); \
-        if (c->kv_bf16) k_attn_mma<HD, true><<<ga, 256, attn_mma_smem<HD>(), st>>>(ap);                                    \
-        else k_attn_mma<HD, false><<<ga, 256, attn_mma_smem<HD>(), st>>>(ap);                                              \
+        if (c->kv_bf16) itb_chain(k_attn_mma<HD, true>, ga, 256, attn_mma_smem<HD>(), st, ap);                                    \
+        else itb_chain(k_attn_mma<HD, false>, ga, 256, attn_mma_smem<HD>(), st, ap);                                              \
         break;
                 switch (d.head_dim) { AM_CASE(64) AM_CASE(128) AM_CASE(256) }
 #undef AM_CASE
                 launches++;
-                k_attn_combine_rows<<<R * d.n_head, d.head_dim, 0, st>>>(e->part_acc, e->part_ml, 1, d.head_dim, e->gate, e->npos, d.n_head, e->aq, e->as); launches++;
+                itb_chain(k_attn_combine_rows, R * d.n_head, d.head_dim, 0, st, e->part_acc, e->part_ml, 1, d.head_dim, e->gate, e->npos, d.n_head, e->aq, e->as); launches++;
             } else if (exact_attention_ok(e) && e->scores_cap >= (size_t)R * d.n_head * scores_stride(e)) {
                 uint32_t top = 0;
                 for (int sq = 0; sq < n_seq; ++sq) top = std::max(top, e->host_pos[sq] + (uint32_t)n_tok);
                 if (n_tok == 1) top = e->n_ctx;        // a decode pass is replayed from a graph: its launches must hold any length
-                enqueue_exact_attention(e, st, false, a.kslab, a.vslab, a.slab_stride, R, n_tok, (int)std::min<uint32_t>(top, e->n_ctx));
+                enqueue_exact_attention(e, st, true, a.kslab, a.vslab, a.slab_stride, R, n_tok, (int)std::min<uint32_t>(top, e->n_ctx));
                 launches += 2;
             } else {
             {
@@ -1360,20 +1361,20 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
 #define ATT_CASE(HD)                                                                                                          \
     case HD:                                                                                                                   \
         set_smem((const void*)k_attn_partial<HD, 8>, smem_a);                                                                  \
-        k_attn_partial<HD, 8><<<grid, nwa * 32, smem_a, st>>>(e->qn, a.kslab, a.vslab, kvd, 0, n_tok, d.n_head, d.n_head_kv,    \
+        itb_chain(k_attn_partial<HD, 8>, grid, nwa * 32, smem_a, st, e->qn, a.kslab, a.vslab, kvd, 0, n_tok, d.n_head, d.n_head_kv,    \
             scale, c->kv_bf16, e->npos, e->part_acc, e->part_ml, n_tok, a.slab_stride);                                        \
         break;
                 switch (d.head_dim) { ATT_CASE(64) ATT_CASE(128) ATT_CASE(256) }
 #undef ATT_CASE
                 launches++;
             }
-            k_attn_combine_rows<<<R * d.n_head, d.head_dim, 0, st>>>(e->part_acc, e->part_ml, ns, d.head_dim, e->gate, e->npos, d.n_head,
+            itb_chain(k_attn_combine_rows, R * d.n_head, d.head_dim, 0, st, e->part_acc, e->part_ml, ns, d.head_dim, e->gate, e->npos, d.n_head,
                                                                     e->aq, e->as); launches++;
             }
             gemm(L.wo, c->quantised(e->aq, e->as), e->x, H, 1);
         }
         // routed FFN
-        k_norm_quant<<<R, 256, smem_nq, st>>>(e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, e->ep ? nullptr : e->xh); launches++;
+        itb_chain(k_norm_quant, R, 256, smem_nq, st, e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, e->ep ? nullptr : e->xh); launches++;
         const QRows xf = c->quantised(e->xq, e->xs);
         if (!L.shared4[0].nib && !L.shared4[1].nib) {
             const DevQ8* ws[2] = {&L.shared_gate, &L.shared_up}; float* os[2] = {e->sg, e->su}; const size_t ss[2] = {(size_t)d.shared_ff, (size_t)d.shared_ff};
@@ -1389,7 +1390,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             const int K = d.n_expert_used, E = d.n_expert, ff = d.expert_ff;
             int32_t* ids = e->route_ids + (size_t)il * e->R * K;
             float* wts = e->route_w + (size_t)il * e->R * K;
-            k_route_rows<<<(R + 3) / 4, 128, (size_t)4 * ((E + 31) & ~31) * 4, st>>>(e->router, R, E, K, ids, wts); launches++;
+            itb_chain(k_route_rows, (R + 3) / 4, 128, (size_t)4 * ((E + 31) & ~31) * 4, st, e->router, R, E, K, ids, wts); launches++;
             // expert parallel: the pairs of every rank's rows, rank-major; otherwise just ours
             const int W = e->ep ? e->ep->world : 1;
             int P = W * R * K, Kt = K;                  // pairs the expert kernels see; pairs per activation row among them
@@ -1464,7 +1465,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                     // the hint: layer il + 1's router on THIS layer's router input, top prefetch_k per row (src/ops/mod.rs:915-924)
                     const int pk = std::min<int>(e->tier->prefetch_k, std::min<int>(16, E));
                     f32mm(m->layers[il + 1].gate_inp, e->xn, e->tier->guess_logits);
-                    k_route_rows<<<(R + 3) / 4, 128, (size_t)4 * ((E + 31) & ~31) * 4, st>>>(e->tier->guess_logits, R, E, pk, e->tier->guess_dev, e->tier->guess_w); launches++;
+                    itb_chain(k_route_rows, (R + 3) / 4, 128, (size_t)4 * ((E + 31) & ~31) * 4, st, e->tier->guess_logits, R, E, pk, e->tier->guess_dev, e->tier->guess_w); launches++;
                     n_guess = (size_t)R * pk;
                 }
                 if (!tier_ensure(e, st, il, ids, (size_t)R * K, n_guess)) return launches;
@@ -1473,7 +1474,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             if (P > 0) {
             const int e_here = e->ep ? std::max(1, E / W) : E;        // an expert-parallel rank serves all the pairs it sees with its own E / W experts
             const int tile_cap = exp_tile_cap(P, e_here, ff, sms), max_tiles = exp_max_tiles(P, E, tile_cap);
-            k_group_pairs_fast<<<1, 1024, (size_t)E * 4, st>>>(ids_src, P, E, e->pair_off, e->pair_list, e->pair_tiles, e->pair_off + E + 1, tile_cap);
+            launch_k(chain, k_group_pairs_fast, 1, 1024, (size_t)E * 4, st, ids_src, P, E, e->pair_off, e->pair_list, e->pair_tiles, e->pair_off + E + 1, tile_cap);
             launches++;
             const cudaStreamCaptureStatus cap_st = cap_rows;
             if (c->fp4tc && n_tok > 1 && !e->ep && !e->tier && cap_st == cudaStreamCaptureStatusNone && itb_tc_shape_ok(Lg) && itb_tc_shape_ok(Lu) && itb_tc_shape_ok(Ld)) {
@@ -1529,23 +1530,23 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                 launches++;
                 o_src = e->ep->o_mine;
             }
-            k_shared_act_rows<<<R, 128, 0, st>>>(e->sg, e->su, d.shared_ff, e->sq, e->ss); launches++;
+            launch_k(chain, k_shared_act_rows, R, 128, 0, st, e->sg, e->su, d.shared_ff, e->sq, e->ss); launches++;
             if (L.shared4[2].nib) gemm_fp4d(L.shared4[2], e->sq, e->ss, e->shd, R, L.has_shared_s[2], L.shared_s[2]);
             else gemm(L.shared_down, c->quantised(e->sq, e->ss), e->shd, H, 0);
             const size_t total = (size_t)R * H;
-            k_moe_finish_rows<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
+            launch_k(chain, k_moe_finish_rows, (unsigned)((total + 255) / 256), 256, 0, st, e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
         }
     }
     // LM head on each sequence's last row
     const float* xl = e->x;
-    if (n_tok > 1) { k_gather_last<<<n_seq, 256, 0, st>>>(e->x, H, n_tok, e->xlast); launches++; xl = e->xlast; }
+    if (n_tok > 1) { itb_chain(k_gather_last, n_seq, 256, 0, st, e->x, H, n_tok, e->xlast); launches++; xl = e->xlast; }
     if (n_seq > 1) {
         // several sequences: one pass over the output matrix for all of them
-        k_norm_quant<<<n_seq, 256, smem_nq, st>>>(xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs); launches++;
+        itb_chain(k_norm_quant, n_seq, 256, smem_nq, st, xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs, nullptr); launches++;
         if (m->output4.nib) gemm_fp4d(m->output4, e->xq, e->xs, e->logits, n_seq, m->has_output_s, m->output_s);
         else gemm_n(m->output, c->quantised(e->xq, e->xs), e->logits, d.n_vocab, 0, n_seq);
     } else if (m->output4.nib) {
-        k_norm_quant<<<1, 256, smem_nq, st>>>(xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs); launches++;
+        itb_chain(k_norm_quant, 1, 256, smem_nq, st, xl, m->output_norm, H, d.rms_eps, nullptr, e->xq, e->xs, nullptr); launches++;
         gemm_fp4d(m->output4, e->xq, e->xs, e->logits, 1, m->has_output_s, m->output_s);
     } else {
         InProj hp{};
@@ -1559,12 +1560,12 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             const int cap = (int)(((SMEM_BUDGET - 256 - (size_t)H * 5 - (size_t)(H / 32) * 4 - (c->exact ? 32 * 33 * 4 : 0) - 64) / (NWG * 4) - CONV_CAP * 8) / (H / 32 + 1));
             hp.br = std::max(pass_in, std::min(hp.br, cap / pass_in * pass_in));
             set_smem((const void*)k_in_proj, 200 * 1024);
-            k_in_proj<<<dim3(gx, n_seq), TPB, in_proj_smem(H, c->exact, hp.br), st>>>(hp); launches++;
+            itb_chain(k_in_proj, dim3(gx, n_seq), TPB, in_proj_smem(H, c->exact, hp.br), st, hp); launches++;
         }
     }
-    k_argmax_partial<<<dim3(ARGMAX_PARTS, n_seq), 256, 0, st>>>(e->logits, d.n_vocab, e->arg_v, e->arg_i); launches++;
-    if (n_tok > 1) { k_advance_pos<<<(n_seq + 127) / 128, 128, 0, st>>>(e->pos, n_seq, n_tok - 1); launches++; }
-    k_argmax_advance<<<n_seq, 32, 0, st>>>(e->arg_v, e->arg_i, ARGMAX_PARTS, e->tokens, e->pos, e->next, e->history, (int)e->history_cap, e->step_counter, n_seq);
+    itb_chain(k_argmax_partial, dim3(ARGMAX_PARTS, n_seq), 256, 0, st, e->logits, d.n_vocab, e->arg_v, e->arg_i); launches++;
+    if (n_tok > 1) { itb_chain(k_advance_pos, (n_seq + 127) / 128, 128, 0, st, e->pos, n_seq, n_tok - 1); launches++; }
+    itb_chain(k_argmax_advance, n_seq, 32, 0, st, e->arg_v, e->arg_i, ARGMAX_PARTS, e->tokens, e->pos, e->next, e->history, (int)e->history_cap, e->step_counter, n_seq);
     launches++;
     return launches;
 }

@@ -130,6 +130,7 @@ __device__ __forceinline__ void exp_stage(const unsigned char* w0, const unsigne
 // Feeding the stages by bulk copies from a ninth warp was slower (1 KB and 128-byte pieces: 102 us against 63 at 32 tokens).
 template <int NJ, bool GLU>
 __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     using C = ExpCfg<NJ>;
     const int k = p.wa.n_in, n_out = p.wa.n_out;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
 template <int NJ, bool GLU>
 static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) {
     itb_raise_smem(k_exp<NJ, GLU>, EX_SMEM);
-    k_exp<NJ, GLU><<<dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st>>>(a);
+    itb_chain(k_exp<NJ, GLU>, dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st, a);
 }
 // The activation scales of a tile's whole rows lie beside the ring: up to 18,944 elements of k with 64 tokens.
 static inline bool exp_k_ok(int k) { return exp_smem<8>(k) <= EX_SMEM; }
@@ -302,6 +303,7 @@ static inline void exp_run(ExpArgs a, bool glu, int max_tiles, int cap, cudaStre
 
 // Q8_0 quantisation of f32 rows as the kernels above read them: f16 values permuted inside blocks, block scales (block per row).
 __global__ void k_quant_rows_h(const float* x, int n, __half* xh, float* xs) {
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int b = wid; b < n / 32; b += nw) {

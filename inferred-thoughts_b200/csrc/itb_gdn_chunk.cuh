@@ -28,6 +28,7 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *(const float4*)p
 template <int SK>
 __global__ void __launch_bounds__(256) k_gdn_chunk_prep(const float* qh, const float* kh, const float* vh, const float* gb, int n_tok, int n_k, int n_v,
                                                         float* scratch) {
+    pdl_wait();
     constexpr int ST = SK + 4;     // shared rows 16-byte aligned and on different banks
     extern __shared__ __align__(16) unsigned char smem[];
     float* Ks = (float*)smem;                  // [GC][ST]
@@ -121,6 +122,7 @@ template <int SK> constexpr size_t gdn_chunk_prep_smem() { return (size_t)(3 * G
 // grid (n_v, SK / 32, n_seq); block 256. The state slice [32 value rows][SK keys] lives in shared memory across the chunks.
 template <int SK>
 __global__ void __launch_bounds__(256) k_gdn_chunk_scan(const float* scratch, int n_tok, int n_v, float* state, size_t state_stride, float* out) {
+    pdl_wait();
     constexpr int ST = SK + 4, DS = GC_VS + 4, PS = GC + 4;
     extern __shared__ __align__(16) unsigned char smem[];
     float* S = (float*)smem;                   // [32][ST]

@@ -7,27 +7,33 @@ namespace {  // each translation unit gets its own copy of these kernels
 
 // ---- elementwise / small ops (one thread per element; src/ops/naive.rs:246-357, src/ops/mod.rs:600-1270) ----
 __global__ void k_silu_mul(float* g, const float* u, size_t n) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) g[i] = silu_f(g[i]) * u[i];
 }
 __global__ void k_sigmoid_mul(float* x, const float* g, size_t n) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] *= sigmoid_f(g[i]);
 }
 __global__ void k_scale(float* x, size_t n, float s) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] *= s;
 }
 __global__ void k_add_assign(float* a, const float* b, size_t n) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] += b[i];
 }
 __global__ void k_add_scaled(float* a, const float* b, size_t n, float s, const float* logit) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (logit) s = sigmoid_f(logit[0]);
     if (i < n) a[i] += b[i] * s;
 }
 __global__ void k_add_scaled_rows(float* acc, size_t n, const float* rows, const float* scales, size_t n_rows) {
+    pdl_wait();
     size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     float v = 0.0f;
@@ -35,20 +41,24 @@ __global__ void k_add_scaled_rows(float* acc, size_t n, const float* rows, const
     acc[j] = v;
 }
 __global__ void k_gather_chunks(const float* src, size_t chunk, size_t stride, size_t offset, float* out, size_t out_len) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < out_len) out[i] = src[(i / chunk) * stride + offset + i % chunk];
 }
 __global__ void k_scatter_chunks(const float* src, size_t src_len, size_t chunk, size_t stride, size_t offset, float* dst) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < src_len) dst[offset + (i / chunk) * stride + i % chunk] = src[i];
 }
 __global__ void k_kv_write(uint16_t* slab, size_t offset, const float* src, size_t n, int bf16) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) slab[offset + i] = bf16 ? f32_to_bf16_bits(src[i]) : f32_to_f16_bits(src[i]);
 }
 
 // RMSNorm over rows of nd (block per row); out may alias x. w has nd entries (src/ops/naive.rs:139-164).
 __global__ void k_rms_norm(const float* x, const float* w, int nd, float eps, float* out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     double* red = (double*)smem;
     float* xn = (float*)(red + 32);
@@ -72,6 +82,7 @@ __global__ void k_l2_norm_heads(float* x, size_t n_heads, int hd, float eps) {
 
 // Row softmax, warp per row: max, exp, serial-order-free sum (tolerance class: expf) (src/ops/naive.rs:362-376).
 __global__ void k_softmax_rows(float* x, size_t n_rows, int row) {
+    pdl_wait();
     size_t r = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_rows) return;
     int lane = threadIdx.x & 31;
@@ -92,6 +103,7 @@ __global__ void k_softmax_rows(float* x, size_t n_rows, int row) {
 // One thread per (row, head, pair). pos_base + row index gives the position; pos_dev (optional)
 // overrides with a per-row device position.
 __global__ void k_rope(float* x, size_t n_rows, int n_heads, int hd, int n_rot, float theta, size_t pos_base, const int* pos_dev) {
+    pdl_wait();
     int half = n_rot / 2;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t total = n_rows * n_heads * half;
@@ -255,6 +267,7 @@ __global__ void k_route(const float* probs, int n_expert, int n_used, int32_t* i
 
 // The same, a warp per token (up to 1,024 experts): no block barriers between the rounds.
 __global__ void __launch_bounds__(128) k_route_warp(const float* probs, int n_tok, int n_expert, int n_used, int32_t* ids_out, float* w_out) {
+    pdl_wait();
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= n_tok) return;
     int32_t ids[16]; float wts[16];
@@ -266,6 +279,7 @@ __global__ void __launch_bounds__(128) k_route_warp(const float* probs, int n_to
 // Weighted expert sum + gated shared expert (src/ops/mod.rs:1134-1171): ascending picks, shared last.
 __global__ void k_moe_finish(float* out, size_t at, int n, const float* rows, const float* wts, int n_used, size_t n_tok,
                              const float* shared, const float* logit, size_t logit_at) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_tok * n) return;
     size_t t = i / n; int j = (int)(i % n);
@@ -278,12 +292,14 @@ __global__ void k_moe_finish(float* out, size_t at, int n, const float* rows, co
 
 // Q8_0 activation quantiser, block per row of n_in (src/ops/naive.rs:653-675).
 __global__ void k_quant_q8(const float* x, int n_in, int8_t* xq, float* xs) {
+    pdl_wait();
     size_t t = blockIdx.x;
     block_quant_q8(x + t * n_in, n_in, xq + t * n_in, xs + t * (n_in / 32));
 }
 
 // ---- op-level matmuls: grid (row blocks, tokens or pairs) ----
 __global__ void k_matmul_q8(DevQ8 w, const int8_t* xq_g, const float* xs_g, float* out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int RP = 4;
     int nb = w.n_in / 32, gsh = lanes_shift(nb);
@@ -305,6 +321,7 @@ __global__ void k_matmul_q8(DevQ8 w, const int8_t* xq_g, const float* xs_g, floa
 // x_row(i) and writes out row i, times the expert's second scale (src/ops/mod.rs:1049-1088).
 // A block takes 32 rows (two 16-row tiles) at a time, four warps to a tile and a quarter of k each.
 __global__ void __launch_bounds__(256) k_matmul_fp4(DevFp4 w, const int32_t* ids, int n_used, int rows_mode, const int8_t* xq_g, const float* xs_g, float* out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int n = w.n_in, nb = n / 32, nsb = n / 16, kgs = n / 64, tid = threadIdx.x, wid = tid >> 5;
     int8_t* xq = (int8_t*)smem;
@@ -335,6 +352,7 @@ __global__ void __launch_bounds__(256) k_matmul_fp4(DevFp4 w, const int32_t* ids
 // The same for a gated pair of stacks and few (token, pick) pairs: 16 gate rows and the same 16 up rows at a time, out = silu(gate) * up
 // (src/ops/mod.rs:1105-1117). grid (ceil(n_out / 16), pairs).
 __global__ void __launch_bounds__(256) k_matmul_fp4_glu(DevFp4 wg, DevFp4 wu, const int32_t* ids, int n_used, int rows_mode, const int8_t* xq_g, const float* xs_g, float* out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int n = wg.n_in, nb = n / 32, nsb = n / 16, kgs = n / 64, tid = threadIdx.x, wid = tid >> 5, row = blockIdx.x * 16;
     int8_t* xq = (int8_t*)smem;
@@ -369,6 +387,7 @@ static inline size_t matmul_fp4_smem(int n) { return (size_t)n + (size_t)(n / 32
 // mode 0: out[t][row] = v; mode 1: out[t][row] += v (residual add).
 template <int NJ>
 __global__ void __launch_bounds__(NJ == 4 ? 256 : 512) k_gemm_q8(DevQ8 w, const int8_t* xq, const float* xs, int n_tok, float* out, size_t out_stride, int mode) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     int8_t* sq = (int8_t*)smem;
     float* ss = (float*)(sq + (size_t)MMA_TOK * mma_act_stride(w.n_in));
@@ -387,6 +406,7 @@ __global__ void __launch_bounds__(NJ == 4 ? 256 : 512) k_gemm_q8(DevQ8 w, const 
 // tensor's second scale).
 __global__ void __launch_bounds__(256) k_gemm_fp4(const uint8_t* nib, const uint8_t* sc, int k, int n_rows, const int8_t* xq, const float* xs,
                                                   int n_tok, float* out, size_t out_stride, float s2, int has_s2) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     int8_t* sq = (int8_t*)smem;
     float* ss = (float*)(sq + (size_t)MMA_TOK * mma_act_stride(k));
@@ -403,6 +423,7 @@ static inline size_t gemm_smem(int k) { return (size_t)MMA_TOK * mma_act_stride(
 
 template <bool EXACT>
 __global__ void k_matmul_f32(DevF32 w, const float* x, float* out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     float* xs = (float*)smem;
     float* tile = xs + w.n_in + (threadIdx.x >> 5) * (32 * 33);

@@ -13,7 +13,7 @@ static inline unsigned blocks_for(size_t n, int per = 256) { return (unsigned)((
 #define EW_LAUNCH(c, kernel, n, ...)                                      \
     do {                                                                  \
         if ((n) > 0) {                                                    \
-            kernel<<<blocks_for(n), 256, 0, (c)->stream>>>(__VA_ARGS__);  \
+            itb_chain(kernel, blocks_for(n), 256, 0, (c)->stream, __VA_ARGS__);  \
             ITB_LAUNCHED(c);                                              \
         }                                                                 \
     } while (0)
@@ -78,14 +78,14 @@ extern "C" void itb_rms_norm(itb_ctx* c, const float* x, size_t x_len, const flo
     const float* xd = itb_mirror_in(c, x, x_len); const float* wd = itb_mirror_in(c, w, nd);
     float* od = itb_mirror_out(c, out, x_len);
     if (!xd || !wd || !od) return;
-    k_rms_norm<<<(unsigned)(x_len / nd), 256, 32 * 8 + nd * 4, c->stream>>>(xd, wd, (int)nd, eps, od);
+    itb_chain(k_rms_norm, (unsigned)(x_len / nd), 256, 32 * 8 + nd * 4, c->stream, xd, wd, (int)nd, eps, od);
     ITB_LAUNCHED(c);
 }
 extern "C" void itb_rms_norm_heads(itb_ctx* c, float* x, size_t len, const float* w, size_t head_dim, float eps) {
     if (head_dim == 0 || len % head_dim) { itb_fail_msg(c, "rms_norm_heads: x is not whole heads"); return; }
     float* xd = itb_mirror_inout(c, x, len); const float* wd = itb_mirror_in(c, w, head_dim);
     if (!xd || !wd) return;
-    k_rms_norm<<<(unsigned)(len / head_dim), 64, 32 * 8 + head_dim * 4, c->stream>>>(xd, wd, (int)head_dim, eps, xd);
+    itb_chain(k_rms_norm, (unsigned)(len / head_dim), 64, 32 * 8 + head_dim * 4, c->stream, xd, wd, (int)head_dim, eps, xd);
     ITB_LAUNCHED(c);
 }
 extern "C" void itb_l2_norm_heads(itb_ctx* c, float* x, size_t len, size_t head_dim, float eps) {
@@ -101,7 +101,7 @@ extern "C" void itb_softmax(itb_ctx* c, float* x, size_t len, size_t row) {
     if (len % row) { itb_fail_msg(c, "softmax: x is not whole rows"); return; }
     float* xd = itb_mirror_inout(c, x, len);
     if (!xd) return;
-    k_softmax_rows<<<blocks_for(len / row, 8), 256, 0, c->stream>>>(xd, len / row, (int)row);
+    itb_chain(k_softmax_rows, blocks_for(len / row, 8), 256, 0, c->stream, xd, len / row, (int)row);
     ITB_LAUNCHED(c);
 }
 extern "C" void itb_rope_neox(itb_ctx* c, float* x, size_t len, size_t pos, size_t head_dim, size_t n_rot, size_t n_heads, float theta) {
@@ -172,8 +172,8 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
         k_gdn_op_pre<<<(unsigned)((nt * kper + 255) / 256), 256, 0, c->stream>>>(q, al, be, sa, dt, nt, n_k * sk, n_v, 1.0f / sqrtf((float)sk), qs, gbd);
         itb_raise_smem(k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>());
         itb_raise_smem(k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
-        k_gdn_chunk_prep<128><<<dim3(n_ch, n_v, 1), 256, gdn_chunk_prep_smem<128>(), c->stream>>>(qs, k, v, gbd, (int)nt, n_k, n_v, scr);
-        k_gdn_chunk_scan<128><<<dim3(n_v, sk / GC_VS, 1), 256, gdn_chunk_scan_smem<128>(), c->stream>>>(scr, (int)nt, n_v, sd, (size_t)n_v * sk * sk, od);
+        itb_chain(k_gdn_chunk_prep<128>, dim3(n_ch, n_v, 1), 256, gdn_chunk_prep_smem<128>(), c->stream, qs, k, v, gbd, (int)nt, n_k, n_v, scr);
+        itb_chain(k_gdn_chunk_scan<128>, dim3(n_v, sk / GC_VS, 1), 256, gdn_chunk_scan_smem<128>(), c->stream, scr, (int)nt, n_v, sd, (size_t)n_v * sk * sk, od);
         ITB_LAUNCHED(c);
         return;
     }
@@ -187,7 +187,7 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
 // Into the context's buffer, over what the call before left there. False: out of memory.
 static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in, QRows* rows) {
     if (!itb_ensure_xq(c, n_rows * n_in)) return false;
-    k_quant_q8<<<(unsigned)n_rows, 256, 0, c->stream>>>(xd, (int)n_in, c->xq, c->xs);
+    itb_chain(k_quant_q8, (unsigned)n_rows, 256, 0, c->stream, xd, (int)n_in, c->xq, c->xs);
     ITB_LAUNCHED(c);
     *rows = c->quantised(c->xq, c->xs);
     return true;
@@ -206,7 +206,7 @@ static void launch_q8(itb_ctx* c, const WeightEntry* w, const QRows& x, size_t n
     size_t smem = w->n_in + nb * 4 + (size_t)nw * terms_floats(4, gsh, nb) * 4;
     dim3 grid(gx, (unsigned)n_tok);
     itb_raise_smem(k_matmul_q8, smem);
-    k_matmul_q8<<<grid, nw * 32, smem, c->stream>>>(dw, x.q, x.s, od);
+    itb_chain(k_matmul_q8, grid, nw * 32, smem, c->stream, dw, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
 
@@ -222,7 +222,7 @@ static bool group_pairs(itb_ctx* c, const int32_t* ids, size_t n_pairs, size_t E
     // the route's pairs stay grouped for the other matmuls over it (gate + up, then down)
     if (c->route_grouped == E && c->route_tile_cap == cap) return true;
     c->route_grouped = E; c->route_tile_cap = cap;
-    k_group_pairs_fast<<<1, 1024, E * 4, c->stream>>>(ids, (int)n_pairs, (int)E, c->pair_off, c->pair_list, (int4*)c->pair_tiles, c->pair_off + E + 1, cap);
+    itb_chain(k_group_pairs_fast, 1, 1024, E * 4, c->stream, ids, (int)n_pairs, (int)E, c->pair_off, c->pair_list, (int4*)c->pair_tiles, c->pair_off + E + 1, cap);
     ITB_LAUNCHED(c);
     return true;
 }
@@ -249,7 +249,7 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const i
         size_t sm = gemm_smem((int)w->n_in);
         itb_raise_smem(k_gemm_fp4, sm);
         dim3 g((unsigned)((w->n_out + MMA_ROWS - 1) / MMA_ROWS), (unsigned)((n_pairs + MMA_TOK - 1) / MMA_TOK));
-        k_gemm_fp4<<<g, 256, sm, c->stream>>>((const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, x.q, x.s,
+        itb_chain(k_gemm_fp4, g, 256, sm, c->stream, (const uint8_t*)w->a, (const uint8_t*)w->b, (int)w->n_in, (int)w->n_out, x.q, x.s,
                                              (int)n_pairs, od, w->n_out, 1.0f, 0);
         ITB_LAUNCHED(c);
         return;
@@ -259,7 +259,7 @@ static void launch_fp4(itb_ctx* c, const WeightEntry* w, const QRows& x, const i
     if (gx < 1) gx = 1;
     const size_t smem = matmul_fp4_smem((int)w->n_in);
     itb_raise_smem(k_matmul_fp4, smem);
-    k_matmul_fp4<<<dim3(gx, (unsigned)n_pairs), 256, smem, c->stream>>>(dw, ids, n_used, rows_mode, x.q, x.s, od);
+    itb_chain(k_matmul_fp4, dim3(gx, (unsigned)n_pairs), 256, smem, c->stream, dw, ids, n_used, rows_mode, x.q, x.s, od);
     ITB_LAUNCHED(c);
 }
 
@@ -282,10 +282,10 @@ static void launch_f32(itb_ctx* c, const WeightEntry* w, const float* xd, size_t
     dim3 grid(gx, (unsigned)n_tok);
     if (c->exact) {
         itb_raise_smem(k_matmul_f32<true>, smem);
-        k_matmul_f32<true><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
+        itb_chain(k_matmul_f32<true>, grid, nw * 32, smem, c->stream, dw, xd, od);
     } else {
         itb_raise_smem(k_matmul_f32<false>, smem);
-        k_matmul_f32<false><<<grid, nw * 32, smem, c->stream>>>(dw, xd, od);
+        itb_chain(k_matmul_f32<false>, grid, nw * 32, smem, c->stream, dw, xd, od);
     }
     ITB_LAUNCHED(c);
 }
@@ -328,7 +328,7 @@ extern "C" void itb_route(itb_ctx* c, float* probs, size_t len, size_t n_expert,
     size_t nt = len / n_expert;
     const float* p = itb_mirror_in(c, probs, len);
     if (!p || !itb_ensure_route(c, nt * n_used)) return;
-    if (n_expert <= 1024) k_route_warp<<<(unsigned)((nt + 3) / 4), 128, 0, c->stream>>>(p, (int)nt, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
+    if (n_expert <= 1024) itb_chain(k_route_warp, (unsigned)((nt + 3) / 4), 128, 0, c->stream, p, (int)nt, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
     else k_route<<<(unsigned)nt, 256, 0, c->stream>>>(p, (int)n_expert, (int)n_used, c->route_ids, c->route_w);
     ITB_LAUNCHED(c);
     c->route_grouped = 0;
@@ -373,7 +373,7 @@ static bool experts_grouped(itb_ctx* c, const itb_experts* g, const itb_experts*
     const int E = (int)g->n_expert, cap = exp_tile_cap((int)n_pairs, E, (int)(u ? g->n_out : g->n_out / 2), c->sm_count);
     if (!itb_ensure_xq(c, rows * k * 2) || !group_pairs(c, c->route_ids, n_pairs, g->n_expert, cap)) return true;
     __half* xh = (__half*)c->xq;
-    k_quant_rows_h<<<(unsigned)rows, 256, 0, c->stream>>>(xd, (int)k, xh, c->xs);
+    itb_chain(k_quant_rows_h, (unsigned)rows, 256, 0, c->stream, xd, (int)k, xh, c->xs);
     ITB_LAUNCHED(c);
     ExpArgs a{};
     a.wa = DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0};
@@ -423,7 +423,7 @@ extern "C" void itb_moe_glu(itb_ctx* c, const itb_experts* gate, const itb_exper
         if (!wg || !wu || !quantize_rows(c, xd, rows, gate->n_in, &xr)) return;
         const size_t smem = matmul_fp4_smem((int)gate->n_in);
         itb_raise_smem(k_matmul_fp4_glu, smem);
-        k_matmul_fp4_glu<<<dim3((unsigned)((gate->n_out + 15) / 16), (unsigned)n_pairs), 256, smem, c->stream>>>(
+        itb_chain(k_matmul_fp4_glu, dim3((unsigned)((gate->n_out + 15) / 16), (unsigned)n_pairs), 256, smem, c->stream,
             DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0},
             DevFp4{(const uint8_t*)wu->a, (const uint8_t*)wu->b, wu->scale2, (int)wu->n_in, (int)wu->n_out, (int)wu->n_expert, 0}, c->route_ids, (int)r->n_used,
             rows == n_pairs ? 0 : rows > 1 ? 1 : 2, xr.q, xr.s, od);
@@ -503,8 +503,8 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
     case HD:                                                                                                                                \
         itb_raise_smem(k_attn_mma<HD, true>, attn_mma_smem<HD>());                                                                          \
         itb_raise_smem(k_attn_mma<HD, false>, attn_mma_smem<HD>());                                                                         \
-        if (c->kv_bf16) k_attn_mma<HD, true><<<ga, 256, attn_mma_smem<HD>(), c->stream>>>(ap);                                              \
-        else k_attn_mma<HD, false><<<ga, 256, attn_mma_smem<HD>(), c->stream>>>(ap);                                                        \
+        if (c->kv_bf16) itb_chain(k_attn_mma<HD, true>, ga, 256, attn_mma_smem<HD>(), c->stream, ap);                                              \
+        else itb_chain(k_attn_mma<HD, false>, ga, 256, attn_mma_smem<HD>(), c->stream, ap);                                                        \
         break;
         switch (hd) { AM_CASE(64) AM_CASE(128) AM_CASE(256) }
 #undef AM_CASE
@@ -532,7 +532,7 @@ extern "C" void itb_attend(itb_ctx* c, const itb_attn* a, float* out, size_t out
         op.n_head_kv = (int)a->n_head_kv; op.bf16 = c->kv_bf16; op.gate = nullptr; op.out = od; op.out_q = nullptr; op.out_s = nullptr;
         if (const int mr = attn_tile_rows((int)n_q, 1, op.hd, op.n_head, op.n_head_kv, c->sm_count)) {
             attn_exact_tiles(sp, AxSoft{c->tmp_f32, (int)s_stride, nullptr, (int)a->n_pos, (int)n_q, (int)a->n_head}, op, mr, 1, (int)n_q, (int)a->n_pos,
-                             [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { k<<<g, b, smem, c->stream>>>(arg); ITB_LAUNCHED(c); });
+                             [&](auto k, dim3 g, dim3 b, size_t smem, const auto& arg) { itb_chain(k, g, b, smem, c->stream, arg); ITB_LAUNCHED(c); });
             return;
         }
         itb_raise_smem(k_attn_scores_exact, attn_scores_exact_smem((int)a->head_dim, group));

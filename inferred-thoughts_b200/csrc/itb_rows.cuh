@@ -44,6 +44,7 @@ __device__ __forceinline__ float warp_sums(const float (&a)[N], int lane) {
 constexpr int F32_TOK = 4;
 template <int NV, int MR>
 __global__ void __launch_bounds__(256) k_matmul_f32_rows(DevF32 w, const float* __restrict__ x, int n_rows, float* out, int tok_blk) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     float* xs = (float*)smem;
     constexpr int n = 128 * NV, N = F32_TOK * MR, PER = F32_TOK * n / 4 / 256;   // PER: float4 per thread of the token tile
@@ -100,7 +101,7 @@ static void f32_tree(cudaStream_t st, int sms, const DevF32& w, const float* x, 
     while (tok < 32 && blocks(mr, 2 * tok) >= 2 * sms) tok *= 2;
     const dim3 g((w.n_out + 8 * mr - 1) / (8 * mr), (n_rows + tok - 1) / tok);
     const size_t sm = (size_t)(tok > F32_TOK ? 2 : 1) * F32_TOK * w.n_in * 4;
-    auto run = [&](auto k) { itb_raise_smem(k, sm); k<<<g, 256, sm, st>>>(w, x, n_rows, out, tok); };
+    auto run = [&](auto k) { itb_raise_smem(k, sm); itb_chain(k, g, 256, sm, st, w, x, n_rows, out, tok); };
     switch (w.n_in / 128) {
 #define F32_CASE(NV) case NV: if (mr == 2) run(k_matmul_f32_rows<NV, 2>); else run(k_matmul_f32_rows<NV, 1>); break;
 #define F32_CASE1(NV) case NV: run(k_matmul_f32_rows<NV, 1>); break;
@@ -122,6 +123,7 @@ static void f32_tree(cudaStream_t st, int sms, const DevF32& w, const float* x, 
 // scheduler has the slots for its warps' reads, products and sums between them; the larger ones the f32 pipe and the reads.
 template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
 __global__ void __launch_bounds__((TO / MO) * (TR / MR)) k_sgemm_chain(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
+    pdl_wait();
     constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, NT = NX * NY, PIECES = (TO + TR) * (KT / 4) / NT;      // a thread per MO x MR outputs
     static_assert((TO + TR) * (KT / 4) % NT == 0, "whole pieces");
     extern __shared__ __align__(16) unsigned char smem[];
@@ -190,7 +192,7 @@ template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
 static void sgemm_tiles(cudaStream_t st, int n_out, int nz, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb, float* ob) {
     constexpr size_t smem = (size_t)NST * (TO + TR) * (KT + 4) * 4;
     itb_raise_smem(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, smem);
-    k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST><<<dim3((n_out + TO - 1) / TO, (n_rows + TR - 1) / TR, nz), (TO / MO) * (TR / MR), smem, st>>>(wa, x, n_rows, oa, wb, ob);
+    itb_chain(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, dim3((n_out + TO - 1) / TO, (n_rows + TR - 1) / TR, nz), (TO / MO) * (TR / MR), smem, st, wa, x, n_rows, oa, wb, ob);
 }
 // One matrix, or two over the same rows. 8 x 8, a chain to a thread, is fastest as long as an SM has no more than four such blocks (32 rows
 // of 257 outputs, 2,048 k: 11.8 us, at 16 x 16 18.5), but it reads every line once per 8 of the others. Large passes: unfused, where a
@@ -217,16 +219,17 @@ static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) itb_raise_smem(f, 200 * 1024);
     const bool skinny = n_rows <= 32;
     const int ns = std::min(k / 256, TILE_STAGES);
-    if (skinny && k % 256 == 0) k_tile_q8<1, 256, 4><<<dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode, ns);
-    else if (k % 256 == 0) k_tile_q8<4, 256, 2><<<dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode, ns);
-    else if (skinny) k_gemm_q8<1><<<dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode);
-    else k_gemm_q8<4><<<dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st>>>(w, x.q, x.s, n_rows, out, stride, mode);
+    if (skinny && k % 256 == 0) itb_chain(k_tile_q8<1, 256, 4>, dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st, w, x.q, x.s, n_rows, out, stride, mode, ns);
+    else if (k % 256 == 0) itb_chain(k_tile_q8<4, 256, 2>, dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st, w, x.q, x.s, n_rows, out, stride, mode, ns);
+    else if (skinny) itb_chain(k_gemm_q8<1>, dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st, w, x.q, x.s, n_rows, out, stride, mode);
+    else itb_chain(k_gemm_q8<4>, dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st, w, x.q, x.s, n_rows, out, stride, mode);
     return true;
 }
 
 // RMSNorm + Q8_0 quantisation of each row (src/ops/naive.rs:139-152, :653-675): normalised f32 row, int8 quants,
 // scales; xh (optional): the quants as f16 for the expert kernels (exp_pos order). grid = rows, block 256.
 __global__ void __launch_bounds__(256) k_norm_quant(const float* x, const float* w, int n, float eps, float* xn_out, int8_t* xq, float* xs, __half* xh = nullptr) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     double* red = (double*)smem;
     float* xn = (float*)(red + 32);
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(256) k_norm_quant(const float* x, const float*
 // the sequence's earlier rows of this pass, or the saved state where it reaches before the pass. Writes the
 // PRE-activation sum to `out` (the input rows stay intact for the neighbours). grid (ceil(nc/128), rows).
 __global__ void k_conv_rows(const float* state, size_t state_stride, const float* x, float* out, int n_tok, int nc, const float* w, int kernel) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     const size_t r = blockIdx.y;
@@ -269,6 +273,7 @@ __global__ void k_conv_rows(const float* state, size_t state_stride, const float
 // are the same expressions in the same order. grid (ceil(nc/128), n_seq * ceil(n_tok / CONV_T)).
 constexpr int CONV_T = 8;
 __global__ void __launch_bounds__(128) k_conv_rows4(const float* state, size_t state_stride, const float* __restrict__ x, float* __restrict__ out, int n_tok, int nc, const float* __restrict__ w) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     const int chunks = (n_tok + CONV_T - 1) / CONV_T, s = blockIdx.y / chunks, t0 = (blockIdx.y % chunks) * CONV_T;
@@ -293,6 +298,7 @@ __global__ void __launch_bounds__(128) k_conv_rows4(const float* state, size_t s
 }
 // The window each sequence leaves behind: its last kernel-1 inputs, oldest first. grid (ceil(nc/128), n_seq).
 __global__ void k_conv_state(float* state, size_t state_stride, const float* x, int n_tok, int nc, int kernel) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
     if (c >= nc) return;
     const int keep = kernel - 1;
@@ -317,6 +323,7 @@ inline unsigned row_share(int rows, int jobs, int sms) { return (unsigned)std::m
 template <int NJ>
 __global__ void __launch_bounds__(256) k_gdn_pre(const float* conv, int cd, const float* alpha, const float* beta, const float* ssm_a, const float* dt_bias,
                           int n_k, int n_v, float eps, float* qh, float* kh, float* vh, float* gb) {
+    pdl_wait();
     constexpr int sk = NJ * 32;
     const size_t r = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, key_dim = n_k * sk, vd = n_v * sk, vjobs = (vd + 127) / 128, jobs = 2 * n_k + vjobs + (n_v + 31) / 32;
@@ -367,6 +374,7 @@ __global__ void __launch_bounds__(256) k_gdn_pre(const float* conv, int cd, cons
 template <int SK>
 __global__ void __launch_bounds__(128) k_gdn_scan(const float* qh, const float* kh, const float* vh, const float* gb, int n_tok, int n_k, int n_v,
                                                   float* state, size_t state_stride, float* out) {
+    pdl_wait();
     constexpr int CW = SK / 4;             // state columns per lane
     constexpr int QS = CW + 4, VEC = 4 * QS;
     constexpr int DEPTH = 5;               // tokens whose operands are in flight or in use (cp.async ring, one group per token)
@@ -483,6 +491,7 @@ __global__ void __launch_bounds__(128) k_gdn_scan(const float* qh, const float* 
 // sequences of 32 heads against 26 us here (134 MB: 20 us at copy speed). Same sums, same order.
 template <int SK>
 __global__ void __launch_bounds__(128, 4) k_gdn_step(const float* qh, const float* kh, const float* vh, const float* gb, int n_k, int n_v, float* state, size_t state_stride, float* out) {
+    pdl_wait();
     constexpr int CW = SK / 4, QS = CW + 4, VEC = 4 * QS;
     __shared__ __align__(16) float st_all[4][8 * VEC], kq_all[4][2 * VEC];
     const int h = blockIdx.x, s = blockIdx.z, khd = h % n_k, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -539,6 +548,7 @@ __global__ void __launch_bounds__(128, 4) k_gdn_step(const float* qh, const floa
 // (src/model/qwen35.rs:1319-1325). Blocks and warps as in k_gdn_pre (75 MB at 2,048 rows of 4,096, 11 us; a block per head 65 us, this 42).
 template <int NJ>
 __global__ void __launch_bounds__(256) k_gdn_post(const float* o, const float* z, const float* norm_w, int n_v, float eps, int8_t* out_q, float* out_s) {
+    pdl_wait();
     constexpr int sv = NJ * 32;
     const size_t r = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -580,6 +590,7 @@ struct AttnPrepRows {
 // Blocks and warps as in k_gdn_pre: the row's rotations once, in double as the CPU takes them, then a warp per head (a block per (row,
 // head) took each rotation 18 times: 116 us at 2,048 rows of 16 + 2 + 2 heads of 256, this 63). Dynamic shared memory: n_rot + 8 * hd floats.
 __global__ void __launch_bounds__(256) k_attn_prep_rows(AttnPrepRows p) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int hd = p.hd, nj = hd / 32, half = p.n_rot / 2, kvd = p.n_head_kv * hd, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     float* cs = (float*)smem; float* sn = cs + half; float* val = sn + half + wid * hd;
@@ -632,6 +643,7 @@ __global__ void __launch_bounds__(256) k_attn_prep_rows(AttnPrepRows p) {
 // Combine of the attention splits per (row, head) with the sigmoid gate and Q8_0 quantisation; positions per row.
 __global__ void k_attn_combine_rows(const float* part_acc, const float* part_ml, int n_split, int hd, const float* gate,
                                     const int* n_pos_row, int n_head, int8_t* out_q, float* out_s) {
+    pdl_wait();
     const size_t th = blockIdx.x;
     const int d = threadIdx.x;
     const size_t r = th / n_head;
@@ -654,11 +666,13 @@ __global__ void k_attn_combine_rows(const float* part_acc, const float* part_ml,
 }
 
 __global__ void k_advance_pos(int* pos, int n_seq, int by) {
+    pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_seq) pos[i] += by;
 }
 // Rows of the last token of each sequence, gathered for the LM head: out[s] = x[s*n_tok + n_tok-1].
 __global__ void k_gather_last(const float* x, int n, int n_tok, float* out) {
+    pdl_wait();
     const int s = blockIdx.x;
     for (int i = threadIdx.x; i < n; i += blockDim.x) out[(size_t)s * n + i] = x[((size_t)s * n_tok + n_tok - 1) * n + i];
 }
@@ -675,6 +689,7 @@ namespace {
 
 // Softmax over all experts + top-k per row (src/model/qwen35.rs:1626-1638, src/ops/mod.rs:1191-1216). One warp per row.
 __global__ void k_route_rows(const float* router, int n_rows, int n_expert, int n_used, int32_t* ids_out, float* w_out) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int ne32 = (n_expert + 31) & ~31;
@@ -701,6 +716,7 @@ __global__ void k_route_rows(const float* router, int n_rows, int n_expert, int 
 
 // silu(gate) * up of the shared expert per row, quantised (src/model/qwen35.rs:1669-1678). block per row.
 __global__ void k_shared_act_rows(const float* sg, const float* su, int n, int8_t* q, float* s) {
+    pdl_wait();
     const size_t r = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int b = wid; b < n / 32; b += nw) {
@@ -712,6 +728,7 @@ __global__ void k_shared_act_rows(const float* sg, const float* su, int n, int8_
 }
 // Weighted expert sum in pick order, gated shared expert, residual add (src/ops/mod.rs:1134-1171, src/model/qwen35.rs:1090).
 __global__ void k_moe_finish_rows(float* x, int n, const float* o, const float* wts, int n_used, const float* shared, const float* logit, size_t total) {
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t r = i / n; const int j = (int)(i % n);
@@ -732,6 +749,7 @@ namespace {
 // tiles (optional): the pairs cut into tiles of at most `cap` (a multiple of 8), an expert's pairs evenly over its tiles, as
 // (expert, first slot, pairs, 0), largest first so that no long tile starts last; *n_tiles of them.
 __global__ void __launch_bounds__(1024) k_group_pairs_fast(const int32_t* ids, int n_pairs, int n_expert, int* off, int* list, int4* tiles = nullptr, int* n_tiles = nullptr, int cap = 64) {
+    pdl_wait();
     extern __shared__ int cnt[];    // [n_expert] counts, then cursors
     __shared__ int s_off[1025];
     __shared__ int s_bucket[9], s_start[9];       // tiles by groups of 8 pairs (1..8)

@@ -222,6 +222,7 @@ struct TcTile { int expert, n0, cnt, npad; unsigned b_off, sf_off; };   // offse
 // pair_off[e .. e+1): the expert's slots. One block; a thread per expert counts its tiles, a block-wide scan places them
 // (tiles in expert order, so the blocks that share an expert's weights run next to each other).
 __global__ void __launch_bounds__(1024) k_tc_build_tiles(const int* pair_off, int n_expert, int expert_lo, int expert_cnt, TcTile* tiles, int* n_tiles_out, int max_tiles, int k_blocks) {
+    pdl_wait();
     __shared__ int s_tiles[1024], s_rows[1024];
     const int e = threadIdx.x;
     int a = 0, z = 0;
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(1024) k_tc_build_tiles(const int* pair_off, in
 // Activation rows -> FP4 records, each row once: codes [row][n_in / 2] (element order, low nibble first), scale codes
 // [row][n_in / 16]. One thread per 16-element block.
 __global__ void k_tc_quant_rows(const float* x, size_t n_blocks, uint8_t* codes, uint8_t* scales) {
+    pdl_wait();
     const size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n_blocks) return;
     uint32_t sc, lo, hi;
@@ -261,6 +263,7 @@ __global__ void k_tc_quant_rows(const float* x, size_t n_blocks, uint8_t* codes,
 // n_used when the rows are tokens shared by a token's picks, 1 when there is a row per pair). Padding rows are written as zeros.
 __global__ void k_tc_gather_tiles(const uint8_t* codes, const uint8_t* scales, int n_in, const int* pair_list, int rows_div, const TcTile* tiles,
                                   const int* n_tiles, uint8_t* b_img, uint8_t* sf_img) {
+    pdl_wait();
     if ((int)blockIdx.x >= *n_tiles) return;
     const TcTile t = tiles[blockIdx.x];
     const int cpr = n_in / 32;                              // 16-byte chunks per row
@@ -331,6 +334,7 @@ __device__ __forceinline__ void tc_bulk(uint32_t dst, const void* src, uint32_t 
 // the same stores without the activation).
 template <bool GLU, bool EXACT_SILU>
 __global__ void __launch_bounds__(320, 1) k_tc_gemm(TcGemm p) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int NST = GLU ? TC_STAGES_GLU : TC_STAGES;
     __shared__ unsigned long long s_full[NST], s_empty[NST], s_acc, s_free;
@@ -596,12 +600,12 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
          tc_grow(&c->tc_codes, &c->tc_cap_codes, (size_t)n_pairs * (wg.n_in / 2), st) && tc_grow(&c->tc_scales, &c->tc_cap_scales, (size_t)n_pairs * (wg.n_in / 16), st);
     if (!ok) return itb_fail_msg(c, "FP4 tensor path: out of device memory for the pass");
     cudaMemsetAsync(c->tc_status, 0, 4, st);
-    k_tc_build_tiles<<<1, 1024, 0, st>>>(pair_off, wg.expert_lo + wg.n_expert, wg.expert_lo, wg.n_expert, tiles, c->tc_n_tiles, (int)max_tiles, (int)kbs);
+    itb_chain(k_tc_build_tiles, 1, 1024, 0, st, pair_off, wg.expert_lo + wg.n_expert, wg.expert_lo, wg.n_expert, tiles, c->tc_n_tiles, (int)max_tiles, (int)kbs);
     const size_t x_rows = rows_div == 1 ? (size_t)n_pairs : rows_div >= n_pairs ? 1 : ((size_t)n_pairs + rows_div - 1) / rows_div;
     const size_t nq = x_rows * (wg.n_in / 16);
-    k_tc_quant_rows<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(x, nq, c->tc_codes, c->tc_scales);
+    itb_chain(k_tc_quant_rows, (unsigned)((nq + 255) / 256), 256, 0, st, x, nq, c->tc_codes, c->tc_scales);
     // scale tiles of a pass are whole 512-byte tiles: rows past npad of a tile's scale tile are never read by a matrix of npad rows
-    k_tc_gather_tiles<<<dim3((unsigned)max_tiles, 4), 256, 0, st>>>(c->tc_codes, c->tc_scales, wg.n_in, pair_list, rows_div, tiles, c->tc_n_tiles, c->tc_b_img, c->tc_b_sf);
+    itb_chain(k_tc_gather_tiles, dim3((unsigned)max_tiles, 4), 256, 0, st, c->tc_codes, c->tc_scales, wg.n_in, pair_list, rows_div, tiles, c->tc_n_tiles, c->tc_b_img, c->tc_b_sf);
     TcGemm g{};
     g.wg_img = tg->img; g.wg_sf = tg->sf; g.wu_img = tu ? tu->img : nullptr; g.wu_sf = tu ? tu->sf : nullptr;
     g.s2g = wg.scale2; g.s2u = wu ? wu->scale2 : nullptr; g.expert_lo = wg.expert_lo;
@@ -614,9 +618,9 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     const dim3 grid((unsigned)n_blocks);
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
-    if (wu && c->exact) k_tc_gemm<true, true><<<grid, 320, tc_gemm_smem(true), st>>>(g);
-    else if (wu) k_tc_gemm<true, false><<<grid, 320, tc_gemm_smem(true), st>>>(g);
-    else k_tc_gemm<false, false><<<grid, 320, tc_gemm_smem(false), st>>>(g);
+    if (wu && c->exact) itb_chain(k_tc_gemm<true, true>, grid, 320, tc_gemm_smem(true), st, g);
+    else if (wu) itb_chain(k_tc_gemm<true, false>, grid, 320, tc_gemm_smem(true), st, g);
+    else itb_chain(k_tc_gemm<false, false>, grid, 320, tc_gemm_smem(false), st, g);
     if (prof_on && g.prof) {
         std::vector<long long> h(n_blocks * 8);
         cudaStreamSynchronize(st);
@@ -697,6 +701,7 @@ template <int NT, int MT> struct Q8Cfg {                                  // tok
 // int8 rows -> K32 block images of tiles of `tile` rows, scales -> f32 per (row tile, block, row). One thread per (row, block); rows
 // past n_rows are zeros. scales16 (f16, per weight row and block) or scales32 (f32, per activation row and block): whichever is not null.
 __global__ void k_q8_tile(const int8_t* q, const uint16_t* scales16, const float* scales32, int n_rows, int n_in, int tile, uint8_t* img, float* sc_out) {
+    pdl_wait();
     const int kbs = n_in / 32;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)((n_rows + tile - 1) / tile) * tile * kbs;
     if (idx >= total) return;
@@ -735,6 +740,7 @@ struct TcQ8 {
 // every row tile by warp / 4), warp 16 fetches operands, warp 17 issues the MMAs.
 template <int NT, int MT>
 __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     using C = Q8Cfg<NT, MT>;
     constexpr int STAGES = C::STAGES, STAGE = C::STAGE, KB = C::KB, ND = C::ND, CW = NT / 4, UW = CW < 16 ? CW : 16, UC = CW / UW, UNITS = KB * MT * UC;     // a unit: UW columns of a block's row tile
@@ -920,7 +926,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
         if (cudaMalloc(&t.sf, rts * kbs * 128 * 4) != cudaSuccess) { cudaFree(t.img); cudaGetLastError(); return itb_fail_msg(c, "Q8_0 tensor path: out of device memory for the tiled weights"); }
         t.bytes = rts * kbs * (Q8_A_BLK + 512);
         const size_t n = rts * 128 * kbs;
-        k_q8_tile<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w.q, w.s, nullptr, w.n_out, w.n_in, 128, t.img, (float*)t.sf);
+        itb_chain(k_q8_tile, (unsigned)((n + 255) / 256), 256, 0, st, w.q, w.s, nullptr, w.n_out, w.n_in, 128, t.img, (float*)t.sf);
         c->launches++;
         it = c->tc_weights.emplace(w.q, t).first;
     }
@@ -930,7 +936,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     // consecutive matmuls over one quantised row set share its image
     if (x.id == 0 || c->tc_q8_src != x.id || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in || c->tc_q8_src_tile != (int)nt) {
         const size_t n = tts * nt * kbs;
-        k_q8_tile<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x.q, nullptr, x.s, n_rows, w.n_in, (int)nt, c->tc_q8_b, c->tc_q8_sx);
+        itb_chain(k_q8_tile, (unsigned)((n + 255) / 256), 256, 0, st, x.q, nullptr, x.s, n_rows, w.n_in, (int)nt, c->tc_q8_b, c->tc_q8_sx);
         c->launches++;
         c->tc_q8_src = x.id; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in; c->tc_q8_src_tile = (int)nt;
     }
@@ -944,7 +950,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = rts / mt * tts;
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
-    kernel<<<dim3((unsigned)(rts / mt), (unsigned)tts), Q8_EPW * 32 + 64, smem, st>>>(g);
+    itb_chain(kernel, dim3((unsigned)(rts / mt), (unsigned)tts), Q8_EPW * 32 + 64, smem, st, g);
     c->launches++;
     if (prof_on && g.prof) {
         std::vector<long long> h(n_blocks * 8);
@@ -990,6 +996,7 @@ __device__ __forceinline__ uint32_t f16x2_rn(float lo, float hi) {
 // scales16 (f16, per weight row and 32-element block) or scales32 (f32, per activation row and block): whichever is not null.
 template <int ROWS>
 __global__ void k_f16_tile(const int8_t* q, const uint16_t* scales16, const float* scales32, int n_rows, int n_in, uint8_t* img) {
+    pdl_wait();
     const int kbs = n_in / 16;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)((n_rows + ROWS - 1) / ROWS) * ROWS * kbs;
     if (idx >= total) return;
@@ -1029,6 +1036,7 @@ struct TcHf {
 // grid: one block per SM (or per work item, if fewer); block 320: warps 0-7 store accumulators (lane quarter = warp % 4, column half
 // = warp / 4), warp 8 fetches operands, warp 9 issues the MMAs.
 __global__ void __launch_bounds__(320, 1) k_tc_f16(TcHf p) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ unsigned long long s_full[HF_STAGES], s_empty[HF_STAGES], s_acc[2], s_free[2];
     __shared__ uint32_t s_tmem;
@@ -1179,7 +1187,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
         if (cudaMalloc(&t.img, rts * kbs * HF_A_BLK) != cudaSuccess) { cudaGetLastError(); return itb_fail_msg(c, "f16 tensor path: out of device memory for the tiled weights"); }
         t.sf = nullptr; t.bytes = rts * kbs * HF_A_BLK;
         const size_t n = rts * 128 * kbs;
-        k_f16_tile<128><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w.q, w.s, nullptr, w.n_out, w.n_in, t.img);
+        itb_chain(k_f16_tile<128>, (unsigned)((n + 255) / 256), 256, 0, st, w.q, w.s, nullptr, w.n_out, w.n_in, t.img);
         c->launches++;
         it = c->tc_weights.emplace(w.s, t).first;
     }
@@ -1189,7 +1197,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     // consecutive matmuls over one quantised row set share its image
     if (x.id == 0 || c->tc_hf_src != x.id || c->tc_hf_src_rows != n_rows || c->tc_hf_src_in != w.n_in) {
         const size_t n = tts * HF_N * kbs;
-        k_f16_tile<HF_N><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x.q, nullptr, x.s, n_rows, w.n_in, c->tc_hf_b);
+        itb_chain(k_f16_tile<HF_N>, (unsigned)((n + 255) / 256), 256, 0, st, x.q, nullptr, x.s, n_rows, w.n_in, c->tc_hf_b);
         c->launches++;
         c->tc_hf_src = x.id; c->tc_hf_src_rows = n_rows; c->tc_hf_src_in = w.n_in;
     }
@@ -1201,7 +1209,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = std::min<size_t>((size_t)c->sm_count, rts * tts);
     if (prof_on) { cudaMalloc(&g.prof, n_blocks * 64); cudaMemsetAsync(g.prof, 0, n_blocks * 64, st); }
-    k_tc_f16<<<(unsigned)n_blocks, 320, tc_f16_smem(), st>>>(g);
+    itb_chain(k_tc_f16, (unsigned)n_blocks, 320, tc_f16_smem(), st, g);
     c->launches++;
     if (prof_on && g.prof) {
         std::vector<long long> h(n_blocks * 8);

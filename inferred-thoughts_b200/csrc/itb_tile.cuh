@@ -133,6 +133,7 @@ __device__ __forceinline__ void tile_foreach(const float (&acc)[NJ][4], int r0, 
 // Dense Q8_0 matmul: grid (ceil(rows/ROWS), ceil(n_tok/TOK)). mode 0: out = v; mode 1: out += v.
 template <int NJ, int KC, int TH>
 __global__ void __launch_bounds__(256) k_tile_q8(DevQ8 w, const int8_t* xq, const float* xs, int n_tok, float* out, size_t out_stride, int mode, int n_stage) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     using C = TileCfg<NJ, KC, TH>;
     int* tok_idx = (int*)smem;
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(256) k_tile_q8(DevQ8 w, const int8_t* xq, cons
 struct Q8Multi { DevQ8 w[3]; float* out[3]; size_t stride[3]; int tiles[3]; int n; };
 template <int NJ, int KC, int TH>
 __global__ void __launch_bounds__(256) k_tile_q8_multi(Q8Multi p, const int8_t* xq, const float* xs, int n_tok, int n_stage) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     using C = TileCfg<NJ, KC, TH>;
     int* tok_idx = (int*)smem;
