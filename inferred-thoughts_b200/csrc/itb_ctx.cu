@@ -107,6 +107,10 @@ extern "C" int itb_create(int device_ordinal, const char* opts, itb_ctx** out) {
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) {
         g_create_error = cudaGetErrorString(e); delete c; return 5;
     }
+    if ((e = cudaHostAlloc((void**)&c->fail_word, 4, cudaHostAllocMapped)) != cudaSuccess) {
+        g_create_error = cudaGetErrorString(e); cudaStreamDestroy(c->stream); delete c; return 6;
+    }
+    *c->fail_word = 0;
     std::string o = opts ? opts : "";
     if (o.find("kv=bf16") != std::string::npos) c->kv_bf16 = true;
     if (o.find("exact=0") != std::string::npos) c->exact = false;
@@ -139,6 +143,7 @@ extern "C" void itb_destroy(itb_ctx* c) {
     itb_tc_free(c);
     cudaFree(c->route_ids); cudaFree(c->route_w); cudaFree(c->xq); cudaFree(c->xs); cudaFree(c->tmp_f32);
     itb_pipe_free(c);
+    cudaFreeHost((void*)c->fail_word);
     cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -148,7 +153,7 @@ extern "C" const char* itb_take_error(itb_ctx* c) {
     if (c->error.empty()) {
         // surface asynchronous failures too
         cudaError_t e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) itb_fail(c, "stream", e);
+        if (e != cudaSuccess) itb_fail(c, "stream", e); else itb_status_ok(c);
         if (c->error.empty()) return nullptr;
     }
     c->error_out.swap(c->error);
@@ -157,6 +162,13 @@ extern "C" const char* itb_take_error(itb_ctx* c) {
 }
 
 extern "C" uint64_t itb_launch_count(itb_ctx* c) { return c->launches; }
+
+bool itb_status_ok(itb_ctx* c) {
+    const int v = *c->fail_word;
+    if (!v) return true;
+    *c->fail_word = 0;
+    return itb_fail_msg(c, std::string("a tensor-core kernel gave up a bounded wait (") + (v == 3 ? "operands" : v == 4 ? "issue" : "accumulators") + "): its results are not there");
+}
 
 // ------------------------------------------------------------------ host transfers
 static void itb_pipe_free(itb_ctx* c) { delete c->pipe; c->pipe = nullptr; }
@@ -172,7 +184,7 @@ bool itb_upload(itb_ctx* c, void* dev, const void* host, size_t bytes) {
 bool itb_download(itb_ctx* c, void* host, const void* dev, size_t bytes) {
     HostPipe* p = pipe_of(c);
     const cudaError_t e = p ? p->down(c->stream, host, dev, bytes) : HostPipe::plain(c->stream, host, dev, bytes, cudaMemcpyDeviceToHost);
-    return e == cudaSuccess || itb_fail(c, "d2h", e);
+    return e == cudaSuccess ? itb_status_ok(c) : itb_fail(c, "d2h", e);
 }
 
 // ------------------------------------------------------------------ mirrors

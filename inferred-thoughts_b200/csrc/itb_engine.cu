@@ -2009,6 +2009,7 @@ static bool ensure_graph(itb_engine* e) {
 // block returns. Turn it into the sticky error and put the grid barrier's counters back.
 // known: the word, where the caller has brought it home with its results.
 static bool check_flag(itb_engine* e, const uint32_t* known = nullptr) {
+    if (!itb_status_ok(e->c)) return false;
     if (e->mega != 1 && !e->c->exact && !(e->ep && (e->ep->p2p || e->ep->p2p_rows))) return true;
     int f = known ? (int)*known : 0;
     if (!known && cudaMemcpy(&f, e->err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return itb_fail_msg(e->c, "engine: cannot read the device status word");

@@ -82,6 +82,7 @@ struct HostPipe;                 // pinned staging and copy threads of one conte
 struct itb_ctx {
     int device = 0;
     HostPipe* pipe = nullptr;
+    volatile int* fail_word = nullptr;   // host memory that the tensor-core kernels store to when a bounded wait runs out (itb_status_ok)
     cudaStream_t stream = nullptr;
     std::string error;       // sticky first error
     std::string error_out;   // storage handed back by take_error
@@ -110,7 +111,7 @@ struct itb_ctx {
     // FP4 tensor-core expert path (itb_tc.cu): expert stacks re-tiled once (keyed by the stack's nibble plane), per-pass scratch
     struct TcWeights { uint8_t* img = nullptr; uint8_t* sf = nullptr; size_t bytes = 0; };
     std::unordered_map<const void*, TcWeights> tc_weights;
-    void* tc_tiles = nullptr; int* tc_n_tiles = nullptr; int* tc_slot_tile = nullptr; uint8_t* tc_b_img = nullptr; uint8_t* tc_b_sf = nullptr; int* tc_status = nullptr;
+    void* tc_tiles = nullptr; int* tc_n_tiles = nullptr; int* tc_slot_tile = nullptr; uint8_t* tc_b_img = nullptr; uint8_t* tc_b_sf = nullptr;
     uint8_t* tc_codes = nullptr; uint8_t* tc_scales = nullptr;      // the pass's activation rows as FP4 records
     size_t tc_cap_tiles = 0, tc_cap_slots = 0, tc_cap_b = 0, tc_cap_sf = 0, tc_cap_codes = 0, tc_cap_scales = 0;
     // Q8_0 tensor path: the pass's activation rows as K32 block images (kept for a following matmul over the same rows)
@@ -144,6 +145,8 @@ bool itb_fail(itb_ctx* c, const char* what, cudaError_t e);
 cudaError_t itb_raise_smem(const void* fn, size_t bytes);
 template <class... A> static inline cudaError_t itb_raise_smem(void (*fn)(A...), size_t bytes) { return itb_raise_smem((const void*)fn, bytes); }
 bool itb_fail_msg(itb_ctx* c, const std::string& msg);
+// After the stream has been waited for: false, with the sticky error set, if a kernel gave up a bounded wait since the last look.
+bool itb_status_ok(itb_ctx* c);
 #define ITB_CUDA(c, call)                                              \
     do {                                                               \
         cudaError_t e__ = (call);                                      \

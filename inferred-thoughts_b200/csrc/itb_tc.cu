@@ -6,7 +6,8 @@
 // by the reference's own method for its sm_120 instructions (tests/cuda_ops.rs:5899-5925 there): back-to-back MMAs on operands
 // that never change, nothing but the MMA in the loop, accumulators verified afterwards.
 //
-// Every wait is bounded; a kernel that gives up frees its tensor memory and reports through its status word.
+// Every wait is bounded; a kernel that gives up frees its tensor memory and reports through its status word (of the GEMMs: host memory,
+// 3 / 4 / 5 for the warp that fetches, issues or reads back; itb_status_ok looks at it behind every wait for the stream).
 #include "itb_internal.cuh"
 #include "itb_gemv.cuh"
 #include "itb_tcgen.cuh"
@@ -318,7 +319,7 @@ struct TcGemm {
     const TcTile* tiles; const int* n_tiles; const int* pair_list;
     int n_out, n_in;                                     // rows of one matrix, K
     float* out; int out_stride;                          // out[pair][n_out]
-    int* status;
+    volatile int* status;
     long long* prof;                                     // optional: 8 clock64 stamps per block (ITB_TC_PROF=1)
 };
 __device__ __forceinline__ void tc_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -378,7 +379,9 @@ __global__ void __launch_bounds__(320, 1) k_tc_gemm(TcGemm p) {
     const uint32_t d_g = tm, d_u = tm + 128, sf0 = tm + 256;
     const unsigned long long limit = 2000000000ull;
     bool ok = true;
-    if (wid == 8 && lane == 0) {
+    // (waits and loops by the whole warp, the instructions themselves by one lane of it: tc_elect)
+    auto wait = [&](unsigned long long* bar, uint32_t phase) { ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(bar), phase, limit)); };
+    if (wid == 8) {
         int it = 0;                                           // stages issued so far, over all items
         for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
             const TcTile t = p.tiles[w / n_mt];
@@ -388,23 +391,26 @@ __global__ void __launch_bounds__(320, 1) k_tc_gemm(TcGemm p) {
             const uint32_t total = a_bytes * (GLU ? 2 : 1) + b_bytes + sf_bytes * (GLU ? 3 : 2);
             for (int st = 0; st < n_stage; ++st, ++it) {
                 const int s = it % NST;
-                if (it >= NST) ok = tc_mbar_wait(tc_smem(&s_empty[s]), ((it / NST) - 1) & 1, limit);
+                if (it >= NST) wait(&s_empty[s], ((it / NST) - 1) & 1);
                 if (!ok) break;
                 const uint32_t full = tc_smem(&s_full[s]), dst = sbase + s * stage_bytes;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(total) : "memory");
                 const size_t kb0 = (size_t)st * TC_KS;
-                tc_bulk(dst, p.wg_img + (w_tile + kb0) * 4096, a_bytes, full);
-                tc_bulk(dst + o_sfg, p.wg_sf + (w_tile + kb0) * 512, sf_bytes, full);
-                if (GLU) {
-                    tc_bulk(dst + o_au, p.wu_img + (w_tile + kb0) * 4096, a_bytes, full);
-                    tc_bulk(dst + o_sfu, p.wu_sf + (w_tile + kb0) * 512, sf_bytes, full);
+                if (tc_elect()) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(total) : "memory");
+                    tc_bulk(dst, p.wg_img + (w_tile + kb0) * 4096, a_bytes, full);
+                    tc_bulk(dst + o_sfg, p.wg_sf + (w_tile + kb0) * 512, sf_bytes, full);
+                    if (GLU) {
+                        tc_bulk(dst + o_au, p.wu_img + (w_tile + kb0) * 4096, a_bytes, full);
+                        tc_bulk(dst + o_sfu, p.wu_sf + (w_tile + kb0) * 512, sf_bytes, full);
+                    }
+                    tc_bulk(dst + o_b, p.b_img + (size_t)t.b_off * (p.n_in / 2) + kb0 * (t.npad * 32), b_bytes, full);
+                    tc_bulk(dst + o_sfb, p.b_sf + ((size_t)t.sf_off + kb0) * 512, sf_bytes, full);
                 }
-                tc_bulk(dst + o_b, p.b_img + (size_t)t.b_off * (p.n_in / 2) + kb0 * (t.npad * 32), b_bytes, full);
-                tc_bulk(dst + o_sfb, p.b_sf + ((size_t)t.sf_off + kb0) * 512, sf_bytes, full);
+                __syncwarp();
             }
         }
-        if (!ok) atomicCAS(p.status, 0, 3);
-    } else if (wid == 9 && lane == 0) {
+        if (!ok && lane == 0) *p.status = 3;
+    } else if (wid == 9) {
         // descriptors of stage slot 0; a slot or K block further on only moves the 14-bit start-address field (address >> 4), which
         // cannot carry out of it (shared memory ends below 256 KB), so the low words are advanced by plain adds
         const uint64_t dA = tc_desc(sbase, 2048, 128), dAu = tc_desc(sbase + o_au, 2048, 128);
@@ -418,39 +424,42 @@ __global__ void __launch_bounds__(320, 1) k_tc_gemm(TcGemm p) {
             const uint32_t b_step = (uint32_t)(t.npad * 32) >> 4;
             if (item) {                                       // the epilogue warps have read the previous item's accumulators
                 const long long c0 = pf ? clock64() : 0;
-                ok = tc_mbar_wait(tc_smem(&s_free), (item - 1) & 1, limit);
+                wait(&s_free, (item - 1) & 1);
                 if (pf) t_free += clock64() - c0;
                 if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tc_fence_after();
             }
             for (int st = 0; st < n_stage; ++st, ++it) {
                 const int s = it % NST;
                 const long long c0 = pf ? clock64() : 0;
-                ok = tc_mbar_wait(tc_smem(&s_full[s]), (it / NST) & 1, limit);
+                wait(&s_full[s], (it / NST) & 1);
                 if (pf) t_load += clock64() - c0;
                 if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tc_fence_after();
                 const uint32_t so = (uint32_t)s * (stage_bytes >> 4), sft = sf0 + s * 48;
+                if (tc_elect()) {
 #pragma unroll
-                for (int k = 0; k < TC_KS; ++k) {
-                    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 4 * k), "l"(dSg + so + 32u * k) : "memory");
-                    if (GLU) asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 16 + 4 * k), "l"(dSu + so + 32u * k) : "memory");
-                    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 32 + 4 * k), "l"(dSb + so + 32u * k) : "memory");
-                }
+                    for (int k = 0; k < TC_KS; ++k) {
+                        asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 4 * k), "l"(dSg + so + 32u * k) : "memory");
+                        if (GLU) asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 16 + 4 * k), "l"(dSu + so + 32u * k) : "memory");
+                        asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(sft + 32 + 4 * k), "l"(dSb + so + 32u * k) : "memory");
+                    }
 #pragma unroll
-                for (int k = 0; k < TC_KS; ++k) {
-                    const uint64_t db = dB + so + b_step * k;
-                    const uint32_t acc = (st | k) ? 1u : 0u;
-                    tc_mma_fp4(d_g, dA + so + 256u * k, db, idesc, sft + 4 * k, sft + 32 + 4 * k, acc);
-                    if (GLU) tc_mma_fp4(d_u, dAu + so + 256u * k, db, idesc, sft + 16 + 4 * k, sft + 32 + 4 * k, acc);
+                    for (int k = 0; k < TC_KS; ++k) {
+                        const uint64_t db = dB + so + b_step * k;
+                        const uint32_t acc = (st | k) ? 1u : 0u;
+                        tc_mma_fp4(d_g, dA + so + 256u * k, db, idesc, sft + 4 * k, sft + 32 + 4 * k, acc);
+                        if (GLU) tc_mma_fp4(d_u, dAu + so + 256u * k, db, idesc, sft + 16 + 4 * k, sft + 32 + 4 * k, acc);
+                    }
+                    tc_commit(tc_smem(&s_empty[s]));
+                    if (st + 1 == n_stage) tc_commit(tc_smem(&s_acc));
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
+                __syncwarp();
             }
             if (!ok) break;
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_acc)) : "memory");
         }
-        if (!ok) atomicCAS(p.status, 0, 4);
-        if (pf) { pf[1] = t_load; pf[2] = t_free; }
+        if (!ok && lane == 0) *p.status = 4;
+        if (pf && lane == 0) { pf[1] = t_load; pf[2] = t_free; }
     } else if (wid < 8) {
         // epilogue: lane quarter `wid % 4` of tensor memory = weight rows 32 * (wid % 4) .. of the tile; the tile's token columns are
         // split between the two warps of a quarter. All of a warp's accumulator reads are issued before the one wait; the values
@@ -471,8 +480,7 @@ __global__ void __launch_bounds__(320, 1) k_tc_gemm(TcGemm p) {
             const float sg = p.s2g ? p.s2g[el] : 1.0f, su = (GLU && p.s2u) ? p.s2u[el] : 1.0f;
             const long long k0 = pf ? clock64() : 0;
             ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_acc), item & 1, limit));      // one answer per warp: the loads below are warp-wide
-            if (!ok && lane == 0) atomicCAS(p.status, 0, 5);                                    // the accumulators never came
-            ok = ok && __shfl_sync(0xffffffffu, *(volatile int*)p.status, 0) == 0;
+            if (!ok && lane == 0) *p.status = 5;                                                // the accumulators never came
             const long long k1 = pf ? clock64() : 0;
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -544,10 +552,10 @@ bool itb_tc_shape_ok(const DevFp4& w) { return w.n_in % (64 * TC_KS) == 0 && w.n
 void itb_tc_free(itb_ctx* c) {
     for (auto& kv : c->tc_weights) { cudaFree(kv.second.img); cudaFree(kv.second.sf); }
     c->tc_weights.clear();
-    cudaFree(c->tc_tiles); cudaFree(c->tc_n_tiles); cudaFree(c->tc_slot_tile); cudaFree(c->tc_b_img); cudaFree(c->tc_b_sf); cudaFree(c->tc_status); cudaFree(c->tc_codes); cudaFree(c->tc_scales); cudaFree(c->tc_q8_b); cudaFree(c->tc_q8_sx); cudaFree(c->tc_hf_b);
+    cudaFree(c->tc_tiles); cudaFree(c->tc_n_tiles); cudaFree(c->tc_slot_tile); cudaFree(c->tc_b_img); cudaFree(c->tc_b_sf); cudaFree(c->tc_codes); cudaFree(c->tc_scales); cudaFree(c->tc_q8_b); cudaFree(c->tc_q8_sx); cudaFree(c->tc_hf_b);
     c->tc_hf_b = nullptr; c->tc_cap_hfb = 0; c->tc_hf_src = 0;
     c->tc_q8_b = nullptr; c->tc_q8_sx = nullptr; c->tc_cap_q8b = c->tc_cap_q8sx = 0; c->tc_q8_src = 0;
-    c->tc_tiles = nullptr; c->tc_n_tiles = nullptr; c->tc_slot_tile = nullptr; c->tc_b_img = nullptr; c->tc_b_sf = nullptr; c->tc_status = nullptr; c->tc_codes = nullptr; c->tc_scales = nullptr; c->tc_cap_codes = c->tc_cap_scales = 0;
+    c->tc_tiles = nullptr; c->tc_n_tiles = nullptr; c->tc_slot_tile = nullptr; c->tc_b_img = nullptr; c->tc_b_sf = nullptr; c->tc_codes = nullptr; c->tc_scales = nullptr; c->tc_cap_codes = c->tc_cap_scales = 0;
     c->tc_cap_tiles = c->tc_cap_slots = c->tc_cap_b = c->tc_cap_sf = 0;
 }
 void itb_free_weight(itb_ctx* c, void* a, void* b, void* scale2) {
@@ -594,12 +602,11 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     size_t cap_t = c->tc_cap_tiles;
     bool ok = tc_grow(&tiles, &cap_t, max_tiles, st);
     c->tc_tiles = tiles; c->tc_cap_tiles = cap_t;
-    size_t cap1 = c->tc_n_tiles ? 1 : 0, cap2 = c->tc_status ? 1 : 0;
-    ok = ok && tc_grow(&c->tc_n_tiles, &cap1, 1, st) && tc_grow(&c->tc_status, &cap2, 1, st) &&
+    size_t cap1 = c->tc_n_tiles ? 1 : 0;
+    ok = ok && tc_grow(&c->tc_n_tiles, &cap1, 1, st) &&
          tc_grow(&c->tc_b_img, &c->tc_cap_b, b_rows * (wg.n_in / 2), st) && tc_grow(&c->tc_b_sf, &c->tc_cap_sf, max_tiles * kbs * 512, st) &&
          tc_grow(&c->tc_codes, &c->tc_cap_codes, (size_t)n_pairs * (wg.n_in / 2), st) && tc_grow(&c->tc_scales, &c->tc_cap_scales, (size_t)n_pairs * (wg.n_in / 16), st);
     if (!ok) return itb_fail_msg(c, "FP4 tensor path: out of device memory for the pass");
-    cudaMemsetAsync(c->tc_status, 0, 4, st);
     itb_chain(k_tc_build_tiles, 1, 1024, 0, st, pair_off, wg.expert_lo + wg.n_expert, wg.expert_lo, wg.n_expert, tiles, c->tc_n_tiles, (int)max_tiles, (int)kbs);
     const size_t x_rows = rows_div == 1 ? (size_t)n_pairs : rows_div >= n_pairs ? 1 : ((size_t)n_pairs + rows_div - 1) / rows_div;
     const size_t nq = x_rows * (wg.n_in / 16);
@@ -610,7 +617,7 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     g.wg_img = tg->img; g.wg_sf = tg->sf; g.wu_img = tu ? tu->img : nullptr; g.wu_sf = tu ? tu->sf : nullptr;
     g.s2g = wg.scale2; g.s2u = wu ? wu->scale2 : nullptr; g.expert_lo = wg.expert_lo;
     g.b_img = c->tc_b_img; g.b_sf = c->tc_b_sf; g.tiles = tiles; g.n_tiles = c->tc_n_tiles; g.pair_list = pair_list;
-    g.n_out = wg.n_out; g.n_in = wg.n_in; g.out = out; g.out_stride = wg.n_out; g.status = c->tc_status;
+    g.n_out = wg.n_out; g.n_in = wg.n_in; g.out = out; g.out_stride = wg.n_out; g.status = c->fail_word;
     itb_raise_smem(k_tc_gemm<true, true>, tc_gemm_smem(true));
     itb_raise_smem(k_tc_gemm<true, false>, tc_gemm_smem(true));
     itb_raise_smem(k_tc_gemm<false, false>, tc_gemm_smem(false));
@@ -642,15 +649,6 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     if (e != cudaSuccess) return itb_fail(c, "FP4 tensor path: launch", e);
     return true;
 }
-// The status word of the last pass: 0 fine; 3 / 4 / 5: a (bounded) wait of the producer / the MMA warp / an epilogue warp ran out.
-int itb_tc_status(itb_ctx* c, cudaStream_t st) {
-    int v = 0;
-    if (!c->tc_status) return 0;
-    cudaMemcpyAsync(&v, c->tc_status, 4, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    return v;
-}
-
 // FP4 activation quantiser on its own (tests against the CPU statement, src/ops/naive.rs:755-788): x[n] (n a multiple of 16) ->
 // one UE4M3 scale code per 16 elements and one E2M1 code per element (a byte each, like the CPU record).
 extern "C" int itb_fp4_quantize(itb_ctx* c, const float* x, size_t n, uint8_t* scales_out, uint8_t* codes_out) {
@@ -732,7 +730,7 @@ struct TcQ8 {
     const uint8_t* b_img; const float* b_sc;      // activations of the pass, the same form over token tiles
     int kbs, n_rows, n_out;
     float* out; size_t stride; int mode;          // out[token][row]; mode 1: += (the residual add of an output projection)
-    int* status;
+    volatile int* status;
     unsigned long long zero2;                     // two f32 zeros the compiler knows nothing about
     long long* prof;                              // optional: 8 words per block, the first its cycles (ITB_TC_PROF=1)
 };
@@ -790,7 +788,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             __syncwarp();
             if (++s == STAGES) { s = 0; phase ^= 1u; }
         }
-        if (!ok && lane == 0) atomicCAS(p.status, 0, 3);
+        if (!ok && lane == 0) *p.status = 3;
     } else if (wid == Q8_EPW + 1) {
         const uint32_t idesc = tc_idesc_f16(128, NT);
         const uint64_t dA = tc_desc(sbase, 2048, 128), dB = tc_desc(sbase + C::O_B, NT * 16, 128);
@@ -815,7 +813,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             if (++s == STAGES) { s = 0; phase ^= 1u; }
             if (++dp == ND) { dp = 0; dphase ^= 1u; }
         }
-        if (!ok && lane == 0) atomicCAS(p.status, 0, 4);
+        if (!ok && lane == 0) *p.status = 4;
     } else {
         const int quarter = wid & 3, col0 = (wid >> 2) * CW, row = quarter * 32 + lane;
         unsigned long long acc[MT * UC][UW / 2];     // f32 pairs: two columns to an instruction
@@ -904,7 +902,7 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
                     }
                 }
             }
-        } else if (lane == 0) atomicCAS(p.status, 0, 5);
+        } else if (lane == 0) *p.status = 5;
     }
     tc_fence_before();
     __syncthreads();
@@ -930,8 +928,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
         c->launches++;
         it = c->tc_weights.emplace(w.q, t).first;
     }
-    size_t cap1 = c->tc_status ? 1 : 0;
-    bool ok = tc_grow(&c->tc_status, &cap1, 1, st) && tc_grow(&c->tc_q8_b, &c->tc_cap_q8b, tts * nt * kbs * 64, st) && tc_grow(&c->tc_q8_sx, &c->tc_cap_q8sx, tts * nt * kbs, st);
+    bool ok = tc_grow(&c->tc_q8_b, &c->tc_cap_q8b, tts * nt * kbs * 64, st) && tc_grow(&c->tc_q8_sx, &c->tc_cap_q8sx, tts * nt * kbs, st);
     if (!ok) return itb_fail_msg(c, "Q8_0 tensor path: out of device memory for the pass");
     // consecutive matmuls over one quantised row set share its image
     if (x.id == 0 || c->tc_q8_src != x.id || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in || c->tc_q8_src_tile != (int)nt) {
@@ -940,10 +937,9 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
         c->launches++;
         c->tc_q8_src = x.id; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in; c->tc_q8_src_tile = (int)nt;
     }
-    cudaMemsetAsync(c->tc_status, 0, 4, st);
     TcQ8 g{};
     g.a_img = it->second.img; g.a_sc = (const float*)it->second.sf; g.b_img = c->tc_q8_b; g.b_sc = c->tc_q8_sx; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_out = w.n_out;
-    g.out = out; g.stride = stride; g.mode = mode; g.status = c->tc_status;
+    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail_word;
     auto kernel = mt == 2 ? k_tc_q8<64, 2> : k_tc_q8<64, 1>;
     const size_t smem = mt == 2 ? Q8Cfg<64, 2>::SMEM : Q8Cfg<64, 1>::SMEM;
     itb_raise_smem(kernel, smem);
@@ -1030,7 +1026,7 @@ struct TcHf {
     const uint8_t* b_img;                         // activations of the pass: [token tile][K16 block][8192 B]
     int kbs, n_rows, n_rt, n_tt;                  // K16 blocks, tokens, row tiles, token tiles
     float* out; size_t stride; int mode;          // out[token][row]; mode 1: += (the residual add of an output projection)
-    int* status;
+    volatile int* status;
     long long* prof;                              // optional: 8 cycle counts per block (ITB_TC_PROF=1)
 };
 // grid: one block per SM (or per work item, if fewer); block 320: warps 0-7 store accumulators (lane quarter = warp % 4, column half
@@ -1068,23 +1064,27 @@ __global__ void __launch_bounds__(320, 1) k_tc_f16(TcHf p) {
     long long* pf = p.prof ? p.prof + (size_t)blockIdx.x * 8 : nullptr;
     if (pf && tid == 0) pf[0] = clock64();
     bool ok = true;
-    if (wid == 8 && lane == 0) {
+    auto wait = [&](unsigned long long* bar, uint32_t phase) { ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(bar), phase, limit)); };      // of a whole warp
+    if (wid == 8) {
         int it = 0;
         for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
             const size_t a0 = (size_t)(w / p.n_tt) * kbs, b0 = (size_t)(w % p.n_tt) * kbs;
             for (int st = 0; st < n_stage; ++st, ++it) {
                 const int s = it % HF_STAGES;
-                if (it >= HF_STAGES) ok = tc_mbar_wait(tc_smem(&s_empty[s]), ((it / HF_STAGES) - 1) & 1, limit);
+                if (it >= HF_STAGES) wait(&s_empty[s], ((it / HF_STAGES) - 1) & 1);
                 if (!ok) break;
                 const uint32_t full = tc_smem(&s_full[s]), dst = sbase + s * HF_STAGE_BYTES;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)HF_STAGE_BYTES) : "memory");
                 const size_t kb0 = (size_t)st * HF_KB;
-                tc_bulk(dst, p.a_img + (a0 + kb0) * HF_A_BLK, HF_KB * HF_A_BLK, full);
-                tc_bulk(dst + HF_KB * HF_A_BLK, p.b_img + (b0 + kb0) * HF_B_BLK, HF_KB * HF_B_BLK, full);
+                if (tc_elect()) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)HF_STAGE_BYTES) : "memory");
+                    tc_bulk(dst, p.a_img + (a0 + kb0) * HF_A_BLK, HF_KB * HF_A_BLK, full);
+                    tc_bulk(dst + HF_KB * HF_A_BLK, p.b_img + (b0 + kb0) * HF_B_BLK, HF_KB * HF_B_BLK, full);
+                }
+                __syncwarp();
             }
         }
-        if (!ok) atomicCAS(p.status, 0, 3);
-    } else if (wid == 9 && lane == 0) {
+        if (!ok && lane == 0) *p.status = 3;
+    } else if (wid == 9) {
         const uint32_t idesc = tc_idesc_f16(128, HF_N);
         const uint64_t dA = tc_desc(sbase, 128 * 16, 128), dB = tc_desc(sbase + HF_KB * HF_A_BLK, HF_N * 16, 128);
         int it = 0, item = 0;
@@ -1093,34 +1093,32 @@ __global__ void __launch_bounds__(320, 1) k_tc_f16(TcHf p) {
             const int buf = item & 1;
             if (item >= 2) {                                  // the warps that store have read this buffer's previous tile
                 const long long c0 = pf ? clock64() : 0;
-                ok = tc_mbar_wait(tc_smem(&s_free[buf]), ((item >> 1) - 1) & 1, limit);
+                wait(&s_free[buf], ((item >> 1) - 1) & 1);
                 if (pf) t_free += clock64() - c0;
                 if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tc_fence_after();
             }
             for (int st = 0; st < n_stage; ++st, ++it) {
                 const int s = it % HF_STAGES;
                 const long long c0 = pf ? clock64() : 0;
-                ok = tc_mbar_wait(tc_smem(&s_full[s]), (it / HF_STAGES) & 1, limit);
+                wait(&s_full[s], (it / HF_STAGES) & 1);
                 if (pf) t_load += clock64() - c0;
                 if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tc_fence_after();
                 const uint32_t so = (uint32_t)s * (HF_STAGE_BYTES >> 4);
+                if (tc_elect()) {
 #pragma unroll
-                for (int k = 0; k < HF_KB; ++k) {
-                    asm volatile(
-                        "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }\n"
-                        ::"r"(tm + (uint32_t)(HF_N * buf)), "l"(dA + so + (uint32_t)(k * (HF_A_BLK >> 4))), "l"(dB + so + (uint32_t)(k * (HF_B_BLK >> 4))), "r"(idesc),
-                          "r"((st | k) ? 1u : 0u) : "memory");
+                    for (int k = 0; k < HF_KB; ++k)
+                        tc_mma_f16(tm + (uint32_t)(HF_N * buf), dA + so + (uint32_t)(k * (HF_A_BLK >> 4)), dB + so + (uint32_t)(k * (HF_B_BLK >> 4)), idesc, (st | k) ? 1u : 0u);
+                    tc_commit(tc_smem(&s_empty[s]));
+                    if (st + 1 == n_stage) tc_commit(tc_smem(&s_acc[buf]));
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_empty[s])) : "memory");
+                __syncwarp();
             }
             if (!ok) break;
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(&s_acc[buf])) : "memory");
         }
-        if (!ok) atomicCAS(p.status, 0, 4);
-        if (pf) { pf[1] = t_load; pf[2] = t_free; }
+        if (!ok && lane == 0) *p.status = 4;
+        if (pf && lane == 0) { pf[1] = t_load; pf[2] = t_free; }
     } else if (wid < 8) {
         const int quarter = wid & 3, half = wid >> 2, row = quarter * 32 + lane;
         int item = 0;
@@ -1129,7 +1127,7 @@ __global__ void __launch_bounds__(320, 1) k_tc_f16(TcHf p) {
             const int buf = item & 1, rt = w / p.n_tt, tt = w % p.n_tt;
             const long long k0 = pf ? clock64() : 0;
             ok = __all_sync(0xffffffffu, tc_mbar_wait(tc_smem(&s_acc[buf]), (item >> 1) & 1, limit));
-            if (!ok || __shfl_sync(0xffffffffu, *(volatile int*)p.status, 0) != 0) break;
+            if (!ok) break;
             const long long k1 = pf ? clock64() : 0;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float* ocol = p.out + (size_t)rt * 128 + row;
@@ -1164,7 +1162,7 @@ __global__ void __launch_bounds__(320, 1) k_tc_f16(TcHf p) {
             }
             if (pf) { t_wait += k1 - k0; t_work += clock64() - k1; }
         }
-        if (!ok) atomicCAS(p.status, 0, 5);
+        if (!ok && lane == 0) *p.status = 5;
         if (pf && tid == 0) { pf[3] = t_wait; pf[4] = t_work; pf[6] = item; }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1191,8 +1189,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
         c->launches++;
         it = c->tc_weights.emplace(w.s, t).first;
     }
-    size_t cap1 = c->tc_status ? 1 : 0;
-    bool ok = tc_grow(&c->tc_status, &cap1, 1, st) && tc_grow(&c->tc_hf_b, &c->tc_cap_hfb, tts * kbs * HF_B_BLK, st);
+    bool ok = tc_grow(&c->tc_hf_b, &c->tc_cap_hfb, tts * kbs * HF_B_BLK, st);
     if (!ok) return itb_fail_msg(c, "f16 tensor path: out of device memory for the pass");
     // consecutive matmuls over one quantised row set share its image
     if (x.id == 0 || c->tc_hf_src != x.id || c->tc_hf_src_rows != n_rows || c->tc_hf_src_in != w.n_in) {
@@ -1201,10 +1198,9 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
         c->launches++;
         c->tc_hf_src = x.id; c->tc_hf_src_rows = n_rows; c->tc_hf_src_in = w.n_in;
     }
-    cudaMemsetAsync(c->tc_status, 0, 4, st);
     TcHf g{};
     g.a_img = it->second.img; g.b_img = c->tc_hf_b; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_rt = (int)rts; g.n_tt = (int)tts;
-    g.out = out; g.stride = stride; g.mode = mode; g.status = c->tc_status;
+    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail_word;
     itb_raise_smem(k_tc_f16, tc_f16_smem());
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = std::min<size_t>((size_t)c->sm_count, rts * tts);
