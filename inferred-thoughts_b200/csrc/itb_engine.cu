@@ -639,6 +639,7 @@ struct itb_engine {
     float *qg = nullptr, *kbuf = nullptr, *vbuf = nullptr, *qn = nullptr, *gate = nullptr, *att = nullptr;
     float *part_acc = nullptr, *part_ml = nullptr;
     uint32_t* words = nullptr;                         // pinned: a step's tokens, next tokens and status word
+    cudaStream_t side = nullptr; cudaEvent_t fork = nullptr, join = nullptr;       // a second stream for what a many-row pass can do beside its main chain (enqueue_rows); null: none
     float* scores = nullptr; size_t scores_cap = 0;    // exact attention: [rows][n_head][n_ctx] scores (grown on demand)
     float *router = nullptr, *shlogit = nullptr, *sg = nullptr, *su = nullptr, *h = nullptr, *logits = nullptr;
     int8_t* xq = nullptr; float* xs = nullptr;
@@ -1216,8 +1217,21 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     cudaStreamCaptureStatus cap_rows = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &cap_rows);
     const bool f16tc = c->f16tc && n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone;
+    // Beside the main chain: alpha and beta while the input projections run, the shared expert while the routed ones do. Each is a few
+    // small kernels that leave most SMs idle, the serial-order chains among them. `beside` runs f on the second stream between two events;
+    // what it writes is read behind `meet`. Only kernels and this engine's buffers are involved, and of the context's scratch the
+    // row images of the dense matmuls, which nothing on the main chain touches between the two.
+    cudaStream_t cur = st;
+    const bool two = chain && e->side;
+    auto beside = [&](auto f) {
+        if (!two) { f(); return; }
+        cudaEventRecord(e->fork, st); cudaStreamWaitEvent(e->side, e->fork, 0);
+        cur = e->side; f(); cur = st;
+        cudaEventRecord(e->join, e->side);
+    };
+    auto meet = [&] { if (two) cudaStreamWaitEvent(st, e->join, 0); };
     auto gemm_n = [&](const DevQ8& w, const QRows& x, float* out, size_t stride, int mode, int R) {
-        dense_q8(c, st, w, x, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone);
+        dense_q8(c, cur, w, x, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone);
         launches++;
     };
     auto gemm = [&](const DevQ8& w, const QRows& x, float* out, size_t stride, int mode) { gemm_n(w, x, out, stride, mode, R); };
@@ -1232,7 +1246,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             int tiles = 0;
             for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; p.tiles[i] = (w[i]->n_out + 31) / 32; tiles += p.tiles[i]; }
             const int k = w[0]->n_in, ns = std::min(k / 256, TILE_STAGES);
-            itb_chain(k_tile_q8_multi<1, 256, 4>, dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), st, p, x.q, x.s, R, ns);
+            itb_chain(k_tile_q8_multi<1, 256, 4>, dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), cur, p, x.q, x.s, R, ns);
             launches++;
             return;
         }
@@ -1243,7 +1257,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     auto gemm_fp4d = [&](const DevFp4& w, const int8_t* xq, const float* xs, float* out, int rows, bool has_s, float sc) {
         if (rows >= 2 && gemm_smem(w.n_in) <= 200 * 1024) {
             set_smem((const void*)k_gemm_fp4, gemm_smem(w.n_in));
-            itb_chain(k_gemm_fp4, dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), st, 
+            itb_chain(k_gemm_fp4, dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(w.n_in), cur, 
                 w.nib, w.sc, w.n_in, w.n_out, xq, xs, rows, out, (size_t)w.n_out, sc, has_s ? 1 : 0);
             launches++;
             return;
@@ -1251,26 +1265,26 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         const int gx = std::max(1, std::min((w.n_out + 31) / 32, 2 * sms));
         const size_t smem = matmul_fp4_smem(w.n_in);
         set_smem((const void*)k_matmul_fp4, smem);
-        itb_chain(k_matmul_fp4, dim3(gx, rows), 256, smem, st, w, nullptr, 1, 0, xq, xs, out);
+        itb_chain(k_matmul_fp4, dim3(gx, rows), 256, smem, cur, w, nullptr, 1, 0, xq, xs, out);
         launches++;
-        if (has_s) { const size_t n = (size_t)rows * w.n_out; k_scale<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, sc); launches++; }
+        if (has_s) { const size_t n = (size_t)rows * w.n_out; k_scale<<<(unsigned)((n + 255) / 256), 256, 0, cur>>>(out, n, sc); launches++; }
     };
     auto f32mm = [&](const DevF32& w, const float* x, float* out) {
-        if (!c->exact && f16tc && sgemm_chain_ok(w.n_in) && R >= 64) { sgemm_chain<true>(st, sms, w, x, R, out); launches++; return; }   // tolerance-class passes: fused multiply-adds
-        if (!c->exact && f32_tree_ok(w.n_in)) { f32_tree(st, sms, w, x, R, out); launches++; return; }
-        if (c->exact && sgemm_chain_ok(w.n_in)) { sgemm_chain<false>(st, sms, w, x, R, out); launches++; return; }   // also for a few rows: the tile's k loop is as long as a row's chain either way
+        if (!c->exact && f16tc && sgemm_chain_ok(w.n_in) && R >= 64) { sgemm_chain<true>(cur, sms, w, x, R, out); launches++; return; }   // tolerance-class passes: fused multiply-adds
+        if (!c->exact && f32_tree_ok(w.n_in)) { f32_tree(cur, sms, w, x, R, out); launches++; return; }
+        if (c->exact && sgemm_chain_ok(w.n_in)) { sgemm_chain<false>(cur, sms, w, x, R, out); launches++; return; }   // also for a few rows: the tile's k loop is as long as a row's chain either way
         const int nw = 4;
         dim3 g(std::max(1, std::min(2 * sms, (w.n_out + 31) / 32)), R);
         size_t sm = (size_t)w.n_in * 4 + (size_t)nw * 32 * 33 * 4;
-        if (c->exact) itb_chain(k_matmul_f32<true>, g, nw * 32, sm, st, w, x, out);
-        else itb_chain(k_matmul_f32<false>, g, nw * 32, sm, st, w, x, out);
+        if (c->exact) itb_chain(k_matmul_f32<true>, g, nw * 32, sm, cur, w, x, out);
+        else itb_chain(k_matmul_f32<false>, g, nw * 32, sm, cur, w, x, out);
         launches++;
     };
     // two F32 matrices over the same rows: one launch where both take the serial-order tiles, else one after the other
     auto f32mm2 = [&](const DevF32& wa, float* oa, const DevF32& wb, float* ob, const float* x) {
         const bool fused = !c->exact && f16tc && R >= 64;
         if ((c->exact || fused) && wa.n_in == wb.n_in && sgemm_chain_ok(wa.n_in)) {
-            if (fused) sgemm_chain<true>(st, sms, wa, x, R, oa, wb, ob); else sgemm_chain<false>(st, sms, wa, x, R, oa, wb, ob);
+            if (fused) sgemm_chain<true>(cur, sms, wa, x, R, oa, wb, ob); else sgemm_chain<false>(cur, sms, wa, x, R, oa, wb, ob);
             launches++;
             return;
         }
@@ -1286,17 +1300,18 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         if (L.recurrent) {
             const int rs = e->slot_of[il];
             const size_t state_stride = (size_t)n_v * sk * sk, conv_stride = (size_t)cd * (d.ssm_d_conv - 1);
+            beside([&] { f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn); });
             {
                 const DevQ8* ws[2] = {&L.wqkv, &L.wgate}; float* os[2] = {e->qkvc, e->z}; const size_t ss[2] = {(size_t)cd, (size_t)vd};
                 gemm_multi(2, ws, os, ss, xa);
             }
-            f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn);
             float* cst = e->conv_state + (size_t)rs * e->B * conv_stride;
             if (d.ssm_d_conv == 4 && n_tok >= CONV_T) itb_chain(k_conv_rows4, dim3((cd + 127) / 128, n_seq * ((n_tok + CONV_T - 1) / CONV_T)), 128, 0, st, cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d);
             else itb_chain(k_conv_rows, dim3((cd + 127) / 128, R), 128, 0, st, cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d, d.ssm_d_conv);
             launches++;
             itb_chain(k_conv_state, dim3((cd + 127) / 128, n_seq), 128, 0, st, cst, conv_stride, e->qkvc, n_tok, cd, d.ssm_d_conv); launches++;
-            itb_chain((sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>), dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st, 
+            meet();
+            launch_k(!two, (sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>), dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st, 
                 e->qkvc2, cd, e->alpha, e->beta, L.ssm_a, L.dt_bias, n_k, n_v, d.rms_eps, e->qh, e->kh, e->vh, e->gb); launches++;
             const size_t chunk_need = (size_t)n_seq * ((n_tok + GC - 1) / GC) * n_v * gdn_chunk_floats<128>();
             if ((c->gdn_chunk || !c->exact) && n_tok >= 32 && sk == 128 && e->gdn_scratch_cap >= chunk_need) {
@@ -1376,15 +1391,23 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         // routed FFN
         itb_chain(k_norm_quant, R, 256, smem_nq, st, e->x, L.ffn_norm, H, d.rms_eps, e->xn, e->xq, e->xs, e->ep ? nullptr : e->xh); launches++;
         const QRows xf = c->quantised(e->xq, e->xs);
-        if (!L.shared4[0].nib && !L.shared4[1].nib) {
-            const DevQ8* ws[2] = {&L.shared_gate, &L.shared_up}; float* os[2] = {e->sg, e->su}; const size_t ss[2] = {(size_t)d.shared_ff, (size_t)d.shared_ff};
-            gemm_multi(2, ws, os, ss, xf);
-        } else {
-            if (L.shared4[0].nib) gemm_fp4d(L.shared4[0], e->xq, e->xs, e->sg, R, L.has_shared_s[0], L.shared_s[0]);
-            else gemm(L.shared_gate, xf, e->sg, d.shared_ff, 0);
-            if (L.shared4[1].nib) gemm_fp4d(L.shared4[1], e->xq, e->xs, e->su, R, L.has_shared_s[1], L.shared_s[1]);
-            else gemm(L.shared_up, xf, e->su, d.shared_ff, 0);
-        }
+        auto shared_in = [&] {
+            if (!L.shared4[0].nib && !L.shared4[1].nib) {
+                const DevQ8* ws[2] = {&L.shared_gate, &L.shared_up}; float* os[2] = {e->sg, e->su}; const size_t ss[2] = {(size_t)d.shared_ff, (size_t)d.shared_ff};
+                gemm_multi(2, ws, os, ss, xf);
+            } else {
+                if (L.shared4[0].nib) gemm_fp4d(L.shared4[0], e->xq, e->xs, e->sg, R, L.has_shared_s[0], L.shared_s[0]);
+                else gemm(L.shared_gate, xf, e->sg, d.shared_ff, 0);
+                if (L.shared4[1].nib) gemm_fp4d(L.shared4[1], e->xq, e->xs, e->su, R, L.has_shared_s[1], L.shared_s[1]);
+                else gemm(L.shared_up, xf, e->su, d.shared_ff, 0);
+            }
+        };
+        auto shared_out = [&] {
+            launch_k(chain, k_shared_act_rows, R, 128, 0, cur, e->sg, e->su, d.shared_ff, e->sq, e->ss); launches++;
+            if (L.shared4[2].nib) gemm_fp4d(L.shared4[2], e->sq, e->ss, e->shd, R, L.has_shared_s[2], L.shared_s[2]);
+            else gemm(L.shared_down, c->quantised(e->sq, e->ss), e->shd, H, 0);
+        };
+        if (two) beside([&] { shared_in(); shared_out(); }); else shared_in();
         f32mm2(L.gate_inp, e->router, L.shared_gate_inp, e->shlogit, e->xn);
         {
             const int K = d.n_expert_used, E = d.n_expert, ff = d.expert_ff;
@@ -1530,11 +1553,9 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                 launches++;
                 o_src = e->ep->o_mine;
             }
-            launch_k(chain, k_shared_act_rows, R, 128, 0, st, e->sg, e->su, d.shared_ff, e->sq, e->ss); launches++;
-            if (L.shared4[2].nib) gemm_fp4d(L.shared4[2], e->sq, e->ss, e->shd, R, L.has_shared_s[2], L.shared_s[2]);
-            else gemm(L.shared_down, c->quantised(e->sq, e->ss), e->shd, H, 0);
+            if (two) meet(); else shared_out();
             const size_t total = (size_t)R * H;
-            launch_k(chain, k_moe_finish_rows, (unsigned)((total + 255) / 256), 256, 0, st, e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
+            launch_k(chain && !two, k_moe_finish_rows, (unsigned)((total + 255) / 256), 256, 0, st, e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
         }
     }
     // LM head on each sequence's last row
@@ -1570,6 +1591,12 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     return launches;
 }
 
+static void drop_side(itb_engine* e) {
+    if (e->side) { cudaStreamSynchronize(e->side); cudaStreamDestroy(e->side); }
+    if (e->fork) cudaEventDestroy(e->fork);
+    if (e->join) cudaEventDestroy(e->join);
+    e->side = nullptr; e->fork = e->join = nullptr;
+}
 static int engine_create(itb_model* m, uint32_t n_ctx, uint32_t n_seq, int world, itb_engine** out, uint32_t rows_cap = 0) {
     *out = nullptr;
     itb_ctx* c = m->c;
@@ -1623,6 +1650,9 @@ static int engine_create(itb_model* m, uint32_t n_ctx, uint32_t n_seq, int world
     }
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) { itb_fail_msg(c, "engine: device error during set-up"); return 1; }
     if (exact_attention_ok(E) && !ensure_scores(E, B)) { for (void* p : e->allocs) cudaFree(p); return 1; }
+    if (world == 1 && cudaStreamCreateWithFlags(&E->side, cudaStreamNonBlocking) == cudaSuccess &&
+        (cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming) != cudaSuccess || cudaEventCreateWithFlags(&E->join, cudaEventDisableTiming) != cudaSuccess)) drop_side(E);
+    cudaGetLastError();                          // refused: the passes stay on one stream
     *out = e.release();
     return 0;
 }
@@ -1776,6 +1806,7 @@ extern "C" void itb_engine_destroy(itb_engine* e) {
     for (void* p : e->allocs) cudaFree(p);
     cudaFreeHost(e->words); cudaFree(e->history); cudaFree(e->prompt); cudaFree(e->scores); cudaFree(e->gdn_scratch);
     cudaEventDestroy(e->ev0); cudaEventDestroy(e->ev1);
+    drop_side(e);
     delete e;
 }
 

@@ -242,6 +242,30 @@ def test_pipelined_rows_batched_decode_equals_single_sequences(mid, n_seq):
     eb.close()
 
 
+@pytest.mark.parametrize("opts", ["exact=1", "exact=1,dense=q8tc"])
+def test_engines_of_one_context_in_turn_equal_each_alone(opts):
+    """Many-row passes run part of a layer on a second stream of the engine's, with the context's scratch: passes of two engines
+    queued in turn, of 1 to 130 rows, give what each gives alone, and so do batched decode steps between them."""
+    from inferred_thoughts_b200 import host
+    ops = host.B200Ops(0, opts)
+    model = host.Model(ops, host_dims(MID)); model.synth(5)
+    parts = [prompt_ids(90 + n, n, MID["n_vocab"]) for n in (130, 65, 7, 100)]
+    batch = np.stack([prompt_ids(70 + b, 70, MID["n_vocab"]) for b in range(3)])
+    alone = [host.Engine(model, 512, 1), host.Engine(model, 512, 3)]
+    want = [alone[0].prefill(p).copy() for p in parts]
+    tok = [alone[1].prefill(batch).reshape(3, -1).argmax(1).astype(np.uint32)]
+    steps = []
+    for _ in range(3):
+        logits, nxt = alone[1].decode(tok[-1]); steps.append(logits.copy()); tok.append(nxt.copy())
+    a, b = host.Engine(model, 512, 1), host.Engine(model, 512, 3)
+    assert a.prefill(parts[0]).tobytes() == want[0].tobytes()
+    b.prefill(batch)
+    for i in range(3):
+        assert a.prefill(parts[i + 1]).tobytes() == want[i + 1].tobytes()
+        assert b.decode(tok[i])[0].tobytes() == steps[i].tobytes()
+    ops.check()
+
+
 def test_tree_mode_rows_equal_single_rows():
     """exact=0 (F32 dots by a shuffle tree, the benchmark's mode): the multi-row F32 kernel keeps the one-token kernel's
     summation order, so batched decode and multi-row prefill still give each row the bits it gets alone."""
