@@ -13,20 +13,23 @@
 
 // A copy from or to pageable memory goes through a staging buffer somewhere: the driver's does it on one thread and asks for a stream
 // synchronise to be sure of it. Here: a small copy is one memcpy into a pinned ring and an asynchronous copy behind it (no
-// synchronise); a large one runs in chunks, the chunk in flight on the bus while the next is copied by four threads. The threads start
+// synchronise); a large one runs in chunks, the chunk in flight on the bus while the next is copied by eight threads. The threads start
 // with the first large copy and end with the context. Nothing here throws, and a refused thread, event or pinned buffer costs only time:
 // the caller copies alone, waits for the stream where an event would have told it, or takes the driver's own copy.
-// One call with its kernel, the driver's copies and a synchronise -> this: 16.8 MB up 1,530 -> 860 us, down 830 -> 490; 0.26 MB up 51 -> 29,
-// down 42 -> 27; 4.2 MB up 420 -> 440 (as long in the driver), down 250 -> 200.
+// Chunks up are small: the bus idles while the first is copied and the threads while the last is sent, and a chunk that waits for a thread
+// to wake holds up less. (4.1 MB up, mean: 2 MB chunks and four threads 437 us, 1 MB and eight 264, 0.5 MB and four 186, six 163, eight 155;
+// 16.8 MB: 895, 883, 712, 633, 588.) Down, large ones want few waits for events: 16.8 MB in 2 MB chunks 491 us, in 0.5 MB ones 611; 4.1 MB 199
+// in three, 157 in 0.5 MB ones. Eight pinned chunks up, three down: 11 MB a context that makes such copies.
 struct HostPipe {
-    static constexpr size_t RING = 1 << 20, SMALL = 128 << 10, CHUNK = 2 << 20;
-    static constexpr int N_CHUNK = 3, N_THREAD = 3;
+    static constexpr size_t RING = 1 << 20, SMALL = 128 << 10, CHUNK = 2 << 20, UP_CHUNK = 512 << 10;
+    static constexpr int N_CHUNK = 3, N_UP = 8, N_THREAD = 7;
     uint8_t* ring = nullptr; size_t ring_at = 0; int ring_half = 0; cudaEvent_t half_ev[2] = {nullptr, nullptr}; bool half_used[2] = {false, false};
     uint8_t* chunk[N_CHUNK] = {nullptr, nullptr, nullptr}; cudaEvent_t chunk_ev[N_CHUNK] = {nullptr, nullptr, nullptr}; bool chunk_used[N_CHUNK] = {false, false, false};
+    uint8_t* up_mem = nullptr; cudaEvent_t up_ev[N_UP] = {}; bool up_used[N_UP] = {};
     // Copy threads. A copy is cut into PARTS; whoever is free takes the next one, the caller included, so a thread that wakes late costs
     // nothing but its help. turn = (copy number << 8) | next part: a part is taken by raising it from the value under which the
     // copy's arguments were read, and the arguments change only after every part of the copy before is done.
-    static constexpr uint64_t PARTS = 8;
+    static constexpr uint64_t PARTS = 16;
     std::vector<std::thread> threads; sem_t wake; std::atomic<bool> quit{false};
     std::atomic<uint64_t> turn{PARTS}, done{0};
     std::atomic<uint8_t*> jd{nullptr}; std::atomic<const uint8_t*> js{nullptr}; std::atomic<size_t> jn{0};
@@ -59,8 +62,9 @@ struct HostPipe {
         }
         return !threads.empty();
     }
+    // below 384 KB waking the threads costs more than they save (0.26 MB up: 29 us alone, 46 with them)
     void copy(void* d, const void* s, size_t n) {
-        if (n < (512 << 10) || !start_threads()) { memcpy(d, s, n); return; }
+        if (n < (384 << 10) || !start_threads()) { memcpy(d, s, n); return; }
         jd.store((uint8_t*)d, std::memory_order_relaxed); js.store((const uint8_t*)s, std::memory_order_relaxed); jn.store(n, std::memory_order_relaxed);
         done.store(0, std::memory_order_relaxed);
         turn.store(((turn.load(std::memory_order_relaxed) >> 8) + 1) << 8, std::memory_order_release);
@@ -88,6 +92,7 @@ struct HostPipe {
         for (int i = 1; i < N_CHUNK; ++i) chunk[i] = chunk[0] + i * CHUNK;
         return true;
     }
+    bool ready_up() { return ready(&up_mem, UP_CHUNK * N_UP, up_ev); }
     // After the copies out of (or into) a staging buffer have been queued: `used` until they have run.
     static cudaError_t queued(cudaStream_t st, cudaEvent_t ev, bool& used) {
         used = true;
@@ -112,7 +117,8 @@ struct HostPipe {
         sem_destroy(&wake);
         for (auto& e : half_ev) if (e) cudaEventDestroy(e);
         for (auto& e : chunk_ev) if (e) cudaEventDestroy(e);
-        cudaFreeHost(ring); cudaFreeHost(chunk[0]);
+        for (auto& e : up_ev) if (e) cudaEventDestroy(e);
+        cudaFreeHost(ring); cudaFreeHost(chunk[0]); cudaFreeHost(up_mem);
     }
     cudaError_t up(cudaStream_t st, void* dev, const void* host, size_t bytes) {
         cudaError_t e = cudaSuccess;
@@ -131,21 +137,21 @@ struct HostPipe {
             ring_at += need;
             return cudaMemcpyAsync(dev, ring + at, bytes, cudaMemcpyHostToDevice, st);
         }
-        if (!ready_large()) return plain(st, dev, host, bytes, cudaMemcpyHostToDevice);
+        if (!ready_up()) return plain(st, dev, host, bytes, cudaMemcpyHostToDevice);
         int i = 0;
-        for (size_t at = 0; at < bytes; at += CHUNK, i = (i + 1) % N_CHUNK) {
-            const size_t n = std::min(CHUNK, bytes - at);
-            if ((e = settle(st, chunk_ev[i], chunk_used[i])) != cudaSuccess) return e;
-            copy(chunk[i], (const uint8_t*)host + at, n);
-            if ((e = cudaMemcpyAsync((uint8_t*)dev + at, chunk[i], n, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
-            if ((e = queued(st, chunk_ev[i], chunk_used[i])) != cudaSuccess) return e;
+        for (size_t at = 0; at < bytes; at += UP_CHUNK, i = (i + 1) % N_UP) {
+            const size_t n = std::min(UP_CHUNK, bytes - at);
+            if ((e = settle(st, up_ev[i], up_used[i])) != cudaSuccess) return e;
+            copy(up_mem + i * UP_CHUNK, (const uint8_t*)host + at, n);
+            if ((e = cudaMemcpyAsync((uint8_t*)dev + at, up_mem + i * UP_CHUNK, n, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
+            if ((e = queued(st, up_ev[i], up_used[i])) != cudaSuccess) return e;
         }
         return e;
     }
     cudaError_t down(cudaStream_t st, void* host, const void* dev, size_t bytes) {
         if (bytes <= (64 << 10) || !ready_large()) return plain(st, host, dev, bytes, cudaMemcpyDeviceToHost);
         cudaError_t e = cudaSuccess;
-        const size_t step = bytes >= 4 * CHUNK ? CHUNK : std::min(CHUNK, (bytes / 3 + 65535) & ~(size_t)65535), n_step = (bytes + step - 1) / step;
+        const size_t step = bytes >= 4 * CHUNK ? CHUNK : std::min(UP_CHUNK, (bytes / 3 + 65535) & ~(size_t)65535), n_step = (bytes + step - 1) / step;
         auto issue = [&](size_t s) {
             const int i = (int)(s % N_CHUNK);
             e = settle(st, chunk_ev[i], chunk_used[i]);
