@@ -869,7 +869,7 @@ static void enqueue_step(itb_engine* e, cudaStream_t st, StepProf* prof = nullpt
             g.state_stride = state_stride; g.state = e->ssm_state + (size_t)rs * B * state_stride;
             g.out_q = e->aq; g.out_s = e->as; g.sk = d.ssm_d_state; g.sv = d.ssm_d_state; g.n_k = d.ssm_n_group; g.n_v = d.ssm_dt_rank; g.eps = d.rms_eps;
             g.tl_slot = tl++;
-            size_t smem_g = (size_t)(g.sv * (g.sk + 1) + 2 * g.sk + g.sv) * 4;
+            size_t smem_g = (size_t)(g.sv * (g.sk + 4) + 2 * g.sk + g.sv) * 4;
             if (d.ssm_d_state == 128) launch_k(pdl, k_gdn_core<128>, dim3(d.ssm_dt_rank, B), 256, smem_g, st, g);
             else launch_k(pdl, k_gdn_core<64>, dim3(d.ssm_dt_rank, B), 256, smem_g, st, g);
             MARK(KC_GDN_CORE, (uint64_t)B * (2ull * g.state_stride * 4 + (cd + 2ull * vd) * 4));

@@ -226,6 +226,10 @@ size_t out_proj_smem(int n, int br) {
 // rule over the head's [sv][sk] state, gated RMSNorm, the SiLU(z) gate, and the Q8_0 quantisation the output
 // projection would apply (src/model/qwen35.rs:1280-1325, src/ops/naive.rs:86-135, :254-273). One thread per
 // value row, keys walked serially so every sum has the CPU's order.
+// What bounds it is latency on 32 SMs: the operands' round trip and exponentials, the l2 norms, two 128-long chains, the norm and the quantisation. What
+// does not wait for the operands is done before them: the state goes through shared memory into registers while the predecessor runs
+// (16-byte accesses on distinct banks; 4-byte ones with four lanes to a bank took 1 us of the kernel), and a warp with one activation
+// instead of two forms the decay. With the routing below: four steps at 6,500 12.12 -> 11.80 ms, generate_tiny 5.20 -> 5.08 ms.
 struct GdnCore {
     const float* conv; int conv_stride;           // [B][conv_dim] = q | k | v conv sums (pre-SiLU)
     const float* z; const float* alpha; const float* beta;
@@ -238,11 +242,11 @@ struct GdnCore {
 template <int SK>
 __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int sk = SK, sv = SK, LD = SK * SK / 4 / 256;   // float4 loads per thread
+    constexpr int sk = SK, sv = SK, LD = SK * SK / 4 / 256, ST = SK + 4;   // float4 loads per thread; floats between state rows (16-byte reads of a row and of a column of rows fall on distinct banks)
     const int h = blockIdx.x, b = blockIdx.y, kh = h % p.n_k, tid = threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
-    float* S = (float*)smem;                 // [sv][sk+1]
-    float* kq = S + sv * (sk + 1);           // k[sk] | q[sk]
+    float* S = (float*)smem;                 // [sv][ST]
+    float* kq = S + sv * ST;                 // k[sk] | q[sk]
     float* o = kq + 2 * sk;                  // [sv]
     __shared__ double red2[8];
     __shared__ float s_gb[2], s_z[SK];
@@ -250,11 +254,20 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     const float* cv = p.conv + (size_t)b * p.conv_stride;
     float* sg = p.state + (size_t)b * p.state_stride + (size_t)h * sv * sk;
     TL(TLK_GDN_CORE, 0);
-    // the state belongs to this layer alone: its loads are in flight while the predecessor kernel finishes
-    float4 ld[LD];
+    // the state belongs to this layer alone: it is a row to a thread, in registers, while the predecessor kernel finishes
+    float R[SK];
+    {
+        float4 ld[LD];
 #pragma unroll
-    for (int i = 0; i < LD; ++i) ld[i] = __ldcs((const float4*)sg + tid + i * 256);
+        for (int i = 0; i < LD; ++i) ld[i] = __ldcs((const float4*)sg + tid + i * 256);
+#pragma unroll
+        for (int i = 0; i < LD; ++i) { const int e = (tid + i * 256) * 4; *(float4*)(S + e / sk * ST + e % sk) = ld[i]; }
+    }
     const float r_dt = p.dt_bias[h], r_a = p.ssm_a[h], r_nw = p.ssm_norm[tid < sv ? tid : 0];
+    __syncthreads();
+    float* row = S + (tid < sv ? tid : 0) * ST;
+#pragma unroll
+    for (int i = 0; i < SK; i += 4) { const float4 v = *(const float4*)(row + i); R[i] = v.x; R[i + 1] = v.y; R[i + 2] = v.z; R[i + 3] = v.w; }
     pdl_wait();
     pdl_trigger();
     TL(TLK_GDN_CORE, 1);
@@ -266,11 +279,14 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     if (tid < 2 * sk) kq[tid] = silu_f(cv[(tid < sk ? key_dim : 0) + kh * sk + (tid < sk ? tid : tid - sk)]);
     float vj = 0.0f;
     if (tid < sv) vj = silu_f(cv[2 * key_dim + h * sv + tid]);
-#pragma unroll
-    for (int i = 0; i < LD; ++i) {
-        int e = (tid + i * 256) * 4, r = e / sk, c0 = e % sk;
-        float* d = S + r * (sk + 1) + c0;
-        d[0] = ld[i].x; d[1] = ld[i].y; d[2] = ld[i].z; d[3] = ld[i].w;
+    if (wid == 7) {
+        // the head's decay and write strength, once, beside the other warps' activations (three library-exact exponentials and a
+        // logarithm: on the f64 unit they were half of the update phase when each of its four warps computed them for itself)
+        float a = r_alpha + r_dt;
+        float sp = a > 20.0f ? a : log_f(1.0f + exp_f(a));
+        float g = exp_f(sp * r_a);
+        float bt = sigmoid_f(r_beta);
+        if (lane == 0) { s_gb[0] = g; s_gb[1] = bt; }
     }
     __syncthreads();
     TL(TLK_GDN_CORE, 2);
@@ -286,24 +302,12 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
             float v = src[i] * sc;
             src[i] = wid == 0 ? v : v * qs;
         }
-    } else if (wid == 2) {
-        // the head's decay and write strength, once (three library-exact exponentials and a logarithm: on the f64 unit they were
-        // half of the update phase when each of its four warps computed them for itself)
-        float a = r_alpha + r_dt;
-        float sp = a > 20.0f ? a : log_f(1.0f + exp_f(a));
-        float g = exp_f(sp * r_a);
-        float bt = sigmoid_f(r_beta);
-        if (lane == 0) { s_gb[0] = g; s_gb[1] = bt; }
     }
     __syncthreads();
     TL(TLK_GDN_CORE, 3);
     if (tid < sv) {
         const float g = s_gb[0], bt = s_gb[1];
         // the thread's state row lives in registers for both passes (src/ops/naive.rs:109-132 order: decay, predict, update, read out)
-        float* row = S + tid * (sk + 1);
-        float R[SK];
-#pragma unroll
-        for (int i = 0; i < SK; ++i) R[i] = row[i];
         float pred = 0.0f;
 #pragma unroll
         for (int i = 0; i < SK; i += 4) {
@@ -324,7 +328,7 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
             R[i + 3] = R[i + 3] + k4.w * d; acc += R[i + 3] * q4.w;
         }
 #pragma unroll
-        for (int i = 0; i < SK; ++i) row[i] = R[i];
+        for (int i = 0; i < SK; i += 4) *(float4*)(row + i) = make_float4(R[i], R[i + 1], R[i + 2], R[i + 3]);
         o[tid] = acc;
     } else if (tid < 2 * sv) s_z[tid - sv] = silu_f(r_z);
     __syncthreads();
@@ -348,9 +352,8 @@ __global__ void __launch_bounds__(256) k_gdn_core(GdnCore p) {
     } else {
 #pragma unroll 8
         for (int i = tid - sv; i < sv * sk / 4; i += 256 - sv) {
-            const int e = i * 4, r = e / sk, c0 = e % sk;
-            const float* s = S + r * (sk + 1) + c0;
-            __stcs((float4*)sg + i, make_float4(s[0], s[1], s[2], s[3]));
+            const int e = i * 4;
+            __stcs((float4*)sg + i, *(const float4*)(S + e / sk * ST + e % sk));
         }
     }
     TL(TLK_GDN_CORE, 5);
@@ -467,10 +470,11 @@ __global__ void k_attn_combine_q(const float* part_acc, const float* part_ml, in
 // ------------------------------------------------------------------------------------------------------
 // Routed experts, gated half. One block per 32 output rows of one pick (so the block can quantise its own
 // Q8_0 block of the result), plus one block per 32 rows of the shared expert's activation.
-// Warp 0 redoes the routing (softmax over all experts, top-k; src/model/qwen35.rs:1626-1638,
-// src/ops/mod.rs:1191-1216) while the others fetch the activation; then
+// Every block redoes the routing (softmax over all experts, top-k; src/model/qwen35.rs:1626-1638, src/ops/mod.rs:1191-1216) as far as it
+// needs it: the picks, from the softmax numerators, without the serial sum (with it and the weights in every block a layer took 0.6 us more);
+// the first block of the shared expert also forms the weights. Then
 // h = silu(gate_e . x * s_g) * (up_e . x * s_u) (src/ops/mod.rs:1105-1117) -> Q8_0.
-constexpr int MOE_CAND = 512;   // 32 groups x 16 picks at most (n_expert <= 1024, n_used <= 16)
+constexpr int MOE_CAND = 544;   // 32 groups x (16 picks and one more) at most (n_expert <= 1024, n_used <= 16)
 struct MoeGlu {
     const float* router; int n_expert, n_used;
     const int8_t* xq; const float* xs; int n_embd;
@@ -500,18 +504,18 @@ __device__ __forceinline__ void ep_wait_flag(const unsigned* flag, unsigned seq,
 }
 __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int32_t s_ids[16];
-    __shared__ float s_wts[16];
+    __shared__ int32_t s_ids[17];
+    __shared__ float s_val[17];
     __shared__ float s_gu[64];
     __shared__ float s_sum;
-    __shared__ float s_cand_p[MOE_CAND];        // the first n_used of every 32-group: probability and id
-    __shared__ int s_cand_i[MOE_CAND];
+    __shared__ __align__(16) unsigned long long s_cand[MOE_CAND];      // the first of every 32-group: value and id as one key
     const int n = p.n_embd, nb = n / 32, nsb = n / 16, ff = p.gate.n_out, upp = ff / 32;
     const int b = blockIdx.y, tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int unit = blockIdx.x, n_units = p.n_used * upp;
     TL(TLK_MOE_GLU, 0);
     pdl_wait(); pdl_trigger();
     TL(TLK_MOE_GLU, 1);
+    const bool writer = unit == n_units;          // of the picks and their weights, for the kernels after this one: not one of the blocks that go on to their rows
     if (unit >= n_units) {
         // shared expert: silu(gate) * up for 32 elements, quantised (src/model/qwen35.rs:1669-1678)
         if (wid == 0 && (p.shared_row < 0 || p.shared_row == b)) {
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
             p.sq[sb * p.sff + k] = q;
             if (lane == 0) p.ss[sb * (p.sff / 32) + (unit - n_units)] = dq;
         }
-        return;
+        if (!writer) return;
     }
     if (p.wait_flags) {
         if (tid == 0) ep_wait_flag(p.wait_flags + b, *p.wait_seq, p.err);
@@ -554,37 +558,13 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     }
     __syncthreads();
     TL(TLK_MOE_GLU, 2);
-    // softmax denominator: serial sum in index order (src/ops/naive.rs:362-376), one thread
-    if (tid == 0) {
-        float sum = 0.0f;
-#pragma unroll 1
-        for (int i0 = 0; i0 < p.n_expert; i0 += 32) {
-            float4 q[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) q[j] = *(const float4*)(probs + i0 + 4 * j);
-            const int lim = p.n_expert - i0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (4 * j < lim) sum += q[j].x;
-                if (4 * j + 1 < lim) sum += q[j].y;
-                if (4 * j + 2 < lim) sum += q[j].z;
-                if (4 * j + 3 < lim) sum += q[j].w;
-            }
-        }
-        s_sum = sum;
-    }
-    __syncthreads();
-    {
-        const float sum = s_sum;
-        for (int i = tid; i < p.n_expert; i += blockDim.x) probs[i] /= sum;
-    }
-    __syncthreads();
-    // top-k without serial rounds, in two stages of counting. An expert's place in an order is the number of experts
-    // that beat it: greater probability, or equal and lower id (src/ops/mod.rs:1191-1216 picks by strict '>' scanning
-    // ascending ids). Stage 1: every 32-group ranks itself by shuffles and keeps its first n_used; stage 2: those
-    // candidates (the overall picks are among them) are ranked against each other.
-    {
-        const int ng = (p.n_expert + 31) >> 5, nu = p.n_used;
+    // Top-k without serial rounds, in two stages of counting. An expert's place in an order is the number of experts that beat it:
+    // greater value, or equal and lower id (src/ops/mod.rs:1191-1216 picks by strict '>' scanning ascending ids) -- one compare of
+    // (value bits, ~id) keys, values being >= 0. Stage 1: every 32-group ranks itself by shuffles and keeps its first `keep`; stage 2: those
+    // candidates (the overall picks are among them) are ranked against each other, eight threads to a candidate.
+    const int ng = (p.n_expert + 31) >> 5, nu = p.n_used, keep = nu + 1;
+    auto select = [&] {
+        if (tid < 17) { s_ids[tid] = -1; s_val[tid] = -1.0f; }
         for (int g = wid; g < ng; g += (int)(blockDim.x >> 5)) {
             const int t = g * 32 + lane;
             const float v = t < p.n_expert ? probs[t] : -1.0f;
@@ -594,36 +574,65 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
                 const float q = __shfl_sync(0xffffffffu, v, j);
                 rank += (int)(q > v) | ((int)(q == v) & (int)(j < lane));   // bitwise: no branches
             }
-            if (rank < nu) { s_cand_p[g * nu + rank] = v; s_cand_i[g * nu + rank] = t < p.n_expert ? t : -1; }
+            if (rank < keep) s_cand[g * keep + rank] = t < p.n_expert ? ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)~t : 0ull;
         }
         __syncthreads();
-        const int cnt = ng * nu;
-        for (int c = tid; c < cnt; c += blockDim.x) {
-            const float v = s_cand_p[c];
-            const int id = s_cand_i[c];
-            if (id < 0) continue;
+        const int cnt = ng * keep;
+        for (int c0 = 0; c0 < cnt; c0 += (int)(blockDim.x >> 3)) {
+            const int c = c0 + (tid >> 3);
+            const unsigned long long key = c < cnt ? s_cand[c] : ~0ull;
             int rank = 0;
-#pragma unroll 8
-            for (int j = 0; j < cnt; ++j) {   // unrolled so the shared-memory reads run ahead of the compares
-                const float q = s_cand_p[j];
-                const int qi = s_cand_i[j];
-                rank += (int)(qi >= 0) & ((int)(q > v) | ((int)(q == v) & (int)(qi < id)));
+#pragma unroll 4
+            for (int j = tid & 7; j < cnt; j += 8) rank += (int)(s_cand[j] > key);
+            rank += __shfl_xor_sync(0xffffffffu, rank, 1); rank += __shfl_xor_sync(0xffffffffu, rank, 2); rank += __shfl_xor_sync(0xffffffffu, rank, 4);
+            if (c < cnt && key && (tid & 7) == 0 && rank < keep) { s_ids[rank] = (int)~(unsigned)key; s_val[rank] = __uint_as_float((unsigned)(key >> 32)); }
+        }
+        __syncthreads();
+    };
+    // The picks are by probability, and probabilities are the numerators over one sum: the same order, unless the division rounds two
+    // different numerators to one value. So the numerators are ranked without waiting for the sum (serial, in index order), and only where
+    // two neighbours among the picks and the first one after them are closer than that could be (or so small that quotients lose bits) are the probabilities ranked
+    // instead. The weights, which need the sum, are one block's work beside the others' rows.
+    select();
+    const float va = lane < nu ? s_val[lane] : 0.0f, vb = lane < nu ? s_val[lane + 1] : 0.0f;
+    const bool close = __any_sync(0xffffffffu, lane < nu && va != vb && (va - vb <= va * 4.8e-7f || va < 1e-30f));      // the same in every warp
+    if (close || writer) {
+        // softmax denominator: serial sum in index order (src/ops/naive.rs:362-376), one thread
+        if (tid == 0) {
+            float sum = 0.0f;
+#pragma unroll 1
+            for (int i0 = 0; i0 < p.n_expert; i0 += 32) {
+                float4 q[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) q[j] = *(const float4*)(probs + i0 + 4 * j);
+                const int lim = p.n_expert - i0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (4 * j < lim) sum += q[j].x;
+                    if (4 * j + 1 < lim) sum += q[j].y;
+                    if (4 * j + 2 < lim) sum += q[j].z;
+                    if (4 * j + 3 < lim) sum += q[j].w;
+                }
             }
-            if (rank < nu) { s_ids[rank] = id; s_wts[rank] = v; }
+            s_sum = sum;
+        }
+        __syncthreads();
+        {
+            const float sum = s_sum;
+            for (int i = tid; i < p.n_expert; i += blockDim.x) probs[i] /= sum;
+        }
+        __syncthreads();
+        if (close) select();
+        if (writer) {
+            if (tid == 0) {
+                float sum = 0.0f;
+                for (int r = 0; r < nu; ++r) sum += s_ids[r] >= 0 ? probs[s_ids[r]] : 0.0f;      // summed in pick order (src/ops/mod.rs:1211)
+                const float denom = fmaxf(sum, 6.103515625e-5f);
+                for (int r = 0; r < nu; ++r) { p.ids_out[(size_t)b * nu + r] = s_ids[r]; p.w_out[(size_t)b * nu + r] = s_ids[r] >= 0 ? probs[s_ids[r]] / denom : 0.0f; }
+            }
+            return;
         }
     }
-    __syncthreads();
-    if (tid == 0) {
-        float sum = 0.0f;
-        for (int r = 0; r < p.n_used; ++r) sum += s_wts[r];                 // summed in pick order (src/ops/mod.rs:1211)
-        const float denom = fmaxf(sum, 6.103515625e-5f);
-        for (int r = 0; r < p.n_used; ++r) {
-            const float w = s_wts[r] / denom;
-            s_wts[r] = w;
-            if (unit == 0) { p.ids_out[(size_t)b * p.n_used + r] = s_ids[r]; p.w_out[(size_t)b * p.n_used + r] = w; }
-        }
-    }
-    __syncthreads();
     TL(TLK_MOE_GLU, 3);
     const int pick = unit / upp, row0 = (unit % upp) * 32;
     const int el = s_ids[pick] - p.gate.expert_lo;

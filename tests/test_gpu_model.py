@@ -114,6 +114,42 @@ def test_loaded_tensors_equal_generated_tensors(oracle, gpu):
     e1.close(); e2.close(); m2.close()
 
 
+@pytest.mark.parametrize("rows", ["zero", "pairs", "one_ulp_apart", "far"])
+def test_one_token_routing_where_probabilities_tie(oracle, gpu, rows):
+    """The one-token step ranks softmax numerators and looks at probabilities only where a division could have made two of them one:
+    experts with equal logits, in equal pairs, an ulp apart, and so far apart that most numerators are zero are picked and weighted
+    as the multi-row pass picks them (which ranks probabilities)."""
+    from inferred_thoughts_b200 import host
+    ops, _ = gpu
+    m = host.Model(ops, host_dims(TINY))
+    for sp in oracle.specs:
+        data, sc = oracle.tensor(sp["name"])
+        if sp["name"].endswith("ffn_gate_inp.weight"):
+            w = data.view(np.float32).reshape(TINY["n_expert"], TINY["n_embd"]).copy()
+            if rows == "zero":
+                w[:] = 0
+            elif rows == "far":
+                w *= 400
+            else:
+                w[1::2] = w[0::2]
+                if rows == "one_ulp_apart":
+                    w[1::2, 7] = np.nextafter(w[1::2, 7], np.float32(1e9))
+            data = np.ascontiguousarray(w).reshape(-1).view(np.uint8)
+        m.set_tensor(sp["name"], sp["ty"], data, sc)
+    prompt = prompt_ids(4, 12, TINY["n_vocab"])
+    a, b = host.Engine(m, 64, 1), host.Engine(m, 64, 1)
+    L, K = TINY["n_layer"], TINY["n_expert_used"]
+    for n in range(2, 12):
+        a.reset(); b.reset()
+        a.prefill(prompt[:n - 1])
+        step, _ = a.decode([prompt[n - 1]])
+        rows_ = b.prefill(prompt[:n])
+        assert a.read_routes(L, K)[:, 0].tolist() == b.read_routes(L, K)[:, 0].tolist(), n
+        assert step.reshape(-1).view(np.uint32).tolist() == rows_.reshape(-1).view(np.uint32).tolist(), n
+    ops.check()
+    a.close(); b.close(); m.close()
+
+
 def test_batch_of_sequences_equals_single_sequences(oracle, gpu):
     """Three sequences in one engine (multi-row passes: int8-MMA matmuls, per-sequence state and KV) give the bits the
     same sequences give alone, through prefill and through decode steps."""
