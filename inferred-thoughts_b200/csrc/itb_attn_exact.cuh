@@ -108,12 +108,55 @@ __device__ __forceinline__ float serial_sum(const float* w, int n) {
     }
     return sum;
 }
+// The same sum, of terms >= 0, when there are many: a warp folds 32 segments at once, each from a guess of the sum before it, and again from
+// better guesses until every segment began where the one before it ended. Then the whole is the left fold from zero, rounding for
+// rounding, however the guesses were made: segment 0 begins at zero, and a segment that begins exactly ends exactly. Each round makes at
+// least one more segment begin exactly (its correction is made of exact zeros), so 32 rounds always do; with terms of one sign the sum's grid
+// seldom coarsens and 5 to 6 do (12 at most in 10^4 softmax rows of 300 to 6,500 terms; terms of both signs take 17, too many). A
+// round is n / 32 adds and two scans: below 640 terms the plain chain is as fast. 6,500 terms: 28,000 cycles of adds -> 8,000; four steps at
+// 6,500 positions 11.80 -> 11.37 ms.
+constexpr int AX_FOLD_MIN = 640;
+__device__ __forceinline__ float fold_sum(const float* w, int n) {
+    if (n < AX_FOLD_MIN) return serial_sum(w, n);
+    const int lane = threadIdx.x & 31, len = ((n + 31) / 32) | 1, lo = lane * len, cnt = min(len, n - lo);      // odd: the lanes' reads fall on distinct banks
+    auto fold = [&](float sum) {
+        const float* t = w + min(lo, n - 1);
+        int i = 0;
+#pragma unroll 1
+        for (; i + 8 <= cnt; i += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = t[i + k];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) sum = __fadd_rn(sum, v[k]);
+        }
+        for (; i < cnt; ++i) sum = __fadd_rn(sum, t[i]);
+        return sum;
+    };
+    auto before = [&](float v) {                     // the sum of the lanes before this one's, by a tree
+        float inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += u; }
+        const float ex = __shfl_up_sync(0xffffffffu, inc, 1);
+        return lane ? ex : 0.0f;
+    };
+    float start = before(fold(0.0f)), end = 0.0f;
+#pragma unroll 1
+    for (int round = 0; round < 32; ++round) {
+        end = fold(start);
+        float left = __shfl_up_sync(0xffffffffu, end, 1);
+        if (lane == 0) left = 0.0f;
+        if (__all_sync(0xffffffffu, left == start)) break;
+        start = left + before(left - start);
+    }
+    return __shfl_sync(0xffffffffu, end, 31);
+}
 // Softmax of one (row, head)'s scores and the weighted sum of the values for 32 dimensions of that head.
 // grid (hd / 32, n_head, rows); block 288: everyone on the maximum, exponentials and divisions, warp 0 on the serial sums: of the
 // exponentials, then of the weighted values, a lane per dimension. Those two chains (n_pos adds of 4 cycles each) bound the kernel, so
 // the chain warp does nothing else: the other eight multiply a tile of AX_VT positions at a time into shared memory, a line per
 // dimension, one tile ahead of it and with the values of AX_AHEAD tiles in flight. With the chain warp converting and multiplying
-// too, and the sum read as it went, 6,500 positions took 124 us; now 46 (the chains alone: 31).
+// too, and the sum read as it went, 6,500 positions took 124 us; with both chains serial 46 (31 of them the chains), now 35.
 // gate != null: times sigmoid(gate) (src/model/qwen35.rs:1216-1218); out_q != null: the result leaves quantised to Q8_0 (the
 // output projection's own quantisation), else as f32 in out.
 // READY (the scores already hold the softmax weights: many rows, where the blocks that share a head would each redo the softmax): no
@@ -189,7 +232,7 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
         for (int s = tid; s < ax_pad(n_pos); s += 288) w[s] = s < n_pos ? exp_f(w[s] - mx) : 0.0f;
         __syncthreads();
         if (wid == 0) {                                               // the sum in position order
-            const float sum = serial_sum(w, n_pos);
+            const float sum = fold_sum(w, n_pos);
             if (lane == 0) s_sum = sum;
         }
         __syncthreads();
@@ -256,7 +299,7 @@ __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
     for (int s = tid; s < ax_pad(n_pos); s += 256) w[s] = s < n_pos ? exp_f(w[s] - mx) : 0.0f;
     __syncthreads();
     if (wid == 0) {
-        const float sum = serial_sum(w, n_pos);
+        const float sum = fold_sum(w, n_pos);
         if (lane == 0) s_sum = sum;
     }
     __syncthreads();

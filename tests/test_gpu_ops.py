@@ -572,6 +572,24 @@ def test_attend_in_exact_mode_equals_the_cpu_path_bit_for_bit(hd, nh, nkv, n_pos
     ops.close()
 
 
+@pytest.mark.parametrize("n_pos,n_q,spread", [(639, 1, 1.0), (640, 1, 1.0), (641, 9, 0.1), (1009, 1, 30.0), (4100, 1, 0.0), (4100, 2, 1.0), (2049, 9, 8.0)])
+def test_attend_exact_with_the_softmax_sum_folded_in_segments(n_pos, n_q, spread):
+    """From 640 positions on the sum of the exponentials is folded in 32 segments until they meet: around that length, with as many
+    terms in every segment as not, scores all equal, close together and far apart (most exponentials zero)."""
+    from inferred_thoughts_b200 import host
+    ops = host.B200Ops(0, "exact=1")
+    hd, nh, nkv = 64, 4, 2
+    kvd = hd * nkv
+    q = noise(n_q * nh * hd, 270, spread)
+    ks = noise(n_pos * kvd, 271).astype(np.float16).view(np.uint16); vs = noise(n_pos * kvd, 272).astype(np.float16).view(np.uint16)
+    want = np.zeros(n_q * nh * hd, np.float32); got = np.zeros_like(want)
+    L.orc_attend(q, q.size, ks, vs, kvd, n_pos, hd, nh, nkv, np.float32(0.125), 0, want)
+    ops.begin_pass(n_q)
+    ops.attend(q, ks, vs, kvd, n_pos, hd, nh, nkv, 0.125, got); ops.host_needs(got); ops.check()
+    assert got.view(np.uint32).tolist() == want.view(np.uint32).tolist()
+    ops.close()
+
+
 @pytest.mark.parametrize("hd,nh,nkv,n_pos,n_q,kv", [(64, 6, 2, 65, 11, "f16"), (128, 8, 1, 131, 131, "bf16"), (256, 16, 2, 200, 33, "f16"), (128, 32, 16, 600, 580, "bf16")])
 def test_attend_of_many_rows_equals_the_cpu_path_bit_for_bit(hd, nh, nkv, n_pos, n_q, kv):
     """The tiled form: head groups that do not divide a tile, a last tile of few tokens, rows from the first position on, and enough
