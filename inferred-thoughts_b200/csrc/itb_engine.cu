@@ -1199,7 +1199,8 @@ static void ep_p2p_setup(itb_engine* e) {
     }
 }
 
-static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_tok, const int32_t* tok_rows) {
+// head: the pass's last rows go through the LM head (all passes of a prompt but its last have no use for it).
+static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_tok, const int32_t* tok_rows, bool head = true) {
     itb_model* m = e->m; itb_ctx* c = e->c;
     const itb_model_dims& d = m->d;
     const int R = n_seq * n_tok, H = d.n_embd, sms = c->sm_count;
@@ -1557,6 +1558,10 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             const size_t total = (size_t)R * H;
             launch_k(chain && !two, k_moe_finish_rows, (unsigned)((total + 255) / 256), 256, 0, st, e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
         }
+    }
+    if (!head) {
+        itb_chain(k_advance_pos, (n_seq + 127) / 128, 128, 0, st, e->pos, n_seq, n_tok);
+        return launches + 1;
     }
     // LM head on each sequence's last row
     const float* xl = e->x;
@@ -2240,7 +2245,7 @@ extern "C" int itb_engine_prefill(itb_engine* e, const uint32_t* tokens, size_t 
             cudaMemcpyAsync(e->tokens, e->prompt + off, e->B * 4, cudaMemcpyDeviceToDevice, st);
             if (!run_steps(e, 1, false)) return 1;
         } else {
-            c->launches += enqueue_rows(e, st, (int)e->B, (int)nt, e->prompt + off);
+            c->launches += enqueue_rows(e, st, (int)e->B, (int)nt, e->prompt + off, t0 + nt == n);
             if (!c->error.empty()) { ep_abort(e); return 1; }
             e->last_n_tok = (uint32_t)nt;
             for (uint32_t b = 0; b < e->B; ++b) e->host_pos[b] += (uint32_t)nt;
