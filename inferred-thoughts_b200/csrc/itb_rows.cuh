@@ -120,18 +120,19 @@ static void f32_tree(cudaStream_t st, int sms, const DevF32& w, const float* x, 
 // gate, or alpha and beta -- each alone is a handful of blocks walking a 2,048-long chain.
 // grid (ceil(n_out / TO), ceil(n_rows / TR), 1 or 2), block (TO / MO) * (TR / MR); n_in a multiple of KT.
 // What bounds the shapes: 8 x 8, a chain to a thread, the chain itself: 4 cycles a step, and with up to four such blocks an SM a
-// scheduler has the slots for its warps' reads, products and sums between them; the larger ones the f32 pipe and the reads.
+// scheduler has the slots for its warps' reads, products and sums between them. The others shared memory: a warp's 16-byte read takes four
+// of its cycles, the same data for several lanes or not, so four k of MO x MR chains are 4 (MO + MR) of those against MO MR operations
+// (fused; twice that unfused) of a scheduler's; and the barrier of a tile, so tiles are 64 k or more. The next four k are read under this four's operations.
 template <bool FUSED, int TO, int TR, int MO, int MR, int KT, int NST>
 __global__ void __launch_bounds__((TO / MO) * (TR / MR)) k_sgemm_chain(DevF32 w0, const float* __restrict__ x, int n_rows, float* out0, DevF32 w1 = DevF32{}, float* out1 = nullptr) {
-    pdl_wait();
-    constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, NT = NX * NY, PIECES = (TO + TR) * (KT / 4) / NT;      // a thread per MO x MR outputs
-    static_assert((TO + TR) * (KT / 4) % NT == 0, "whole pieces");
+    constexpr int ST = KT + 4, NX = TO / MO, NY = TR / MR, NT = NX * NY, PIECES = (TO + TR) * (KT / 4) / NT, W_PIECES = TO * (KT / 4) / NT;      // a thread per MO x MR outputs
+    static_assert((TO + TR) * (KT / 4) % NT == 0 && TO * (KT / 4) % NT == 0, "whole pieces");
     extern __shared__ __align__(16) unsigned char smem[];
     float* ring = (float*)smem;                    // [stage][TO weight lines | TR activation lines][ST]
     const DevF32 w = blockIdx.z ? w1 : w0;
     float* out = blockIdx.z ? out1 : out0;
     const int o0 = blockIdx.x * TO, r0 = blockIdx.y * TR, n = w.n_in, nk = n / KT;
-    if (o0 >= w.n_out) return;
+    if (o0 >= w.n_out) { pdl_wait(); return; }
     const int tx = threadIdx.x % NX, ty = threadIdx.x / NX;
     const float* src[PIECES];
 #pragma unroll
@@ -139,52 +140,63 @@ __global__ void __launch_bounds__((TO / MO) * (TR / MR)) k_sgemm_chain(DevF32 w0
         const int c = threadIdx.x + NT * i, line = c / (KT / 4), k4 = (c % (KT / 4)) * 4;
         src[i] = (line < TO ? w.w + (size_t)min(o0 + line, w.n_out - 1) * n : x + (size_t)min(r0 + line - TO, n_rows - 1) * n) + k4;
     }
-    auto fetch = [&](int t) {
-        if (t < nk) {
-            float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
+    auto fetch = [&](int t, int from, int to) {
+        float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
 #pragma unroll
-            for (int i = 0; i < PIECES; ++i) {
-                const int c = threadIdx.x + NT * i;
-                cp_async16(st + (c / (KT / 4)) * ST + (c % (KT / 4)) * 4, src[i] + (size_t)t * KT, true);
+        for (int i = 0; i < PIECES; ++i) {
+            const int c = threadIdx.x + NT * i;
+            if (i >= from && i < to) cp_async16(st + (c / (KT / 4)) * ST + (c % (KT / 4)) * 4, src[i] + (size_t)t * KT, true);
+        }
+    };
+    // the weights of the first stages are requested before the rows they will meet are there
+    for (int t = 0; t < NST - 1; ++t) if (t < nk) fetch(t, 0, W_PIECES);
+    pdl_wait();
+    for (int t = 0; t < NST - 1; ++t) { if (t < nk) fetch(t, W_PIECES, PIECES); cp_async_commit(); }
+    // ML of the thread's MO outputs exist: where a matrix has no more than one per thread (the shared expert's gate), the others are not walked
+    auto walk = [&](auto live) {
+        constexpr int ML = decltype(live)::value;
+        float acc[MR][ML];
+#pragma unroll
+        for (int i = 0; i < MR; ++i)
+#pragma unroll
+            for (int j = 0; j < ML; ++j) acc[i][j] = 0.0f;
+        for (int t = 0; t < nk; ++t) {
+            cp_async_wait<NST - 2>();
+            __syncthreads();                       // tile t has landed for everyone; everyone is done with tile t - 1
+            if (t + NST - 1 < nk) fetch(t + NST - 1, 0, PIECES);      // into the slot tile t - 1 used
+            cp_async_commit();
+            const float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
+            const float* wr = st + tx * ST; const float* xr = st + (TO + ty) * ST;
+            float4 a[2][ML], c[2][MR];
+            auto read = [&](int kk, float4 (&a)[ML], float4 (&c)[MR]) {
+#pragma unroll
+                for (int j = 0; j < ML; ++j) a[j] = *(const float4*)(wr + j * NX * ST + kk);
+#pragma unroll
+                for (int i = 0; i < MR; ++i) c[i] = *(const float4*)(xr + i * NY * ST + kk);
+            };
+            read(0, a[0], c[0]);
+#pragma unroll(ML * MR <= 8 ? KT / 4 : 4)
+            for (int kk = 0; kk < KT; kk += 4) {
+                const int u = (kk >> 2) & 1;
+                if (kk + 4 < KT) read(kk + 4, a[u ^ 1], c[u ^ 1]);
+                auto step = [&](auto get) {
+#pragma unroll
+                    for (int i = 0; i < MR; ++i)
+#pragma unroll
+                        for (int j = 0; j < ML; ++j) acc[i][j] = FUSED ? fmaf(get(a[u][j]), get(c[u][i]), acc[i][j]) : __fadd_rn(acc[i][j], __fmul_rn(get(a[u][j]), get(c[u][i])));
+                };
+                step([](const float4& v) { return v.x; }); step([](const float4& v) { return v.y; });
+                step([](const float4& v) { return v.z; }); step([](const float4& v) { return v.w; });
             }
         }
-        cp_async_commit();
+        cp_async_wait<0>();
+#pragma unroll
+        for (int i = 0; i < MR; ++i)
+#pragma unroll
+            for (int j = 0; j < ML; ++j)
+                if (r0 + ty + i * NY < n_rows && o0 + tx + j * NX < w.n_out) out[(size_t)(r0 + ty + i * NY) * w.n_out + o0 + tx + j * NX] = acc[i][j];
     };
-    for (int t = 0; t < NST - 1; ++t) fetch(t);
-    float acc[MR][MO];
-#pragma unroll
-    for (int i = 0; i < MR; ++i)
-#pragma unroll
-        for (int j = 0; j < MO; ++j) acc[i][j] = 0.0f;
-    for (int t = 0; t < nk; ++t) {
-        cp_async_wait<NST - 2>();
-        __syncthreads();                           // tile t has landed for everyone; everyone is done with tile t - 1
-        fetch(t + NST - 1);                        // into the slot tile t - 1 used
-        const float* st = ring + (size_t)(t % NST) * (TO + TR) * ST;
-        const float* wr = st + tx * ST; const float* xr = st + (TO + ty) * ST;
-#pragma unroll(MO * MR <= 2 ? KT / 4 : 4)
-        for (int kk = 0; kk < KT; kk += 4) {
-            float4 a[MO], c[MR];
-#pragma unroll
-            for (int j = 0; j < MO; ++j) a[j] = *(const float4*)(wr + j * NX * ST + kk);
-#pragma unroll
-            for (int i = 0; i < MR; ++i) c[i] = *(const float4*)(xr + i * NY * ST + kk);
-            auto step = [&](float (&acc)[MR][MO], auto get) {
-#pragma unroll
-                for (int i = 0; i < MR; ++i)
-#pragma unroll
-                    for (int j = 0; j < MO; ++j) acc[i][j] = FUSED ? fmaf(get(a[j]), get(c[i]), acc[i][j]) : __fadd_rn(acc[i][j], __fmul_rn(get(a[j]), get(c[i])));
-            };
-            step(acc, [](const float4& v) { return v.x; }); step(acc, [](const float4& v) { return v.y; });
-            step(acc, [](const float4& v) { return v.z; }); step(acc, [](const float4& v) { return v.w; });
-        }
-    }
-    cp_async_wait<0>();
-#pragma unroll
-    for (int i = 0; i < MR; ++i)
-#pragma unroll
-        for (int j = 0; j < MO; ++j)
-            if (r0 + ty + i * NY < n_rows && o0 + tx + j * NX < w.n_out) out[(size_t)(r0 + ty + i * NY) * w.n_out + o0 + tx + j * NX] = acc[i][j];
+    if (MO > 1 && w.n_out - o0 <= NX) walk(std::integral_constant<int, 1>{}); else walk(std::integral_constant<int, MO>{});
 }
 constexpr int SG_KT = 64;
 inline bool sgemm_chain_ok(int n_in) { return n_in % SG_KT == 0; }
@@ -194,17 +206,23 @@ static void sgemm_tiles(cudaStream_t st, int n_out, int nz, const DevF32& wa, co
     itb_raise_smem(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, smem);
     itb_chain(k_sgemm_chain<FUSED, TO, TR, MO, MR, KT, NST>, dim3((n_out + TO - 1) / TO, (n_rows + TR - 1) / TR, nz), (TO / MO) * (TR / MR), smem, st, wa, x, n_rows, oa, wb, ob);
 }
-// One matrix, or two over the same rows. 8 x 8, a chain to a thread, is fastest as long as an SM has no more than four such blocks (32 rows
-// of 257 outputs, 2,048 k: 11.8 us, at 16 x 16 18.5), but it reads every line once per 8 of the others. Large passes: unfused, where a
-// step is two operations, 2 x 2 chains and twice the warps (2,048 rows: 145 us, at 4 x 4 173); fused, fewer reads (119, at 2 x 2 149).
+// One matrix, or two over the same rows. 8 x 8, a chain to a thread, is fastest as long as an SM has no more than four such blocks, but it
+// reads every line once per 8 of the others; beyond that, of the tiles that read less the largest of which every SM still gets three or four.
+// Measured (us, 257 outputs, 2,048 k; in parentheses the next best): 32 rows 8 x 8 11.4 (16 x 16 18.5); 256 rows 16 x 16 with 2 x 2 chains to a
+// thread 30.1 (1 x 2 33.4); 512 rows the same 38.0 (43.0); 1,024 rows 16 x 32 with 2 x 2 59.9 (16 x 16 69.3, 32 x 32 90); 2,048 rows 32 x 32
+// with 2 x 4 99.4 (16 x 32 116, 64 x 64 with 4 x 4 111; 32 x 32 with 2 x 2 and tiles of 32 k 145). Fused, 512 rows 16 x 32 with 2 x 4 42.6 (32 x 64
+// 49.4), 2,048 rows 32 x 64 with 4 x 4 79.7 (64 x 64 with 4 x 4 88.9; tiles of 32 k 116).
 template <bool FUSED>
 static void sgemm_chain(cudaStream_t st, int sms, const DevF32& wa, const float* x, int n_rows, float* oa, const DevF32& wb = DevF32{}, float* ob = nullptr) {
     const int n_out = std::max(wa.n_out, wb.w ? wb.n_out : 0), nz = wb.w ? 2 : 1, n_all = wa.n_out + (wb.w ? wb.n_out : 0);
     auto blocks = [&](int to, int tr) { return (long long)((n_all + to - 1) / to) * ((n_rows + tr - 1) / tr); };
-    if (blocks(8, 8) <= 4 * sms) sgemm_tiles<FUSED, 8, 8, 1, 1, 64, 8>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
-    else if (FUSED && blocks(32, 64) >= sms) sgemm_tiles<FUSED, 32, 64, 4, 4, 32, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
-    else if (!FUSED && blocks(32, 32) >= 2 * sms) sgemm_tiles<FUSED, 32, 32, 2, 2, 32, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
-    else sgemm_tiles<FUSED, 16, 16, 1, 2, 64, 6>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    if (blocks(8, 8) <= 4 * sms && wa.n_in % 128 == 0) sgemm_tiles<FUSED, 8, 8, 1, 1, 128, 5>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (blocks(8, 8) <= 4 * sms) sgemm_tiles<FUSED, 8, 8, 1, 1, 64, 8>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (FUSED && 2 * blocks(32, 64) >= 3 * sms) sgemm_tiles<FUSED, 32, 64, 4, 4, 64, 3>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (FUSED) sgemm_tiles<FUSED, 16, 32, 2, 4, 64, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (2 * blocks(32, 32) >= 7 * sms) sgemm_tiles<FUSED, 32, 32, 2, 4, 64, 3>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else if (2 * blocks(16, 32) >= 7 * sms) sgemm_tiles<FUSED, 16, 32, 2, 2, 64, 4>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
+    else sgemm_tiles<FUSED, 16, 16, 2, 2, 64, 6>(st, n_out, nz, wa, x, n_rows, oa, wb, ob);
 }
 
 // A dense Q8_0 matrix against n_rows >= 1 quantised rows: out[row][n_out] = or += (mode). tc: the tensor-core forms the context's
