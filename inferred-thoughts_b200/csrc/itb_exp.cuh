@@ -301,17 +301,10 @@ static inline void exp_run(ExpArgs a, bool glu, int max_tiles, int cap, cudaStre
     else { if (glu) exp_launch<8, true>(a, max_tiles, st); else exp_launch<8, false>(a, max_tiles, st); }
 }
 
-// Q8_0 quantisation of f32 rows as the kernels above read them: f16 values permuted inside blocks, block scales (block per row).
-__global__ void k_quant_rows_h(const float* x, int n, __half* xh, float* xs) {
+// Q8_0 quantisation of f32 rows as the kernels above read them: f16 values permuted inside blocks, block scales.
+__global__ void __launch_bounds__(256) k_quant_rows_h(const float* x, size_t n_blocks, __half* xh, float* xs) {
     pdl_wait();
-    const size_t r = blockIdx.x;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int b = wid; b < n / 32; b += nw) {
-        float d;
-        const int8_t q = warp_quant_q8(x[r * n + b * 32 + lane], &d);
-        xh[r * n + b * 32 + exp_pos(lane)] = __int2half_rn((int)q);
-        if (lane == 0) xs[r * (n / 32) + b] = d;
-    }
+    quant_blocks(x, n_blocks, xs, [&](size_t, size_t b, int lane, int8_t q) { xh[b * 32 + exp_pos(lane)] = __int2half_rn((int)q); });
 }
 // int8 rows (already quantised) to the same form; a thread per 16 bytes.
 __global__ void k_q8_to_h(const int8_t* xq, size_t n16, __half* xh) {

@@ -81,12 +81,34 @@ __global__ void k_l2_norm_heads(float* x, size_t n_heads, int hd, float eps) {
 }
 
 // Row softmax, warp per row: max, exp, serial-order-free sum (tolerance class: expf) (src/ops/naive.rs:362-376).
-__global__ void k_softmax_rows(float* x, size_t n_rows, int row) {
+constexpr size_t SOFTMAX_STAGED = 1024;      // rows up to this long go through shared memory, where the serial sum reads ahead of its adds
+__global__ void __launch_bounds__(256) k_softmax_rows(float* x, size_t n_rows, int row) {
     pdl_wait();
+    extern __shared__ __align__(16) unsigned char smem[];
     size_t r = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= n_rows) return;
     int lane = threadIdx.x & 31;
     float* p = x + r * row;
+    if (row <= (int)SOFTMAX_STAGED) {
+        const int n32 = (row + 31) & ~31;
+        float* w = (float*)smem + (threadIdx.x >> 5) * n32;
+        float mx = -INFINITY;
+        for (int i = lane; i < row; i += 32) { const float v = p[i]; w[i] = v; mx = fmaxf(mx, v); }
+        mx = warp_max(mx);
+        for (int i = lane; i < n32; i += 32) w[i] = i < row ? exp_f(w[i] - mx) : 0.0f;      // behind the end: terms that change no sum
+        __syncwarp();
+        float sum = 0.0f;
+#pragma unroll 1
+        for (int i = 0; i < n32; i += 32) {
+            float4 a[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[j] = *(const float4*)(w + i + 4 * j);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { sum += a[j].x; sum += a[j].y; sum += a[j].z; sum += a[j].w; }
+        }
+        for (int i = lane; i < row; i += 32) p[i] = w[i] / sum;
+        return;
+    }
     float mx = -INFINITY;
     for (int i = lane; i < row; i += 32) mx = fmaxf(mx, p[i]);
     mx = warp_max(mx);
@@ -283,18 +305,37 @@ __global__ void k_moe_finish(float* out, size_t at, int n, const float* rows, co
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_tok * n) return;
     size_t t = i / n; int j = (int)(i % n);
-    float g = sigmoid_f(logit[logit_at + t]);
+    const float lg = logit[logit_at + t], sh = shared[t * n + j];
     float v = 0.0f;
-    for (int e = 0; e < n_used; ++e) v += wts[t * n_used + e] * rows[(t * n_used + e) * n + j];
-    v += shared[t * n + j] * g;
+    for (int e0 = 0; e0 < n_used; e0 += 8) {         // eight picks' loads in flight, and the exponential under the first eight's
+        float wv[8], rv[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e0 + e < n_used) { wv[e] = wts[t * n_used + e0 + e]; rv[e] = rows[(t * n_used + e0 + e) * n + j]; }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (e0 + e < n_used) v += wv[e] * rv[e];
+    }
+    v += sh * sigmoid_f(lg);
     out[at + t * n + j] = v;
 }
 
-// Q8_0 activation quantiser, block per row of n_in (src/ops/naive.rs:653-675).
-__global__ void k_quant_q8(const float* x, int n_in, int8_t* xq, float* xs) {
+// Q8_0 activation quantiser over whole rows, which are blocks of 32 one after the other (src/ops/naive.rs:653-675): a warp per block, so that one
+// row is spread over many SMs (a row to a thread block had a warp quantise eight blocks of 32 one after the other).
+__host__ inline unsigned quant_grid(size_t n_blocks, int sms) { return (unsigned)std::min<size_t>((n_blocks + 7) / 8, (size_t)16 * sms); }
+template <class Put>
+__device__ __forceinline__ void quant_blocks(const float* x, size_t n_blocks, float* xs, Put put) {
+    const int lane = threadIdx.x & 31;
+    for (size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); b < n_blocks; b += (size_t)gridDim.x * 8) {
+        float d;
+        const int8_t q = warp_quant_q8(x[b * 32 + lane], &d);
+        put(b * 32 + lane, b, lane, q);
+        if (lane == 0) xs[b] = d;
+    }
+}
+__global__ void __launch_bounds__(256) k_quant_q8(const float* x, size_t n_blocks, int8_t* xq, float* xs) {
     pdl_wait();
-    size_t t = blockIdx.x;
-    block_quant_q8(x + t * n_in, n_in, xq + t * n_in, xs + t * (n_in / 32));
+    quant_blocks(x, n_blocks, xs, [&](size_t i, size_t, int, int8_t q) { xq[i] = q; });
 }
 
 // ---- op-level matmuls: grid (row blocks, tokens or pairs) ----

@@ -101,7 +101,7 @@ extern "C" void itb_softmax(itb_ctx* c, float* x, size_t len, size_t row) {
     if (len % row) { itb_fail_msg(c, "softmax: x is not whole rows"); return; }
     float* xd = itb_mirror_inout(c, x, len);
     if (!xd) return;
-    itb_chain(k_softmax_rows, blocks_for(len / row, 8), 256, 0, c->stream, xd, len / row, (int)row);
+    itb_chain(k_softmax_rows, blocks_for(len / row, 8), 256, row <= SOFTMAX_STAGED ? (size_t)8 * ((row + 31) & ~(size_t)31) * 4 : 0, c->stream, xd, len / row, (int)row);
     ITB_LAUNCHED(c);
 }
 extern "C" void itb_rope_neox(itb_ctx* c, float* x, size_t len, size_t pos, size_t head_dim, size_t n_rot, size_t n_heads, float theta) {
@@ -187,7 +187,7 @@ extern "C" void itb_delta_rule(itb_ctx* c, const itb_delta* d, float* state, siz
 // Into the context's buffer, over what the call before left there. False: out of memory.
 static bool quantize_rows(itb_ctx* c, const float* xd, size_t n_rows, size_t n_in, QRows* rows) {
     if (!itb_ensure_xq(c, n_rows * n_in)) return false;
-    itb_chain(k_quant_q8, (unsigned)n_rows, 256, 0, c->stream, xd, (int)n_in, c->xq, c->xs);
+    itb_chain(k_quant_q8, quant_grid(n_rows * (n_in / 32), c->sm_count), 256, 0, c->stream, xd, n_rows * (n_in / 32), c->xq, c->xs);
     ITB_LAUNCHED(c);
     *rows = c->quantised(c->xq, c->xs);
     return true;
@@ -314,6 +314,15 @@ extern "C" void itb_matmul_pair(itb_ctx* c, const itb_weights* a, const itb_weig
     const float* xd = itb_mirror_in(c, x, x_len);
     float* oa = itb_mirror_out(c, out_a, out_a_len); float* ob = itb_mirror_out(c, out_b, out_b_len);
     if (!xd || !oa || !ob) return;
+    const bool f32 = a->ggml_type != ITB_Q8_0 && a->ggml_type != ITB_NVFP4 && b->ggml_type != ITB_Q8_0 && b->ggml_type != ITB_NVFP4;
+    if (f32 && c->exact && sgemm_chain_ok((int)a->n_in)) {       // the chains of both side by side: one launch, not one after the other
+        const WeightEntry* wa = itb_weight(c, a->data, a->bytes, a->ggml_type, a->n_in, a->n_out, 1, nullptr, 0);
+        const WeightEntry* wb = wa ? itb_weight(c, b->data, b->bytes, b->ggml_type, b->n_in, b->n_out, 1, nullptr, 0) : nullptr;
+        if (!wb) return;
+        sgemm_chain<false>(c->stream, c->sm_count, DevF32{(const float*)wa->a, (int)wa->n_in, (int)wa->n_out}, xd, (int)nt, oa, DevF32{(const float*)wb->a, (int)wb->n_in, (int)wb->n_out}, ob);
+        ITB_LAUNCHED(c);
+        return;
+    }
     QRows rows;
     matmul_dev(c, a, xd, nt, oa, &rows);
     if (!c->error.empty()) return;
@@ -373,7 +382,7 @@ static bool experts_grouped(itb_ctx* c, const itb_experts* g, const itb_experts*
     const int E = (int)g->n_expert, cap = exp_tile_cap((int)n_pairs, E, (int)(u ? g->n_out : g->n_out / 2), c->sm_count);
     if (!itb_ensure_xq(c, rows * k * 2) || !group_pairs(c, c->route_ids, n_pairs, g->n_expert, cap)) return true;
     __half* xh = (__half*)c->xq;
-    itb_chain(k_quant_rows_h, (unsigned)rows, 256, 0, c->stream, xd, (int)k, xh, c->xs);
+    itb_chain(k_quant_rows_h, quant_grid(rows * (k / 32), c->sm_count), 256, 0, c->stream, xd, rows * (k / 32), xh, c->xs);
     ITB_LAUNCHED(c);
     ExpArgs a{};
     a.wa = DevFp4{(const uint8_t*)wg->a, (const uint8_t*)wg->b, wg->scale2, (int)wg->n_in, (int)wg->n_out, (int)wg->n_expert, 0};
