@@ -31,9 +31,9 @@ template <int NJ> struct ExpCfg {
     static constexpr int OFF_S = EX_WROWS * EX_KC / 2;
     static constexpr int OFF_X = OFF_S + EX_WROWS * (EX_KC / 16);
     static constexpr int STAGE = OFF_X + TOK * EX_XSTR;
-    static constexpr int NST = NJ >= 8 ? 2 : 3;          // stages
+    static constexpr int NST = NJ <= 2 ? 4 : 3;          // stages: what two blocks to an SM leave room for
 };
-constexpr int EX_VS = 132;                               // floats per token of the gate and up tiles (they reuse the ring: 2 x 64 x 132 x 4 bytes fit two stages)
+constexpr int EX_VS = 132;                               // floats per token of the gate and up tiles (they reuse the ring: 2 x 48 x 132 x 4 bytes fit three stages)
 constexpr size_t EX_SMEM = 224 * 1024;
 template <int NJ> static inline size_t exp_smem(int k) { return (size_t)ExpCfg<NJ>::NST * ExpCfg<NJ>::STAGE + (size_t)(k / 32) * ExpCfg<NJ>::TOK * 4; }
 
@@ -122,14 +122,15 @@ __device__ __forceinline__ void exp_stage(const unsigned char* w0, const unsigne
 }
 // grid (tiles, ceil(n_out / (GLU ? 128 : 256))), block 256: a block is one tile of an expert's pairs; a warp owns 16 gate rows and the same 16 up rows, or 32 rows of the
 // down matrix, and all tokens of the tile (up to 8 * NJ); groups of 8 tokens past the tile's last pair are
-// skipped, so a tile costs what it holds. k in stages of 128 through a cp.async ring. Any n_in that is a multiple of 64.
+// skipped, so a tile costs what it holds. k in stages of 128 through a cp.async ring, whose first weights are asked for before the
+// pair list is read (they need the expert alone). Any n_in that is a multiple of 64.
 // What bounds it: with 1-2 pairs per expert (batched decode) the start of a tile -- a block serves one and begins with an empty ring:
 // at 32 rows gate + up stream their 197 MB at 42 % of DRAM's peak with 64 % of the issue slots and 20 % of the tensor pipe busy, down
 // its 98 MB at 34 %; with many pairs the MMAs and the f32 operations behind them, which overlap only in part (3.8 cycles per MMA
 // and SM in the loop alone, against 2.0 for the MMAs and as much for the f32 pipe; 2,048 rows: tensor pipe 34 %, f32 pipe 45 %).
 // Feeding the stages by bulk copies from a ninth warp was slower (1 KB and 128-byte pieces: 102 us against 63 at 32 tokens).
 template <int NJ, bool GLU>
-__global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
+__global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     using C = ExpCfg<NJ>;
@@ -148,8 +149,6 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
     const bool rows_live = r0 + (GLU ? wid * 16 : wid * 32) < n_out;
     const bool has_a = p.wa.scale2 != nullptr, has_b = GLU && p.wb.scale2 != nullptr;
     const float s2a = has_a ? p.wa.scale2[el] : 1.0f, s2b = has_b ? p.wb.scale2[el] : 1.0f;
-    if (tid < n) { const int pr = p.list[t0 + tid]; s_pair[tid] = pr; s_row[tid] = pr / p.div; }
-    __syncthreads();
     // source addresses of this thread's pieces, advanced by a stage's bytes per stage. Weights: 16 tiles x 1 KB per stage (64 lanes x
     // 16 bytes to a tile), scales: 16 tiles x 128 bytes; rows past the matrix read its last tile. Tokens past the last are not
     // staged: what stands in their place reaches only their own results, which nobody reads.
@@ -160,13 +159,8 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) wsrc[i] = (GLU && i >= 2 ? p.wb.nib : p.wa.nib) + tile_row((tid >> 6) + i * 4) * (k / 2) + (tid & 63) * 16;
         ssrc = (GLU && tid >= 64 ? p.wb.sc : p.wa.sc) + tile_row((tid >> 3) & 15) * (k / 16) + (tid & 7) * 16;
-#pragma unroll
-        for (int i = 0; i < XP; ++i) {               // activations: 16 tokens x 16 pieces of 16 bytes
-            const int tk = (tid >> 4) + i * 16;
-            xsrc[i] = tk < n ? p.xh + (size_t)s_row[tk] * k + (tid & 15) * 8 : nullptr;
-        }
     }
-    auto load = [&](int c) {
+    auto load_w = [&](int c) {
         unsigned char* st = smem + (c % C::NST) * C::STAGE;
         const bool half = 2 * c + 2 > kgs;           // the last stage of a row that ends with 64 elements
         if (!half || (tid & 63) < 32) {
@@ -174,14 +168,30 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
             for (int i = 0; i < 4; ++i) cp_async16(st + tid * 16 + i * 4096, wsrc[i] + (size_t)c * 1024, true);
         }
         if (tid < 128 && (!half || (tid & 7) < 4)) cp_async16(st + C::OFF_S + tid * 16, ssrc + (size_t)c * 128, true);
+    };
+    auto load_x = [&](int c) {
+        unsigned char* st = smem + (c % C::NST) * C::STAGE;
+        const bool half = 2 * c + 2 > kgs;
         if (!half || (tid & 15) < 8) {
 #pragma unroll
             for (int i = 0; i < XP; ++i)
                 if (xsrc[i]) cp_async16(st + C::OFF_X + ((tid >> 4) + i * 16) * EX_XSTR + (tid & 15) * 16, xsrc[i] + (size_t)c * EX_KC, true);
         }
     };
+    auto load = [&](int c) { load_w(c); load_x(c); };
+    int pr = 0;
+    if (tid < n) pr = p.list[t0 + tid];
 #pragma unroll
-    for (int c = 0; c < C::NST - 1; ++c) { if (c < n_chunk) load(c); cp_async_commit(); }
+    for (int c = 0; c < C::NST - 1; ++c) if (c < n_chunk) load_w(c);
+    if (tid < n) { s_pair[tid] = pr; s_row[tid] = pr / p.div; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < XP; ++i) {                   // activations: 16 tokens x 16 pieces of 16 bytes
+        const int tk = (tid >> 4) + i * 16;
+        xsrc[i] = tk < n ? p.xh + (size_t)s_row[tk] * k + (tid & 15) * 8 : nullptr;
+    }
+#pragma unroll
+    for (int c = 0; c < C::NST - 1; ++c) { if (c < n_chunk) load_x(c); cp_async_commit(); }
     for (int tk = wid; tk < n; tk += 8)               // the tile's activation scales, [block][token]
         for (int b2 = lane; b2 < nb / 2; b2 += 32) {
             const float2 v = *(const float2*)(p.xs + (size_t)s_row[tk] * nb + 2 * b2);
@@ -216,7 +226,7 @@ __global__ void __launch_bounds__(256, NJ >= 8 ? 2 : 3) k_exp(ExpArgs p) {
     };
     switch (nja) {
 #define EX_CASE(N) case N: if constexpr (N <= NJ) walk(std::integral_constant<int, N>{}); break;
-        EX_CASE(1) EX_CASE(2) EX_CASE(3) EX_CASE(4) EX_CASE(5) EX_CASE(6) EX_CASE(7) EX_CASE(8)
+        EX_CASE(1) EX_CASE(2) EX_CASE(3) EX_CASE(4) EX_CASE(5) EX_CASE(6)
 #undef EX_CASE
     }
     cp_async_wait<0>();
@@ -283,22 +293,27 @@ static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) 
     itb_raise_smem(k_exp<NJ, GLU>, EX_SMEM);
     itb_chain(k_exp<NJ, GLU>, dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st, a);
 }
-// The activation scales of a tile's whole rows lie beside the ring: up to 18,944 elements of k with 64 tokens.
-static inline bool exp_k_ok(int k) { return exp_smem<8>(k) <= EX_SMEM; }
-// Pairs per tile. Up to 4 per expert on average nearly every expert holds at most 16: tiles of 16, whose kernel keeps three stages
-// of the weight stream in flight in each of three blocks to an SM. More: 64, so that an expert's weights are decoded once for
-// most of its pairs -- unless that leaves SMs without a block (few experts or short rows): then as many as give every SM four.
+// The activation scales of a tile's whole rows lie beside the ring: up to 22,464 elements of k with 48 tokens.
+static inline bool exp_k_ok(int k) { return exp_smem<6>(k) <= EX_SMEM; }
+// Pairs per tile: 16, 32 or 48. A larger tile decodes an expert's weights once for more of its pairs; a smaller one has fewer
+// accumulators and less of shared memory in activations, and an expert's pairs are cut evenly, so tiles of 32 end less unevenly than
+// tiles of 48. Gate + up and down of 256 experts (2048 x 512), 8 pairs to a row, in us with 16 / 32 / 48 pairs: 128 rows 129 / 132 /
+// 138, 256 rows 154 / 156 / 162, 384 rows 189 / 187 / 192, 512 rows 236 / 213 / 218, 768 rows 321 / 278 / 279, 1,024 rows 406 / 358 /
+// 334, 5,548 rows 1909 / 1606 / 1497: 16 up to 8 pairs per expert on average, 32 up to 24. (64 pairs leave room for two stages only and
+// spill: 180, 214, 240, 304, 365 and 1565 us from 256 rows on.) Where that leaves SMs without a block (few experts or short rows):
+// as many pairs as give every SM four blocks.
 static inline int exp_tile_cap(int n_pairs, int n_expert, int ff, int sms) {
-    if (n_pairs <= 4 * n_expert) return 16;
+    const int cap = n_pairs <= 8 * n_expert ? 16 : n_pairs <= 24 * n_expert ? 32 : 48;
     const int want = 4 * sms / ((ff + 127) / 128);                        // tiles, at (ff / 128) blocks each
-    if (n_expert >= want) return 64;
-    return std::min(64, std::max(16, (n_pairs / std::max(want, 1) + 7) & ~7));
+    if (n_expert >= want) return cap;
+    return std::min(cap, std::max(16, (n_pairs / std::max(want, 1) + 7) & ~7));
 }
 static inline int exp_max_tiles(int n_pairs, int n_expert, int cap) { return std::min(n_pairs, n_expert + n_pairs / cap); }
 static inline void exp_run(ExpArgs a, bool glu, int max_tiles, int cap, cudaStream_t st) {
     a.zero2 = 0;
     if (cap <= 16) { if (glu) exp_launch<2, true>(a, max_tiles, st); else exp_launch<2, false>(a, max_tiles, st); }
-    else { if (glu) exp_launch<8, true>(a, max_tiles, st); else exp_launch<8, false>(a, max_tiles, st); }
+    else if (cap <= 32) { if (glu) exp_launch<4, true>(a, max_tiles, st); else exp_launch<4, false>(a, max_tiles, st); }
+    else { if (glu) exp_launch<6, true>(a, max_tiles, st); else exp_launch<6, false>(a, max_tiles, st); }
 }
 
 // Q8_0 quantisation of f32 rows as the kernels above read them: f16 values permuted inside blocks, block scales.

@@ -330,7 +330,7 @@ def cfg2_experts():
 @pytest.mark.parametrize("n_tok", [1, 8, 32, 200])
 def test_grouped_expert_matmuls_config2_exact(ops, cfg2_experts, n_tok):
     """gate/up/SiLU and down over Zipf-skewed routing at the microbenchmark's shapes: 1 and 8 tokens take the per-pair
-    dequant-and-dot kernels, 32 and 200 the expert-grouped int8-MMA tiles (8- and 16-token tiles); routing ids bit-exact,
+    dequant-and-dot kernels, 32 and 200 the expert-grouped tiles (16 pairs); routing ids bit-exact,
     the down matmul bit-exact on the same inputs, gate/up within the exp tolerance."""
     from inferred_thoughts_b200 import host
     H, ff, E, K, (gb, gs), (ub, us), (db, ds) = cfg2_experts
@@ -355,7 +355,7 @@ def test_grouped_expert_matmuls_config2_exact(ops, cfg2_experts, n_tok):
 
 @pytest.mark.parametrize("E,H,ff", [(5, 192, 64), (20, 192, 4160)])
 def test_grouped_expert_tiles_at_their_edges(ops, E, H, ff):
-    """Tiles of up to 16 pairs (few experts: spread over the SMs) and of up to 64: experts with no pair, 1, 8, 9, 64, 65 and 130 of them,
+    """Tiles of up to 16 pairs (few experts: spread over the SMs) and of up to 32: experts with no pair, 1, 8, 9, 64, 65 and 130 of them,
     rows that end inside a block of rows and a stage of k."""
     from inferred_thoughts_b200 import host
     gb, gs = nvfp4_weights(E, ff, H, 150); ub, us = nvfp4_weights(E, ff, H, 151); db, ds = nvfp4_weights(E, H, ff, 152)
@@ -377,7 +377,31 @@ def test_grouped_expert_tiles_at_their_edges(ops, E, H, ff):
     exact(o, o_want, "matmul_experts(down)")
 
 
-@pytest.mark.parametrize("n_in", [18944, 19008])
+@pytest.mark.parametrize("counts", [[0, 1, 8, 9, 31, 32, 33, 64, 65] + [1] * 11, [0, 1, 7, 8, 40, 41, 47, 48, 49, 96, 97, 130] + [5] * 8])
+def test_grouped_expert_tiles_of_32_and_of_48_pairs(ops, counts):
+    """12.7 pairs per expert on average (tiles of up to 32) and 30.2 (up to 48), with long enough outputs that the tiles are not made smaller
+    for want of blocks: experts of one pair less and one more than a tile, and of two and three tiles."""
+    from inferred_thoughts_b200 import host
+    E, H, ff, N = len(counts), 192, 4160, 8320
+    gb, gs = nvfp4_weights(E, ff, H, 250); ub, us = nvfp4_weights(E, ff, H, 251); db, ds = nvfp4_weights(E, N, H, 252)
+    gs *= 300; us *= 300; ds *= 300
+    ids = np.random.default_rng(6).permutation(np.repeat(np.arange(E), counts)).astype(np.int32)
+    n = ids.size
+    x = noise(n * H, 253)
+    h = keep(np.zeros(n * ff, np.float32)); scratch = keep(np.zeros_like(h)); o = keep(np.zeros(n * N, np.float32))
+    ops.begin_pass(n)
+    route = host.Route.host(ids.astype(np.uint64), None, 1)
+    ops.moe_glu(host.Experts(gb, host.NVFP4, H, ff, E, gs), host.Experts(ub, host.NVFP4, H, ff, E, us), route, x, h, scratch)
+    ops.matmul_experts(host.Experts(db, host.NVFP4, H, N, E, ds), route, x, o)
+    ops.host_needs(h); ops.host_needs(o); ops.check()
+    h_want = np.zeros_like(h); o_want = np.zeros_like(o)
+    L.orc_moe_glu(gb, gs.ctypes.data, ub, us.ctypes.data, H, ff, E, ids, n, 1, x, x.size, h_want, 0)
+    close(h, h_want, 8 * EPS, "moe_glu (through silu)")
+    L.orc_matmul_experts(db, H, N, E, ds.ctypes.data, ids, n, 1, x, x.size, o_want, 0)
+    exact(o, o_want, "matmul_experts(long rows)")
+
+
+@pytest.mark.parametrize("n_in", [18944, 19008, 22464, 22528])
 def test_grouped_experts_with_rows_as_long_as_the_tiles_hold_and_longer(ops, n_in):
     """The grouped form keeps a tile's activation scales in shared memory; longer rows take the form without tiles."""
     from inferred_thoughts_b200 import host
