@@ -1210,7 +1210,6 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     const int TPB = NWG * 32;
     uint64_t launches = 0;
     const bool chain = !e->ep && !e->tier;       // with them, copies, events and collectives come between the kernels: the first one behind such orders itself as ever
-    set_smem((const void*)k_tile_q8_multi<1, 256, 4>, 226 * 1024);
     set_smem((const void*)k_gdn_chunk_prep<128>, gdn_chunk_prep_smem<128>()); set_smem((const void*)k_gdn_chunk_scan<128>, gdn_chunk_scan_smem<128>());
     set_smem((const void*)k_matmul_f32<true>, 100 * 1024); set_smem((const void*)k_matmul_f32<false>, 100 * 1024);
     // Pipelined tile kernels when k is a multiple of the chunk (every matrix of the 35B and 177B shapes); the
@@ -1244,10 +1243,8 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         if (one) {
             Q8Multi p{};
             p.n = n;
-            int tiles = 0;
-            for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; p.tiles[i] = (w[i]->n_out + 31) / 32; tiles += p.tiles[i]; }
-            const int k = w[0]->n_in, ns = std::min(k / 256, TILE_STAGES);
-            itb_chain(k_tile_q8_multi<1, 256, 4>, dim3(tiles, (R + 31) / 32), 256, tile_smem<1, 256, 4>(k), cur, p, x.q, x.s, R, ns);
+            for (int i = 0; i < n; ++i) { p.w[i] = *w[i]; p.out[i] = out[i]; p.stride[i] = stride[i]; }
+            tile_q8(cur, sms, p, x.q, x.s, R, 0);
             launches++;
             return;
         }

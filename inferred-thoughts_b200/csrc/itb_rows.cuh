@@ -233,12 +233,13 @@ static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, x, n_rows, out, stride, mode);
     // many rows, dense=q8tc: exact integer dots of 128 x 128 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
     if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, x, n_rows, out, stride, mode);
-    for (const void* f : {(const void*)k_tile_q8<1, 256, 4>, (const void*)k_tile_q8<4, 256, 2>}) itb_raise_smem(f, 226 * 1024);
     for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) itb_raise_smem(f, 200 * 1024);
     const bool skinny = n_rows <= 32;
-    const int ns = std::min(k / 256, TILE_STAGES);
-    if (skinny && k % 256 == 0) itb_chain(k_tile_q8<1, 256, 4>, dim3((w.n_out + 31) / 32, (n_rows + 31) / 32), 256, tile_smem<1, 256, 4>(k), st, w, x.q, x.s, n_rows, out, stride, mode, ns);
-    else if (k % 256 == 0) itb_chain(k_tile_q8<4, 256, 2>, dim3((w.n_out + 63) / 64, (n_rows + 63) / 64), 256, tile_smem<4, 256, 2>(k), st, w, x.q, x.s, n_rows, out, stride, mode, ns);
+    if (k % 256 == 0) {
+        Q8Multi p{};
+        p.n = 1; p.w[0] = w; p.out[0] = out; p.stride[0] = stride;
+        tile_q8(st, c->sm_count, p, x.q, x.s, n_rows, mode);
+    }
     else if (skinny) itb_chain(k_gemm_q8<1>, dim3((w.n_out + 63) / 64, 1), 512, gemm_smem(k), st, w, x.q, x.s, n_rows, out, stride, mode);
     else itb_chain(k_gemm_q8<4>, dim3((w.n_out + MMA_ROWS - 1) / MMA_ROWS, (n_rows + MMA_TOK - 1) / MMA_TOK), 256, gemm_smem(k), st, w, x.q, x.s, n_rows, out, stride, mode);
     return true;

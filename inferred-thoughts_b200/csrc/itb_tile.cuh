@@ -1,18 +1,12 @@
-// Pipelined multi-token matmuls: a block owns 64 weight rows x TOK tokens and walks k in chunks of KC elements
-// through a ring of cp.async stages (weights, their scales, the Q8_0 activations and their scales all arrive by
-// 16-byte asynchronous copies, several chunks in flight), so DRAM latency is paid once per block instead of once
-// per k-block. The arithmetic is the exact chain of itb_mma.cuh: one int8 MMA per quantisation block, its int32
-// sum scaled and added to an f32 accumulator in ascending block order (src/ops/naive.rs:691-734).
-//
-// 8 warps, split TH ways over the tile's tokens and 8/TH ways over its rows: TH=2 -> 64 rows x 16*NJ tokens (wide token
-// tiles); TH=4 -> 32 rows x 32*NJ tokens (batched decode: small blocks, so every SM gets several and their pipelines
-// overlap). NJ = groups of 8 tokens per warp. (Routed experts: itb_exp.cuh.)
+// Pipelined multi-token matmuls, Q8_0 weights x Q8_0-quantised rows in the CPU path's arithmetic: a block owns 16 RG weight rows x 8 NJ TG
+// tokens and walks k in chunks of 256 elements through a ring of cp.async stages (weights, their scales, the activations and theirs),
+// several chunks in flight. One int8 MMA per quantisation block, its int32 sum scaled and added to an f32 accumulator in ascending
+// block order (src/ops/naive.rs:691-734).
 #pragma once
+#include <type_traits>
 #include "itb_mma.cuh"
 
 namespace {
-
-constexpr int TILE_STAGES = 4;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -23,152 +17,143 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
-template <int NJ, int KC, int TH = 2>
-struct TileCfg {
-    static constexpr int ROWS = 128 / TH;
-    static constexpr int TOK = 8 * NJ * TH;
-    static constexpr int WB = KC;            // weight bytes per row and chunk
-    static constexpr int WSTR = WB + 32;       // padded row stride: fragment reads hit distinct banks
-    static constexpr int SB = KC / 32 * 2;  // scale bytes per row and chunk
-    static constexpr int XSTR = KC + 32;
-    static constexpr int XSB = KC / 32 * 4;                           // activation scale bytes per token and chunk
-    static constexpr int XSF = KC / 32 + 4;                           // padded scale row in floats (distinct banks for the 4 token pairs)
-    static constexpr int OFF_WS = ROWS * WSTR;
-    static constexpr int OFF_XQ = OFF_WS + ROWS * SB;
-    static constexpr int OFF_XS = OFF_XQ + TOK * XSTR;
-    static constexpr int STAGE = OFF_XS + TOK * XSF * 4;
-    static_assert(WB % 16 == 0 && SB % 16 == 0 && XSB % 16 == 0 && STAGE % 16 == 0, "16-byte copies");
+constexpr int TQ_KC = 256;                       // elements of k per stage
+template <int RG, int TG, int NJ> struct TileCfg {
+    static constexpr int ROWS = 16 * RG, TOK = 8 * NJ * TG, THREADS = 32 * RG * TG;
+    static constexpr int STR = TQ_KC + 32;           // padded line: fragment reads hit distinct banks
+    static constexpr int XSF = TQ_KC / 32 + 4;       // floats per token's line of scales, padded likewise
+    static constexpr int OFF_S = ROWS * STR, OFF_X = OFF_S + ROWS * 16, OFF_XS = OFF_X + TOK * STR, STAGE = OFF_XS + TOK * XSF * 4;
 };
-template <int NJ, int KC, int TH = 2>
-static inline size_t tile_smem(int k) {
-    int n = k / KC; if (n > TILE_STAGES) n = TILE_STAGES; if (n < 1) n = 1;
-    return (size_t)n * TileCfg<NJ, KC, TH>::STAGE + 64 * 4;
-}
+// Up to three dense Q8_0 matrices over the same quantised rows in one launch (the input projections of a layer; the shared
+// expert's gate and up): grid.x runs over the matrices' row tiles one after the other. A matrix of 512 rows alone is 32 blocks.
+struct Q8Multi { DevQ8 w[3]; float* out[3]; size_t stride[3]; int tiles[3]; int n; };
 
-// One (ROWS-row, TOK-token) tile. wq/ws: the matrix's quants and scales (row-major, k elements per row); rows
-// [r0, r0+ROWS) clamped to n_rows-1. tok_idx[TOK] (shared memory): activation row of each tile token or -1.
-// Results in acc[NJ][4] in the MMA C layout for the warp's rows {g, g+8} and tokens 8*j + 2t, +1 of its token share.
-template <int NJ, int KC, int TH>
-__device__ __forceinline__ void tile_gemm(const uint8_t* wq, const uint8_t* ws, int k, int n_rows, int r0, const int8_t* xq, const float* xs,
-                                          const int* tok_idx, unsigned char* ring, int n_stage, float (&acc)[NJ][4]) {
-    using C = TileCfg<NJ, KC, TH>;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int n_chunk = k / KC, nb = k / 32;
-    const size_t wrow = (size_t)k, srow = (size_t)nb * 2;
-    auto load = [&](int c) {
-        unsigned char* st = ring + (size_t)(c % n_stage) * C::STAGE;
-        constexpr int WP = C::WB / 16, SP = C::SB / 16, XP = KC / 16, XSP = C::XSB / 16;
-        for (int i = tid; i < C::ROWS * WP; i += 256) {
-            const int r = i / WP, p = i % WP, row = min(r0 + r, n_rows - 1);
-            cp_async16(st + r * C::WSTR + p * 16, wq + (size_t)row * wrow + (size_t)c * C::WB + p * 16, true);
+// RG x TG warps, each 16 rows x 8 NJ tokens; groups of 8 tokens past the last row are neither staged nor multiplied. mode 0: out = v;
+// mode 1: out += v. n_in a multiple of 256. grid (row tiles of all matrices, ceil(n_tok / TOK)).
+// What bounds it, at 32 tokens: with many rows shared memory and the issue slots (LM head, 248,320 x 2048: a 16 x 8 product costs 8 cycles of
+// an SM's shared-memory pipe -- fragments, scales, the staging itself -- and 27 issue slots; 176 us against 82 for the bytes); with few
+// the latency of a stage and of the dot -> scale -> add chain, which is why all eight blocks of a stage are unrolled (a chunk's MMAs go out
+// back to back), the scales of a row are one 16-byte read per chunk, and the first stages' weights are asked for before the rows are there.
+template <int RG, int TG, int NJ, int NST>
+__global__ void __launch_bounds__(32 * RG * TG, 3) k_tile_q8(Q8Multi p, const int8_t* xq, const float* xs, int n_tok, int mode) {
+    using C = TileCfg<RG, TG, NJ>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    int m = 0, bx = blockIdx.x;
+    while (m + 1 < p.n && bx >= p.tiles[m]) { bx -= p.tiles[m]; ++m; }
+    const DevQ8 w = p.w[m];
+    const int k = w.n_in, nb = k / 32, n_chunk = k / TQ_KC, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int r0 = bx * C::ROWS, t0 = blockIdx.y * C::TOK, n = min(C::TOK, n_tok - t0);
+    auto load_w = [&](int c) {
+        unsigned char* st = smem + (c % NST) * C::STAGE;
+#pragma unroll
+        for (int i0 = 0; i0 < C::ROWS * 16; i0 += C::THREADS) {
+            const int i = i0 + tid, r = i >> 4, q = i & 15, row = min(r0 + r, w.n_out - 1);
+            cp_async16(st + r * C::STR + q * 16, (const uint8_t*)w.q + (size_t)row * k + (size_t)c * TQ_KC + q * 16, true);
         }
-        for (int i = tid; i < C::ROWS * SP; i += 256) {
-            const int r = i / SP, p = i % SP, row = min(r0 + r, n_rows - 1);
-            cp_async16(st + C::OFF_WS + r * C::SB + p * 16, ws + (size_t)row * srow + (size_t)c * C::SB + p * 16, true);
+        if (tid < C::ROWS) cp_async16(st + C::OFF_S + tid * 16, (const uint8_t*)w.s + (size_t)min(r0 + tid, w.n_out - 1) * nb * 2 + (size_t)c * 16, true);
+    };
+    auto load_x = [&](int c) {
+        unsigned char* st = smem + (c % NST) * C::STAGE;
+#pragma unroll
+        for (int i0 = 0; i0 < C::TOK * 16; i0 += C::THREADS) {
+            const int i = i0 + tid, tk = i >> 4, q = i & 15;
+            if (tk < n) cp_async16(st + C::OFF_X + tk * C::STR + q * 16, xq + (size_t)(t0 + tk) * k + (size_t)c * TQ_KC + q * 16, true);
         }
-        for (int i = tid; i < C::TOK * XP; i += 256) {
-            const int tk = i / XP, p = i % XP, src = tok_idx[tk];
-            cp_async16(st + C::OFF_XQ + tk * C::XSTR + p * 16, xq + (size_t)max(src, 0) * k + (size_t)c * KC + p * 16, src >= 0);
-        }
-        for (int i = tid; i < C::TOK * XSP; i += 256) {
-            const int tk = i / XSP, p = i % XSP, src = tok_idx[tk];
-            cp_async16(st + C::OFF_XS + tk * C::XSF * 4 + p * 16, (const unsigned char*)(xs + (size_t)max(src, 0) * nb) + (size_t)c * C::XSB + p * 16, src >= 0);
+#pragma unroll
+        for (int i0 = 0; i0 < C::TOK * 2; i0 += C::THREADS) {
+            const int i = i0 + tid, tk = i >> 1, q = i & 1;
+            if (tk < n) cp_async16(st + C::OFF_XS + tk * C::XSF * 4 + q * 16, (const unsigned char*)(xs + (size_t)(t0 + tk) * nb) + (size_t)c * 32 + q * 16, true);
         }
     };
+#pragma unroll
+    for (int c = 0; c < NST - 1; ++c) if (c < n_chunk) load_w(c);
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < NST - 1; ++c) { if (c < n_chunk) load_x(c); cp_async_commit(); }
+    // this warp's rows and tokens inside the tile, and how many groups of 8 of its tokens exist
+    const int rw = (wid % RG) * 16, tb = (wid / RG) * NJ * 8;
+    const int nja = min(NJ, (n - tb + 7) >> 3);
+    float acc[NJ][4];
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[j][i] = 0.0f;
-    for (int c = 0; c < n_stage - 1; ++c) { if (c < n_chunk) load(c); cp_async_commit(); }
-    constexpr int RG = 8 / TH;   // row groups of 16 among the 8 warps
-    const int rw = (wid % RG) * 16, tb = (wid / RG) * NJ * 8;
-    for (int c = 0; c < n_chunk; ++c) {
-        if (n_stage == 1) { __syncthreads(); load(c); cp_async_commit(); }
-        if (n_stage >= 4) cp_async_wait<2>(); else if (n_stage == 3) cp_async_wait<1>(); else cp_async_wait<0>();
-        __syncthreads();
-        if (n_stage > 1) { if (c + n_stage - 1 < n_chunk) load(c + n_stage - 1); cp_async_commit(); }
-        const unsigned char* st = ring + (size_t)(c % n_stage) * C::STAGE;
-        const unsigned char* wa = st + (rw + g) * C::WSTR;
-        const unsigned char* wb = wa + 8 * C::WSTR;
-        const unsigned char* sa = st + C::OFF_WS + (rw + g) * C::SB;
-        const unsigned char* sb = sa + 8 * C::SB;
-        const unsigned char* xq_s = st + C::OFF_XQ;
-        const float* xs_s = (const float*)(st + C::OFF_XS);
-#pragma unroll 2
-        for (int b = 0; b < KC / 32; ++b) {
-            const uint2 va = *(const uint2*)(wa + b * 32 + 8 * t), vb = *(const uint2*)(wb + b * 32 + 8 * t);
-            const float dwa = f16_bits_to_f32(*(const uint16_t*)(sa + 2 * b)), dwb = f16_bits_to_f32(*(const uint16_t*)(sb + 2 * b));
+    // the whole k loop per group count (a compile-time count: the loads, MMAs and sums of all groups interleave)
+    auto walk = [&](auto count) {
+        constexpr int NJA = decltype(count)::value;
+        for (int c = 0; c < n_chunk; ++c) {
+            cp_async_wait<NST - 2>();
+            __syncthreads();                         // stage c has landed; everyone is done with stage c - 1
+            if (c + NST - 1 < n_chunk) { load_w(c + NST - 1); load_x(c + NST - 1); }
+            cp_async_commit();
+            if (NJA == 0) continue;
+            const unsigned char* st = smem + (c % NST) * C::STAGE;
+            const unsigned char* wa = st + (rw + g) * C::STR + 8 * t;
+            const unsigned char* xr = st + C::OFF_X + (tb + g) * C::STR + 8 * t;
+            const float* xsr = (const float*)(st + C::OFF_XS) + (tb + 2 * t) * C::XSF;
+            const uint4 sa = *(const uint4*)(st + C::OFF_S + (rw + g) * 16), sb = *(const uint4*)(st + C::OFF_S + (rw + g + 8) * 16);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const int tj = tb + 8 * j;
-                const uint2 x = *(const uint2*)(xq_s + (tj + g) * C::XSTR + b * 32 + 8 * t);
-                int cc[4];
-                mma_s8_k32(cc, va.x, vb.x, va.y, vb.y, x.x, x.y);
-                const float dx0 = xs_s[(tj + 2 * t) * C::XSF + b], dx1 = xs_s[(tj + 2 * t + 1) * C::XSF + b];
-                acc[j][0] += i2f_small(cc[0]) * (dwa * dx0);
-                acc[j][1] += i2f_small(cc[1]) * (dwa * dx1);
-                acc[j][2] += i2f_small(cc[2]) * (dwb * dx0);
-                acc[j][3] += i2f_small(cc[3]) * (dwb * dx1);
+            for (int h = 0; h < 2; ++h) {
+                float dx[NJA > 0 ? NJA : 1][2][4];
+#pragma unroll
+                for (int j = 0; j < NJA; ++j)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) { const float4 v = *(const float4*)(xsr + (8 * j + q) * C::XSF + 4 * h); dx[j][q][0] = v.x; dx[j][q][1] = v.y; dx[j][q][2] = v.z; dx[j][q][3] = v.w; }
+                const uint2 s2a = h ? make_uint2(sa.z, sa.w) : make_uint2(sa.x, sa.y), s2b = h ? make_uint2(sb.z, sb.w) : make_uint2(sb.x, sb.y);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const uint2 va = *(const uint2*)(wa + (4 * h + b) * 32), vb = *(const uint2*)(wa + 8 * C::STR + (4 * h + b) * 32);
+                    const float da = f16_bits_to_f32((uint16_t)((b < 2 ? s2a.x : s2a.y) >> (16 * (b & 1)))), db = f16_bits_to_f32((uint16_t)((b < 2 ? s2b.x : s2b.y) >> (16 * (b & 1))));
+#pragma unroll
+                    for (int j = 0; j < NJA; ++j) {
+                        const uint2 x = *(const uint2*)(xr + 8 * j * C::STR + (4 * h + b) * 32);
+                        int cc[4];
+                        mma_s8_k32(cc, va.x, vb.x, va.y, vb.y, x.x, x.y);
+                        acc[j][0] += i2f_small(cc[0]) * (da * dx[j][0][b]);
+                        acc[j][1] += i2f_small(cc[1]) * (da * dx[j][1][b]);
+                        acc[j][2] += i2f_small(cc[2]) * (db * dx[j][0][b]);
+                        acc[j][3] += i2f_small(cc[3]) * (db * dx[j][1][b]);
+                    }
+                }
             }
         }
-    }
+    };
+    if (nja <= 0) walk(std::integral_constant<int, 0>{});
+    else if (NJ == 1 || nja == 1) walk(std::integral_constant<int, 1>{});
+    else walk(std::integral_constant<int, NJ>{});
     cp_async_wait<0>();
-    __syncthreads();   // the ring may be refilled by the caller's next tile
-}
-
-// Visit this warp's results: f(token_in_tile, row, value).
-template <int NJ, int TH, class F>
-__device__ __forceinline__ void tile_foreach(const float (&acc)[NJ][4], int r0, int n_rows, F f) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    constexpr int RG = 8 / TH;
-    const int ra = r0 + (wid % RG) * 16 + g, rb = ra + 8, tb = (wid / RG) * NJ * 8;
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-        const int tj = tb + 8 * j + 2 * t;
-        if (ra < n_rows) { f(tj, ra, acc[j][0]); f(tj + 1, ra, acc[j][1]); }
-        if (rb < n_rows) { f(tj, rb, acc[j][2]); f(tj + 1, rb, acc[j][3]); }
-    }
-}
-
-// Dense Q8_0 matmul: grid (ceil(rows/ROWS), ceil(n_tok/TOK)). mode 0: out = v; mode 1: out += v.
-template <int NJ, int KC, int TH>
-__global__ void __launch_bounds__(256) k_tile_q8(DevQ8 w, const int8_t* xq, const float* xs, int n_tok, float* out, size_t out_stride, int mode, int n_stage) {
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char smem[];
-    using C = TileCfg<NJ, KC, TH>;
-    int* tok_idx = (int*)smem;
-    const int t0 = blockIdx.y * C::TOK, r0 = blockIdx.x * C::ROWS;
-    if ((int)threadIdx.x < C::TOK) { const int ti = t0 + (int)threadIdx.x; tok_idx[threadIdx.x] = ti < n_tok ? ti : -1; }
-    __syncthreads();
-    float acc[NJ][4];
-    tile_gemm<NJ, KC, TH>((const uint8_t*)w.q, (const uint8_t*)w.s, w.n_in, w.n_out, r0, xq, xs, tok_idx, smem + 256, n_stage, acc);
-    tile_foreach<NJ, TH>(acc, r0, w.n_out, [&](int t, int row, float v) {
-        if (t0 + t < n_tok) { float* o = out + (size_t)(t0 + t) * out_stride + row; *o = mode ? *o + v : v; }
-    });
-}
-
-// Up to three dense Q8_0 matrices over the same quantised rows in one launch (the input projections of a layer; the shared
-// expert's gate and up): grid.x runs over the matrices' row tiles one after the other. A matrix of 512 rows alone is 16 blocks.
-struct Q8Multi { DevQ8 w[3]; float* out[3]; size_t stride[3]; int tiles[3]; int n; };
-template <int NJ, int KC, int TH>
-__global__ void __launch_bounds__(256) k_tile_q8_multi(Q8Multi p, const int8_t* xq, const float* xs, int n_tok, int n_stage) {
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char smem[];
-    using C = TileCfg<NJ, KC, TH>;
-    int* tok_idx = (int*)smem;
-    int m = 0, bx = blockIdx.x;
-    while (m + 1 < p.n && bx >= p.tiles[m]) { bx -= p.tiles[m]; ++m; }
-    const DevQ8 w = p.w[m];
     float* out = p.out[m];
-    const size_t out_stride = p.stride[m];
-    const int t0 = blockIdx.y * C::TOK, r0 = bx * C::ROWS;
-    if ((int)threadIdx.x < C::TOK) { const int ti = t0 + (int)threadIdx.x; tok_idx[threadIdx.x] = ti < n_tok ? ti : -1; }
-    __syncthreads();
-    float acc[NJ][4];
-    tile_gemm<NJ, KC, TH>((const uint8_t*)w.q, (const uint8_t*)w.s, w.n_in, w.n_out, r0, xq, xs, tok_idx, smem + 256, n_stage, acc);
-    tile_foreach<NJ, TH>(acc, r0, w.n_out, [&](int t, int row, float v) {
-        if (t0 + t < n_tok) out[(size_t)(t0 + t) * out_stride + row] = v;
-    });
+    const int ra = r0 + rw + g, rb = ra + 8;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int tk = t0 + tb + 8 * j + 2 * t + (i & 1), row = i < 2 ? ra : rb;
+            if (tk < n_tok && row < w.n_out) { float* o = out + (size_t)tk * p.stride[m] + row; *o = mode ? *o + acc[j][i] : acc[j][i]; }
+        }
+}
+template <int RG, int TG, int NJ, int NST>
+static void tile_q8_launch(cudaStream_t st, Q8Multi p, const int8_t* xq, const float* xs, int n_tok, int mode) {
+    using C = TileCfg<RG, TG, NJ>;
+    static_assert(NJ <= 2, "the group counts k_tile_q8 walks");
+    int tiles = 0;
+    for (int i = 0; i < p.n; ++i) { p.tiles[i] = (p.w[i].n_out + C::ROWS - 1) / C::ROWS; tiles += p.tiles[i]; }
+    itb_raise_smem(k_tile_q8<RG, TG, NJ, NST>, NST * C::STAGE);
+    itb_chain(k_tile_q8<RG, TG, NJ, NST>, dim3((unsigned)tiles, (unsigned)((n_tok + C::TOK - 1) / C::TOK)), C::THREADS, (size_t)NST * C::STAGE, st, p, xq, xs, n_tok, mode);
+}
+// Tiles by how many there are, all of 32 tokens and three blocks to an SM: 16 rows while all fit the SMs at once, then 32 rows, and 64 (half
+// the reads of the activations again) where even those are several to an SM. Measured (us, 16 / 32 / 64 rows; k 2048 unless said; in
+// parentheses the kernel with 32 x 32 tiles, one group of 8 tokens to a warp and 64 x 64 tiles past 32 tokens that this one replaced):
+// 32 tokens: 2,048 outputs of k 4096 7.6 / 10.7 / 17.8 (17.9), 4,096 6.6 / 6.6 / 10.0 (9.8), 6,144 9.3 / 10.2 / 10.4 (13.1), 12,288 16.1 / 13.6 / 16.3
+// (21.1), 24,576 28.4 / 23.8 / 22.8 (36.9), 248,320 243 / 187 / 176 (311); 8 tokens: 2,048 of k 4096 6.4 / 7.9 / 13.6 (18.1), 12,288 12.0 / 8.8 / 10.0 (21.2),
+// 24,576 20.3 / 15.5 / 12.5 (36.9), 248,320 181 / 118 / 102 (311); 200 tokens: 2,048 of k 4096 28.5 / 23.6 / 29.3 (34.4), 12,288 79 / 63 / 58 (103).
+static void tile_q8(cudaStream_t st, int sms, const Q8Multi& p, const int8_t* xq, const float* xs, int n_tok, int mode) {
+    long long blocks = 0;                                 // of 16 rows x 32 tokens
+    for (int i = 0; i < p.n; ++i) blocks += (p.w[i].n_out + 15) / 16;
+    blocks *= (n_tok + 31) / 32;
+    if (blocks <= 3 * sms) tile_q8_launch<1, 4, 1, 4>(st, p, xq, xs, n_tok, mode);
+    else if (blocks <= 8 * sms) tile_q8_launch<2, 2, 2, 3>(st, p, xq, xs, n_tok, mode);
+    else tile_q8_launch<4, 2, 2, 2>(st, p, xq, xs, n_tok, mode);
 }
 
 }  // namespace

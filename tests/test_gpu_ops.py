@@ -79,6 +79,13 @@ def test_matmul_q8_0_exact(ops, n_in, n_out, n_tok):
     exact(out, want, "Q8_0 matmul")
 
 
+@pytest.mark.parametrize("n_in,n_out,n_tok", [(256, 17, 2), (2048, 48, 9), (1280, 3540, 64), (1280, 7205, 17), (768, 3557, 63), (512, 3001, 250), (256, 19001, 8)])
+def test_matmul_q8_0_tiles_of_16_32_and_64_rows_exact(ops, n_in, n_out, n_tok):
+    """Few row tiles (16 rows), more (32) and many (64): one stage of k, fewer than the ring holds and more; a last tile of one row, of
+    one token and of one group of 8 tokens."""
+    test_matmul_q8_0_exact(ops, n_in, n_out, n_tok)
+
+
 @pytest.mark.parametrize("n_in,n_out,n_tok", [(512, 256, 150), (2048, 384, 700), (256, 128, 64), (4096, 128, 257)])
 def test_matmul_q8_0_as_f16_tensor_core_gemm(n_in, n_out, n_tok):
     """opts dense=f16tc: a many-row Q8_0 matmul as one tcgen05 kind::f16 GEMM over operands dequantised to f16 (weights and the
