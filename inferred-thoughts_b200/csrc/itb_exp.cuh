@@ -24,16 +24,18 @@
 namespace {
 
 constexpr int EX_KC = 128;                               // elements of k per pipeline stage
-constexpr int EX_WROWS = 256;                            // weight rows per block: 128 gate + 128 up, or 256 of the down matrix
 constexpr int EX_XSTR = EX_KC * 2 + 64;                  // padded token stride: the fragment reads of a warp hit distinct banks
 template <int NJ> struct ExpCfg {
     static constexpr int TOK = 8 * NJ;
-    static constexpr int OFF_S = EX_WROWS * EX_KC / 2;
-    static constexpr int OFF_X = OFF_S + EX_WROWS * (EX_KC / 16);
+    static constexpr int W = NJ <= 2 ? 4 : 8;            // warps
+    static constexpr int WROWS = 32 * W;                 // weight rows per block: half gate and half up, or all of the down matrix
+    static constexpr int BLOCKS = NJ <= 2 ? 4 : 2;       // to an SM
+    static constexpr int VS = 16 * W + 4;                // floats per token of the gate and up tiles, which reuse the ring
+    static constexpr int OFF_S = WROWS * EX_KC / 2;
+    static constexpr int OFF_X = OFF_S + WROWS * (EX_KC / 16);
     static constexpr int STAGE = OFF_X + TOK * EX_XSTR;
-    static constexpr int NST = NJ <= 2 ? 4 : 3;          // stages: what two blocks to an SM leave room for
+    static constexpr int NST = 3;                        // stages
 };
-constexpr int EX_VS = 132;                               // floats per token of the gate and up tiles (they reuse the ring: 2 x 48 x 132 x 4 bytes fit three stages)
 constexpr size_t EX_SMEM = 224 * 1024;
 template <int NJ> static inline size_t exp_smem(int k) { return (size_t)ExpCfg<NJ>::NST * ExpCfg<NJ>::STAGE + (size_t)(k / 32) * ExpCfg<NJ>::TOK * 4; }
 
@@ -120,17 +122,19 @@ __device__ __forceinline__ void exp_stage(const unsigned char* w0, const unsigne
         }
     }
 }
-// grid (tiles, ceil(n_out / (GLU ? 128 : 256))), block 256: a block is one tile of an expert's pairs; a warp owns 16 gate rows and the same 16 up rows, or 32 rows of the
-// down matrix, and all tokens of the tile (up to 8 * NJ); groups of 8 tokens past the tile's last pair are
+// grid (tiles, ceil(n_out / (GLU ? 16 W : 32 W))), block 32 W: a block is one tile of an expert's pairs; a warp owns 16 gate rows and the same
+// 16 up rows, or 32 rows of the down matrix, and all tokens of the tile (up to 8 * NJ); groups of 8 tokens past the tile's last pair are
 // skipped, so a tile costs what it holds. k in stages of 128 through a cp.async ring, whose first weights are asked for before the
 // pair list is read (they need the expert alone). Any n_in that is a multiple of 64.
-// What bounds it: with 1-2 pairs per expert (batched decode) the start of a tile -- a block serves one and begins with an empty ring:
-// at 32 rows gate + up stream their 197 MB at 42 % of DRAM's peak with 64 % of the issue slots and 20 % of the tensor pipe busy, down
-// its 98 MB at 34 %; with many pairs the MMAs and the f32 operations behind them, which overlap only in part (3.8 cycles per MMA
-// and SM in the loop alone, against 2.0 for the MMAs and as much for the f32 pipe; 2,048 rows: tensor pipe 34 %, f32 pipe 45 %).
+// What bounds it: with 1-2 pairs per expert (batched decode) the start of a tile -- a block serves one and begins with an empty ring -- and
+// the last round of blocks: four warps to a block and four blocks to an SM leave less of both than eight and two do (256 experts of
+// 2048 x 512, 8 pairs to a row, gate + up and down: 32 rows 77 us against 85, 64 rows 106 and 116, 128 rows 122 and 128; 43 us are the
+// bytes at 32 rows; blocks for 8 pairs, five to an SM: 75, 103, 118, but 164 against 152 at 256 rows). With many pairs: the MMAs and
+// the f32 operations behind them, which overlap only in part (3.8 cycles per MMA and SM in the loop alone, against 2.0 for the MMAs and
+// as much for the f32 pipe); there four warps to a block are the slower ones (512 rows, tiles of 32 pairs: 232 us against 213).
 // Feeding the stages by bulk copies from a ninth warp was slower (1 KB and 128-byte pieces: 102 us against 63 at 32 tokens).
 template <int NJ, bool GLU>
-__global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
+__global__ void __launch_bounds__(32 * ExpCfg<NJ>::W, ExpCfg<NJ>::BLOCKS) k_exp(ExpArgs p) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     using C = ExpCfg<NJ>;
@@ -142,32 +146,32 @@ __global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
     __shared__ int s_pair[C::TOK], s_row[C::TOK];
     float* s_xs = (float*)(smem + C::NST * C::STAGE);    // [k / 32][TOK]: the tile's activation scales
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
-    constexpr int RB = GLU ? 128 : 256, XP = (C::TOK + 15) / 16;
+    constexpr int W = C::W, VS = C::VS, RB = GLU ? 16 * W : 32 * W, XP = (C::TOK + 2 * W - 1) / (2 * W);
     const int r0 = blockIdx.y * RB, nb = k / 32, kgs = k / 64, n_chunk = (kgs + 1) / 2;
-    // this warp's two row tiles of 16 inside the staged 256 rows
-    const int wr0 = GLU ? wid * 16 : wid * 32, wr1 = GLU ? 128 + wid * 16 : wid * 32 + 16;
+    // this warp's two row tiles of 16 inside the staged rows
+    const int wr0 = GLU ? wid * 16 : wid * 32, wr1 = GLU ? 16 * W + wid * 16 : wid * 32 + 16;
     const bool rows_live = r0 + (GLU ? wid * 16 : wid * 32) < n_out;
     const bool has_a = p.wa.scale2 != nullptr, has_b = GLU && p.wb.scale2 != nullptr;
     const float s2a = has_a ? p.wa.scale2[el] : 1.0f, s2b = has_b ? p.wb.scale2[el] : 1.0f;
-    // source addresses of this thread's pieces, advanced by a stage's bytes per stage. Weights: 16 tiles x 1 KB per stage (64 lanes x
-    // 16 bytes to a tile), scales: 16 tiles x 128 bytes; rows past the matrix read its last tile. Tokens past the last are not
+    // source addresses of this thread's pieces, advanced by a stage's bytes per stage. Weights: 2 W tiles x 1 KB per stage (64 lanes x
+    // 16 bytes to a tile), scales: 2 W tiles x 128 bytes; rows past the matrix read its last tile. Tokens past the last are not
     // staged: what stands in their place reaches only their own results, which nobody reads.
     const uint8_t* wsrc[4]; const uint8_t* ssrc; const __half* xsrc[XP];
     {
         const size_t eo = (size_t)el * n_out;
-        auto tile_row = [&](int tile) { return eo + min(r0 + (GLU ? (tile & 7) : tile) * 16, n_out - 16); };
+        auto tile_row = [&](int tile) { return eo + min(r0 + (GLU ? (tile & (W - 1)) : tile) * 16, n_out - 16); };
 #pragma unroll
-        for (int i = 0; i < 4; ++i) wsrc[i] = (GLU && i >= 2 ? p.wb.nib : p.wa.nib) + tile_row((tid >> 6) + i * 4) * (k / 2) + (tid & 63) * 16;
-        ssrc = (GLU && tid >= 64 ? p.wb.sc : p.wa.sc) + tile_row((tid >> 3) & 15) * (k / 16) + (tid & 7) * 16;
+        for (int i = 0; i < 4; ++i) wsrc[i] = (GLU && i >= 2 ? p.wb.nib : p.wa.nib) + tile_row((tid >> 6) + i * (W / 2)) * (k / 2) + (tid & 63) * 16;
+        ssrc = (GLU && tid >= 8 * W ? p.wb.sc : p.wa.sc) + tile_row((tid >> 3) & (2 * W - 1)) * (k / 16) + (tid & 7) * 16;
     }
     auto load_w = [&](int c) {
         unsigned char* st = smem + (c % C::NST) * C::STAGE;
         const bool half = 2 * c + 2 > kgs;           // the last stage of a row that ends with 64 elements
         if (!half || (tid & 63) < 32) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cp_async16(st + tid * 16 + i * 4096, wsrc[i] + (size_t)c * 1024, true);
+            for (int i = 0; i < 4; ++i) cp_async16(st + tid * 16 + i * W * 512, wsrc[i] + (size_t)c * 1024, true);
         }
-        if (tid < 128 && (!half || (tid & 7) < 4)) cp_async16(st + C::OFF_S + tid * 16, ssrc + (size_t)c * 128, true);
+        if (tid < 16 * W && (!half || (tid & 7) < 4)) cp_async16(st + C::OFF_S + tid * 16, ssrc + (size_t)c * 128, true);
     };
     auto load_x = [&](int c) {
         unsigned char* st = smem + (c % C::NST) * C::STAGE;
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
         if (!half || (tid & 15) < 8) {
 #pragma unroll
             for (int i = 0; i < XP; ++i)
-                if (xsrc[i]) cp_async16(st + C::OFF_X + ((tid >> 4) + i * 16) * EX_XSTR + (tid & 15) * 16, xsrc[i] + (size_t)c * EX_KC, true);
+                if (xsrc[i]) cp_async16(st + C::OFF_X + ((tid >> 4) + i * 2 * W) * EX_XSTR + (tid & 15) * 16, xsrc[i] + (size_t)c * EX_KC, true);
         }
     };
     auto load = [&](int c) { load_w(c); load_x(c); };
@@ -186,13 +190,13 @@ __global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
     if (tid < n) { s_pair[tid] = pr; s_row[tid] = pr / p.div; }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < XP; ++i) {                   // activations: 16 tokens x 16 pieces of 16 bytes
-        const int tk = (tid >> 4) + i * 16;
+    for (int i = 0; i < XP; ++i) {                   // activations: 2 W tokens x 16 pieces of 16 bytes
+        const int tk = (tid >> 4) + i * 2 * W;
         xsrc[i] = tk < n ? p.xh + (size_t)s_row[tk] * k + (tid & 15) * 8 : nullptr;
     }
 #pragma unroll
     for (int c = 0; c < C::NST - 1; ++c) { if (c < n_chunk) load_x(c); cp_async_commit(); }
-    for (int tk = wid; tk < n; tk += 8)               // the tile's activation scales, [block][token]
+    for (int tk = wid; tk < n; tk += W)               // the tile's activation scales, [block][token]
         for (int b2 = lane; b2 < nb / 2; b2 += 32) {
             const float2 v = *(const float2*)(p.xs + (size_t)s_row[tk] * nb + 2 * b2);
             s_xs[(2 * b2) * C::TOK + tk] = v.x; s_xs[(2 * b2 + 1) * C::TOK + tk] = v.y;
@@ -231,29 +235,29 @@ __global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
     }
     cp_async_wait<0>();
     if (GLU) {
-        // the gate and up results go to [token][128 rows] tiles in the ring's memory; from there a warp takes a token's 32 rows:
+        // the gate and up results go to [token][16 W rows] tiles in the ring's memory; from there a warp takes a token's 32 rows:
         // silu(gate * s_g) * (up * s_u) (src/ops/mod.rs:1105-1117), quantised to Q8_0 where the consumer is the down projection (it
         // would do the same), stored in whole pieces. (The library-exact exponential is a call: made here it has no accumulators to save.)
-        float* vg = (float*)smem; float* vu = vg + C::TOK * EX_VS;
+        float* vg = (float*)smem; float* vu = vg + C::TOK * VS;
         __syncthreads();                             // every warp is done with the ring
         if (rows_live) {
-            const int o = 2 * t * EX_VS + wid * 16 + g;
+            const int o = 2 * t * VS + wid * 16 + g;
 #pragma unroll
             for (int j = 0; j < NJ; ++j) {
                 if (NJ > 1 && j >= nja) break;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int at = o + (8 * j + (i & 1)) * EX_VS + (i >> 1) * 8;
+                    const int at = o + (8 * j + (i & 1)) * VS + (i >> 1) * 8;
                     vg[at] = f32_of_pair(acc[0][j][i >> 1], i & 1); vu[at] = f32_of_pair(acc[1][j][i >> 1], i & 1);
                 }
             }
         }
         __syncthreads();
-        const int q = wid & 3, row = r0 + q * 32;    // the warp's 32 rows, every other token
+        const int q = wid % (W / 2), row = r0 + q * 32;    // the warp's 32 rows, every other token
         if (row < n_out)
 #pragma unroll 1
-            for (int tk = wid >> 2; tk < n; tk += 2) {
-                float gv = vg[tk * EX_VS + q * 32 + lane], uv = vu[tk * EX_VS + q * 32 + lane];
+            for (int tk = wid / (W / 2); tk < n; tk += 2) {
+                float gv = vg[tk * VS + q * 32 + lane], uv = vu[tk * VS + q * 32 + lane];
                 if (has_a) gv = gv * s2a;
                 if (has_b) uv = uv * s2b;
                 const float val = silu_f(gv) * uv;
@@ -291,14 +295,15 @@ __global__ void __launch_bounds__(256, 2) k_exp(ExpArgs p) {
 template <int NJ, bool GLU>
 static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) {
     itb_raise_smem(k_exp<NJ, GLU>, EX_SMEM);
-    itb_chain(k_exp<NJ, GLU>, dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + (GLU ? 127 : 255)) / (GLU ? 128 : 256))), 256, exp_smem<NJ>(a.wa.n_in), st, a);
+    constexpr int W = ExpCfg<NJ>::W, RB = GLU ? 16 * W : 32 * W;
+    itb_chain(k_exp<NJ, GLU>, dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + RB - 1) / RB)), 32 * W, exp_smem<NJ>(a.wa.n_in), st, a);
 }
 // The activation scales of a tile's whole rows lie beside the ring: up to 22,464 elements of k with 48 tokens.
 static inline bool exp_k_ok(int k) { return exp_smem<6>(k) <= EX_SMEM; }
 // Pairs per tile: 16, 32 or 48. A larger tile decodes an expert's weights once for more of its pairs; a smaller one has fewer
 // accumulators and less of shared memory in activations, and an expert's pairs are cut evenly, so tiles of 32 end less unevenly than
-// tiles of 48. Gate + up and down of 256 experts (2048 x 512), 8 pairs to a row, in us with 16 / 32 / 48 pairs: 128 rows 129 / 132 /
-// 138, 256 rows 154 / 156 / 162, 384 rows 189 / 187 / 192, 512 rows 236 / 213 / 218, 768 rows 321 / 278 / 279, 1,024 rows 406 / 358 /
+// tiles of 48. Gate + up and down of 256 experts (2048 x 512), 8 pairs to a row, in us with 16 / 32 / 48 pairs: 128 rows 122 / 132 /
+// 138, 256 rows 152 / 156 / 162, 384 rows 188 / 187 / 192, 512 rows 233 / 213 / 218, 768 rows 321 / 278 / 279, 1,024 rows 399 / 358 /
 // 334, 5,548 rows 1909 / 1606 / 1497: 16 up to 8 pairs per expert on average, 32 up to 24. (64 pairs leave room for two stages only and
 // spill: 180, 214, 240, 304, 365 and 1565 us from 256 rows on.) Where that leaves SMs without a block (few experts or short rows):
 // as many pairs as give every SM four blocks.
