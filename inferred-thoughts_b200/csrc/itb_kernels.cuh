@@ -243,10 +243,10 @@ __device__ __forceinline__ void block_topk(const float* p, int n_expert, int n_u
     __syncthreads();
 }
 // The same rule inside ONE warp, probabilities in registers (expert e = lane + 32*j), no block barrier:
-// every round is a lane-local scan plus a five-step shuffle reduction. All lanes return the picks in
-// ids/wts (arrays of 16). p may be shared or global memory; n_expert <= 32*EPL.
+// every round is a lane-local scan plus a five-step shuffle reduction. Lane k returns pick k and its weight (n_used <= 16), so the
+// divisions are one. p may be shared or global memory; n_expert <= 32*EPL.
 template <int EPL>
-__device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_used, int32_t* ids, float* wts) {
+__device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_used, int32_t& id, float& w) {
     const int lane = threadIdx.x & 31;
     float v[EPL];
 #pragma unroll
@@ -255,6 +255,7 @@ __device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_us
 #pragma unroll
     for (int j = 0; j < EPL; ++j) if (lane + 32 * j >= n_expert) taken |= 1u << j;
     float sum = 0.0f;
+    id = 0; w = 0.0f;
     for (int r = 0; r < n_used; ++r) {
         float bv = -INFINITY; int bi = 0x7fffffff;
 #pragma unroll
@@ -266,18 +267,17 @@ __device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_us
             if (oi != 0x7fffffff && (bi == 0x7fffffff || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
         }
         if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
-        ids[r] = bi; wts[r] = bv;
+        if (lane == r) { id = bi; w = bv; }
         sum += bv;                      // summed in pick order (src/ops/mod.rs:1211)
     }
-    float denom = fmaxf(sum, 6.103515625e-5f);
-    for (int r = 0; r < n_used; ++r) wts[r] = wts[r] / denom;
+    w = w / fmaxf(sum, 6.103515625e-5f);
 }
-__device__ __forceinline__ void warp_topk_any(const float* p, int n_expert, int n_used, int32_t* ids, float* wts) {
-    if (n_expert <= 32) warp_topk<1>(p, n_expert, n_used, ids, wts);
-    else if (n_expert <= 128) warp_topk<4>(p, n_expert, n_used, ids, wts);
-    else if (n_expert <= 256) warp_topk<8>(p, n_expert, n_used, ids, wts);
-    else if (n_expert <= 512) warp_topk<16>(p, n_expert, n_used, ids, wts);
-    else warp_topk<32>(p, n_expert, n_used, ids, wts);
+__device__ __forceinline__ void warp_topk_any(const float* p, int n_expert, int n_used, int32_t& id, float& w) {
+    if (n_expert <= 32) warp_topk<1>(p, n_expert, n_used, id, w);
+    else if (n_expert <= 128) warp_topk<4>(p, n_expert, n_used, id, w);
+    else if (n_expert <= 256) warp_topk<8>(p, n_expert, n_used, id, w);
+    else if (n_expert <= 512) warp_topk<16>(p, n_expert, n_used, id, w);
+    else warp_topk<32>(p, n_expert, n_used, id, w);
 }
 
 __global__ void k_route(const float* probs, int n_expert, int n_used, int32_t* ids, float* wts) {
@@ -292,10 +292,9 @@ __global__ void __launch_bounds__(128) k_route_warp(const float* probs, int n_to
     pdl_wait();
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= n_tok) return;
-    int32_t ids[16]; float wts[16];
-    warp_topk_any(probs + (size_t)t * n_expert, n_expert, n_used, ids, wts);
-    if (lane == 0)
-        for (int k = 0; k < n_used; ++k) { ids_out[(size_t)t * n_used + k] = ids[k]; w_out[(size_t)t * n_used + k] = wts[k]; }
+    int32_t id; float w;
+    warp_topk_any(probs + (size_t)t * n_expert, n_expert, n_used, id, w);
+    if (lane < n_used) { ids_out[(size_t)t * n_used + lane] = id; w_out[(size_t)t * n_used + lane] = w; }
 }
 
 // Weighted expert sum + gated shared expert (src/ops/mod.rs:1134-1171): ascending picks, shared last.

@@ -706,8 +706,9 @@ __global__ void k_gather_last(const float* x, int n, int n_tok, float* out) {
 // =====================================================================================================
 namespace {
 
-// Softmax over all experts + top-k per row (src/model/qwen35.rs:1626-1638, src/ops/mod.rs:1191-1216). One warp per row.
-__global__ void k_route_rows(const float* router, int n_rows, int n_expert, int n_used, int32_t* ids_out, float* w_out) {
+// Softmax over all experts + top-k per row (src/model/qwen35.rs:1626-1638, src/ops/mod.rs:1191-1216). One warp per row. What bounds it is
+// the one chain after another: the sum (in index order; its terms are read 32 ahead, or each add would wait for its own read) and the rounds of picks.
+__global__ void __launch_bounds__(128) k_route_rows(const float* router, int n_rows, int n_expert, int n_used, int32_t* ids_out, float* w_out) {
     pdl_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -717,20 +718,26 @@ __global__ void k_route_rows(const float* router, int n_rows, int n_expert, int 
     if (r >= n_rows) return;
     const float* lg = router + (size_t)r * n_expert;
     float mx = -INFINITY;
-    for (int i = lane; i < n_expert; i += 32) mx = fmaxf(mx, lg[i]);
+#pragma unroll 4
+    for (int i = lane; i < n_expert; i += 32) { const float v = lg[i]; probs[i] = v; mx = fmaxf(mx, v); }
     mx = warp_max(mx);
-    for (int i = lane; i < ne32; i += 32) probs[i] = i < n_expert ? exp_f(lg[i] - mx) : 0.0f;
+    for (int i = lane; i < ne32; i += 32) probs[i] = i < n_expert ? exp_f(probs[i] - mx) : 0.0f;       // behind the end: terms that change no sum
     __syncwarp();
     float sum = 0.0f;
-    if (lane == 0) for (int i = 0; i < n_expert; ++i) sum += probs[i];
-    sum = __shfl_sync(0xffffffffu, sum, 0);
+#pragma unroll 1
+    for (int i = 0; i < ne32; i += 32) {
+        float4 a[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = *(const float4*)(probs + i + 4 * j);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { sum += a[j].x; sum += a[j].y; sum += a[j].z; sum += a[j].w; }
+    }
+    __syncwarp();                                    // every lane has read all of them
     for (int i = lane; i < n_expert; i += 32) probs[i] /= sum;
     __syncwarp();
-    int32_t ids[16];
-    float wts[16];
-    warp_topk_any(probs, n_expert, n_used, ids, wts);
-    if (lane == 0)
-        for (int k = 0; k < n_used; ++k) { ids_out[(size_t)r * n_used + k] = ids[k]; w_out[(size_t)r * n_used + k] = wts[k]; }
+    int32_t id; float w;
+    warp_topk_any(probs, n_expert, n_used, id, w);
+    if (lane < n_used) { ids_out[(size_t)r * n_used + lane] = id; w_out[(size_t)r * n_used + lane] = w; }
 }
 
 // silu(gate) * up of the shared expert per row, quantised (src/model/qwen35.rs:1669-1678). block per row.
@@ -751,11 +758,19 @@ __global__ void k_moe_finish_rows(float* x, int n, const float* o, const float* 
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t r = i / n; const int j = (int)(i % n);
-    const float g = sigmoid_f(logit[r]);
+    const float lg = logit[r], sh = shared[r * n + j], xv = x[i];
     float v = 0.0f;
-    for (int k = 0; k < n_used; ++k) v += wts[r * n_used + k] * o[(r * n_used + k) * n + j];
-    v += shared[r * n + j] * g;
-    x[i] += v;
+    for (int k0 = 0; k0 < n_used; k0 += 8) {         // eight picks' loads in flight, and the exponential under the first eight's
+        float wv[8], rv[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < n_used) { wv[k] = wts[r * n_used + k0 + k]; rv[k] = o[(r * n_used + k0 + k) * n + j]; }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < n_used) v += wv[k] * rv[k];
+    }
+    v += sh * sigmoid_f(lg);
+    x[i] = xv + v;
 }
 
 }  // namespace
