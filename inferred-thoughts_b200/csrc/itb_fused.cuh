@@ -590,12 +590,13 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
         __syncthreads();
     };
     // The picks are by probability, and probabilities are the numerators over one sum: the same order, unless the division rounds two
-    // different numerators to one value. So the numerators are ranked without waiting for the sum (serial, in index order), and only where
-    // two neighbours among the picks and the first one after them are closer than that could be (or so small that quotients lose bits) are the probabilities ranked
-    // instead. The weights, which need the sum, are one block's work beside the others' rows.
+    // different numerators to one value. So the numerators are ranked without waiting for the sum (serial, in index order), and the probabilities
+    // instead only where two neighbours among the picks and the first one after them differ by less than that could take (or are so small that
+    // quotients lose bits), or where the last pick and that one are equal: one behind them, which is not looked at, may be close to both.
+    // The weights, which need the sum, are one block's work beside the others' rows.
     select();
     const float va = lane < nu ? s_val[lane] : 0.0f, vb = lane < nu ? s_val[lane + 1] : 0.0f;
-    const bool close = __any_sync(0xffffffffu, lane < nu && va != vb && (va - vb <= va * 4.8e-7f || va < 1e-30f));      // the same in every warp
+    const bool close = __any_sync(0xffffffffu, lane < nu && (va == vb ? lane == nu - 1 : va - vb <= va * 4.8e-7f || va < 1e-30f));      // the same in every warp
     if (close || writer) {
         // softmax denominator: serial sum in index order (src/ops/naive.rs:362-376), one thread
         if (tid == 0) {

@@ -150,6 +150,48 @@ def test_one_token_routing_where_probabilities_tie(oracle, gpu, rows):
     a.close(); b.close(); m.close()
 
 
+def test_one_token_routing_where_the_last_pick_ties_with_two_behind_it(oracle, gpu):
+    """At the cut two experts have equal router logits and a third of lower id has the next smaller one: for some sums the division makes
+    the three one probability, and the third is the pick. Layer 0's logits are made by hand (its FFN's input is the embedding, of which the
+    router reads one element), a token per sum; picks and logits as the multi-row pass has them."""
+    from inferred_thoughts_b200 import host
+    ops, _ = gpu
+    m = host.Model(ops, host_dims(TINY))
+    E, H, L, K = TINY["n_expert"], TINY["n_embd"], TINY["n_layer"], TINY["n_expert_used"]
+    w = np.zeros((E, H), np.float32)
+    w[:, 0] = np.linspace(0.01, 0.04, E)
+    w[[13, 14, 15], 0] = 0.055, 0.057, 0.059
+    w[[5, 9], 0] = 0.05
+    w[1, 0] = np.nextafter(w[5, 0], np.float32(0))
+    x = np.zeros((TINY["n_vocab"], H), np.float32)
+    x[:, 0] = 1
+    x[:, 1] = np.linspace(0, 0.8, TINY["n_vocab"])
+    made = {"blk.0.ffn_gate_inp.weight": w, "token_embd.weight": x, "blk.0.post_attention_norm.weight": np.ones(H, np.float32)}
+    for sp in oracle.specs:
+        data, sc = oracle.tensor(sp["name"])
+        if sp["name"] in made:
+            assert data.size == made[sp["name"]].nbytes
+            data = made[sp["name"]].reshape(-1).view(np.uint8)
+        elif sp["name"] == "blk.0.ssm_out.weight":
+            data = np.zeros_like(data)
+        m.set_tensor(sp["name"], sp["ty"], data, sc)
+    a, b = host.Engine(m, 16, 1), host.Engine(m, 16, 1)
+    third = 0
+    for tok in range(0, TINY["n_vocab"], 4):
+        a.reset(); b.reset()
+        a.prefill(np.array([tok], np.uint32))
+        step, _ = a.decode([tok])
+        rows = b.prefill(np.array([tok, tok], np.uint32))
+        want = b.read_routes(L, K)[:, 0].tolist()
+        assert a.read_routes(L, K)[:, 0].tolist() == want, tok
+        assert step.reshape(-1).view(np.uint32).tolist() == rows.reshape(-1).view(np.uint32).tolist(), tok
+        assert set(want[0][:3]) == {13, 14, 15} and want[0][3] in (1, 5), want[0]
+        third += want[0][3] == 1
+    assert 8 <= third <= 248, third                   # both outcomes were there
+    ops.check()
+    a.close(); b.close(); m.close()
+
+
 def test_batch_of_sequences_equals_single_sequences(oracle, gpu):
     """Three sequences in one engine (multi-row passes: int8-MMA matmuls, per-sequence state and KV) give the bits the
     same sequences give alone, through prefill and through decode steps."""
