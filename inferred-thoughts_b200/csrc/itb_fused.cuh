@@ -560,21 +560,22 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     TL(TLK_MOE_GLU, 2);
     // Top-k without serial rounds, in two stages of counting. An expert's place in an order is the number of experts that beat it:
     // greater value, or equal and lower id (src/ops/mod.rs:1191-1216 picks by strict '>' scanning ascending ids) -- one compare of
-    // (value bits, ~id) keys, values being >= 0. Stage 1: every 32-group ranks itself by shuffles and keeps its first `keep`; stage 2: those
+    // (value bits, ~id) keys, values being >= 0. By bits also inside a group: a row that holds a NaN is NaN throughout, and compares of such
+    // would leave places without an expert. Stage 1: every 32-group ranks itself by shuffles and keeps its first `keep`; stage 2: those
     // candidates (the overall picks are among them) are ranked against each other, eight threads to a candidate.
     const int ng = (p.n_expert + 31) >> 5, nu = p.n_used, keep = nu + 1;
     auto select = [&] {
         if (tid < 17) { s_ids[tid] = -1; s_val[tid] = -1.0f; }
         for (int g = wid; g < ng; g += (int)(blockDim.x >> 5)) {
             const int t = g * 32 + lane;
-            const float v = t < p.n_expert ? probs[t] : -1.0f;
+            const int v = t < p.n_expert ? __float_as_int(probs[t]) : INT_MIN;
             int rank = 0;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-                const float q = __shfl_sync(0xffffffffu, v, j);
+                const int q = __shfl_sync(0xffffffffu, v, j);
                 rank += (int)(q > v) | ((int)(q == v) & (int)(j < lane));   // bitwise: no branches
             }
-            if (rank < keep) s_cand[g * keep + rank] = t < p.n_expert ? ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)~t : 0ull;
+            if (rank < keep) s_cand[g * keep + rank] = t < p.n_expert ? ((unsigned long long)(unsigned)v << 32) | (unsigned)~t : 0ull;
         }
         __syncthreads();
         const int cnt = ng * keep;
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(NWG * 32) k_moe_glu(MoeGlu p) {
     // The weights, which need the sum, are one block's work beside the others' rows.
     select();
     const float va = lane < nu ? s_val[lane] : 0.0f, vb = lane < nu ? s_val[lane + 1] : 0.0f;
-    const bool close = __any_sync(0xffffffffu, lane < nu && (va == vb ? lane == nu - 1 : va - vb <= va * 4.8e-7f || va < 1e-30f));      // the same in every warp
+    const bool close = __any_sync(0xffffffffu, lane < nu && (va == vb ? lane == nu - 1 : !(va - vb > va * 4.8e-7f) || va < 1e-30f));      // the same in every warp; a NaN is close to anything
     if (close || writer) {
         // softmax denominator: serial sum in index order (src/ops/naive.rs:362-376), one thread
         if (tid == 0) {

@@ -244,13 +244,14 @@ __device__ __forceinline__ void block_topk(const float* p, int n_expert, int n_u
 }
 // The same rule inside ONE warp, probabilities in registers (expert e = lane + 32*j), no block barrier:
 // every round is a lane-local scan plus a five-step shuffle reduction. Lane k returns pick k and its weight (n_used <= 16), so the
-// divisions are one. p may be shared or global memory; n_expert <= 32*EPL.
+// divisions are one. p may be shared or global memory; n_expert <= 32*EPL. A NaN (a softmax row that holds one is NaN throughout) ranks below
+// everything, so that lanes agree on each pick and every pick is an expert; its weight is NaN.
 template <int EPL>
 __device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_used, int32_t& id, float& w) {
     const int lane = threadIdx.x & 31;
     float v[EPL];
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) v[j] = lane + 32 * j < n_expert ? p[lane + 32 * j] : 0.0f;
+    for (int j = 0; j < EPL; ++j) { const float a = lane + 32 * j < n_expert ? p[lane + 32 * j] : 0.0f; v[j] = a == a ? a : -INFINITY; }
     uint32_t taken = 0;
 #pragma unroll
     for (int j = 0; j < EPL; ++j) if (lane + 32 * j >= n_expert) taken |= 1u << j;
@@ -267,6 +268,7 @@ __device__ __forceinline__ void warp_topk(const float* p, int n_expert, int n_us
             if (oi != 0x7fffffff && (bi == 0x7fffffff || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
         }
         if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
+        if (bv == -INFINITY) bv = p[bi];
         if (lane == r) { id = bi; w = bv; }
         sum += bv;                      // summed in pick order (src/ops/mod.rs:1211)
     }

@@ -869,33 +869,34 @@ __device__ __forceinline__ void mg_stage_glu(const MegaParams& p, MegaCtl* ctl, 
     }
     csync();
     {
-        // top-k in two stages of counting (an expert's place = how many beat it: greater, or equal with a lower id)
+        // top-k in two stages of counting (an expert's place = how many beat it: greater, or equal with a lower id). Probabilities are >= 0 and
+        // are compared by their bits: in a row that holds a NaN all are NaN, and compares of such would leave places without an expert.
         const int ng = (ne + 31) >> 5;
         for (int g = wid; g < ng; g += MG_NW) {
             const int t = g * 32 + lane;
-            const float v = t < ne ? probs[t] : -1.0f;
+            const int v = t < ne ? __float_as_int(probs[t]) : INT_MIN;
             int rank = 0;
 #pragma unroll 8
             for (int j = 0; j < 32; ++j) {
-                const float q = __shfl_sync(0xffffffffu, v, j);
+                const int q = __shfl_sync(0xffffffffu, v, j);
                 rank += (int)(q > v) | ((int)(q == v) & (int)(j < lane));
             }
-            if (rank < nu) { cand_p[g * nu + rank] = v; cand_i[g * nu + rank] = t < ne ? t : -1; }
+            if (rank < nu) { cand_p[g * nu + rank] = __int_as_float(v); cand_i[g * nu + rank] = t < ne ? t : -1; }
         }
         csync();
         const int cnt = ng * nu;
         for (int c = tid; c < cnt; c += MG_CT) {
-            const float v = cand_p[c];
+            const int v = __float_as_int(cand_p[c]);
             const int id = cand_i[c];
             if (id < 0) continue;
             int rank = 0;
 #pragma unroll 8
             for (int j = 0; j < cnt; ++j) {
-                const float q = cand_p[j];
+                const int q = __float_as_int(cand_p[j]);
                 const int qi = cand_i[j];
                 rank += (int)(qi >= 0) & ((int)(q > v) | ((int)(q == v) & (int)(qi < id)));
             }
-            if (rank < nu) { ctl->ids[rank] = min(max(id, 0), ne - 1); s_wts[rank] = v; }   // in range whatever the logits were (a NaN ranks first everywhere)
+            if (rank < nu) { ctl->ids[rank] = id; s_wts[rank] = __int_as_float(v); }
         }
     }
     csync();

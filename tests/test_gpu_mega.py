@@ -134,3 +134,25 @@ def test_a_wait_that_runs_out_fails_the_call_and_leaves_the_engine_usable():
     assert np.isfinite(lg).all()
     ops.check()
     stuck.close(); good.close(); model.close(); ops.close()
+
+
+def test_picks_of_a_row_that_holds_a_nan_are_experts():
+    """One NaN in a layer's router makes its softmax rows NaN throughout: every path picks the first experts from there on, whatever the numbers are."""
+    from inferred_thoughts_b200 import host
+    ops = host.B200Ops(0, "exact=1")
+    model = host.Model(ops, host_dims(MID)); model.synth(configs.SEEDS["mid"])
+    E, H, L, K = MID["n_expert"], MID["n_embd"], MID["n_layer"], MID["n_expert_used"]
+    w = np.zeros((E, H), np.float32)
+    w[7, 3] = np.nan
+    model.set_tensor("blk.1.ffn_gate_inp.weight", host.F32, w.reshape(-1))
+    prompt = prompt_ids(44, 3, MID["n_vocab"])
+    first = list(range(K))
+    for eng in (_engine(host, model, 16, False), _engine(host, model, 16, True)):
+        logits = eng.prefill(prompt)
+        assert np.isnan(logits).all() and eng.read_routes(L, K)[1:, 0].tolist() == [first] * (L - 1)
+        logits, nxt = eng.decode([prompt[0]])
+        assert np.isnan(logits).all() and eng.read_routes(L, K)[1:, 0].tolist() == [first] * (L - 1)
+        assert 0 <= int(nxt[0]) < MID["n_vocab"]
+        eng.close()
+    ops.check()
+    model.close(); ops.close()

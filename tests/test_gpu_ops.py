@@ -317,6 +317,22 @@ def test_route_exact_including_tie_tables(ops):
     assert ids.tolist() == tied[:10]
 
 
+@pytest.mark.parametrize("E,K", [(16, 4), (50, 10), (64, 4), (256, 8), (512, 10), (1000, 16)])
+def test_route_of_rows_that_hold_a_nan(ops, E, K):
+    """A softmax row that holds one is NaN throughout: the picks are the first experts, as the scan of the CPU path has them, the weights NaN."""
+    p = np.exp(noise(5 * E, 121)).astype(np.float32).reshape(5, E)
+    p /= p.sum(1, keepdims=True)
+    p[[1, 4]] = np.nan
+    probs = keep(p.reshape(-1).copy())
+    ops.begin_pass(5)
+    r = ops.route(probs, E, K); ids, w = ops.read_route(r); ops.check()
+    wi = np.zeros(5 * K, np.int32); ww = np.zeros(5 * K, np.float32)
+    L.orc_route(probs, probs.size, E, K, wi, ww)
+    assert wi.reshape(5, K)[[1, 4]].tolist() == [list(range(K))] * 2
+    assert ids.tolist() == wi.tolist()
+    assert ((w.view(np.uint32) == ww.view(np.uint32)) | (np.isnan(w) & np.isnan(ww))).all()
+
+
 def _zipf_logits(n_tok, n_expert, seed, s=1.1):
     """Router logits whose softmax is Zipf(s) over a per-token random ranking of the experts (BASELINE config 2's skew)."""
     rng = np.random.default_rng(seed)
