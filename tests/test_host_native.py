@@ -147,6 +147,41 @@ def test_transfers_whose_events_cannot_be_recorded_or_waited_for(tmp_path):
     run(tmp_path, FAKE_RUNTIME + "int main() { no_record = true; transfers(); no_record = false; no_wait = true; transfers(); return 0; }")
 
 
+def test_copy_threads_are_counted_by_the_cpus_and_woken_once(tmp_path):
+    """Half of the CPUs copy, the caller's own among them, and the caller pays for one wake a piece at most (for none of the pieces that
+    find the threads still looking): threads by the dozen, each woken for each piece, made a copy on eight CPUs slower than one memcpy."""
+    run(tmp_path, FAKE_RUNTIME + r"""
+#include <unistd.h>
+static int cpus = 1, wakes = 0;
+static pthread_t caller;
+extern "C" {
+int get_nprocs() noexcept { return cpus; }
+int sem_post(sem_t* s) noexcept { wakes += pthread_equal(pthread_self(), caller) != 0; return ((int (*)(sem_t*))dlsym(RTLD_NEXT, "sem_post"))(s); }
+}
+int main() {
+    caller = pthread_self();
+    const int want[][2] = {{1, 0}, {2, 0}, {4, 1}, {8, 3}, {16, 7}, {128, 7}};
+    std::vector<uint8_t> h((size_t)16 << 20), d(h.size()), back(h.size());
+    for (size_t i = 0; i < h.size(); ++i) h[i] = (uint8_t)(i * 2654435761u >> 13);
+    for (auto& w : want) {
+        HostPipe p;
+        cpus = w[0]; wakes = 0;
+        memset(d.data(), 0, d.size()); memset(back.data(), 0, back.size());
+        CHECK(p.up(nullptr, d.data(), h.data(), h.size()) == cudaSuccess);
+        run_to(issued);
+        CHECK((int)p.threads.size() == w[1]);
+        CHECK(wakes <= (int)(h.size() / HostPipe::UP_CHUNK));
+        usleep(2000);                                          // they sleep again, and are woken for the way down
+        wakes = 0;
+        CHECK(p.down(nullptr, back.data(), d.data(), h.size()) == cudaSuccess);
+        CHECK(wakes <= (int)(h.size() / HostPipe::CHUNK));
+        CHECK(d == h && back == h);
+    }
+    return 0;
+}
+""")
+
+
 def test_shares_whose_thread_is_refused_run_on_the_caller(tmp_path):
     """The correction table of log is built on all host threads inside a C entry point: a refused thread must not end the program."""
     run(tmp_path, FAKE_RUNTIME + r"""
