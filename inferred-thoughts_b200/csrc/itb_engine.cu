@@ -23,6 +23,7 @@ void itb_synth_fp4_raw(cudaStream_t st, uint64_t key, size_t per_expert, size_t 
                        unsigned* amax_tmp, float* scale2, uint8_t* raw);
 
 #include "itb_fused.cuh"
+#include "itb_side.h"
 #include "itb_mega.cuh"
 #include "itb_rows.cuh"
 #include "itb_exp.cuh"
@@ -1218,18 +1219,11 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
     cudaStreamIsCapturing(st, &cap_rows);
     const bool f16tc = c->f16tc && n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone;
     // Beside the main chain: alpha and beta while the input projections run, the shared expert while the routed ones do. Each is a few
-    // small kernels that leave most SMs idle, the serial-order chains among them. `beside` runs f on the second stream between two events;
-    // what it writes is read behind `meet`. Only kernels and this engine's buffers are involved, and of the context's scratch the
+    // small kernels that leave most SMs idle, the serial-order chains among them (SideStream). Only kernels and this engine's buffers are involved, and of the context's scratch the
     // row images of the dense matmuls, which nothing on the main chain touches between the two.
-    cudaStream_t cur = st;
     const bool two = chain && e->side;
-    auto beside = [&](auto f) {
-        if (!two) { f(); return; }
-        cudaEventRecord(e->fork, st); cudaStreamWaitEvent(e->side, e->fork, 0);
-        cur = e->side; f(); cur = st;
-        cudaEventRecord(e->join, e->side);
-    };
-    auto meet = [&] { if (two) cudaStreamWaitEvent(st, e->join, 0); };
+    SideStream sides(st, two ? e->side : nullptr, e->fork, e->join);
+    cudaStream_t& cur = sides.cur;
     auto gemm_n = [&](const DevQ8& w, const QRows& x, float* out, size_t stride, int mode, int R) {
         dense_q8(c, cur, w, x, R, out, stride, mode, n_tok > 1 && cap_rows == cudaStreamCaptureStatusNone);
         launches++;
@@ -1298,7 +1292,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
         if (L.recurrent) {
             const int rs = e->slot_of[il];
             const size_t state_stride = (size_t)n_v * sk * sk, conv_stride = (size_t)cd * (d.ssm_d_conv - 1);
-            beside([&] { f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn); });
+            sides.beside([&] { f32mm2(L.ssm_alpha, e->alpha, L.ssm_beta, e->beta, e->xn); });
             {
                 const DevQ8* ws[2] = {&L.wqkv, &L.wgate}; float* os[2] = {e->qkvc, e->z}; const size_t ss[2] = {(size_t)cd, (size_t)vd};
                 gemm_multi(2, ws, os, ss, xa);
@@ -1308,7 +1302,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             else itb_chain(k_conv_rows, dim3((cd + 127) / 128, R), 128, 0, st, cst, conv_stride, e->qkvc, e->qkvc2, n_tok, cd, L.conv1d, d.ssm_d_conv);
             launches++;
             itb_chain(k_conv_state, dim3((cd + 127) / 128, n_seq), 128, 0, st, cst, conv_stride, e->qkvc, n_tok, cd, d.ssm_d_conv); launches++;
-            meet();
+            sides.meet();
             launch_k(!two, (sk == 128 ? k_gdn_pre<4> : k_gdn_pre<2>), dim3(R, row_share(R, 2 * n_k + (n_v * sk + 127) / 128 + (n_v + 31) / 32, sms)), 256, 0, st, 
                 e->qkvc2, cd, e->alpha, e->beta, L.ssm_a, L.dt_bias, n_k, n_v, d.rms_eps, e->qh, e->kh, e->vh, e->gb); launches++;
             const size_t chunk_need = (size_t)n_seq * ((n_tok + GC - 1) / GC) * n_v * gdn_chunk_floats<128>();
@@ -1405,7 +1399,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
             if (L.shared4[2].nib) gemm_fp4d(L.shared4[2], e->sq, e->ss, e->shd, R, L.has_shared_s[2], L.shared_s[2]);
             else gemm(L.shared_down, c->quantised(e->sq, e->ss), e->shd, H, 0);
         };
-        if (two) beside([&] { shared_in(); shared_out(); }); else shared_in();
+        if (two) sides.beside([&] { shared_in(); shared_out(); }); else shared_in();
         f32mm2(L.gate_inp, e->router, L.shared_gate_inp, e->shlogit, e->xn);
         {
             const int K = d.n_expert_used, E = d.n_expert, ff = d.expert_ff;
@@ -1551,7 +1545,7 @@ static uint64_t enqueue_rows(itb_engine* e, cudaStream_t st, int n_seq, int n_to
                 launches++;
                 o_src = e->ep->o_mine;
             }
-            if (two) meet(); else shared_out();
+            if (two) sides.meet(); else shared_out();
             const size_t total = (size_t)R * H;
             launch_k(chain && !two, k_moe_finish_rows, (unsigned)((total + 255) / 256), 256, 0, st, e->x, H, o_src, wts, K, e->shd, e->shlogit, total); launches++;
         }

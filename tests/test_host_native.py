@@ -227,3 +227,46 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_work_beside_the_main_stream_is_met_on_every_way_out(tmp_path):
+    """A pass that ends early between beside and meet leaves the main stream waiting for the second one, whatever call was refused."""
+    run(tmp_path, CHECK + r"""
+#include <stdexcept>
+#include "itb_side.h"
+struct CUstream_st { int seen[2] = {0, 0}, done = 0; };      // per stream: work queued; of each stream's work, how much is ordered before what comes next
+struct CUevent_st { int at[2] = {0, 0}; };
+static CUstream_st S[2];
+static int refuse = 0, calls = 0;
+static bool no() { return ++calls == refuse; }
+extern "C" {
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { if (no()) return cudaErrorInvalidResourceHandle; const int i = (int)(s - S); for (int k = 0; k < 2; ++k) e->at[k] = k == i ? s->done : s->seen[k]; return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { if (no()) return cudaErrorInvalidResourceHandle; for (int k = 0; k < 2; ++k) if (s->seen[k] < e->at[k]) s->seen[k] = e->at[k]; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { const int i = (int)(s - S); S[1 - i].seen[i] = s->done; return cudaSuccess; }
+}
+static bool pass(bool two, int leave) {
+    CUevent_st fork, join;
+    SideStream x(&S[0], two ? &S[1] : nullptr, &fork, &join);
+    for (int layer = 0; layer < 3; ++layer) {
+        CHECK(S[0].seen[1] == S[1].done);                    // this layer's main chain comes behind all of the last one's side work
+        S[0].done++;
+        x.beside([&] { if (x.cur == &S[1]) CHECK(S[1].seen[0] == S[0].done); x.cur->done++; });
+        CHECK(x.cur == &S[0]);
+        S[0].done++;
+        if (layer == leave) return false;
+        if (layer == leave - 10) throw std::runtime_error("out");
+        x.meet();
+    }
+    return true;
+}
+int main() {
+    for (bool two : {false, true})
+        for (int r = 0; r < 12; ++r)
+            for (int leave : {-1, 0, 1, 2, 10, 11, 12}) {
+                S[0] = S[1] = CUstream_st(); refuse = r; calls = 0;
+                try { pass(two, leave); } catch (const std::exception&) {}
+                CHECK(S[0].seen[1] == S[1].done);            // the next pass too
+            }
+    return 0;
+}
+""")
