@@ -315,7 +315,9 @@ extern "C" void itb_matmul_pair(itb_ctx* c, const itb_weights* a, const itb_weig
     float* oa = itb_mirror_out(c, out_a, out_a_len); float* ob = itb_mirror_out(c, out_b, out_b_len);
     if (!xd || !oa || !ob) return;
     const bool f32 = a->ggml_type != ITB_Q8_0 && a->ggml_type != ITB_NVFP4 && b->ggml_type != ITB_Q8_0 && b->ggml_type != ITB_NVFP4;
-    if (f32 && c->exact && sgemm_chain_ok((int)a->n_in)) {       // the chains of both side by side: one launch, not one after the other
+    // the chains of both side by side: one launch, not one after the other. (Two shapes at one address, a matrix and its first rows: looking
+    // the second up drops the upload of the first, which therefore has to be launched before.)
+    if (f32 && c->exact && a->data != b->data && sgemm_chain_ok((int)a->n_in)) {
         const WeightEntry* wa = itb_weight(c, a->data, a->bytes, a->ggml_type, a->n_in, a->n_out, 1, nullptr, 0);
         const WeightEntry* wb = wa ? itb_weight(c, b->data, b->bytes, b->ggml_type, b->n_in, b->n_out, 1, nullptr, 0) : nullptr;
         if (!wb) return;

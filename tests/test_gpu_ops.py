@@ -317,6 +317,22 @@ def test_route_exact_including_tie_tables(ops):
     assert ids.tolist() == tied[:10]
 
 
+def test_matmul_pair_of_a_matrix_and_its_first_rows(ops):
+    """Two F32 matrices that begin at one address: weights are kept by address, so looking the second up frees the first's upload."""
+    from inferred_thoughts_b200 import host
+    n_in, n_tok = 128, 3
+    w = keep(noise(40 * n_in, 126)); x = keep(noise(n_tok * n_in, 127))
+    for na, nb in ((40, 8), (8, 40), (40, 40)):
+        a, b = (host.Weights(w[:n * n_in], host.F32, n_in, n) for n in (na, nb))
+        oa, ob = np.zeros(n_tok * na, np.float32), np.zeros(n_tok * nb, np.float32)
+        ops.begin_pass(n_tok)
+        ops.matmul_pair(a, b, x, oa, ob); ops.host_needs(oa); ops.host_needs(ob); ops.check()
+        for n, o in ((na, oa), (nb, ob)):
+            want = np.zeros_like(o)
+            L.orc_matmul(0, w[:n * n_in].view(np.uint8), n_in, n, x, x.size, want, 0)
+            exact(o, want, f"{na} and {nb} rows: the one of {n}")
+
+
 @pytest.mark.parametrize("E,K", [(16, 4), (50, 10), (64, 4), (256, 8), (512, 10), (1000, 16)])
 def test_route_of_rows_that_hold_a_nan(ops, E, K):
     """A softmax row that holds one is NaN throughout: the picks are the first experts, as the scan of the CPU path has them, the weights NaN."""
