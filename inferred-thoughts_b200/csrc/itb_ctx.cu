@@ -107,10 +107,10 @@ extern "C" int itb_create(int device_ordinal, const char* opts, itb_ctx** out) {
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) {
         g_create_error = cudaGetErrorString(e); delete c; return 5;
     }
-    if ((e = cudaHostAlloc((void**)&c->fail_word, 4, cudaHostAllocMapped)) != cudaSuccess) {
+    if ((e = c->fail.open()) != cudaSuccess) {
         g_create_error = cudaGetErrorString(e); cudaStreamDestroy(c->stream); delete c; return 6;
     }
-    *c->fail_word = 0;
+    if (const char* v = getenv("ITB_TEST_FAIL_WORD")) c->fail.set(atoi(v));      // tests: as if a kernel of the first call had given up
     std::string o = opts ? opts : "";
     if (o.find("kv=bf16") != std::string::npos) c->kv_bf16 = true;
     if (o.find("exact=0") != std::string::npos) c->exact = false;
@@ -143,7 +143,7 @@ extern "C" void itb_destroy(itb_ctx* c) {
     itb_tc_free(c);
     cudaFree(c->route_ids); cudaFree(c->route_w); cudaFree(c->xq); cudaFree(c->xs); cudaFree(c->tmp_f32);
     itb_pipe_free(c);
-    cudaFreeHost((void*)c->fail_word);
+    c->fail.close();
     cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -164,9 +164,8 @@ extern "C" const char* itb_take_error(itb_ctx* c) {
 extern "C" uint64_t itb_launch_count(itb_ctx* c) { return c->launches; }
 
 bool itb_status_ok(itb_ctx* c) {
-    const int v = *c->fail_word;
+    const int v = c->fail.take();
     if (!v) return true;
-    *c->fail_word = 0;
     return itb_fail_msg(c, std::string("a tensor-core kernel gave up a bounded wait (") + (v == 3 ? "operands" : v == 4 ? "issue" : "accumulators") + "): its results are not there");
 }
 

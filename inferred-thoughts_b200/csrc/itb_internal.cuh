@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/itb.h"
+#include "itb_failword.h"
 
 // ------------------------------------------------------------------ device-side weight layouts
 // Q8_0 matrix repacked from 34-byte blocks (src/quant/mod.rs:90-106) into two planes so rows can be
@@ -82,7 +83,7 @@ struct HostPipe;                 // pinned staging and copy threads of one conte
 struct itb_ctx {
     int device = 0;
     HostPipe* pipe = nullptr;
-    volatile int* fail_word = nullptr;   // host memory that the tensor-core kernels store to when a bounded wait runs out (itb_status_ok)
+    FailWord fail;           // what the tensor-core kernels store to when a bounded wait runs out (itb_status_ok)
     cudaStream_t stream = nullptr;
     std::string error;       // sticky first error
     std::string error_out;   // storage handed back by take_error

@@ -617,7 +617,7 @@ bool itb_tc_experts(itb_ctx* c, cudaStream_t st, const DevFp4& wg, const DevFp4*
     g.wg_img = tg->img; g.wg_sf = tg->sf; g.wu_img = tu ? tu->img : nullptr; g.wu_sf = tu ? tu->sf : nullptr;
     g.s2g = wg.scale2; g.s2u = wu ? wu->scale2 : nullptr; g.expert_lo = wg.expert_lo;
     g.b_img = c->tc_b_img; g.b_sf = c->tc_b_sf; g.tiles = tiles; g.n_tiles = c->tc_n_tiles; g.pair_list = pair_list;
-    g.n_out = wg.n_out; g.n_in = wg.n_in; g.out = out; g.out_stride = wg.n_out; g.status = c->fail_word;
+    g.n_out = wg.n_out; g.n_in = wg.n_in; g.out = out; g.out_stride = wg.n_out; g.status = c->fail.word;
     itb_raise_smem(k_tc_gemm<true, true>, tc_gemm_smem(true));
     itb_raise_smem(k_tc_gemm<true, false>, tc_gemm_smem(true));
     itb_raise_smem(k_tc_gemm<false, false>, tc_gemm_smem(false));
@@ -939,7 +939,7 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     }
     TcQ8 g{};
     g.a_img = it->second.img; g.a_sc = (const float*)it->second.sf; g.b_img = c->tc_q8_b; g.b_sc = c->tc_q8_sx; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_out = w.n_out;
-    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail_word;
+    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail.word;
     auto kernel = mt == 2 ? k_tc_q8<64, 2> : k_tc_q8<64, 1>;
     const size_t smem = mt == 2 ? Q8Cfg<64, 2>::SMEM : Q8Cfg<64, 1>::SMEM;
     itb_raise_smem(kernel, smem);
@@ -1200,7 +1200,7 @@ bool itb_tc_f16_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     }
     TcHf g{};
     g.a_img = it->second.img; g.b_img = c->tc_hf_b; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_rt = (int)rts; g.n_tt = (int)tts;
-    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail_word;
+    g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail.word;
     itb_raise_smem(k_tc_f16, tc_f16_smem());
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = std::min<size_t>((size_t)c->sm_count, rts * tts);

@@ -317,6 +317,41 @@ def test_route_exact_including_tie_tables(ops):
     assert ids.tolist() == tied[:10]
 
 
+@pytest.mark.parametrize("word,what", [(3, "operands"), (4, "issue"), (5, "accumulators")])
+def test_wait_that_ran_out_fails_the_call_that_waits_for_it_and_no_other(monkeypatch, word, what):
+    """The word that a tensor-core kernel leaves when it gives up a wait, stored from the host before the first call: a download, a prefill
+    and a look at the error each report it, and what comes next runs and is right."""
+    from inferred_thoughts_b200 import configs, host
+    from tests.util import host_dims
+    monkeypatch.setenv("ITB_TEST_FAIL_WORD", str(word))
+    made = [host.B200Ops(0, "exact=1,dense=q8tc") for _ in range(3)]
+    monkeypatch.delenv("ITB_TEST_FAIL_WORD")
+    down, pre, look = made
+    x = keep(noise(64, 125)); y = keep(x.copy())
+    down.begin_pass(1)
+    down.scale(y, 2.0); down.host_needs(y)
+    with pytest.raises(RuntimeError, match=f"gave up a bounded wait .{what}"):
+        down.check()
+    y[:] = x
+    down.begin_pass(1)
+    down.scale(y, 2.0); down.host_needs(y); down.check()
+    exact(y, 2 * x, "the call after it")
+    model = host.Model(pre, host_dims(configs.TINY)); model.synth(0)
+    eng = host.Engine(model, 16, 1)
+    with pytest.raises(RuntimeError, match="gave up a bounded wait"):
+        eng.prefill(np.arange(4, dtype=np.uint32))
+    eng.reset()
+    again = eng.prefill(np.arange(4, dtype=np.uint32)); pre.check()
+    eng.reset()
+    exact(again, eng.prefill(np.arange(4, dtype=np.uint32)), "logits after it")
+    with pytest.raises(RuntimeError, match="gave up a bounded wait"):
+        look.check()
+    look.check()
+    eng.close(); model.close()
+    for o in made:
+        o.close()
+
+
 def test_matmul_pair_of_a_matrix_and_its_first_rows(ops):
     """Two F32 matrices that begin at one address: weights are kept by address, so looking the second up frees the first's upload."""
     from inferred_thoughts_b200 import host

@@ -270,3 +270,36 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_word_of_a_wait_that_ran_out_where_pinned_memory_is_refused(tmp_path):
+    """Host memory or, without it, device memory: the word reads as stored, once, and a context needs both refused to fail."""
+    run(tmp_path, CHECK + r"""
+#include <string.h>
+#include "itb_failword.h"
+static bool no_pinned = false, no_device = false; static int alive = 0, device_reads = 0;
+extern "C" {
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { if (no_pinned) return cudaErrorMemoryAllocation; ++alive; *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { if (p) { --alive; free(p); } return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { if (no_device) return cudaErrorMemoryAllocation; ++alive; *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { if (p) { --alive; free(p); } return cudaSuccess; }
+cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { ++device_reads; memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+}
+int main() {
+    for (bool refused : {false, true}) {
+        no_pinned = refused;
+        FailWord f;
+        CHECK(f.take() == 0 && f.open() == cudaSuccess && f.on_device == refused && f.take() == 0);
+        for (int v : {3, 4, 5}) { *f.word = v; CHECK(f.take() == v && f.take() == 0); }
+        CHECK(refused == (device_reads > 0));
+        f.close();
+        CHECK(alive == 0 && !f.word);
+    }
+    no_device = true;
+    FailWord f;
+    CHECK(f.open() == cudaErrorMemoryAllocation && !f.word && f.take() == 0 && alive == 0);
+    return 0;
+}
+""")
