@@ -298,7 +298,7 @@ static inline void exp_launch(const ExpArgs& a, int max_tiles, cudaStream_t st) 
     constexpr int W = ExpCfg<NJ>::W, RB = GLU ? 16 * W : 32 * W;
     itb_chain(k_exp<NJ, GLU>, dim3((unsigned)max_tiles, (unsigned)((a.wa.n_out + RB - 1) / RB)), 32 * W, exp_smem<NJ>(a.wa.n_in), st, a);
 }
-// The activation scales of a tile's whole rows lie beside the ring: up to 22,464 elements of k with 48 tokens.
+// The activation scales of a tile's whole rows lie beside the ring: up to 21,312 elements of k with 48 tokens.
 static inline bool exp_k_ok(int k) { return exp_smem<6>(k) <= EX_SMEM; }
 // Pairs per tile: 16, 32 or 48. A larger tile decodes an expert's weights once for more of its pairs; a smaller one has fewer
 // accumulators and less of shared memory in activations, and an expert's pairs are cut evenly, so tiles of 32 end less unevenly than

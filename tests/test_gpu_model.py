@@ -375,6 +375,27 @@ def test_tree_mode_rows_equal_single_rows():
     eb.close(); model.close(); ops.close()
 
 
+def test_tolerance_class_router_tiles_of_many_rows_equal_those_of_few(monkeypatch):
+    """A pass of 1,700 rows takes the router's fused chains in tiles of 32 x 64, passes of 448 rows in 16 x 32: a chain is walked in the order of
+    k in either, and everything else of a pass is by token or by 64 tokens, so picks, logits and state are the same to the bit."""
+    from inferred_thoughts_b200 import host
+    dims = dict(MID, n_expert=257)
+    ops = host.B200Ops(0, "exact=0,dense=f16tc")
+    m = host.Model(ops, host_dims(dims)); m.synth(7)
+    prompt = prompt_ids(45, 1700, dims["n_vocab"])
+    seen = []
+    for rows in (448, 1728):
+        monkeypatch.setenv("ITB_ROWS", str(rows))
+        eng = host.Engine(m, 1728, 1)
+        logits = eng.prefill(prompt)
+        seen.append((logits.view(np.uint32).tolist(), eng.read_routes(dims["n_layer"], dims["n_expert_used"]).tolist(),
+                     [eng.read_ssm_state(il).view(np.uint32).tolist() for il in range(3)]))
+        ops.check(); eng.close()
+    assert seen[0][1] == seen[1][1]
+    assert seen[0] == seen[1]
+    m.close(); ops.close()
+
+
 def test_phase_timeline_records_every_structured_launch(oracle, gpu):
     """itb_timeline_arm/read: one decode step of the tiny model (3 GDN layers + 1 attention layer) fills one slot per structured
     launch, phase stamps ascending inside a launch and launches in order; disarmed, nothing is written."""

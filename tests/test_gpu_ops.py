@@ -475,9 +475,9 @@ def test_grouped_expert_tiles_of_32_and_of_48_pairs(ops, counts):
     exact(o, o_want, "matmul_experts(long rows)")
 
 
-@pytest.mark.parametrize("n_in", [18944, 19008, 22464, 22528])
+@pytest.mark.parametrize("n_in", [18944, 21312, 21376, 22528])
 def test_grouped_experts_with_rows_as_long_as_the_tiles_hold_and_longer(ops, n_in):
-    """The grouped form keeps a tile's activation scales in shared memory; longer rows take the form without tiles."""
+    """The grouped form keeps a tile's activation scales in shared memory, of rows of up to 21,312; longer ones take the form without tiles."""
     from inferred_thoughts_b200 import host
     E, n_out, n = 3, 32, 16
     wb, sc = nvfp4_weights(E, n_out, n_in, 171)
@@ -490,10 +490,12 @@ def test_grouped_experts_with_rows_as_long_as_the_tiles_hold_and_longer(ops, n_i
     exact(out, want, "experts of long rows")
 
 
-@pytest.mark.parametrize("n_tok,n_in,n_out", [(1, 64, 1), (15, 384, 16), (17, 2048, 33), (33, 448, 129), (300, 64, 1000), (321, 2048, 993)])
+@pytest.mark.parametrize("n_tok,n_in,n_out", [(1, 64, 1), (15, 384, 16), (17, 2048, 33), (33, 448, 129), (300, 64, 1000), (321, 2048, 993),
+                                              (200, 64, 257), (201, 448, 257), (2049, 64, 257), (2047, 448, 259)])
 def test_f32_matmul_tiles_at_their_edges(ops, n_tok, n_in, n_out):
-    """Chains per output in 16 x 16 and 32 x 64 tiles: fewer k steps than the ring has stages, ragged rows and outputs; inputs and outputs
-    on both sides of the sizes at which the copies to and from the host change."""
+    """Chains per output in tiles of 8 x 8 (few rows), 16 x 16 (200 of 257), 16 x 32 (300 of 1,000) and 32 x 32 (2,049 of 257): fewer k steps
+    than the ring has stages, ragged rows and outputs; inputs and outputs on both sides of the sizes at which the copies to and from the
+    host change."""
     from inferred_thoughts_b200 import host
     w, x = keep(noise(n_in * n_out, 160)), keep(noise(n_tok * n_in, 161))
     out = keep(np.zeros(n_tok * n_out, np.float32)); want = np.zeros_like(out)
@@ -503,6 +505,21 @@ def test_f32_matmul_tiles_at_their_edges(ops, n_tok, n_in, n_out):
         ops.matmul(host.Weights(w, host.F32, n_in, n_out), x, out); ops.host_needs(out); ops.check()
         L.orc_matmul(0, w.view(np.uint8), n_in, n_out, x, x.size, want, 0)
         exact(out, want, "F32 matmul")
+
+
+@pytest.mark.parametrize("n_tok,n_in", [(5, 192), (201, 448), (1000, 64), (2049, 128)])
+def test_f32_matmul_pair_of_257_and_one_outputs(ops, n_tok, n_in):
+    """Router and gate in one launch, in tiles of each size: the gate's blocks walk one output a thread."""
+    from inferred_thoughts_b200 import host
+    wa, wb, x = keep(noise(257 * n_in, 164)), keep(noise(n_in, 165)), keep(noise(n_tok * n_in, 166))
+    oa, ob = keep(np.zeros(n_tok * 257, np.float32)), keep(np.zeros(n_tok, np.float32))
+    ops.begin_pass(n_tok)
+    ops.matmul_pair(host.Weights(wa, host.F32, n_in, 257), host.Weights(wb, host.F32, n_in, 1), x, oa, ob)
+    ops.host_needs(oa); ops.host_needs(ob); ops.check()
+    for w, n, o in ((wa, 257, oa), (wb, 1, ob)):
+        want = np.zeros_like(o)
+        L.orc_matmul(0, w.view(np.uint8), n_in, n, x, x.size, want, 0)
+        exact(o, want, f"{n} outputs")
 
 
 @pytest.mark.parametrize("n_tok,n_in,n_out", [(64, 512, 1), (65, 2048, 257), (300, 2048, 257), (3001, 1536, 9), (127, 4096, 33),
