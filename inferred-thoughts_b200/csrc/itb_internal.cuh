@@ -117,7 +117,7 @@ struct itb_ctx {
     size_t tc_cap_tiles = 0, tc_cap_slots = 0, tc_cap_b = 0, tc_cap_sf = 0, tc_cap_codes = 0, tc_cap_scales = 0;
     // Q8_0 tensor path: the pass's activation rows as K32 block images (kept for a following matmul over the same rows)
     uint8_t* tc_q8_b = nullptr; float* tc_q8_sx = nullptr; size_t tc_cap_q8b = 0, tc_cap_q8sx = 0;
-    uint64_t tc_q8_src = 0; int tc_q8_src_rows = 0, tc_q8_src_in = 0, tc_q8_src_tile = 0;      // the quantisation (QRows::id) they were made from
+    uint64_t tc_q8_src = 0; int tc_q8_src_rows = 0, tc_q8_src_in = 0;      // the quantisation (QRows::id) they were made from
     uint8_t* tc_hf_b = nullptr; size_t tc_cap_hfb = 0;                 // dense=f16tc: the pass's activation rows as f16 operand tiles
     uint64_t tc_hf_src = 0; int tc_hf_src_rows = 0, tc_hf_src_in = 0;
     bool f16tc = false;     // opts dense=f16tc: many-row passes run the dense Q8_0 matmuls as f16 tcgen05 GEMMs over dequantised operands (tolerance class)

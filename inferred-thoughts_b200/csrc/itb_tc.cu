@@ -672,9 +672,9 @@ extern "C" int itb_fp4_quantize(itb_ctx* c, const float* x, size_t n, uint8_t* s
 // Dense Q8_0 matmuls of many-row passes on the tensor cores, bit for bit
 // =====================================================================================================
 // The CPU path's Q8_0 dot (src/ops/naive.rs:676-712) is, per 32-element block, an integer dot product, converted to f32,
-// times (weight scale * activation scale), added to the row's sum in block order. The dot of 128 weight rows against NT activation
-// rows is two tcgen05.mma kind::f16 (M 128, N NT, K 16 each, f32 accumulators in tensor memory, the second accumulating): int8 values
-// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. The accumulators of two to four
+// times (weight scale * activation scale), added to the row's sum in block order. The dot of 128 weight rows against 64 activation
+// rows is two tcgen05.mma kind::f16 (M 128, N 64, K 16 each, f32 accumulators in tensor memory, the second accumulating): int8 values
+// are exact in f16, products and sums are integers below 2^20, so the f32 accumulator IS the converted integer dot. The accumulators of two
 // stages fill tensor memory, so the tensor core runs blocks ahead while sixteen warps read a finished block back (tcgen05.ld) and apply the two
 // scales and the addition in the CPU's own order and rounding, two columns to an instruction (the products as fma with a zero the compiler
 // cannot see: the assembler fuses a packed multiply into the packed add behind it). The result equals the CPU path to the bit. What bounds it:
@@ -688,9 +688,11 @@ namespace {
 
 constexpr int Q8_EPW = 16;         // warps that read accumulators back
 constexpr int Q8_A_BLK = 128 * 64;                                         // bytes of a weight K32 block
-template <int NT, int MT> struct Q8Cfg {                                  // tokens and 128-row weight tiles of a block
-    static constexpr int KB = MT == 1 ? 256 / NT : 2;                     // K32 blocks per pipeline stage
+constexpr int Q8_NT = 64;          // tokens of a block
+template <int MT> struct Q8Cfg {                                          // 128-row weight tiles of a block
+    static constexpr int NT = Q8_NT, KB = MT == 1 ? 4 : 2;                // K32 blocks per pipeline stage
     static constexpr int ND = 512 / (MT * NT * KB);                       // stages whose accumulators tensor memory holds
+    static_assert(ND == 2, "two sets of accumulators take turns");
     static constexpr int B_BLK = NT * 64, O_B = MT * KB * Q8_A_BLK, O_SA = O_B + KB * B_BLK, O_SB = O_SA + MT * KB * 512, STAGE = O_SB + KB * NT * 4;      // A | B | weight scales | activation scales
     static constexpr int STAGES = 200 * 1024 / STAGE;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE + 128;
@@ -734,14 +736,14 @@ struct TcQ8 {
     unsigned long long zero2;                     // two f32 zeros the compiler knows nothing about
     long long* prof;                              // optional: 8 words per block, the first its cycles (ITB_TC_PROF=1)
 };
-// grid (weight rows / (128 MT), token tiles of NT); block 576: warps 0-15 read accumulators back and scale (lane quarter = warp % 4, NT / 4 columns of
+// grid (weight rows / (128 MT), token tiles of 64); block 576: warps 0-15 read accumulators back and scale (lane quarter = warp % 4, 16 columns of
 // every row tile by warp / 4), warp 16 fetches operands, warp 17 issues the MMAs.
-template <int NT, int MT>
+template <int MT>
 __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
-    using C = Q8Cfg<NT, MT>;
-    constexpr int STAGES = C::STAGES, STAGE = C::STAGE, KB = C::KB, ND = C::ND, CW = NT / 4, UW = CW < 16 ? CW : 16, UC = CW / UW, UNITS = KB * MT * UC;     // a unit: UW columns of a block's row tile
+    using C = Q8Cfg<MT>;
+    constexpr int NT = C::NT, STAGES = C::STAGES, STAGE = C::STAGE, KB = C::KB, ND = C::ND, CW = NT / 4, UNITS = KB * MT;     // a unit: this warp's CW columns of a block's row tile
     __shared__ unsigned long long s_full[STAGES], s_empty[STAGES], s_dfull[ND], s_dfree[ND];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
@@ -816,14 +818,14 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
         if (!ok && lane == 0) *p.status = 4;
     } else {
         const int quarter = wid & 3, col0 = (wid >> 2) * CW, row = quarter * 32 + lane;
-        unsigned long long acc[MT * UC][UW / 2];     // f32 pairs: two columns to an instruction
+        unsigned long long acc[MT][CW / 2];          // f32 pairs: two columns to an instruction
 #pragma unroll
-        for (int m = 0; m < MT * UC; ++m)
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int j = 0; j < UW / 2; ++j) acc[m][j] = 0;
-        uint32_t d0[UW], d1[UW];
+            for (int j = 0; j < CW / 2; ++j) acc[m][j] = 0;
+        uint32_t d0[CW], d1[CW];
         // A stage's blocks are waited for, handed back and released together. open: its accumulators and scales are there. Unit i of
-        // it: UW of this warp's columns of row tile i / UC % MT of block i / (UC MT); load starts reading them (asynchronous: tc_wait_ld ends it).
+        // it: row tile i % MT of block i / MT; load starts reading them (asynchronous: tc_wait_ld ends it).
         int s_next = 0, dp = 0, dp_cur = 0, s_cur = 0; uint32_t p_next = 0, dphase = 0;
         auto open = [&] {
             wait(tc_smem(&s_dfull[dp]), dphase, tc_smem(&s_full[s_next]), p_next);
@@ -832,28 +834,28 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
             if (++s_next == STAGES) { s_next = 0; p_next ^= 1u; }
             if (++dp == ND) { dp = 0; dphase ^= 1u; }
         };
-        auto load = [&](int i, uint32_t (&d)[UW]) {
-            tc_ld(d, tm + (uint32_t)(MT * NT * KB * dp_cur + i / UC * NT + col0 + UW * (i % UC)) + ((uint32_t)(quarter * 32) << 16));
+        auto load = [&](int i, uint32_t (&d)[CW]) {
+            tc_ld(d, tm + (uint32_t)(MT * NT * KB * dp_cur + i * NT + col0) + ((uint32_t)(quarter * 32) << 16));
         };
         // the scales of a unit's columns: read once for a block's row tiles (a value for every lane: 32 lanes x 16 bytes are four cycles of the
         // block's shared memory, 512 for 128 x 128 outputs, more than their f32 operations)
-        ulonglong2 dx[UC][UW / 4];
+        ulonglong2 dx[CW / 4];
         // scale and add a unit in the CPU's order: sum += dot * (dw * dx)
-        auto scale_add = [&](const unsigned char* stage, int i, const uint32_t (&d)[UW]) {
-            const int blk = i / (UC * MT), m = i / UC % MT, u = i % UC;
+        auto scale_add = [&](const unsigned char* stage, int i, const uint32_t (&d)[CW]) {
+            const int blk = i / MT, m = i % MT;
             if (m == 0)
 #pragma unroll
-                for (int j = 0; j < UW / 4; ++j) dx[u][j] = *(const ulonglong2*)(stage + C::O_SB + (blk * NT + col0 + UW * u + 4 * j) * 4);
+                for (int j = 0; j < CW / 4; ++j) dx[j] = *(const ulonglong2*)(stage + C::O_SB + (blk * NT + col0 + 4 * j) * 4);
             const float dw = ((const float*)(stage + C::O_SA))[(m * KB + blk) * 128 + row];
             unsigned long long dw2;
             asm("mov.b64 %0, {%1, %1};" : "=l"(dw2) : "f"(dw));
 #pragma unroll
-            for (int j = 0; j < UW / 2; ++j)
+            for (int j = 0; j < CW / 2; ++j)
                 asm volatile("{ .reg .b64 s, q;\n"
                     "mov.b64 q, {%1, %2};\n"
                     "fma.rn.f32x2 s, %3, %4, %5; fma.rn.f32x2 q, q, s, %5;\n"
                     "add.rn.f32x2 %0, %0, q; }"
-                    : "+l"(acc[m * UC + u][j]) : "r"(d[2 * j]), "r"(d[2 * j + 1]), "l"(dw2), "l"(j & 1 ? dx[u][j / 2].y : dx[u][j / 2].x), "l"(p.zero2));
+                    : "+l"(acc[m][j]) : "r"(d[2 * j]), "r"(d[2 * j + 1]), "l"(dw2), "l"(j & 1 ? dx[j / 2].y : dx[j / 2].x), "l"(p.zero2));
         };
         long long* pf = p.prof ? p.prof + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 : nullptr;
         const long long t_begin = clock64();
@@ -883,23 +885,20 @@ __global__ void __launch_bounds__(Q8_EPW * 32 + 64, 1) k_tc_q8(TcQ8 p) {
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const size_t orow = ((size_t)rt * MT + m) * 128 + row;
-                auto column = [&](int j) { const unsigned long long v = acc[m * UC + j / UW][j % UW / 2]; return __uint_as_float((uint32_t)(j & 1 ? v >> 32 : v)); };
+                auto column = [&](int j) { const unsigned long long v = acc[m][j / 2]; return __uint_as_float((uint32_t)(j & 1 ? v >> 32 : v)); };
                 // mode 1 reads what it adds to: all of a batch's reads first, then the stores (a read placed after a store that may
                 // alias it waits for nothing, but the compiler keeps their order, and one read-add-store at a time is a memory round
                 // trip per column)
+                float old[CW];
 #pragma unroll
-                for (int j0 = 0; j0 < CW; j0 += UW) {
-                    float old[UW];
+                for (int j = 0; j < CW; ++j) {
+                    const int tok = tt * NT + col0 + j;
+                    old[j] = (p.mode && tok < p.n_rows) ? p.out[(size_t)tok * p.stride + orow] : 0.0f;
+                }
 #pragma unroll
-                    for (int j = 0; j < UW; ++j) {
-                        const int tok = tt * NT + col0 + j0 + j;
-                        old[j] = (p.mode && tok < p.n_rows) ? p.out[(size_t)tok * p.stride + orow] : 0.0f;
-                    }
-#pragma unroll
-                    for (int j = 0; j < UW; ++j) {
-                        const int tok = tt * NT + col0 + j0 + j;
-                        if (tok < p.n_rows) p.out[(size_t)tok * p.stride + orow] = p.mode ? __fadd_rn(old[j], column(j0 + j)) : column(j0 + j);
-                    }
+                for (int j = 0; j < CW; ++j) {
+                    const int tok = tt * NT + col0 + j;
+                    if (tok < p.n_rows) p.out[(size_t)tok * p.stride + orow] = p.mode ? __fadd_rn(old[j], column(j)) : column(j);
                 }
             }
         } else if (lane == 0) *p.status = 5;
@@ -916,7 +915,7 @@ bool itb_tc_q8_shape_ok(const DevQ8& w) { return w.n_in % 128 == 0 && w.n_out % 
 bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x, int n_rows, float* out, size_t stride, int mode) {
     if (!itb_tc_q8_shape_ok(w) || n_rows <= 0) return false;
     // 256 rows x 64 tokens to a block; half as much where that would leave half of the SMs without one (an output projection over 512 rows)
-    const size_t kbs = w.n_in / 32, rts = w.n_out / 128, nt = 64, tts = ((size_t)n_rows + nt - 1) / nt, mt = rts % 2 == 0 && rts / 2 * tts > (size_t)c->sm_count / 2 ? 2 : 1;
+    const size_t kbs = w.n_in / 32, rts = w.n_out / 128, nt = Q8_NT, tts = ((size_t)n_rows + nt - 1) / nt, mt = rts % 2 == 0 && rts / 2 * tts > (size_t)c->sm_count / 2 ? 2 : 1;
     auto it = c->tc_weights.find(w.q);
     if (it == c->tc_weights.end()) {
         itb_ctx::TcWeights t;
@@ -931,17 +930,17 @@ bool itb_tc_q8_gemm(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x,
     bool ok = tc_grow(&c->tc_q8_b, &c->tc_cap_q8b, tts * nt * kbs * 64, st) && tc_grow(&c->tc_q8_sx, &c->tc_cap_q8sx, tts * nt * kbs, st);
     if (!ok) return itb_fail_msg(c, "Q8_0 tensor path: out of device memory for the pass");
     // consecutive matmuls over one quantised row set share its image
-    if (x.id == 0 || c->tc_q8_src != x.id || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in || c->tc_q8_src_tile != (int)nt) {
+    if (x.id == 0 || c->tc_q8_src != x.id || c->tc_q8_src_rows != n_rows || c->tc_q8_src_in != w.n_in) {
         const size_t n = tts * nt * kbs;
         itb_chain(k_q8_tile, (unsigned)((n + 255) / 256), 256, 0, st, x.q, nullptr, x.s, n_rows, w.n_in, (int)nt, c->tc_q8_b, c->tc_q8_sx);
         c->launches++;
-        c->tc_q8_src = x.id; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in; c->tc_q8_src_tile = (int)nt;
+        c->tc_q8_src = x.id; c->tc_q8_src_rows = n_rows; c->tc_q8_src_in = w.n_in;
     }
     TcQ8 g{};
     g.a_img = it->second.img; g.a_sc = (const float*)it->second.sf; g.b_img = c->tc_q8_b; g.b_sc = c->tc_q8_sx; g.kbs = (int)kbs; g.n_rows = n_rows; g.n_out = w.n_out;
     g.out = out; g.stride = stride; g.mode = mode; g.status = c->fail.word;
-    auto kernel = mt == 2 ? k_tc_q8<64, 2> : k_tc_q8<64, 1>;
-    const size_t smem = mt == 2 ? Q8Cfg<64, 2>::SMEM : Q8Cfg<64, 1>::SMEM;
+    auto kernel = mt == 2 ? k_tc_q8<2> : k_tc_q8<1>;
+    const size_t smem = mt == 2 ? Q8Cfg<2>::SMEM : Q8Cfg<1>::SMEM;
     itb_raise_smem(kernel, smem);
     static const bool prof_on = getenv("ITB_TC_PROF") != nullptr;
     const size_t n_blocks = rts / mt * tts;
