@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(288) k_attn_out_exact(AxOut p) {
 }
 // The softmax of one (row, head)'s scores on its own, in place (many-row passes: the eight blocks that share a head's weights in
 // k_attn_out_exact would each recompute them, and the library-exact exponential is the expensive part): maximum, exponentials,
-// the sum in position order by one thread, the division. grid (n_head, rows), block 256; dynamic shared memory n_pos_max floats.
+// the sum in position order by one warp (fold_sum), the division. grid (n_head, rows), block 256; dynamic shared memory n_pos_max floats.
 struct AxSoft { float* scores; int s_stride; const int* n_pos_dev; int n_pos_last, n_q, n_head; };
 __global__ void __launch_bounds__(256) k_attn_softmax_exact(AxSoft p) {
     pdl_wait();

@@ -189,9 +189,10 @@ void itb_f16_to_f32(cudaStream_t st, const uint16_t* raw, float* out, size_t n);
 #ifdef __CUDACC__
 // A launch that is prepared while the kernel before it in the stream still runs. Only for kernels that begin with pdl_wait(), which returns
 // once that kernel has ended and its writes are visible; kernels that do not take part order themselves as ever. Kernels of many-row
-// passes and of the op seam give no early go-ahead (pdl_trigger) themselves: the next one's blocks are then placed when all SMs are free
-// and not wherever the first blocks happened to end -- with it, a scan of 128 blocks shared SMs and prefill of 512 tokens took 41.4 ms
-// instead of 32.8 (34.5 with ordinary launches). An op-seam row: 16 launches, 134 -> 102 us; prefill_odd's 98 kernels 1,055 -> 881 us.
+// passes and of the op seam give no early go-ahead (pdl_trigger) themselves, but for those they share with the one-token step (the exact and
+// the split attention, the LM head's projection, the arg-max): the next one's blocks are then placed when all SMs are free
+// and not wherever the first blocks happened to end -- with it everywhere, a scan of 128 blocks shared SMs and prefill of 512 tokens took
+// 41.4 ms instead of 32.8 (34.5 with ordinary launches). An op-seam row: 16 launches, 134 -> 102 us; prefill_odd's 98 kernels 1,055 -> 881 us.
 template <class... KA, class... A>
 static void itb_chain(void (*k)(KA...), dim3 g, dim3 b, size_t sm, cudaStream_t st, A&&... a) {
     cudaLaunchConfig_t cfg{};

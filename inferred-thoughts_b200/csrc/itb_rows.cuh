@@ -231,7 +231,7 @@ static bool dense_q8(itb_ctx* c, cudaStream_t st, const DevQ8& w, const QRows& x
     const int k = w.n_in;
     // many rows, dense=f16tc (tolerance class): both operands dequantised to f16, one tcgen05 GEMM with f32 accumulators
     if (tc && c->f16tc && n_rows >= 64 && itb_tc_f16_shape_ok(w)) return itb_tc_f16_gemm(c, st, w, x, n_rows, out, stride, mode);
-    // many rows, dense=q8tc: exact integer dots of 128 x 128 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
+    // many rows, dense=q8tc: exact integer dots of 256 x 64 or 128 x 64 (row, token) pairs on tcgen05, scaled and summed in the CPU's order
     if (tc && c->q8tc && n_rows >= 64 && itb_tc_q8_shape_ok(w)) return itb_tc_q8_gemm(c, st, w, x, n_rows, out, stride, mode);
     for (const void* f : {(const void*)k_gemm_q8<1>, (const void*)k_gemm_q8<4>}) itb_raise_smem(f, 200 * 1024);
     const bool skinny = n_rows <= 32;

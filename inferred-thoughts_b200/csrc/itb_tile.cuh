@@ -146,7 +146,8 @@ static void tile_q8_launch(cudaStream_t st, Q8Multi p, const int8_t* xq, const f
 // parentheses the kernel with 32 x 32 tiles, one group of 8 tokens to a warp and 64 x 64 tiles past 32 tokens that this one replaced):
 // 32 tokens: 2,048 outputs of k 4096 7.6 / 10.7 / 17.8 (17.9), 4,096 6.6 / 6.6 / 10.0 (9.8), 6,144 9.3 / 10.2 / 10.4 (13.1), 12,288 16.1 / 13.6 / 16.3
 // (21.1), 24,576 28.4 / 23.8 / 22.8 (36.9), 248,320 243 / 187 / 176 (311); 8 tokens: 2,048 of k 4096 6.4 / 7.9 / 13.6 (18.1), 12,288 12.0 / 8.8 / 10.0 (21.2),
-// 24,576 20.3 / 15.5 / 12.5 (36.9), 248,320 181 / 118 / 102 (311); 200 tokens: 2,048 of k 4096 28.5 / 23.6 / 29.3 (34.4), 12,288 79 / 63 / 58 (103).
+// 24,576 20.3 / 15.5 / 12.5 (36.9), 248,320 181 / 118 / 102 (311); 200 tokens: 2,048 of k 4096 28.5 / 23.6 / 29.3 (34.4), 12,288 79 / 63 / 58 (103). Passes without the
+// tensor cores, under ncu, 64 rows: 512 tokens 8,192 101 (127), 4,096 53 (72); 2,048 tokens 8,192 380 (491), 4,096 195 (250).
 static void tile_q8(cudaStream_t st, int sms, const Q8Multi& p, const int8_t* xq, const float* xs, int n_tok, int mode) {
     long long blocks = 0;                                 // of 16 rows x 32 tokens
     for (int i = 0; i < p.n; ++i) blocks += (p.w[i].n_out + 15) / 16;
